@@ -20,7 +20,7 @@ from ctypes import c_float, c_int, c_int64, c_void_p
 import numpy as np
 import torch
 
-from .library import OPS_SOURCES, KernelBuildError, load_library, require_cuda
+from .library import GEMM_SOURCES, OPS_SOURCES, KernelBuildError, load_library, require_cuda
 
 SS_F32, SS_BF16 = 0, 1
 
@@ -148,6 +148,7 @@ _ATTN_SIGNATURES["ss_attn_decode_across"] = [c_void_p, c_int64, c_void_p, c_void
                                              c_void_p]
 
 _GEMM_SIGNATURES = {
+    "ss_gemm_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_void_p, c_void_p],
     "ss_gemm_tc5_many": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int64, c_int64, c_int64,
                          c_int, c_int, c_int, c_void_p, c_void_p],
     "ss_gemm_tc5_many_tile_cols": [c_int, c_int, c_int],
@@ -200,7 +201,7 @@ def gemm_library() -> ctypes.CDLL:
     lib = _state.get("gemm")
     if lib is None:
         require_cuda()
-        lib = load_library("slipstream_gemm", ["gemm_tc5.cu"])
+        lib = load_library("slipstream_gemm", GEMM_SOURCES)
         _declare(lib, _GEMM_SIGNATURES)
         _state["gemm"] = lib
     return lib  # type: ignore[return-value]
@@ -574,6 +575,31 @@ def gemm_simt(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None =
             raise KernelError("bias has the wrong size or dtype")
     _check(ops_library().ss_gemm_simt(x.data_ptr(), weight.data_ptr(), _ptr(bias), bias_f32, out.data_ptr(),
                                       m, n, k, k, n, _code(x.dtype), _code(out_dtype), _stream()), "gemm_simt")
+    return out
+
+
+def gemm_float32(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+    """``x @ weight.T + bias`` for float32 tensors, every value carrying its 24 bits: the tensor-core kernel that cuts
+    each operand into three bfloat16 parts (`csrc/gemm_f32.cu`) where rows start on 16 bytes, else the CUDA-core kernel.
+    The rule asks nothing about the number of rows, and either kernel gives a row the same bits whatever rows stand
+    beside it, so a token's values do not depend on the rest of its step.  The tensor-core kernel is the faster one at
+    every size (us against the CUDA-core kernel's: 1 row of 896 x 896 15 / 57, 4 of 17,920 x 1,536 30 / 201, 777 of
+    4,608 x 3,584 171 / 1,191)."""
+    _need(x, torch.float32, "x")
+    _need(weight, torch.float32, "weight")
+    m, k = x.shape
+    n = weight.shape[0]
+    if k == 0 or k % 4 or x.data_ptr() % 16 or weight.data_ptr() % 16 or (bias is not None and bias.dtype != torch.float32):
+        return gemm_simt(x, weight, bias)
+    if weight.shape[1] != k:
+        raise KernelError(f"weight {tuple(weight.shape)} does not match x {tuple(x.shape)}")
+    if bias is not None:
+        _need(bias, torch.float32, "bias")
+        if bias.numel() != n:
+            raise KernelError("bias has the wrong size or dtype")
+    out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+    _check(gemm_library().ss_gemm_f32(x.data_ptr(), weight.data_ptr(), _ptr(bias), out.data_ptr(), m, n, k, n,
+                                      error_word(x.device).data_ptr(), _stream()), "gemm_f32")
     return out
 
 
@@ -1536,7 +1562,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
            out_dtype: torch.dtype | None = None) -> torch.Tensor:
     """A projection ``x @ weight.T + bias``.
 
-    float32 runs the CUDA-core kernel (no reduced-precision matrix mode).  bfloat16 with few tokens (decode
+    float32 runs `gemm_float32` (every value with its 24 bits).  bfloat16 with few tokens (decode
     steps) and a large weight runs the hand-written tcgen05 kernel, which streams the weights once and
     overlaps its first fetches with the kernel before it; from ``MANY_TOKENS`` tokens (prompt portions) and with
     enough output tiles (``many_tokens_fits``) the persistent two-SM tcgen05 kernel; everything else runs the
@@ -1549,6 +1575,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
             return gemm_tcgen05(x, weight, bias, out_dtype)
         else:
             return gemm_tcgen05_many(x, weight, bias, out_dtype)
+    if x.dtype == torch.float32 and out_dtype in (None, torch.float32):
+        return gemm_float32(x, weight, bias)
     if x.dtype == torch.float32:
         return gemm_simt(x, weight, bias, out_dtype)
     sms = sm_count(x.device)
@@ -2618,7 +2646,7 @@ def set_programmatic_launch(enabled: bool) -> None:
 
 
 __all__ = ["KernelError", "KernelBuildError", "embedding", "add_rmsnorm", "hc_norm", "linear_hc_rmsnorm", "rope_norm_cache", "glu_limited", "gate_up_glu", "sigmoid_gate", "key_span", "rope_and_cache", "swiglu",
-           "gemm_simt", "paged_attention_simt", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "paged_attention_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
+           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "paged_attention_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
            "attention_library", "group_norm", "round_stream", "conv_silu", "ssm_scan", "router", "moe_experts", "moe_combine",
            "norm_rope_cache", "turn_heads", "soft_cap", "embed_sum", "matrix_cell", "cell_output", "gated_recurrence", "xielu",
            "DiffPair", "diff_in_attention", "diff_combine", "heads_to_pages", "branch_norm", "PairedOutput", "WeighedTerms",

@@ -133,6 +133,51 @@ def test_float32_matrix_product_is_exact_to_rounding_and_independent_of_the_batc
     assert torch.equal(alone, got[:1])
 
 
+# widths at the edges of the 128-row weight tiles, K at the edges of the 64-wide steps and 256-wide chunks, rows at the edges of
+# every token tile (16, 32, 64 and the wider ones), K's chunks on one to eight blocks of a cluster and more than fit 64 columns
+@pytest.mark.parametrize("n, k", [(1, 4), (128, 64), (129, 68), (300, 252), (257, 260), (1000, 2304), (70, 8960), (40, 18944)])
+def test_float32_product_on_tensor_cores_carries_24_bits_and_is_independent_of_the_batch(n, k):
+    torch.manual_seed(n)
+    x, w, b = torch.randn(300, k, device=DEV), torch.randn(n, k, device=DEV), torch.randn(n, device=DEV)
+    x[7] *= 1e-30
+    x[8] *= 1e20
+    whole = ops().gemm_float32(x, w, b)
+    ref = x.double() @ w.double().T + b.double()
+    # parts left out: 2^-23 of |x| |w|; a chunk's sum: 16 additions that truncate, 2^-23 each at most; the chunks' sums: a
+    # rounding of 2^-24 each, with random signs
+    bound = (18 + (k / 256) ** 0.5) * 2.0 ** -23 * (x.abs().double() @ w.abs().double().T + b.abs())
+    assert ((whole.double() - ref).abs() <= bound).all()
+    # beside the size of such a sum (random signs): 8 truncations of half a unit of 2^-23 in a chunk on average, each of a part
+    # of the chunk's sum, make less than 5e-7; a 32-bit chain shows up to 1.7e-6 at these K
+    typical = x.double().norm(dim=1, keepdim=True) * w.double().norm(dim=1) * k ** -0.5 + b.double().abs()
+    assert ((whole.double() - ref) / typical).square().mean().sqrt() < 5e-7
+    for m in (1, 2, 16, 17, 32, 33, 64, 65, 80, 113, 129):
+        assert torch.equal(ops().gemm_float32(x[:m].contiguous(), w, b), whole[:m]), m
+    ops().check_errors(DEV)
+
+
+def test_float32_product_passes_infinities_and_nan_on_as_cuda_cores_do():
+    torch.manual_seed(0)
+    w = torch.randn(200, 512, device=DEV)
+    w[5, 9] = -float("inf")
+    for m in (6, 90):
+        x = torch.randn(m, 512, device=DEV)
+        x[1, 3], x[2, 7], x[3, 0], x[4] = float("inf"), float("nan"), 3.4e38, -float("inf")
+        got, want = ops().gemm_float32(x, w), ops().gemm_simt(x, w)
+        odd = ~torch.isfinite(want)
+        assert torch.equal(torch.nan_to_num(got[odd], 1.5, 2.5, 3.5), torch.nan_to_num(want[odd], 1.5, 2.5, 3.5))
+        assert torch.isfinite(got[~odd]).all() and rel_err(got[~odd], want[~odd]) < 2e-6
+    ops().check_errors(DEV)
+
+
+def test_float32_product_without_16_byte_rows_takes_the_cuda_cores():
+    x, w = torch.randn(5, 70, device=DEV), torch.randn(33, 70, device=DEV)
+    assert torch.equal(ops().gemm_float32(x, w), ops().gemm_simt(x, w))
+    flat = torch.randn(5 * 72 + 1, device=DEV)
+    x, w = flat[1:].view(5, 72), torch.randn(33, 72, device=DEV)
+    assert torch.equal(ops().gemm_float32(x, w), ops().gemm_simt(x, w))
+
+
 def test_bfloat16_linear_gives_float32_logits():
     x, w = torch.randn(5, 200, device=DEV).bfloat16(), torch.randn(1001, 200, device=DEV).bfloat16()
     got = ops().linear(x, w, None, out_dtype=torch.float32)

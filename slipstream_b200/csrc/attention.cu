@@ -1,5 +1,6 @@
 // Attention library for one head size: compiled with -DHEAD_DIM=<multiple of 16>,
 // once for each head size a loaded model uses.
+#include "attention_f32.cuh"
 #include "attention_simt.cuh"
 
 #ifndef HEAD_DIM
@@ -25,6 +26,24 @@ extern "C" int ss_attn_simt(const void* q, int64_t q_stride, void* out, int64_t 
     return launch_attn_simt<float, HEAD_DIM>(q, q_stride, out, out_stride, kv, block_tables, max_blocks,
                                              tile_req, tile_q0, n_tiles, q_start, seq_lens, n_q, n_kv,
                                              page_size, num_pages, scale, window, gate, err, stream, softcap, sinks, keep, across);
+}
+
+// tile_req null: a decode step (one token a request).  parts > 1: a row's slices of keys on that many blocks; `part` and
+// `part_ml` then hold max_slices slices a (row, output head), at least as many as the longest request has.
+extern "C" int ss_attn_f32(const float* q, int64_t q_stride, float* out, int64_t out_stride, const float* kv,
+                           const int32_t* tables, int max_blocks, const int32_t* tile_req, const int32_t* tile_q0, int n_tiles,
+                           const int32_t* q_start, const int32_t* seq_lens, int n_requests, int n_q, int n_kv, int page_size,
+                           int64_t num_pages, float scale, int window, const float* gate, int* err, cudaStream_t stream,
+                           float softcap, const float* sinks, int keep, int across, float* part, float2* part_ml,
+                           int max_slices, int n_rows, int parts) {
+    if (n_tiles <= 0 || n_rows <= 0 || n_requests <= 0) return 0;
+    if (keep < 0 || (keep > 0 && window <= 0) || (across && gate) || parts < 1 || parts > 65535 || (parts > 1) != (part != nullptr) ||
+        (part != nullptr && part_ml == nullptr) || ((uintptr_t)kv & 15) != 0)
+        return (int)cudaErrorInvalidValue;
+    const AttnF32Args g{q, q_stride, out, out_stride, kv, tables, max_blocks, tile_req, tile_q0, q_start, seq_lens, n_requests,
+                        n_q, n_kv, page_size, num_pages, scale, window, err, gate, softcap, sinks, keep, across, part, part_ml,
+                        max_slices, n_rows};
+    return launch_attn_f32<HEAD_DIM>(g, n_tiles, parts, stream);
 }
 
 #include "attention_mma.cuh"

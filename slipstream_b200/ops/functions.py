@@ -122,6 +122,9 @@ _OPS_SIGNATURES = {
 }
 
 _ATTN_SIGNATURES = {
+    "ss_attn_f32": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
+                    c_int, c_int, c_int, c_int, c_int64, c_float, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int,
+                    c_int, c_void_p, c_void_p, c_int, c_int, c_int],
     "ss_attn_simt": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p,
                      c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_float,
                      c_int, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int],
@@ -689,6 +692,54 @@ def paged_attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: 
            "paged_attention_simt")
 
 
+FLOAT32_GROUP = 128  # query heads a kv head up to which a captured step has room for the lists of 64-row tiles
+FLOAT32_SLICE = 128  # keys of a slice of the float32 kernel (csrc/attention_f32.cuh)
+FLOAT32_SCRATCH = 128 << 20  # bytes of slices that a call may leave in scratch memory
+
+
+def float32_key_parts(blocks: int, slices: int, rows: int, heads: int, head_dim: int, sms: int | None = None) -> int:
+    """Blocks that share the ``slices`` slices of a row's keys in the float32 kernel where ``blocks`` would walk all of
+    theirs: as many as make two blocks an SM, the most that do not wait for one another.  The slices then go through
+    scratch memory, which is bounded.  Only the time depends on it: a row's slices are joined in the same order."""
+    parts = min(slices, 2 * (sms or sm_count()) // max(blocks, 1))
+    return parts if parts > 1 and rows * heads * slices * (head_dim + 2) * 4 <= FLOAT32_SCRATCH else 1
+
+
+def paged_attention_float32(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, block_tables: torch.Tensor, ctx, n_q: int,
+                            n_kv: int, head_dim: int, scale: float, window: int = 0, chunk: int = 0,
+                            gate: torch.Tensor | None = None, softcap: float = 0.0, sinks: torch.Tensor | None = None,
+                            keep: int = 0, across: bool = False) -> None:
+    """`paged_attention_simt` for the rows of a step in float32, with the arguments of `paged_attention`: the kernel that
+    tiles 64 rows of a kv head's group with 32 keys and splits a row's keys over several blocks where there are few rows."""
+    _need(out, torch.float32, "attention output")
+    _check_sinks(sinks, n_q)
+    _need(kv, torch.float32, "kv pages")
+    group, heads = n_q // n_kv, n_kv * n_q if across else n_q
+    if ctx.is_decode_only:
+        tile_req = tile_row0 = None
+        tiles = ctx.num_requests * ((group + 15) // 16)
+        longest = ctx.extras.get("static_max_seq_len") or ctx.max_seq_len
+    else:
+        tile_req, tile_row0 = ctx.query_tiles(64, group)
+        tiles, longest = tile_req.numel(), ctx.max_seq_len  # 0 in a captured step, whose lengths the host does not know
+    for name, t in (("block_tables", block_tables), ("q_start", ctx.q_start), ("seq_lens", ctx.seq_lens)):
+        _need(t, torch.int32, name)
+    slices = max(1, -(-longest // FLOAT32_SLICE))
+    parts = float32_key_parts(tiles * heads // group, slices, qkv.shape[0], heads, head_dim, sm_count(qkv.device))
+    part = part_ml = None
+    if parts > 1:
+        part = torch.empty((qkv.shape[0], heads, slices, head_dim), dtype=torch.float32, device=qkv.device)
+        part_ml = torch.empty((qkv.shape[0], heads, slices, 2), dtype=torch.float32, device=qkv.device)
+    _check(attention_library(head_dim).ss_attn_f32(
+        qkv.data_ptr(), qkv.shape[1], out.data_ptr(), out.shape[1], kv.data_ptr(), block_tables.data_ptr(),
+        block_tables.shape[1], _ptr(tile_req), _ptr(tile_row0), tiles, ctx.q_start.data_ptr(), ctx.seq_lens.data_ptr(),
+        ctx.num_requests, n_q, n_kv, kv.shape[3], kv.shape[0], float(scale), key_span(window, chunk),
+        _gate_ptr(gate, qkv, qkv.shape[1]), error_word(qkv.device).data_ptr(), _stream(), float(softcap or 0.0), _ptr(sinks),
+        _kept(keep, window), int(across), _ptr(part), _ptr(part_ml), slices, qkv.shape[0], parts), "attn_f32")
+    if parts > 1:
+        _launches[0] += 1  # the kernel that joins the slices
+
+
 def paged_attention_prefill(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torch.Tensor,
                             block_tables: torch.Tensor, tile_req: torch.Tensor, tile_row0: torch.Tensor,
                             q_start: torch.Tensor, seq_lens: torch.Tensor, n_q: int, n_kv: int, head_dim: int,
@@ -940,7 +991,7 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, bloc
 
     ``qkv`` is the stacked projection output [N, (n_q + 2 n_kv) * D] whose first n_q heads are the
     rotated queries; ``ctx`` gives the rows of each request (``q_start``), the cached lengths after
-    this step (``seq_lens``) and the lists of query tiles.  float32 runs the CUDA-core kernel;
+    this step (``seq_lens``) and the lists of query tiles.  float32 runs the CUDA-core kernels (`paged_attention_float32`);
     bfloat16 the tensor-core kernels: the split decode kernel when every request brings one token, else
     the tcgen05 kernel (head size 64 or 128; windows, chunked masks and soft caps included) or the mma.sync tiled kernel.
 
@@ -968,10 +1019,14 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, bloc
     if rope is not None and not (qkv.dtype == torch.bfloat16 and ctx.is_decode_only):
         raise KernelError("only bfloat16 decode steps rotate inside the attention kernel")
     if qkv.dtype == torch.float32:
-        tile_req, tile_q0 = ctx.query_tiles(16)
         heads = out if diff is None else _heads_f32(out, n_q, head_dim)
-        paged_attention_simt(qkv, qkv.shape[1], heads, kv, block_tables, tile_req, tile_q0, ctx.q_start,
-                             ctx.seq_lens, n_q, n_kv, head_dim, scale, window, chunk, gate, softcap, sinks, keep, across)
+        if n_q // n_kv <= FLOAT32_GROUP:
+            paged_attention_float32(qkv, heads, kv, block_tables, ctx, n_q, n_kv, head_dim, scale, window, chunk, gate, softcap,
+                                    sinks, keep, across)
+        else:
+            tile_req, tile_q0 = ctx.query_tiles(16)
+            paged_attention_simt(qkv, qkv.shape[1], heads, kv, block_tables, tile_req, tile_q0, ctx.q_start,
+                                 ctx.seq_lens, n_q, n_kv, head_dim, scale, window, chunk, gate, softcap, sinks, keep, across)
         if diff is not None:
             diff_combine(heads, diff, n_q // 2, out)
         return
@@ -2646,7 +2701,7 @@ def set_programmatic_launch(enabled: bool) -> None:
 
 
 __all__ = ["KernelError", "KernelBuildError", "embedding", "add_rmsnorm", "hc_norm", "linear_hc_rmsnorm", "rope_norm_cache", "glu_limited", "gate_up_glu", "sigmoid_gate", "key_span", "rope_and_cache", "swiglu",
-           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "paged_attention_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
+           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "paged_attention_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
            "attention_library", "group_norm", "round_stream", "conv_silu", "ssm_scan", "router", "moe_experts", "moe_combine",
            "norm_rope_cache", "turn_heads", "soft_cap", "embed_sum", "matrix_cell", "cell_output", "gated_recurrence", "xielu",
            "DiffPair", "diff_in_attention", "diff_combine", "heads_to_pages", "branch_norm", "PairedOutput", "WeighedTerms",

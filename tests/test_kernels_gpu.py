@@ -153,7 +153,7 @@ def test_float32_product_on_tensor_cores_carries_24_bits_and_is_independent_of_t
     assert ((whole.double() - ref) / typical).square().mean().sqrt() < 5e-7
     for m in (1, 2, 16, 17, 32, 33, 64, 65, 80, 113, 129):
         assert torch.equal(ops().gemm_float32(x[:m].contiguous(), w, b), whole[:m]), m
-    ops().check_errors(DEV)
+    ops().check_errors(torch.device(DEV))
 
 
 def test_float32_product_passes_infinities_and_nan_on_as_cuda_cores_do():
@@ -167,7 +167,7 @@ def test_float32_product_passes_infinities_and_nan_on_as_cuda_cores_do():
         odd = ~torch.isfinite(want)
         assert torch.equal(torch.nan_to_num(got[odd], 1.5, 2.5, 3.5), torch.nan_to_num(want[odd], 1.5, 2.5, 3.5))
         assert torch.isfinite(got[~odd]).all() and rel_err(got[~odd], want[~odd]) < 2e-6
-    ops().check_errors(DEV)
+    ops().check_errors(torch.device(DEV))
 
 
 def test_float32_product_without_16_byte_rows_takes_the_cuda_cores():
@@ -813,4 +813,46 @@ def test_what_a_pages_last_owner_left_behind_reaches_nobody(n_q, n_kv, d, page):
                                          n_slices=slices, tma=tma)
             assert torch.isfinite(outd).all(), (tma, slices)
             assert rel_err(outd.cpu(), refd) < 1e-2, (tma, slices)
+    ops().check_errors(torch.device(DEV))
+
+
+# 64-row tiles whose groups straddle tokens, heads beyond 128 (tiles of 32 rows), one head a group, more heads than a decode
+# tile has rows; contexts at the edges of key tiles (32) and slices (128); windows, kept keys and chunks
+@pytest.mark.parametrize("d, n_q, n_kv, window, chunk, keep", [
+    (128, 14, 2, 0, 0, 0), (16, 3, 3, 0, 0, 0), (64, 40, 2, 0, 0, 0), (160, 6, 1, 0, 0, 0), (256, 8, 4, 150, 0, 0),
+    (80, 5, 1, 40, 0, 3), (96, 4, 4, 0, 64, 0)])
+def test_float32_attention_gives_a_row_the_same_bits_however_its_step_was_cut(monkeypatch, d, n_q, n_kv, window, chunk, keep):
+    from types import SimpleNamespace
+    from slipstream_b200.engine.context import query_tiles_host
+    from slipstream_b200.ops import functions
+    lens = [1, 31, 32, 129, 300, 517]
+    page, rule = 16, functions.float32_key_parts
+    q, kv, table, q_start, seq_lens = make_attention_case(torch.float32, lens, lens, n_q, n_kv, d, page, seed=d)
+    sinks = torch.randn(n_q, device=DEV) if d == 64 else None
+
+    def run(rows, q_lens, ends, static=None, parts=None):
+        as_dev = lambda a: torch.tensor(np.asarray(a, dtype=np.int32), device=DEV)  # noqa: E731
+        ctx = SimpleNamespace(
+            is_decode_only=max(q_lens) == 1, num_requests=len(lens), max_seq_len=max(ends), seq_lens=as_dev(ends),
+            q_start=as_dev(np.concatenate([[0], np.cumsum(q_lens)])), extras={"static_max_seq_len": static} if static else {},
+            query_tiles=lambda n, g: tuple(as_dev(t) for t in query_tiles_host(np.asarray(q_lens) * g, n)))
+        out = torch.full((rows.shape[0], n_q * d), 7.0, device=DEV)
+        monkeypatch.setattr(functions, "float32_key_parts", rule if parts is None else lambda *a, **k: parts)
+        ops().paged_attention_float32(rows.reshape(rows.shape[0], -1).contiguous(), out, kv, table, ctx, n_q, n_kv, d, 0.3, window,
+                                      chunk, None, 0.0, sinks, keep)
+        return out
+
+    whole = run(q, lens, lens, parts=1)
+    if not chunk and not keep:
+        want = attention_reference(q, kv, table, q_start, seq_lens, n_kv, page, 0.3, window, sinks)
+        # chains of up to 256 (scores) and 128 (outputs of a slice) roundings of 2^-24 with random signs, and exponentials
+        # of scores up to 40 in size, whose rounding of 2^-24 they pass on times 40
+        assert rel_err(whole.cpu(), want.reshape(whole.shape)) < 5e-6
+    assert torch.equal(run(q, lens, lens, parts=3), whole)  # a row's slices on three blocks
+    last = [int(b) - 1 for b in np.cumsum(lens)]
+    for static, parts in ((None, None), (4096, None), (None, 1)):  # a decode step: split, as captured, not split
+        assert torch.equal(run(q[last], [1] * len(lens), lens, static, parts), whole[last]), (static, parts)
+    tail = [min(n, 37) for n in lens]  # the last portion of every request
+    rows = [r for b, t in zip(np.cumsum(lens), tail) for r in range(int(b) - t, int(b))]
+    assert torch.equal(run(q[rows], tail, lens), whole[rows])
     ops().check_errors(torch.device(DEV))

@@ -4,8 +4,8 @@
 //
 // Rows are (token, query head of a kv head's group) pairs, so a group shares every tile of keys and values.  A block takes
 // RT rows of one request and walks tiles of 32 keys that start at multiples of 32 from the request's first token, copied
-// ahead by cp.async into one of two buffers; a thread forms 4 x (RT / 16) scores and (RT / 8) x 4 ceil(D / 64) outputs in
-// registers, so that a 16-byte read of shared memory feeds eight to sixteen multiply-adds.
+// ahead by cp.async (keys into one of two buffers, values while the scores are formed); a thread forms 4 x (RT / 16) scores
+// and (RT / 8) x 4 ceil(D / 64) outputs in registers.
 //
 // The order of the arithmetic behind one row is the same however the prompt was cut, whatever else is in the step and
 // however many blocks share a row's keys: keys fall into slices of AF_SLICE from the request's first token, every slice has
@@ -13,8 +13,10 @@
 // walks all slices of its rows joins them in registers; with more than one block to a row (gridDim.z) every slice's
 // maximum, sum and output go to scratch memory and attn_f32_join_kernel joins them, with the same operations.
 //
-// Bound by the multiply-adds and the shared-memory reads that feed them (two 16-byte reads a 16 multiply-adds for the
-// scores, four a 64 for the outputs with 64 rows).  AF_FIGURES
+// Bound by issue: 70 % of its instructions are the multiply-adds, and three blocks of four warps an SM issue on about half
+// of the cycles.  Against attention_simt.cuh (a tile of 16 tokens of one query head, keys in series, no copies ahead):
+// 777 tokens of two requests, one behind 300 cached ones, 28 heads of 128 on 4: 551 -> 209 us; four decoded tokens behind
+// 500 on average, 12 heads of 128 on 2: 266 -> 33 us; 20 behind 800, 28 on 4: 602 -> 102 us.
 #pragma once
 
 #include "common.cuh"
@@ -70,36 +72,38 @@ __device__ __forceinline__ float af_finish(float v, float l, const float* gate) 
 
 template <int D, int RT>
 constexpr int af_smem_bytes() {
-    return (RT * (D + 4) + 2 * AF_BN * (D + 4) + 2 * AF_BN * D + AF_BN * (RT + 4) + 2 * RT) * 4;
+    return (RT * (D + 4) + 2 * AF_BN * (D + 4) + AF_BN * D + AF_BN * (RT + 4) + 2 * RT) * 4;
 }
 
 template <int D, int RT>
-__global__ void __launch_bounds__(AF_THREADS) attn_f32_kernel(const AttnF32Args g) {
+__global__ void __launch_bounds__(AF_THREADS, D <= 128 ? 3 : 1) attn_f32_kernel(const AttnF32Args g) {
     constexpr int KS = D + 4, PS = RT + 4;             // row strides in shared memory: rows 16 bytes further round the banks
-    constexpr int KPT = RT / 16, TX = AF_BN / KPT, TY = AF_THREADS / TX;  // scores: rows ty + TY i (i < 4), keys tx + TX j
-    constexpr int RP = RT / 8, NC = (D + 63) / 64;     // outputs: rows py RP + i, elements 4 (px + 16 c) .. + 3
+    constexpr int KPT = RT * AF_BN / AF_THREADS / 4, TX = AF_BN / KPT, TY = AF_THREADS / TX;  // scores: rows ty + TY i (i < 4), keys tx + TX j
+    constexpr int RP = RT / (AF_THREADS / 16), NC = (D + 63) / 64;     // outputs: rows py RP + i, elements 4 (px + 16 c) .. + 3
     extern __shared__ __align__(16) float af_smem[];
     float* Qs = af_smem;
     float* Ks = Qs + RT * KS;
     float* Vs = Ks + 2 * AF_BN * KS;
-    float* Ps = Vs + 2 * AF_BN * D;   // [key][row]
+    float* Ps = Vs + AF_BN * D;   // [key][row]
     float* alpha_s = Ps + AF_BN * PS; // by row: the factor of what was summed before the tile, and the maximum so far
     float* max_s = alpha_s + RT;
 
     pdl_launch_dependents();
     pdl_wait();
     const int tid = threadIdx.x;
-    const int G = g.n_q / g.n_kv, u = blockIdx.y;
+    // the kv head runs fastest and a request's later tiles, which see more keys, come first: the longest blocks start first
+    const int G = g.n_q / g.n_kv, n_heads = g.across ? g.n_kv * g.n_kv : g.n_kv, u = blockIdx.x % n_heads;
+    const int block = ((int)gridDim.x - 1 - (int)blockIdx.x) / n_heads;
     const HeadPair hp = head_pair(u, g.n_kv, g.across);
     int r, row0;
     if (g.tile_req != nullptr) {
         constexpr int SUB = 64 / RT;  // blocks of a tile of the list
-        r = g.tile_req[blockIdx.x / SUB];
-        row0 = g.tile_q0[blockIdx.x / SUB] + (blockIdx.x % SUB) * RT;
+        r = g.tile_req[block / SUB];
+        row0 = g.tile_q0[block / SUB] + (block % SUB) * RT;
     } else {
         const int per_request = (G + RT - 1) / RT;
-        r = blockIdx.x / per_request;
-        row0 = (blockIdx.x % per_request) * RT;
+        r = block / per_request;
+        row0 = (block % per_request) * RT;
     }
     const int qs = g.q_start[r], q_len = g.q_start[r + 1] - qs, seq_len = g.seq_lens[r];
     const int rows = min(RT, q_len * G - row0);
@@ -130,28 +134,36 @@ __global__ void __launch_bounds__(AF_THREADS) attn_f32_kernel(const AttnF32Args 
         }
         *reinterpret_cast<float4*>(&Qs[row * KS + d4 * 4]) = v;
     }
-    // four threads copy a key and its value; rows outside [lo_min, p_max] that are not kept are zero
-    auto fetch = [&](int j) {
-        const int row = tid >> 2, key = tile_at(j) * AF_BN + row, buf = j & 1;
-        int64_t page = -1;
-        if ((key >= lo_min || key < g.keep) && key <= p_max) {
-            page = table[key / g.page_size];
-            if (page >= g.num_pages) {
-                if ((tid & 3) == 0) atomicOr(g.err, SS_ERR_PAGE_RANGE);
-                page = -1;
-            }
+    constexpr int TPR = AF_THREADS / AF_BN;  // threads that copy a key and its value; rows outside [lo_min, p_max] that are not kept are zero
+    // (the page of the tile after is looked up a tile ahead)
+    const int copy_row = tid / TPR;
+    auto page_of = [&](int j) -> int64_t {
+        const int key = tile_at(j) * AF_BN + copy_row;
+        if (j >= n_tiles || !((key >= lo_min || key < g.keep) && key <= p_max)) return -1;
+        return table[key / g.page_size];
+    };
+    int64_t next_page = page_of(0);
+    int64_t value_at = -1;  // where the value of the key that was fetched last stands
+    auto fetch_key = [&](int j) {
+        int64_t page = next_page;
+        next_page = page_of(j + 1);
+        if (page >= g.num_pages) {
+            if (tid % TPR == 0) atomicOr(g.err, SS_ERR_PAGE_RANGE);
+            page = -1;
         }
         const bool live = page >= 0;
-        const int64_t off = live ? (int64_t)(key % g.page_size) * D : 0;
-        const float* kp = g.kv + (live ? ((page * 2 + 0) * g.n_kv + hp.key) * g.page_size * (int64_t)D + off : 0);
-        const float* vp = g.kv + (live ? ((page * 2 + 1) * g.n_kv + hp.value) * g.page_size * (int64_t)D + off : 0);
-        float* kd = Ks + (buf * AF_BN + row) * KS;
-        float* vd = Vs + (buf * AF_BN + row) * D;
+        const int64_t off = live ? (int64_t)((tile_at(j) * AF_BN + copy_row) % g.page_size) * D : 0;
+        const float* src = g.kv + (live ? ((page * 2 + 0) * g.n_kv + hp.key) * g.page_size * (int64_t)D + off : 0);
+        value_at = live ? ((page * 2 + 1) * g.n_kv + hp.value) * g.page_size * (int64_t)D + off : -1;
+        float* dst = Ks + ((j & 1) * AF_BN + copy_row) * KS;
 #pragma unroll
-        for (int d = (tid & 3) * 4; d < D; d += 16) {
-            cp_async16(kd + d, kp + (live ? d : 0), live);
-            cp_async16(vd + d, vp + (live ? d : 0), live);
-        }
+        for (int d = (tid % TPR) * 4; d < D; d += 4 * TPR) cp_async16(dst + d, src + (live ? d : 0), live);
+    };
+    auto fetch_value = [&]() {
+        const bool live = value_at >= 0;
+        const float* src = g.kv + (live ? value_at : 0);
+#pragma unroll
+        for (int d = (tid % TPR) * 4; d < D; d += 4 * TPR) cp_async16(Vs + copy_row * D + d, src + (live ? d : 0), live);
     };
 
     const int tx = tid % TX, ty = tid / TX, px = tid & 15, py = tid >> 4;
@@ -166,15 +178,17 @@ __global__ void __launch_bounds__(AF_THREADS) attn_f32_kernel(const AttnF32Args 
 #pragma unroll
         for (int c = 0; c < NC * 4; ++c) tot[i][c] = 0.f;
     }
-    if (n_tiles > 0) fetch(0);
+    if (n_tiles > 0) fetch_key(0);
     cp_async_commit();
 
     for (int j = 0; j < n_tiles; ++j) {
         const int kt = tile_at(j), buf = j & 1;
         const bool opens = j == 0 || tile_at(j - 1) / TPS != kt / TPS, closes = j + 1 == n_tiles || tile_at(j + 1) / TPS != kt / TPS;
         cp_async_wait<0>();
-        __syncthreads();  // the tile is there, and everyone is done with the tile before it
-        if (j + 1 < n_tiles) fetch(j + 1);
+        __syncthreads();  // the tile's keys are there, and everyone is done with the values before it
+        fetch_value();
+        cp_async_commit();
+        if (j + 1 < n_tiles) fetch_key(j + 1);
         cp_async_commit();
 
         // ---- scores
@@ -226,6 +240,7 @@ __global__ void __launch_bounds__(AF_THREADS) attn_f32_kernel(const AttnF32Args 
             }
             m[i] = now;
         }
+        cp_async_wait<1>();  // the values; the next keys may still be under way
         __syncthreads();
 
         // ---- outputs
@@ -236,7 +251,7 @@ __global__ void __launch_bounds__(AF_THREADS) attn_f32_kernel(const AttnF32Args 
 #pragma unroll
             for (int c = 0; c < NC * 4; ++c) acc[i][c] = opens ? 0.f : __fmul_rn(acc[i][c], a);
         }
-        const float* vb = Vs + buf * AF_BN * D;
+        const float* vb = Vs;
 #pragma unroll 4
         for (int k = 0; k < AF_BN; ++k) {
             float p[RP];
@@ -275,7 +290,7 @@ __global__ void __launch_bounds__(AF_THREADS) attn_f32_kernel(const AttnF32Args 
 #pragma unroll
                 for (int c = 0; c < NC * 4; ++c) tot[i][c] = af_mix(tot[i][c], f, acc[i][c]);
             } else if (row < rows) {
-                const int64_t at = ((int64_t)(qs + (row0 + row) / G) * (gridDim.y * G) + u * G + (row0 + row) % G) * g.max_slices + kt / TPS;
+                const int64_t at = ((int64_t)(qs + (row0 + row) / G) * (n_heads * G) + u * G + (row0 + row) % G) * g.max_slices + kt / TPS;
                 if (px == 0) g.part_ml[at] = make_float2(slice_m, l[i]);
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
@@ -382,7 +397,7 @@ int launch_attn_f32_rows(const AttnF32Args& g, int n_tiles, int parts, cudaStrea
     if (int rc = ss_opt_in_smem(attn_f32_kernel<D, RT>, smem, opted)) return rc;
     const int blocks = g.tile_req ? n_tiles * (64 / RT) : g.n_requests * ((g.n_q / g.n_kv + RT - 1) / RT);
     const int heads = g.across ? g.n_kv * g.n_kv : g.n_kv;
-    ss_launch(attn_f32_kernel<D, RT>, dim3(blocks, heads, parts), dim3(AF_THREADS), smem, stream, g);
+    ss_launch(attn_f32_kernel<D, RT>, dim3(blocks * heads, 1, parts), dim3(AF_THREADS), smem, stream, g);
     if (g.part) {
         const int64_t items = (int64_t)g.n_rows * heads * (g.n_q / g.n_kv);
         ss_launch(attn_f32_join_kernel<D>, dim3((unsigned)((items + AF_THREADS / 32 - 1) / (AF_THREADS / 32))), dim3(AF_THREADS), 0, stream, g);
@@ -390,10 +405,10 @@ int launch_attn_f32_rows(const AttnF32Args& g, int n_tiles, int parts, cudaStrea
     return SS_LAUNCH_CHECK();
 }
 
-// 64 rows of a prompt portion to a block (32 beyond 128 elements a head: 64 would need 256 output registers a thread); a
-// decode step's rows of one request in tiles of 16.
+// 32 rows of a prompt portion to a block (64, with 8 warps and half the blocks: 257 us where 32 take 209, 777 tokens at the 7B sizes); a decode
+// step's rows of one request in tiles of 16.
 template <int D>
 int launch_attn_f32(const AttnF32Args& g, int n_tiles, int parts, cudaStream_t stream) {
     if (g.tile_req == nullptr) return launch_attn_f32_rows<D, 16>(g, n_tiles, parts, stream);
-    return launch_attn_f32_rows<D, D <= 128 ? 64 : 32>(g, n_tiles, parts, stream);
+    return launch_attn_f32_rows<D, 32>(g, n_tiles, parts, stream);
 }

@@ -141,6 +141,33 @@ def test_sampling_kernel_at_random_settings():
             assert np.isfinite(kept[got[i]]) and score[got[i]] >= score.max() - 1e-3, (trial, i, r, got[i])
 
 
+# what the passes over a histogram cannot settle (more values in the threshold's bin than the list holds, infinities), what they
+# settle by different rules (top-k alone, top-p alone, both, more than the list holds under both), one, some and eight blocks a row
+@pytest.mark.parametrize("m, vocab", [(1, 50000), (20, 9001), (150, 4099)])
+def test_sampling_where_the_threshold_falls_among_many_or_odd_values(m, vocab):
+    torch.manual_seed(m)
+    logits = torch.randn(m, vocab) * 2.0
+    kinds = [dict(top_k=-1, top_p=0.8), dict(top_k=40, top_p=1.0), dict(top_k=3000, top_p=1.0), dict(top_k=3000, top_p=0.7),
+             dict(top_k=1000, top_p=0.7), dict(top_k=2, top_p=1e-6)]
+    rows = [dict(temperature=0.9, seed=i, draw=i % 3, min_p=0.0, repetition_penalty=1.0, **kinds[(i + m) % len(kinds)]) for i in range(m)]
+    for i in range(m):
+        if i % 4 == 1:
+            logits[i] = logits[i].round()  # every value in a few bins
+        if i % 4 == 2:
+            logits[i, ::2] = -float("inf")
+        if i % 4 == 3:
+            logits[i] = 1.0 + 1e-6 * logits[i]
+    dev = logits.to(DEV)
+    got = run_sample(dev, rows)
+    for i, r in enumerate(rows):
+        values = logits[i] / np.float32(r["temperature"])  # the kernel's own rounding decides which values are equal
+        kept = plain.filtered_logits(values, temperature=1.0, top_k=r["top_k"], top_p=r["top_p"], min_p=0.0)
+        kept = np.where(values.numpy() >= float(kept[torch.isfinite(kept)].min()), values.double().numpy(), -np.inf)  # ties stay
+        score = kept + gumbel_noise(r["seed"], r["draw"], vocab)
+        assert np.isfinite(kept[got[i]]) and score[got[i]] >= score.max() - 1e-3, (i, r, got[i])
+    ops().check_errors(torch.device(DEV))
+
+
 def test_engine_under_random_schedules_gives_the_tokens_of_the_engine_with_room(model_folders):
     """2 to 10 requests with prompts of 1 to 75 tokens and 1 to 40 new tokens, greedy or sampled with seeds,
     filters and penalty; pools of pages from barely enough for the longest request to three times that, at most

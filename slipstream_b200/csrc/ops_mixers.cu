@@ -512,131 +512,10 @@ ssm_scan_kernel(const T* __restrict__ xbc, int C, const T* __restrict__ dt_raw, 
     }
 }
 
-// The same recurrence for bfloat16 rows whose parts start on 16-byte boundaries: the tokens' B, C and x are copied
-// to shared memory as they are (cp.async, 16 bytes a copy) one batch of tokens ahead of the arithmetic, into two
-// buffers that take turns, and widened to float32 as they are read (8 values a 16-byte load).
-__device__ __forceinline__ void cp_async_16_on(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
-}
-template <int PER>
-__global__ void __launch_bounds__(SCAN_PT * SCAN_NS)
-ssm_scan_bf16_kernel(const bf16* __restrict__ xbc, int C, const bf16* __restrict__ dt_raw, int64_t dt_stride,
-                     const float* __restrict__ dt_bias, const float* __restrict__ a_log,
-                     const float* __restrict__ d_skip, float* __restrict__ state, float* __restrict__ y,
-                     const int32_t* __restrict__ q_start, const int32_t* __restrict__ seq_lens,
-                     const int32_t* __restrict__ slots, int heads, int groups, int P, int N, int PT, int n_slots,
-                     int* err) {
-    pdl_wait();
-    constexpr int TB = PER >= 64 ? 16 : 32;
-    constexpr int SEGB = PER * 2 + 16, ROWB = SCAN_NS * SEGB;  // bytes: a lane's segment (16 apart from the next), a token's row
-    extern __shared__ __align__(16) unsigned char raw_sm[];
-    // per stage: B rows, C rows, x rows; behind both stages: the step sizes and decays of both
-    const int stage_bytes = 2 * TB * ROWB + TB * PT * 2;
-    float* dts = reinterpret_cast<float*>(raw_sm + 2 * stage_bytes);  // [2][TB]
-    float* decs = dts + 2 * TB;                                        // [2][TB]
-    const int r = blockIdx.x, h = blockIdx.y, p0 = blockIdx.z * PT;
-    const int q0 = q_start[r], q_len = q_start[r + 1] - q0;
-    if (q_len <= 0 || seq_lens[r] <= 0) return;
-    const int slot = slots[r];
-    if (slot < 0 || slot >= n_slots) {
-        if (threadIdx.x == 0) atomicOr(err, SS_ERR_SLOT_RANGE);
-        return;
-    }
-    const int tid = threadIdx.x, pl = tid / SCAN_NS, ns = tid % SCAN_NS;
-    const int p = p0 + pl, n0 = ns * PER;
-    const bool valid = p < P;
-    const int g = h / (heads / groups);
-    const int inner = heads * P;
-    float* st = state + (((int64_t)slot * heads + h) * P + (valid ? p : 0)) * N;
-    float S[PER];
-#pragma unroll
-    for (int i = 0; i < PER; i += 4) {  // N is a multiple of 8 here
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (valid && n0 + i < N) v = *reinterpret_cast<const float4*>(st + n0 + i);
-        S[i] = v.x; S[i + 1] = v.y; S[i + 2] = v.z; S[i + 3] = v.w;
-    }
-    const float rate = expf(a_log[h]), bias = dt_bias[h], skip = d_skip[h];
-    for (int i = tid * 16; i < 2 * stage_bytes; i += blockDim.x * 16)  // what no copy writes (n beyond N) stays zero
-        *reinterpret_cast<uint4*>(raw_sm + i) = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-    const int chunks = N >> 3, x_chunks = PT >> 3;
-    auto issue = [&](int stage, int t0, int nt) {
-        unsigned char* base = raw_sm + stage * stage_bytes;
-        for (int idx = tid; idx < nt * 2 * chunks; idx += blockDim.x) {
-            const int tt = idx / (2 * chunks), rem = idx - tt * 2 * chunks;
-            const int which = rem >= chunks, n = (rem - which * chunks) << 3;
-            cp_async_16_on(base + which * TB * ROWB + tt * ROWB + (n / PER) * SEGB + (n % PER) * 2,
-                           xbc + (int64_t)(q0 + t0 + tt) * C + inner + which * groups * N + g * N + n);
-        }
-        for (int idx = tid; idx < nt * x_chunks; idx += blockDim.x) {
-            const int tt = idx / x_chunks, c = idx - tt * x_chunks;
-            if (p0 + 8 * c < P)
-                cp_async_16_on(base + 2 * TB * ROWB + (tt * PT + 8 * c) * 2, xbc + (int64_t)(q0 + t0 + tt) * C + h * P + p0 + 8 * c);
-        }
-    };
-    const int n_batches = (q_len + TB - 1) / TB;
-    issue(0, 0, min(TB, q_len));
-    cp_async_commit();
-    float dt_next = (tid < min(TB, q_len)) ? to_float(dt_raw[(int64_t)(q0 + tid) * dt_stride + h]) : 0.f;
-    for (int k = 0; k < n_batches; ++k) {
-        const int t0 = k * TB, nt = min(TB, q_len - t0), buf = k & 1;
-        if (tid < nt) {
-            const float z = dt_next + bias;
-            const float dt = z > 20.f ? z : log1pf(expf(z));
-            dts[buf * TB + tid] = dt;
-            decs[buf * TB + tid] = expf(-rate * dt);
-        }
-        if (k + 1 < n_batches) {
-            const int nt1 = min(TB, q_len - t0 - TB);
-            issue(buf ^ 1, t0 + TB, nt1);
-            if (tid < nt1) dt_next = to_float(dt_raw[(int64_t)(q0 + t0 + TB + tid) * dt_stride + h]);
-        }
-        cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        const unsigned char* base = raw_sm + buf * stage_bytes;
-        const bf16* xs = reinterpret_cast<const bf16*>(base + 2 * TB * ROWB);
-        float* yp = y + (int64_t)(q0 + t0) * inner + h * P + p;
-#pragma unroll 2
-        for (int tt = 0; tt < nt; ++tt, yp += inner) {
-            const float dec = decs[buf * TB + tt], xv = to_float(xs[tt * PT + pl]);
-            const float dx = dts[buf * TB + tt] * xv;
-            const uint4* b8 = reinterpret_cast<const uint4*>(base + tt * ROWB + ns * SEGB);
-            const uint4* c8 = reinterpret_cast<const uint4*>(base + TB * ROWB + tt * ROWB + ns * SEGB);
-            float acc0 = 0.f, acc1 = 0.f;
-#pragma unroll
-            for (int i = 0; i < PER; i += 8) {
-                const uint4 bw = b8[i >> 3], cw = c8[i >> 3];
-                const uint32_t bb[4] = {bw.x, bw.y, bw.z, bw.w}, cc[4] = {cw.x, cw.y, cw.z, cw.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float b_lo = __uint_as_float(bb[e] << 16), b_hi = __uint_as_float(bb[e] & 0xffff0000u);
-                    const float c_lo = __uint_as_float(cc[e] << 16), c_hi = __uint_as_float(cc[e] & 0xffff0000u);
-                    S[i + 2 * e] = fmaf(dec, S[i + 2 * e], dx * b_lo);
-                    S[i + 2 * e + 1] = fmaf(dec, S[i + 2 * e + 1], dx * b_hi);
-                    acc0 = fmaf(S[i + 2 * e], c_lo, acc0);
-                    acc1 = fmaf(S[i + 2 * e + 1], c_hi, acc1);
-                }
-            }
-            float acc = acc0 + acc1;
-            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-            if (ns == 0 && valid) *yp = fmaf(skip, xv, acc);
-        }
-        __syncthreads();  // the buffer is free for the copies of the batch after next
-    }
-    cp_async_wait<0>();
-    if (valid) {
-#pragma unroll
-        for (int i = 0; i < PER; i += 4)
-            if (n0 + i < N) *reinterpret_cast<float4*>(st + n0 + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
-    }
-}
-
 extern "C" int ss_ssm_scan(const void* xbc, int C, const void* dt_raw, int64_t dt_stride, const float* dt_bias,
                            const float* a_log, const float* d_skip, float* state, float* y, const int32_t* q_start,
                            const int32_t* seq_lens, const int32_t* slots, int R, int heads, int groups, int P, int N,
-                           int n_slots, int dtype, int* err, cudaStream_t stream, int long_rows) {
+                           int n_slots, int dtype, int* err, cudaStream_t stream) {
     if (R <= 0) return 0;
     if (N < 1 || N > 256 || P < 1 || groups < 1 || heads % groups) return (int)cudaErrorInvalidValue;
     const int PT = P >= SCAN_PT ? SCAN_PT : (P + 7) / 8 * 8;  // a block of PT * 4 threads: whole warps
@@ -644,20 +523,6 @@ extern "C" int ss_ssm_scan(const void* xbc, int C, const void* dt_raw, int64_t d
     const int per = N <= 32 ? 8 : (N <= 64 ? 16 : (N <= 128 ? 32 : 64));
     const int tb = per >= 64 ? 16 : 32;
     const int smem = (2 * tb * SCAN_NS * (per + 4) + tb * PT + 2 * tb) * 4;
-    if (long_rows && dtype == SS_BF16 && C % 8 == 0 && (heads * P) % 8 == 0 && N % 8 == 0 && P % 8 == 0 && ((uintptr_t)xbc & 15) == 0 &&
-        ((uintptr_t)state & 15) == 0) {
-        const int stage = 2 * tb * SCAN_NS * (per * 2 + 16) + tb * PT * 2;
-        const int smem16 = 2 * stage + 4 * tb * 4;
-#define SCAN16_GO(PER)                                                                                                  \
-    ss_launch(ssm_scan_bf16_kernel<PER>, grid, block, smem16, stream, (const bf16*)xbc, C, (const bf16*)dt_raw, dt_stride,  \
-              dt_bias, a_log, d_skip, state, y, q_start, seq_lens, slots, heads, groups, P, N, PT, n_slots, err)
-        if (per == 8) SCAN16_GO(8);
-        else if (per == 16) SCAN16_GO(16);
-        else if (per == 32) SCAN16_GO(32);
-        else SCAN16_GO(64);
-#undef SCAN16_GO
-        return SS_LAUNCH_CHECK();
-    }
 #define SCAN_GO(T, PER)                                                                                                 \
     ss_launch(ssm_scan_kernel<T, PER>, grid, block, smem, stream, (const T*)xbc, C, (const T*)dt_raw, dt_stride, dt_bias,     \
               a_log, d_skip, state, y, q_start, seq_lens, slots, heads, groups, P, N, PT, n_slots, err)

@@ -64,8 +64,12 @@ _OPS_SIGNATURES = {
     "ss_round_stream": [c_void_p, c_void_p, c_int64, c_void_p],
     "ss_conv_silu": [c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                      c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int],
+    "ss_ssm_scan_chunks": [c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                           c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    "ss_matrix_cell_chunks": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_float, c_float, c_void_p, c_void_p, c_void_p,
+                              c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "ss_ssm_scan": [c_void_p, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                    c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int],
+                    c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "ss_router": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p,
                   c_int, c_int, c_void_p, c_int, c_void_p],
     "ss_moe_plan": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int],
@@ -1853,12 +1857,13 @@ def conv_silu(proj: torch.Tensor, col0: int, channels: int, taps: torch.Tensor, 
 
 
 def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
-             state: torch.Tensor, ctx, heads: int, groups: int, head_dim: int, state_dim: int) -> torch.Tensor:
+             state: torch.Tensor, ctx, heads: int, groups: int, head_dim: int, state_dim: int, chunks: bool = True) -> torch.Tensor:
     """The diagonal state-space recurrence over each request's tokens, continued from and left in ``state``
     (float32 [slots, heads, head_dim, state_dim]).  ``xbc`` [N, heads * head_dim + 2 * groups * state_dim] holds x, then
     B, then C; ``dt`` [N, heads] is a view of the raw step sizes (unit inner stride).  Per head h (group
     ``h // (heads / groups)``): ``dt' = softplus(dt + dt_bias[h])``, ``S <- exp(-exp(a_log[h]) dt') S + dt' B x^T``,
-    ``y = S^T C + d_skip[h] x``.  Returns y float32 [N, heads * head_dim]."""
+    ``y = S^T C + d_skip[h] x``.  Returns y float32 [N, heads * head_dim].  Steps with prompt portions run the kernel that takes
+    chunks of tokens on the tensor cores where it can (``chunks`` False: never): bfloat16 rows, sizes in steps of 8."""
     _need(xbc, None, "x, B and C")
     for name, t in (("dt_bias", dt_bias), ("a_log", a_log), ("d_skip", d_skip), ("state", state)):
         _need(t, torch.float32, name)
@@ -1869,11 +1874,19 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
     if tuple(state.shape[1:]) != (heads, head_dim, state_dim) or state_dim > 256:
         raise KernelError("ssm_scan: the state must be [slots, heads, head_dim, state_dim] with state_dim <= 256")
     y = torch.empty((n, inner), dtype=torch.float32, device=xbc.device)
+    if (chunks and not ctx.is_decode_only and xbc.dtype == torch.bfloat16 and head_dim % 8 == state_dim % 8 == xbc.shape[1] % 8 == 0
+            and xbc.data_ptr() % 16 == 0):
+        _check(ops_library().ss_ssm_scan_chunks(xbc.data_ptr(), xbc.shape[1], dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(),
+                                                a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), y.data_ptr(),
+                                                ctx.q_start.data_ptr(), ctx.seq_lens.data_ptr(), ctx.state_slots.data_ptr(),
+                                                ctx.num_requests, heads, groups, head_dim, state_dim, state.shape[0],
+                                                error_word(xbc.device).data_ptr(), _stream()), "ssm_scan_chunks")
+        return y
     _check(ops_library().ss_ssm_scan(xbc.data_ptr(), xbc.shape[1], dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(),
                                      a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), y.data_ptr(),
                                      ctx.q_start.data_ptr(), ctx.seq_lens.data_ptr(), ctx.state_slots.data_ptr(),
                                      ctx.num_requests, heads, groups, head_dim, state_dim, state.shape[0], _code(xbc.dtype),
-                                     error_word(xbc.device).data_ptr(), _stream(), int(not ctx.is_decode_only)), "ssm_scan")
+                                     error_word(xbc.device).data_ptr(), _stream()), "ssm_scan")
     return y
 
 
@@ -2109,7 +2122,7 @@ def embed_sum(token_ids: torch.Tensor, table: torch.Tensor, ctx, *, pair_table: 
 
 
 def matrix_cell(qkv: torch.Tensor, gates: torch.Tensor, bias_i: torch.Tensor | None, bias_f: torch.Tensor | None, cap: float,
-                q_scale: float, memory: torch.Tensor, peak: torch.Tensor, ctx, heads: int, dim: int, vdim: int
+                q_scale: float, memory: torch.Tensor, peak: torch.Tensor, ctx, heads: int, dim: int, vdim: int, chunks: bool = True
                 ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """The matrix-memory recurrence over each request's tokens, continued from and left in ``memory`` (float32
     [slots, heads, vdim + 1, dim]: S column by column, the last column the normaliser n) and ``peak`` (float32
@@ -2117,7 +2130,9 @@ def matrix_cell(qkv: torch.Tensor, gates: torch.Tensor, bias_i: torch.Tensor | N
     k: heads * dim | v: heads * vdim]; ``gates`` float32 [N, >= 2 heads] holds the raw input and forget gates.  With
     ``i = cap tanh((a + bias_i) / cap)`` and ``f = logsigmoid(cap tanh((b + bias_f) / cap))``:
     ``m' = max(f + m, i)``, ``S <- exp(f + m - m') S + exp(i - m') k v^T``, n likewise with k alone.
-    Returns (``S^T (q_scale q)`` float32 [N, heads * vdim], ``n . (q_scale q)`` [N, heads], m [N, heads])."""
+    Returns (``S^T (q_scale q)`` float32 [N, heads * vdim], ``n . (q_scale q)`` [N, heads], m [N, heads]).  Steps with prompt
+    portions run the kernel that takes chunks of tokens on the tensor cores where it can (``chunks`` False: never): bfloat16
+    rows, sizes in steps of 8."""
     _need(qkv, None, "q, k and v")
     _need(gates, torch.float32, "gates")
     _need(memory, torch.float32, "memory")
@@ -2133,6 +2148,14 @@ def matrix_cell(qkv: torch.Tensor, gates: torch.Tensor, bias_i: torch.Tensor | N
     num = torch.empty((n, heads * vdim), dtype=torch.float32, device=qkv.device)
     nq = torch.empty((n, heads), dtype=torch.float32, device=qkv.device)
     peaks = torch.empty((n, heads), dtype=torch.float32, device=qkv.device)
+    if (chunks and not ctx.is_decode_only and qkv.dtype == torch.bfloat16 and dim % 8 == vdim % 8 == qkv.stride(0) % 8 == 0
+            and qkv.data_ptr() % 16 == 0 and cap > 0.0):
+        _check(ops_library().ss_matrix_cell_chunks(
+            qkv.data_ptr(), qkv.stride(0), gates.data_ptr(), gates.stride(0), _ptr(bias_i), _ptr(bias_f), float(cap), float(q_scale),
+            memory.data_ptr(), peak.data_ptr(), num.data_ptr(), nq.data_ptr(), peaks.data_ptr(), ctx.q_start.data_ptr(),
+            ctx.seq_lens.data_ptr(), ctx.state_slots.data_ptr(), ctx.num_requests, heads, dim, vdim, memory.shape[0],
+            error_word(qkv.device).data_ptr(), _stream()), "matrix_cell_chunks")
+        return num, nq, peaks
     _check(ops_library().ss_matrix_cell(qkv.data_ptr(), qkv.stride(0), gates.data_ptr(), gates.stride(0), _ptr(bias_i),
                                         _ptr(bias_f), float(cap), float(q_scale), memory.data_ptr(), peak.data_ptr(),
                                         num.data_ptr(), nq.data_ptr(), peaks.data_ptr(), ctx.q_start.data_ptr(),

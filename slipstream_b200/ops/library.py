@@ -26,7 +26,7 @@ import time
 from pathlib import Path
 
 # the row-wise operations and recurrences of every design: one library
-OPS_SOURCES = ["ops.cu", "ops_streams.cu", "ops_mixers.cu", "ops_cells.cu", "ops_gated.cu", "ops_heads.cu", "ops_retention.cu",
+OPS_SOURCES = ["ops.cu", "ops_streams.cu", "ops_mixers.cu", "ops_cells.cu", "ops_gated.cu", "ops_heads.cu", "ops_retention.cu", "ops_scan.cu",
                "sampling.cu"]
 # the tensor-core matrix products
 GEMM_SOURCES = ["gemm_tc5.cu", "gemm_f32.cu"]

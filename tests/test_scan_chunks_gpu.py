@@ -1,0 +1,129 @@
+"""The state-space scan and the matrix memory over prompt portions in chunks on the tensor cores, against the recurrence token by
+token in double precision: key and value sizes at the edges of the kernel's tiles, requests at the edges of its chunks of 64
+tokens, whole and cut, and values that are not finite."""
+import types
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+# Every float32 factor is carried with its 24 bits; sums of 64 to 256 products truncate by 2^-23 of a partial sum at a time and the
+# decays of a chunk are off by a few 2^-24: a few 1e-7 of the result.  The token-by-token kernels show 1e-7 to 5e-7.
+TOLERANCE = 1e-6
+
+
+def step_ctx(q_lens, slots):
+    as_dev = lambda a: torch.tensor(np.asarray(a, dtype=np.int32), device=DEV)  # noqa: E731
+    return types.SimpleNamespace(q_start=as_dev(np.concatenate([[0], np.cumsum(q_lens)])), seq_lens=as_dev(np.maximum(q_lens, 1)),
+                                 state_slots=as_dev(slots), num_requests=len(q_lens), is_decode_only=False)
+
+
+def off(got, want):
+    return float((got.double().cpu() - want).norm() / want.norm())
+
+
+def walk(decay, k, x, q, state):
+    """S <- decay S + k x^T, y = S^T q, head by head in double precision: decay [n, h], k and q [n, h, a], x [n, h, b], S [h, b, a]."""
+    out = []
+    for t in range(decay.shape[0]):
+        state = decay[t][:, None, None] * state + x[t][:, :, None] * k[t][:, None, :]
+        out.append((state * q[t][:, None, :]).sum(-1))
+    return torch.stack(out), state
+
+
+@pytest.mark.parametrize("heads, groups, p, n, bias", [(4, 2, 64, 128, -1.0), (3, 1, 8, 8, 3.0), (2, 2, 72, 64, -4.0), (2, 1, 40, 72, 0.0),
+                                                       (3, 3, 128, 136, -1.0), (2, 1, 32, 256, 1.0)])
+def test_state_space_scan_in_chunks(heads, groups, p, n, bias):
+    from slipstream_b200 import ops
+    g = torch.Generator().manual_seed(n + p)
+    lens, slots, inner = [1, 63, 64, 65, 0, 150], [5, 0, 3, 1, 2, 4], heads * p
+    xbc = [torch.randn(t, inner + 2 * groups * n, generator=g).bfloat16() for t in lens]
+    dt = [torch.randn(t, heads + 3, generator=g).bfloat16() for t in lens]
+    dt_bias, a_log, d = torch.randn(heads, generator=g) * 0.5 + bias, torch.randn(heads, generator=g) * 0.5 - 0.5, torch.randn(heads, generator=g)
+    start = torch.randn(7, heads, p, n, generator=g)
+    want, states = [], start.double().clone()
+    for rows, steps, slot in zip(xbc, dt, slots):
+        v, t = rows.double(), rows.shape[0]
+        if t == 0:
+            continue
+        x = v[:, :inner].reshape(t, heads, p)
+        b, c = (v[:, inner + i * groups * n: inner + (i + 1) * groups * n].reshape(t, groups, n).repeat_interleave(heads // groups, 1) for i in range(2))
+        w = torch.nn.functional.softplus(steps[:, 3:].double() + dt_bias.double())
+        y, states[slot] = walk(torch.exp(-a_log.double().exp() * w), b, w[..., None] * x, c, states[slot])
+        want.append((y + d.double()[:, None] * x).reshape(t, inner))
+    want = torch.cat(want)
+    consts = [v.to(DEV) for v in (dt_bias, a_log, d)]
+    for cut in (None, 33):  # whole, and every request in two portions
+        state, outs = start.to(DEV), [[] for _ in lens]
+        for part in ([(0, None)] if cut is None else [(0, cut), (cut, None)]):
+            rows, steps = ([v[part[0]: part[1]] for v in s] for s in (xbc, dt))
+            counts = [v.shape[0] for v in rows]
+            y = ops.ssm_scan(torch.cat(rows).to(DEV), torch.cat(steps).to(DEV)[:, 3:], *consts, state, step_ctx(counts, slots), heads, groups, p, n)
+            for i, piece in enumerate(y.split(counts)):
+                outs[i].append(piece)
+        assert off(torch.cat([torch.cat(o) for o in outs]), want) < TOLERANCE, cut
+        assert off(state, states) < TOLERANCE and torch.equal(state[6].cpu(), start[6]), cut
+    ops.check_errors(DEV)
+
+
+@pytest.mark.parametrize("heads, dim, vdim, bias", [(3, 128, 128, 3.0), (2, 8, 8, 0.0), (2, 64, 72, 8.0), (3, 96, 64, -3.0), (2, 256, 40, 4.0), (1, 136, 200, 3.0)])
+def test_matrix_memory_in_chunks(heads, dim, vdim, bias):
+    from slipstream_b200 import ops
+    g = torch.Generator().manual_seed(dim + vdim)
+    lens, slots, cap, scale = [1, 63, 64, 65, 0, 150], [5, 0, 3, 1, 2, 4], 6.0, dim ** -0.5
+    qkv = [torch.randn(t, heads * (2 * dim + vdim) + 8, generator=g).bfloat16()[:, : heads * (2 * dim + vdim) + 8] for t in lens]
+    gates = [torch.randn(t, 2 * heads + 1, generator=g) * 4 for t in lens]
+    bias_i, bias_f = torch.randn(heads, generator=g), torch.randn(heads, generator=g) + bias
+    memory0, peak0 = torch.randn(7, heads, vdim + 1, dim, generator=g), torch.randn(7, heads, generator=g)
+    want, memories, peaks = [], memory0.double().clone(), peak0.double().clone()
+    for rows, gate, slot in zip(qkv, gates, slots):
+        v, t = rows.double(), rows.shape[0]
+        if t == 0:
+            continue
+        q, k, x = (v[:, o: o + heads * w].reshape(t, heads, w) for o, w in ((0, dim), (heads * dim, dim), (2 * heads * dim, vdim)))
+        i = cap * torch.tanh((gate[:, :heads].double() + bias_i.double()) / cap)
+        f = torch.nn.functional.logsigmoid(cap * torch.tanh((gate[:, heads: 2 * heads].double() + bias_f.double()) / cap))
+        m, ms = peaks[slot], []
+        for step in range(t):
+            m = torch.maximum(f[step] + m, i[step])
+            ms.append(m)
+        ms = torch.stack(ms)
+        before = torch.cat([peaks[slot][None], ms[:-1]])
+        grown = torch.exp(i - ms)[..., None] * torch.cat([x, torch.ones_like(x[..., :1])], -1)
+        y, memories[slot] = walk(torch.exp(f + before - ms), k, grown, q * scale, memories[slot])
+        peaks[slot] = ms[-1]
+        want.append((y[..., :vdim].reshape(t, -1), y[..., vdim], ms))
+    want = [torch.cat(v) for v in zip(*want)]
+    for cut in (None, 33):
+        memory, peak, outs = memory0.to(DEV), peak0.to(DEV), [[] for _ in lens]
+        for part in ([(0, None)] if cut is None else [(0, cut), (cut, None)]):
+            rows, gate = ([v[part[0]: part[1]] for v in s] for s in (qkv, gates))
+            counts = [v.shape[0] for v in rows]
+            got = ops.matrix_cell(torch.cat(rows).to(DEV), torch.cat(gate).to(DEV), bias_i.to(DEV), bias_f.to(DEV), cap, scale, memory, peak,
+                                  step_ctx(counts, slots), heads, dim, vdim)
+            for i, piece in enumerate(zip(*(v.split(counts) for v in got))):
+                outs[i].append(piece)
+        for which in range(3):
+            assert off(torch.cat([piece[which] for o in outs for piece in o]), want[which]) < TOLERANCE, (cut, which)
+        assert off(memory, memories) < TOLERANCE and off(peak, peaks) < TOLERANCE and torch.equal(memory[6].cpu(), memory0[6]), cut
+    ops.check_errors(DEV)
+
+
+@pytest.mark.parametrize("token, column, value", [(0, 3, "inf"), (70, 5, "nan"), (63, 2, "-inf"), (100, 256 + 7, "nan"), (130, 512 + 9, "inf")])
+def test_what_is_not_finite_reaches_what_it_reaches_token_by_token(token, column, value):
+    """An infinity or a NaN among the values (columns up to 256), B (then 256) and C of one token."""
+    from slipstream_b200 import ops
+    torch.manual_seed(0)
+    heads, groups, p, n, t = 4, 2, 64, 128, 150
+    xbc, dt = torch.randn(t, heads * p + 2 * groups * n, device=DEV).bfloat16(), torch.randn(t, heads, device=DEV).bfloat16()
+    consts = [torch.randn(heads, device=DEV) * 0.5 for _ in range(3)]
+    xbc[token, column] = float(value)
+    got, want = (ops.ssm_scan(xbc, dt, *consts, torch.zeros(1, heads, p, n, device=DEV), step_ctx([t], [0]), heads, groups, p, n, chunks=c)
+                 for c in (True, False))
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), finite) and 0 < int((~finite).sum()) < finite.numel()
+    assert off(got[finite], want[finite].double().cpu()) < 2 * TOLERANCE
+    ops.check_errors(DEV)

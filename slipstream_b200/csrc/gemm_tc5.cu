@@ -1182,6 +1182,167 @@ extern "C" int ss_gemm_tc5_grouped(const void* A, const void* B, void* C, int to
     return launch_pair<0>(ma, mb, g, tiles2 < max_pairs ? tiles2 : max_pairs, stream);
 }
 
+// ---------------------------------------------------------------- grouped products with few rows an expert
+//
+// The experts' products of decode steps: out[s] = act(W[e] A[s]) for the rows s of the plan's tiles (tile_expert, tile_row0,
+// tile_rows; rows sorted by expert, at most BN a tile).  As in the swapped form above the weight's rows fill the 128 lanes of
+// the product and the tile's rows are its BN columns; a block takes one tile of rows and 128 weight rows, over all of K.  B is
+// read from tile_row0 on, so columns beyond the tile's rows hold other experts' rows (or nothing) and are not stored.
+// MODE: 0 float32 out[perm[s]][m]; 1 rows alternate 64 gate and 64 up features, bfloat16 out[s][m / 2] = silu(gate) * up; 2
+// bfloat16 out[s][m] = max(z, 0)^2.
+// Bound by the weights' way from memory.  Up and down products with plan and gather at 8 experts of 4,736 x 3,584 and two
+// choices, against mma.sync tiles of 32 or 128 rows fed by cp.async, whose threads spend their time on the copies' addresses:
+// 4 tokens 181 -> 79 us (62 at the copy bandwidth), 12 220 -> 124 (109), 64 221 -> 138 (124), 256 483 -> 153, 500 726 -> 207.
+struct ExpertsArgs {
+    void* out;
+    const int32_t* perm;
+    const int32_t* tile_expert;
+    const int32_t* tile_row0;
+    const int32_t* tile_rows;
+    int M, K;        // weight rows of an expert, and their length
+    int64_t ldc;
+    int* err;
+};
+
+template <int BN, int STAGES, int MODE>
+__global__ void __launch_bounds__(TC_THREADS)
+gemm_tc5_experts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const ExpertsArgs g) {
+    constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2, STAGE = A_BYTES + B_BYTES;
+    constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
+    static_assert(BN * TC_BM * 4 <= STAGES * STAGE, "a tile of sums fits the ring");
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = reinterpret_cast<uint64_t*>(ring + STAGES * STAGE);
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_ready = empty + STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_ready + 1);
+    volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    pdl_wait();  // the plan is an earlier kernel's
+    const int e = g.tile_expert[blockIdx.x];
+    if (e < 0) return;  // (the whole block; nothing has been set up)
+    const int row0 = g.tile_row0[blockIdx.x], rows = min(BN, g.tile_rows[blockIdx.x]), m0 = blockIdx.y * TC_BM;
+    const int k_iters = (g.K + TC_BK - 1) / TC_BK;
+    if (threadIdx.x == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(acc_ready, 1);
+        *gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_addr(tmem_slot)), "r"(TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0 && lane == 0) {
+        const uint64_t once = l2_evict_first_policy();
+        for (int it = 0; it < k_iters; ++it) {
+            const int s = it % STAGES;
+            if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, gave_up)) break;
+            mbar_expect_tx(&full[s], STAGE);
+            tma_load_2d_once(ring + s * STAGE, &map_w, it * TC_BK, e * g.M + m0, &full[s], once);
+            tma_load_2d(ring + s * STAGE + A_BYTES, &map_x, it * TC_BK, row0, &full[s]);
+        }
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+        for (int it = 0; it < k_iters; ++it) {
+            const int s = it % STAGES;
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (it / STAGES) & 1, gave_up))) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t a_desc = smem_desc(ring + s * STAGE), b_desc = smem_desc(ring + s * STAGE + A_BYTES);
+            if (elect_one()) {
+#pragma unroll
+                for (int kk = 0; kk < TC_BK / 16; ++kk)
+                    umma_f16(tmem, a_desc + (uint64_t)(kk * 2), b_desc + (uint64_t)(kk * 2), idesc, (it | kk) != 0);
+                umma_commit(&empty[s]);
+            }
+            __syncwarp();
+        }
+        if (elect_one()) umma_commit(acc_ready);
+        __syncwarp();
+    } else if (warp >= 2) {
+        const int quarter = warp & 3, t = quarter * 32 + lane, m = m0 + t;
+        const bool good = __all_sync(0xffffffffu, mbar_wait(acc_ready, 0, gave_up));
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        float* sums = reinterpret_cast<float*>(ring);  // MODE 1: all stages have been consumed, gate and up meet here
+#pragma unroll 1
+        for (int c = 0; c < rows; c += 16) {
+            uint32_t r[16];
+            tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + c, r);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                if constexpr (MODE == 1) {
+                    sums[(c + j) * TC_BM + t] = __uint_as_float(r[j]);
+                } else {
+                    if (c + j >= rows || m >= g.M || !good) continue;
+                    const float v = __uint_as_float(r[j]);
+                    if constexpr (MODE == 0) ((float*)g.out)[(int64_t)g.perm[row0 + c + j] * g.ldc + m] = v;
+                    else ((bf16*)g.out)[(int64_t)(row0 + c + j) * g.ldc + m] = __float2bfloat16_rn(v > 0.f ? v * v : 0.f);
+                }
+            }
+        }
+        if constexpr (MODE == 1) {
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            const int ml = t & 63;  // gate and up feature ml of the tile, every other row
+            for (int c = t >> 6; c < rows && good; c += 2)
+                ((bf16*)g.out)[(int64_t)(row0 + c) * g.ldc + (m0 >> 1) + ml] =
+                    __float2bfloat16_rn(silu_mul<true>(sums[c * TC_BM + ml], sums[c * TC_BM + ml + 64]));
+        }
+    }
+    if (*gave_up && threadIdx.x == 0) atomicOr(g.err, SS_ERR_WAIT_LIMIT);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+    }
+}
+
+template <int BN, int STAGES, int MODE>
+static int launch_experts(const CUtensorMap& mw, const CUtensorMap& mx, const ExpertsArgs& g, int n_tiles, cudaStream_t stream) {
+    constexpr int smem = STAGES * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + 1024 + 256;
+    static SsPerDevice opted;
+    if (int rc = ss_opt_in_smem(gemm_tc5_experts_kernel<BN, STAGES, MODE>, smem, opted)) return rc;
+    ss_launch(gemm_tc5_experts_kernel<BN, STAGES, MODE>, dim3(n_tiles, (g.M + TC_BM - 1) / TC_BM), dim3(TC_THREADS), smem, stream, mw, mx, g);
+    return SS_LAUNCH_CHECK();
+}
+template <int MODE>
+static int launch_experts_rows(const CUtensorMap& mw, const CUtensorMap& mx, const ExpertsArgs& g, int tile, int n_tiles, cudaStream_t stream) {
+    switch (tile) {
+        case 16: return launch_experts<16, 4, MODE>(mw, mx, g, n_tiles, stream);
+        case 32: return launch_experts<32, 4, MODE>(mw, mx, g, n_tiles, stream);
+        case 64: return launch_experts<64, 4, MODE>(mw, mx, g, n_tiles, stream);
+        case 128: return launch_experts<128, 3, MODE>(mw, mx, g, n_tiles, stream);
+        default: return -2011;
+    }
+}
+
+// rows [total, K] bfloat16 sorted by expert, W [experts, M, K]; the plan's tiles hold at most `tile` (16, 32, 64 or 128) rows.
+// mode as above; out float32 [..][M] (0), bfloat16 [total][M / 2] (1, M a multiple of 128) or [total][M] (2).
+extern "C" int ss_gemm_tc5_experts(const void* rows, const void* W, void* out, int total, int M, int K, int experts, int mode, int tile,
+                                   const int32_t* perm, const int32_t* tile_expert, const int32_t* tile_row0, const int32_t* tile_rows,
+                                   int n_tiles, int* err, cudaStream_t stream) {
+    if (total <= 0 || M <= 0 || n_tiles <= 0) return 0;
+    if (K <= 0 || K % 8 != 0) return -2003;
+    if (((uintptr_t)rows & 15) || ((uintptr_t)W & 15)) return -2004;
+    if (mode == 1 && M % 128 != 0) return -2007;
+    if (!perm || !tile_expert || !tile_row0 || !tile_rows || mode < 0 || mode > 2) return -2010;
+    CUtensorMap mw, mx;
+    if (int rc = make_map(&mw, W, (int64_t)experts * M, K, K, TC_BM)) return rc;
+    if (int rc = make_map(&mx, rows, total, K, K, tile)) return rc;
+    const ExpertsArgs g{out, perm, tile_expert, tile_row0, tile_rows, M, K, mode == 1 ? M / 2 : M, err};
+    return mode == 0 ? launch_experts_rows<0>(mw, mx, g, tile, n_tiles, stream)
+                     : mode == 1 ? launch_experts_rows<1>(mw, mx, g, tile, n_tiles, stream) : launch_experts_rows<2>(mw, mx, g, tile, n_tiles, stream);
+}
+
 // The same product with the fused gated unit of other constants than SwiGLU's.
 extern "C" int ss_gemm_tc5_many_glu(const void* A, const void* B, const void* bias, int bias_f32, void* C, int M, int N,
                                     int K, int64_t lda, int64_t ldb, int64_t ldc, float alpha, float limit, float shift,

@@ -1010,8 +1010,7 @@ moe_gemm_mma_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, cons
         for (int half = 0; half < 2; ++half) {
             const int m = wm * TM + i * 16 + (lane >> 2) + half * 8;
             if (m >= rows) continue;
-            const bool squared = !UP && hidden != nullptr;  // an expert without a gate branch: relu(z)^2 into the hidden rows
-            const int64_t out_row = (UP || squared) ? (int64_t)(row0 + m) : (int64_t)perm[row0 + m];
+            const int64_t out_row = UP ? (int64_t)(row0 + m) : (int64_t)perm[row0 + m];
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
                 const int n = n0 + wn * TN + j * 8 + ((lane & 3) << 1);
@@ -1020,9 +1019,6 @@ moe_gemm_mma_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, cons
                     const float h0 = silu_mul<true>(acc[0][i][j][half * 2], acc[U - 1][i][j][half * 2]);
                     const float h1 = silu_mul<true>(acc[0][i][j][half * 2 + 1], acc[U - 1][i][j][half * 2 + 1]);
                     *reinterpret_cast<__nv_bfloat162*>(hidden + out_row * n_out + n) = __floats2bfloat162_rn(h0, h1);
-                } else if (squared) {
-                    *reinterpret_cast<__nv_bfloat162*>(hidden + out_row * n_out + n) =
-                        __floats2bfloat162_rn(relu_square(acc[0][i][j][half * 2]), relu_square(acc[0][i][j][half * 2 + 1]));
                 } else {
                     *reinterpret_cast<float2*>(y + out_row * n_out + n) = make_float2(acc[0][i][j][half * 2], acc[0][i][j][half * 2 + 1]);
                 }

@@ -176,6 +176,8 @@ _GEMM_SIGNATURES = {
     "ss_gemm_tc5_scaled_glu": [c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                                c_int64, c_int64, c_int64, c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_void_p,
                                c_void_p, c_void_p, c_void_p],
+    "ss_gemm_tc5_experts": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                            c_void_p, c_int, c_void_p, c_void_p],
     "ss_gemm_tc5_grouped": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int64, c_int64, c_int, c_void_p,
                             c_void_p, c_void_p, c_int, c_void_p, c_void_p],
     "ss_gemm_tc5_scaled": [c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
@@ -1932,6 +1934,18 @@ MOE_TILE = 64  # rows of one expert that a block of the grouped products takes
 GROUPED_TCGEN05_ROWS = 1024  # from this many (token, choice) pairs the experts' products run the two-SM tcgen05 kernel
 
 
+def expert_tile(pairs: int, experts: int, tensor_cores: bool, tcgen05: bool, few: bool) -> int:
+    """Rows of a tile of the experts' plan for ``pairs`` (token, choice) pairs: 256 for the two-SM tcgen05 kernel, the width of the
+    one-SM form for ``few`` rows an expert, 32 or 128 for the mma.sync kernel, 64 on CUDA cores.
+
+    The one-SM form: the narrowest tile that holds about two even shares, so that most experts' weights are read once.  Up
+    and down of 8 experts of 4,736 x 3,584 (us at widths 16, 32, 64, 128): 8 pairs 80, 81, 97, 137; 64 136, 137, 136, 139; 256 170,
+    161, 141, 147; 512 225, 181, 168, 153; 1,000 390, 301, 207, 206."""
+    if few:
+        return 16 if pairs <= 8 * experts else (32 if pairs <= 16 * experts else (64 if pairs <= 32 * experts else 128))
+    return MOE_TILE if not tensor_cores else (256 if tcgen05 else (128 if pairs >= 96 * experts else 32))
+
+
 def moe_experts(x: torch.Tensor, ids: torch.Tensor, scores: torch.Tensor | None, gate_up: torch.Tensor, down: torch.Tensor,
                 run: int | None = None) -> tuple[torch.Tensor, torch.Tensor | None]:
     """The chosen experts of every token: ``y[t, k] = W_down[e] (silu(W_gate[e] a) * (W_up[e] a))`` with
@@ -1943,9 +1957,9 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, scores: torch.Tensor | None,
     [N * top, hidden] in sorted order with int32 [N * top] saying where pair (t, k) stands (`group_norm` and
     `moe_combine` take both forms).  The same launches whatever the routing: the plan (pairs sorted by expert and cut
     into tiles), a gather of the scaled activations into sorted order, the up product with the activation, the down
-    product.  bfloat16 with sizes in steps of 8 runs the products on the tensor cores: mma.sync tiles of 32 or 128
-    sorted rows, or, with runs of 64 and many pairs, the grouped form of the two-SM tcgen05 kernel over tiles of 256;
-    everything else runs them on CUDA cores."""
+    product.  bfloat16 with sizes in steps of 8 runs the products on the tensor cores: with runs of 64 the tcgen05 kernels (with
+    many pairs the grouped form of the two-SM one over tiles of 256 sorted rows, else the one whose columns are a tile's
+    rows), otherwise mma.sync tiles of 32 or 128; everything else runs them on CUDA cores."""
     n, hidden = x.shape
     experts, two_ff, _ = gate_up.shape
     ff, top = two_ff // 2, ids.shape[1]
@@ -1961,7 +1975,8 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, scores: torch.Tensor | None,
     a = n * top
     tensor_cores = x.dtype == torch.bfloat16 and hidden % 8 == 0 and ff % 8 == 0
     tcgen05 = tensor_cores and run == 64 and hidden % 16 == 0 and a >= GROUPED_TCGEN05_ROWS
-    tile = MOE_TILE if not tensor_cores else (256 if tcgen05 else (128 if a >= 96 * experts else 32))
+    few = tensor_cores and run == 64 and not tcgen05
+    tile = expert_tile(a, experts, tensor_cores, tcgen05, few)
     max_tiles = (a + tile - 1) // tile + experts
     plan = torch.empty(2 * a + 3 * max_tiles, dtype=torch.int32, device=x.device)
     perm, place, tile_expert = plan[:a], plan[a: 2 * a], plan[2 * a: 2 * a + max_tiles]
@@ -1986,6 +2001,13 @@ def moe_experts(x: torch.Tensor, ids: torch.Tensor, scores: torch.Tensor | None,
                "moe_down")
         return y_sorted, place
     y = torch.empty((n, top, hidden), dtype=torch.float32, device=x.device)
+    if few:
+        err = error_word(x.device).data_ptr()
+        _check(gemm_library().ss_gemm_tc5_experts(gathered.data_ptr(), gate_up.data_ptr(), hidden_act.data_ptr(), a, two_ff, hidden,
+                                                  experts, 1, tile, *lists, max_tiles, err, _stream()), "moe_up")
+        _check(gemm_library().ss_gemm_tc5_experts(hidden_act.data_ptr(), down.data_ptr(), y.data_ptr(), a, hidden, ff, experts, 0,
+                                                  tile, *lists, max_tiles, err, _stream()), "moe_down")
+        return y, None
     if tensor_cores:
         _check(lib.ss_moe_gemm_mma(gathered.data_ptr(), gate_up.data_ptr(), *lists, hidden_act.data_ptr(), None, hidden, ff,
                                    max_tiles, tile, 1, run, int(a <= 4), _stream()), "moe_up")
@@ -2460,7 +2482,7 @@ def moe_experts_single(x: torch.Tensor, ids: torch.Tensor, up: torch.Tensor, dow
     with ``e = ids[t, k]``; no weight is applied here (`moe_mix` weighs the outputs).  ``up`` [experts, ff, hidden],
     ``down`` [experts, hidden, ff].  ``slots`` (default: experts): ids from ``experts`` up to ``slots`` name experts
     without weights; their terms are not computed (and must not be read).  Returns what `moe_experts` returns, by the
-    same three routes (CUDA cores; mma.sync tiles; the grouped two-SM tcgen05 kernel with the activation behind it)."""
+    routes for runs of 64 (CUDA cores; the tcgen05 kernel for few rows; the grouped two-SM one with the activation behind it)."""
     n, hidden = x.shape
     experts, ff, _ = up.shape
     top = ids.shape[1]
@@ -2474,7 +2496,8 @@ def moe_experts_single(x: torch.Tensor, ids: torch.Tensor, up: torch.Tensor, dow
     a = n * top
     tensor_cores = x.dtype == torch.bfloat16 and hidden % 8 == 0 and ff % 8 == 0
     tcgen05 = tensor_cores and hidden % 16 == 0 and ff % 16 == 0 and a >= GROUPED_TCGEN05_ROWS
-    tile = MOE_TILE if not tensor_cores else (256 if tcgen05 else (128 if a >= 96 * experts else 32))
+    few = tensor_cores and not tcgen05
+    tile = expert_tile(a, experts, tensor_cores, tcgen05, few)
     max_tiles = (a + tile - 1) // tile + slots
     plan = torch.empty(2 * a + 3 * max_tiles, dtype=torch.int32, device=x.device)
     perm, place, tile_expert = plan[:a], plan[a: 2 * a], plan[2 * a: 2 * a + max_tiles]
@@ -2500,11 +2523,12 @@ def moe_experts_single(x: torch.Tensor, ids: torch.Tensor, up: torch.Tensor, dow
                "moe_down")
         return y_sorted, place
     y = torch.empty((n, top, hidden), dtype=torch.float32, device=x.device)
-    if tensor_cores:
-        _check(lib.ss_moe_gemm_mma(gathered.data_ptr(), up.data_ptr(), *lists, hidden_act.data_ptr(), None, hidden, ff,
-                                   max_tiles, tile, 0, 0, int(a <= 4), _stream()), "moe_up")
-        _check(lib.ss_moe_gemm_mma(hidden_act.data_ptr(), down.data_ptr(), *lists, None, y.data_ptr(), ff, hidden,
-                                   max_tiles, tile, 0, 0, int(a <= 4), _stream()), "moe_down")
+    if few:
+        err = error_word(x.device).data_ptr()
+        _check(gemm_library().ss_gemm_tc5_experts(gathered.data_ptr(), up.data_ptr(), hidden_act.data_ptr(), a, ff, hidden, experts, 2,
+                                                  tile, *lists, max_tiles, err, _stream()), "moe_up")
+        _check(gemm_library().ss_gemm_tc5_experts(hidden_act.data_ptr(), down.data_ptr(), y.data_ptr(), a, hidden, ff, experts, 0,
+                                                  tile, *lists, max_tiles, err, _stream()), "moe_down")
         return y, None
     _check(lib.ss_moe_gemm(x.data_ptr(), None, up.data_ptr(), *lists, hidden_act.data_ptr(), None, top, hidden, ff,
                            max_tiles, 0, _code(x.dtype), 0, _stream(), 1), "moe_up")

@@ -856,3 +856,38 @@ def test_float32_attention_gives_a_row_the_same_bits_however_its_step_was_cut(mo
     rows = [r for b, t in zip(np.cumsum(lens), tail) for r in range(int(b) - t, int(b))]
     assert torch.equal(run(q[rows], tail, lens), whole[rows])
     ops().check_errors(torch.device(DEV))
+
+
+# widths and depths off the 128-row weight tiles and 64-wide steps of K; tokens that make every tile width (16, 32, 64, 128), all on
+# one expert (several tiles of it) or spread out, some experts without a token
+@pytest.mark.parametrize("hidden, ff, experts, top, gated", [(200, 64, 5, 2, True), (72, 192, 3, 1, True), (264, 320, 8, 3, True),
+                                                             (136, 40, 4, 2, False), (64, 200, 6, 1, False)])
+@pytest.mark.parametrize("tokens", [1, 9, 33, 70, 150])
+def test_experts_with_few_rows_on_tensor_cores(hidden, ff, experts, top, gated, tokens):
+    g = torch.Generator().manual_seed(hidden + tokens)
+    x = torch.randn(tokens, hidden, generator=g).bfloat16()
+    first = (torch.randn(experts, (2 if gated else 1) * ff, hidden, generator=g) * hidden ** -0.5).bfloat16()
+    down = (torch.randn(experts, hidden, ff, generator=g) * ff ** -0.5).bfloat16()
+    scores = torch.rand(tokens, top, generator=g)
+    for spread in (True, False):
+        ids = torch.stack([torch.randperm(experts, generator=g)[:top] if spread else torch.arange(top) for _ in range(tokens)]).int()
+        dev = [t.to(DEV) for t in (x, ids, scores, first, down)]
+        if gated:
+            y, rows = ops().moe_experts(*dev, 64)
+        else:
+            y, rows = ops().moe_experts_single(dev[0], dev[1], dev[3], dev[4])
+        assert rows is None and tuple(y.shape) == (tokens, top, hidden)
+        want = torch.empty(tokens, top, hidden, dtype=torch.float64)
+        for t in range(tokens):
+            for k in range(top):
+                e = int(ids[t, k])
+                a = (x[t].float() * scores[t, k]).bfloat16().double() if gated else x[t].double()
+                z = first[e].double() @ a
+                if gated:
+                    gate, up = (z.view(ff // 64, 2, 64)[:, i].reshape(-1) for i in (0, 1))
+                    z = gate * torch.sigmoid(gate) * up
+                else:
+                    z = torch.relu(z).square()
+                want[t, k] = down[e].double() @ z.bfloat16().double()
+        assert rel_err(y.cpu(), want) < 8e-3  # a hidden value may round to either of two bfloat16 neighbours, 2^-8 apart
+    ops().check_errors(torch.device(DEV))

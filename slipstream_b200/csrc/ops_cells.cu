@@ -474,12 +474,62 @@ cell_output_kernel(const float* __restrict__ num, const float* __restrict__ nq, 
     }
 }
 
+// The same for bfloat16 with heads of up to 256 elements in steps of 4: the head stays in registers, 4 elements a load (1,900
+// rows of 28 heads of 128: 37 us read twice element by element, 21 here).
+__global__ void __launch_bounds__(128)
+cell_output_x4_kernel(const float* __restrict__ num, const float* __restrict__ nq, const float* __restrict__ peaks,
+                      const float* __restrict__ weight, const bf16* __restrict__ gate, int64_t gate_stride, bf16* __restrict__ out,
+                      int n_pairs, int H, int V, float eps) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, pair = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (pair >= n_pairs) return;
+    const int row = pair / H, h = pair - row * H;
+    const float* src = num + (int64_t)pair * V;
+    const bf16* gt = gate + (int64_t)row * gate_stride + (int64_t)h * V;
+    float4 o[2];
+    uint2 z[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int v = (lane + 32 * u) * 4;
+        o[u] = v < V ? *reinterpret_cast<const float4*>(src + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+        z[u] = v < V ? *reinterpret_cast<const uint2*>(gt + v) : make_uint2(0u, 0u);
+    }
+    const float den = fmaxf(fabsf(nq[pair]), expf(-peaks[pair])) + 1e-6f;
+    float ss = 0.f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        if (u * 128 >= V) break;
+        o[u].x /= den; o[u].y /= den; o[u].z /= den; o[u].w /= den;
+        ss = fmaf(o[u].x, o[u].x, ss);
+        ss = fmaf(o[u].y, o[u].y, ss);
+        ss = fmaf(o[u].z, o[u].z, ss);
+        ss = fmaf(o[u].w, o[u].w, ss);
+    }
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)V + eps);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int v = (lane + 32 * u) * 4;
+        if (v >= V) break;
+        const float4 w = *reinterpret_cast<const float4*>(weight + h * V + v);
+        const __nv_bfloat162 a = __floats2bfloat162_rn(o[u].x * inv * w.x * sigmoid_exact(__uint_as_float(z[u].x << 16)),
+                                                       o[u].y * inv * w.y * sigmoid_exact(__uint_as_float(z[u].x & 0xffff0000u)));
+        const __nv_bfloat162 b = __floats2bfloat162_rn(o[u].z * inv * w.z * sigmoid_exact(__uint_as_float(z[u].y << 16)),
+                                                       o[u].w * inv * w.w * sigmoid_exact(__uint_as_float(z[u].y & 0xffff0000u)));
+        *reinterpret_cast<uint2*>(out + (int64_t)pair * V + v) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+}
+
 extern "C" int ss_cell_output(const float* num, const float* nq, const float* peaks, const float* weight, const void* gate,
                               int64_t gate_stride, void* out, int n_rows, int H, int V, float eps, int dtype,
                               cudaStream_t stream) {
     if (n_rows <= 0) return 0;
     const dim3 grid((unsigned)(((int64_t)n_rows * H + 3) / 4));
-    if (dtype == SS_BF16)
+    if (dtype == SS_BF16 && V % 4 == 0 && V <= 256 && gate_stride % 4 == 0 && (int64_t)n_rows * H < (1ll << 31) - 4 &&
+        (((uintptr_t)num | (uintptr_t)weight) & 15) == 0 && (((uintptr_t)gate | (uintptr_t)out) & 7) == 0)
+        ss_launch(cell_output_x4_kernel, grid, dim3(128), 0, stream, num, nq, peaks, weight, (const bf16*)gate, gate_stride, (bf16*)out,
+                  n_rows * H, H, V, eps);
+    else if (dtype == SS_BF16)
         ss_launch(cell_output_kernel<bf16>, grid, dim3(128), 0, stream, num, nq, peaks, weight, (const bf16*)gate, gate_stride,
                   (bf16*)out, n_rows, H, V, eps);
     else

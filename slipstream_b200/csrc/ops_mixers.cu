@@ -113,6 +113,56 @@ group_norm_kernel(const TI* __restrict__ in, int64_t in_stride, int terms, const
     }
 }
 
+// The gated form (MODE 1) for float32 rows and bfloat16 gates, 4 elements a load: a block per row and group, its values read and
+// gated once and kept in registers between the sum of squares and the output (element by element and twice over, 2,045 rows
+// of 7,168 in one group took 85 us; 34 here, bound by the exact exponential and division of the gate).
+template <int NV>
+__global__ void __launch_bounds__(256)
+gated_norm_kernel(const float* __restrict__ in, const bf16* __restrict__ gate, int64_t gate_stride, const float* __restrict__ weight,
+                  bf16* __restrict__ out, int hidden, int groups, float eps) {
+    pdl_launch_dependents();
+    pdl_wait();
+    __shared__ float scratch[33];
+    const int row = blockIdx.x / groups, g = blockIdx.x - row * groups, gs = hidden / groups;
+    const float* src = in + (int64_t)row * hidden + g * gs;
+    const bf16* gt = gate + (int64_t)row * gate_stride + g * gs;
+    float4 x[NV];
+    uint2 z[NV];
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+        const int i = (threadIdx.x + u * blockDim.x) * 4;
+        x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        z[u] = make_uint2(0u, 0u);
+        if (i < gs) {
+            x[u] = *reinterpret_cast<const float4*>(src + i);
+            z[u] = *reinterpret_cast<const uint2*>(gt + i);
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+        x[u].x *= silu_exact(__uint_as_float(z[u].x << 16));
+        x[u].y *= silu_exact(__uint_as_float(z[u].x & 0xffff0000u));
+        x[u].z *= silu_exact(__uint_as_float(z[u].y << 16));
+        x[u].w *= silu_exact(__uint_as_float(z[u].y & 0xffff0000u));
+        ss = fmaf(x[u].x, x[u].x, ss);
+        ss = fmaf(x[u].y, x[u].y, ss);
+        ss = fmaf(x[u].z, x[u].z, ss);
+        ss = fmaf(x[u].w, x[u].w, ss);
+    }
+    const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)gs + eps);
+#pragma unroll
+    for (int u = 0; u < NV; ++u) {
+        const int i = (threadIdx.x + u * blockDim.x) * 4;
+        if (i >= gs) break;
+        const float4 w = *reinterpret_cast<const float4*>(weight + g * gs + i);
+        const __nv_bfloat162 a = __floats2bfloat162_rn(x[u].x * rstd * w.x, x[u].y * rstd * w.y);
+        const __nv_bfloat162 b = __floats2bfloat162_rn(x[u].z * rstd * w.z, x[u].w * rstd * w.w);
+        *reinterpret_cast<uint2*>(out + (int64_t)row * hidden + g * gs + i) =
+            make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+}
+
 // in_type: 0 the compute type, 1 float32.  dtype: the compute type (of out, extra and gate).
 extern "C" int ss_group_norm(const void* in, int in_f32, int64_t in_stride, int terms, const void* extra, const void* gate,
                              int64_t gate_stride, const float* weight, float* residual, void* out, const int32_t* rows,
@@ -121,6 +171,21 @@ extern "C" int ss_group_norm(const void* in, int in_f32, int64_t in_stride, int 
     if (n_out <= 0) return 0;
     if (groups < 1 || hidden % groups || terms < 1) return (int)cudaErrorInvalidValue;
     const int mode = (terms == 1 && !term_rows && !extra) ? (gate ? 1 : 0) : 2;
+    const int gs = hidden / groups;
+    if (mode == 1 && dtype == SS_BF16 && in_f32 && !residual && !rows && out && gs % 4 == 0 && gs <= 8192 && in_stride == hidden &&
+        gate_stride % 4 == 0 && (((uintptr_t)in | (uintptr_t)weight) & 15) == 0 && (((uintptr_t)gate | (uintptr_t)out) & 7) == 0 &&
+        (int64_t)n_out * groups < (1ll << 31)) {
+        const int threads = gs >= 1024 ? 256 : (gs / 4 + 31) / 32 * 32, nv = (gs / 4 + threads - 1) / threads;
+        const dim3 grid(n_out * groups), block(threads);
+#define GG_GO(NV) ss_launch(gated_norm_kernel<NV>, grid, block, 0, stream, (const float*)in, (const bf16*)gate, gate_stride, weight, \
+                            (bf16*)out, hidden, groups, eps)
+        if (nv == 1) GG_GO(1);
+        else if (nv == 2) GG_GO(2);
+        else if (nv <= 4) GG_GO(4);
+        else GG_GO(8);
+#undef GG_GO
+        return SS_LAUNCH_CHECK();
+    }
 #define GN_LAUNCH(TI, T, MODE)                                                                                        \
     ss_launch(group_norm_kernel<TI, T, T, MODE>, dim3(n_out), dim3(256), 0, stream, (const TI*)in, in_stride, terms,  \
               (const T*)extra, (const T*)gate, gate_stride, weight, residual, (T*)out, rows, hidden, groups, eps, term_rows)
@@ -224,40 +289,40 @@ conv_silu_kernel(const T* __restrict__ proj, int64_t stride, int col0, const flo
     }
 }
 
-// The same for bfloat16 with channels in steps of 8 (and the projection's rows and the first channel on 16-byte
-// boundaries) and at most 4 taps: a thread takes 8 neighbouring channels, 16 bytes a load and a store, over
-// CONV_ROWS rows.  The window of a row that is not a request's first in this tile is already in registers.
+// The same for bfloat16 with channels in steps of 4 (and the projection's rows and the first channel on 8-byte boundaries) and
+// at most 4 taps: a thread takes 4 neighbouring channels, 8 bytes a load and a store, over CONV_ROWS rows, the loads of 4 rows
+// in flight.  The window of a row that is not a request's first in this tile is already in registers.  Bound by the exact
+// exponentials and divisions of silu, so by how many warps an SM holds: 2,045 rows of 9,216 channels took 60 us with 8 channels a
+// thread and a row at a time, 81 with 8 channels and 8 rows in flight (164 registers), 56 so.
 __global__ void __launch_bounds__(128)
-conv_silu_bf16x8_kernel(const bf16* __restrict__ proj, int64_t stride, int col0, const float* __restrict__ taps,
-                        const float* __restrict__ bias, float* __restrict__ state, bf16* __restrict__ out,
+conv_silu_bf16x4_kernel(const bf16* __restrict__ proj, int64_t stride, int col0, const float* __restrict__ taps,
+                        const float* __restrict__ bias, const float* __restrict__ state, bf16* __restrict__ out,
                         const int32_t* __restrict__ q_start, const int32_t* __restrict__ seq_lens,
-                        const int32_t* __restrict__ slots, int R, int n_rows, int C, int n_taps, int n_slots,
-                        int fused_update, int* err, int plus_input) {
+                        const int32_t* __restrict__ slots, int R, int n_rows, int C, int n_taps, int n_slots, int* err, int plus_input) {
+    pdl_launch_dependents();
     pdl_wait();
-    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (c >= C) return;
     constexpr int MAXB = 3;  // taps - 1 at most
     const int back = n_taps - 1;
-    float w[8][MAXB + 1], x[8][MAXB], b[8];
+    float w[4][MAXB + 1], x[4][MAXB], b[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < 4; ++e) {
         b[e] = bias ? bias[c + e] : 0.f;
 #pragma unroll
         for (int j = 0; j <= MAXB; ++j) w[e][j] = j < n_taps ? taps[(int64_t)(c + e) * n_taps + j] : 0.f;
 #pragma unroll
         for (int j = 0; j < MAXB; ++j) x[e][j] = 0.f;
     }
-    auto widen = [](const uint4& raw, float (&v)[8]) {
-        const uint32_t q[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { v[2 * e] = __uint_as_float(q[e] << 16); v[2 * e + 1] = __uint_as_float(q[e] & 0xffff0000u); }
+    auto widen = [](const uint2& raw, float (&v)[4]) {
+        v[0] = __uint_as_float(raw.x << 16); v[1] = __uint_as_float(raw.x & 0xffff0000u);
+        v[2] = __uint_as_float(raw.y << 16); v[3] = __uint_as_float(raw.y & 0xffff0000u);
     };
     const int row_first = blockIdx.x * CONV_ROWS, row_end = min(n_rows, row_first + CONV_ROWS);
     int r = -1, r_end = -1;
     bool on = false;
-    float* st = state;
-    for (int row = row_first; row < row_end; ++row) {
-        bool fresh = row == row_first;
+    constexpr int BATCH = 4;  // rows of a request whose loads are in flight before the first is used
+    for (int row = row_first; row < row_end;) {
         if (row >= r_end) {
             r = request_of_row(q_start, R, row);
             if (r < 0) break;
@@ -265,59 +330,60 @@ conv_silu_bf16x8_kernel(const bf16* __restrict__ proj, int64_t stride, int col0,
             const int slot = slots[r];
             on = seq_lens[r] > 0 && slot >= 0 && slot < n_slots;
             if (seq_lens[r] > 0 && !on && threadIdx.x == 0) atomicOr(err, SS_ERR_SLOT_RANGE);
-            st = state + (int64_t)(on ? slot : 0) * back * C + c;
-            fresh = true;
-        }
-        if (!on) continue;
-        if (fresh) {
+            const float* st = state + (int64_t)(on ? slot : 0) * back * C + c;
             const int i = row - q_start[r];
 #pragma unroll
             for (int j = 0; j < MAXB; ++j) {
-                if (j >= back) break;
+                if (j >= back || !on) break;
                 const int src = i - (back - j);
-                float v[8];
+                float v[4];
                 if (src >= 0) {
-                    widen(*reinterpret_cast<const uint4*>(proj + (int64_t)(row - (back - j)) * stride + col0 + c), v);
+                    widen(*reinterpret_cast<const uint2*>(proj + (int64_t)(row - (back - j)) * stride + col0 + c), v);
                 } else {
-                    const float4 lo = *reinterpret_cast<const float4*>(st + (int64_t)(back + src) * C);
-                    const float4 hi = *reinterpret_cast<const float4*>(st + (int64_t)(back + src) * C + 4);
-                    v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w; v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+                    const float4 old = *reinterpret_cast<const float4*>(st + (int64_t)(back + src) * C);
+                    v[0] = old.x; v[1] = old.y; v[2] = old.z; v[3] = old.w;
                 }
 #pragma unroll
-                for (int e = 0; e < 8; ++e) x[e][j] = v[e];
+                for (int e = 0; e < 4; ++e) x[e][j] = v[e];
             }
         }
-        float cur[8];
-        widen(*reinterpret_cast<const uint4*>(proj + (int64_t)row * stride + col0 + c), cur);
-        uint32_t packed[4];
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-            float o2[2];
-#pragma unroll
-            for (int d = 0; d < 2; ++d) {
-                float acc = b[e + d];
-#pragma unroll
-                for (int j = 0; j <= MAXB; ++j)
-                    if (j <= back) acc = fmaf(w[e + d][j], j < back ? x[e + d][j < MAXB ? j : 0] : cur[e + d], acc);
-                o2[d] = plus_input == 1 ? cur[e + d] + acc : (plus_input == 2 ? acc : silu_exact(acc));
-            }
-            const __nv_bfloat162 h2 = __floats2bfloat162_rn(o2[0], o2[1]);
-            packed[e >> 1] = *reinterpret_cast<const uint32_t*>(&h2);
+        const int n = min(min(row_end, r_end) - row, BATCH);
+        if (!on) {
+            row += n;
+            continue;
         }
-        *reinterpret_cast<uint4*>(out + (int64_t)row * C + c) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        uint2 raw[BATCH];
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
+        for (int u = 0; u < BATCH; ++u)
+            if (u < n) raw[u] = *reinterpret_cast<const uint2*>(proj + (int64_t)(row + u) * stride + col0 + c);
 #pragma unroll
-            for (int j = 0; j < MAXB; ++j)
-                if (j < back) x[e][j] = (j + 1 < back) ? x[e][j + 1 < MAXB ? j + 1 : 0] : cur[e];
-        if (fused_update) {
+        for (int u = 0; u < BATCH; ++u) {
+            if (u >= n) break;
+            float cur[4];
+            widen(raw[u], cur);
+            uint32_t packed[2];
 #pragma unroll
-            for (int j = 0; j < MAXB; ++j)
-                if (j < back) {
-                    *reinterpret_cast<float4*>(st + (int64_t)j * C) = make_float4(x[0][j], x[1][j], x[2][j], x[3][j]);
-                    *reinterpret_cast<float4*>(st + (int64_t)j * C + 4) = make_float4(x[4][j], x[5][j], x[6][j], x[7][j]);
+            for (int e = 0; e < 4; e += 2) {
+                float o2[2];
+#pragma unroll
+                for (int d = 0; d < 2; ++d) {
+                    float acc = b[e + d];
+#pragma unroll
+                    for (int j = 0; j <= MAXB; ++j)
+                        if (j <= back) acc = fmaf(w[e + d][j], j < back ? x[e + d][j < MAXB ? j : 0] : cur[e + d], acc);
+                    o2[d] = plus_input == 1 ? cur[e + d] + acc : (plus_input == 2 ? acc : silu_exact(acc));
                 }
+                const __nv_bfloat162 h2 = __floats2bfloat162_rn(o2[0], o2[1]);
+                packed[e >> 1] = *reinterpret_cast<const uint32_t*>(&h2);
+            }
+            *reinterpret_cast<uint2*>(out + (int64_t)(row + u) * C + c) = make_uint2(packed[0], packed[1]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int j = 0; j < MAXB; ++j)
+                    if (j < back) x[e][j] = (j + 1 < back) ? x[e][j + 1 < MAXB ? j + 1 : 0] : cur[e];
         }
+        row += n;
     }
 }
 
@@ -348,11 +414,11 @@ extern "C" int ss_conv_silu(const void* proj, int64_t stride, int col0, const fl
     if (n_rows <= 0 || R <= 0) return 0;
     if (n_taps < 1 || n_taps > CONV_MAX_TAPS) return (int)cudaErrorInvalidValue;
     const dim3 grid((n_rows + CONV_ROWS - 1) / CONV_ROWS, (C + 127) / 128);
-    if (dtype == SS_BF16 && !fused_update && n_taps <= 4 && C % 8 == 0 && col0 % 8 == 0 && stride % 8 == 0 && ((uintptr_t)proj & 15) == 0 &&
-        ((uintptr_t)out & 15) == 0 && ((uintptr_t)state & 15) == 0) {
-        const dim3 grid8((n_rows + CONV_ROWS - 1) / CONV_ROWS, (C / 8 + 127) / 128);
-        ss_launch(conv_silu_bf16x8_kernel, grid8, dim3(128), 0, stream, (const bf16*)proj, stride, col0, taps, bias, state,
-                  (bf16*)out, q_start, seq_lens, slots, R, n_rows, C, n_taps, n_slots, fused_update, err, plus_input);
+    if (dtype == SS_BF16 && !fused_update && n_taps <= 4 && C % 4 == 0 && col0 % 4 == 0 && stride % 4 == 0 && ((uintptr_t)proj & 7) == 0 &&
+        ((uintptr_t)out & 7) == 0 && ((uintptr_t)state & 15) == 0) {
+        const dim3 grid4((n_rows + CONV_ROWS - 1) / CONV_ROWS, (C / 4 + 127) / 128);
+        ss_launch(conv_silu_bf16x4_kernel, grid4, dim3(128), 0, stream, (const bf16*)proj, stride, col0, taps, bias, state,
+                  (bf16*)out, q_start, seq_lens, slots, R, n_rows, C, n_taps, n_slots, err, plus_input);
     } else if (dtype == SS_BF16)
         ss_launch(conv_silu_kernel<bf16>, grid, dim3(128), 0, stream, (const bf16*)proj, stride, col0, taps, bias, state,
                   (bf16*)out, q_start, seq_lens, slots, R, n_rows, C, n_taps, n_slots, fused_update, err, plus_input);
@@ -579,34 +645,78 @@ __device__ __forceinline__ float router_dot(const bf16* __restrict__ w, const fl
     return acc;
 }
 
-template <typename T>
+// The parts of w . x of TT tokens (x in shared memory as bfloat16, rows `stride` apart): a weight is read once for all of them,
+// and a token's sum is the one that router_dot forms.
+template <int TT>
+__device__ __forceinline__ void router_dots(const bf16* __restrict__ w, const bf16* xs, int stride, int hidden, int lane, float (&acc)[TT]) {
+#pragma unroll
+    for (int t = 0; t < TT; ++t) acc[t] = 0.f;
+#pragma unroll 2
+    for (int i = lane * 8; i < hidden; i += 256) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(w + i);
+        const uint32_t q[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+        for (int t = 0; t < TT; ++t) {
+            const uint4 xr = *reinterpret_cast<const uint4*>(xs + t * stride + i);
+            const uint32_t p[4] = {xr.x, xr.y, xr.z, xr.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                acc[t] = fmaf(__uint_as_float(q[e] << 16), __uint_as_float(p[e] << 16), acc[t]);
+                acc[t] = fmaf(__uint_as_float(q[e] & 0xffff0000u), __uint_as_float(p[e] & 0xffff0000u), acc[t]);
+            }
+        }
+    }
+}
+
+// TT: tokens of a block (1, or 4 with many bfloat16 tokens: 2,000 tokens of 3,584 with 8 experts 42 -> 17 us; a block a token
+// read every expert's weights for one token).
+template <typename T, int TT>
 __global__ void __launch_bounds__(ROUTER_THREADS)
 router_kernel(const T* __restrict__ x, const T* __restrict__ w_router, int32_t* __restrict__ ids,
               float* __restrict__ weights, int hidden, int experts, int top, int renormalize, int softmax,
               const float* __restrict__ correction, int groups, int keep, float* __restrict__ extra_out, int extra,
-              const float* __restrict__ bias) {
+              const float* __restrict__ bias, int n_tokens) {
     pdl_wait();
     extern __shared__ __align__(16) float rsm[];
-    float* xs = rsm;                  // [hidden] (rounded up to a multiple of 4)
-    float* z = rsm + ((hidden + 3) & ~3);  // [experts] scores
-    float* c = z + experts;           // [experts] choice scores
-    float* gb = c + experts;          // [groups] the groups' scores
-    const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < hidden; i += blockDim.x) xs[i] = to_float(x[(int64_t)t * hidden + i]);
-    __syncthreads();
-    const int n_warps = blockDim.x >> 5;
-    for (int e = warp; e < experts + extra; e += n_warps) {
-        const T* w = w_router + (int64_t)e * hidden;
-        float acc = router_dot(w, xs, hidden, lane);
-        acc = warp_sum(acc);
-        if (lane == 0) {
-            if (e < experts && bias) acc += bias[e];
-            if (e >= experts) extra_out[(int64_t)t * extra + (e - experts)] = acc;
-            else z[e] = softmax ? acc : 1.0f / (1.0f + expf(-acc));  // the choice below is among scores
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5, t0 = blockIdx.x * TT;
+    const int row = TT > 1 ? hidden : (hidden + 3) & ~3;  // x: TT rows of T, or one of float32 rounded up to a multiple of 4
+    float* z0 = rsm + (TT > 1 ? TT * row / 2 : row);
+    const int per_token = 2 * experts + groups;
+    auto note = [&](int t, int e, float acc) {  // the logit of token t0 + t
+        if (e < experts && bias) acc += bias[e];
+        if (e >= experts) extra_out[(int64_t)(t0 + t) * extra + (e - experts)] = acc;
+        else z0[t * per_token + e] = softmax ? acc : 1.0f / (1.0f + expf(-acc));  // the choice below is among scores
+    };
+    if constexpr (TT > 1) {
+        bf16* xs = reinterpret_cast<bf16*>(rsm);
+        for (int i = tid * 8; i < TT * hidden; i += blockDim.x * 8) {
+            const int t = i / hidden;
+            *reinterpret_cast<uint4*>(xs + i) = t0 + t < n_tokens ? *reinterpret_cast<const uint4*>(x + (int64_t)t0 * hidden + i) : make_uint4(0u, 0u, 0u, 0u);
+        }
+        __syncthreads();
+        for (int e = warp; e < experts + extra; e += n_warps) {
+            float acc[TT];
+            router_dots<TT>(w_router + (int64_t)e * hidden, xs, row, hidden, lane, acc);
+#pragma unroll
+            for (int t = 0; t < TT; ++t) {
+                acc[t] = warp_sum(acc[t]);
+                if (lane == 0 && t0 + t < n_tokens) note(t, e, acc[t]);
+            }
+        }
+    } else {
+        for (int i = tid; i < hidden; i += blockDim.x) rsm[i] = to_float(x[(int64_t)t0 * hidden + i]);
+        __syncthreads();
+        for (int e = warp; e < experts + extra; e += n_warps) {
+            const float acc = warp_sum(router_dot(w_router + (int64_t)e * hidden, rsm, hidden, lane));
+            if (lane == 0) note(0, e, acc);
         }
     }
     __syncthreads();
-    if (warp != 0) return;
+    if (warp >= TT || t0 + warp >= n_tokens) return;
+    const int t = t0 + warp;              // a warp a token
+    float* z = z0 + warp * per_token;     // [experts] scores
+    float* c = z + experts;               // [experts] choice scores
+    float* gb = c + experts;              // [groups] the groups' scores
     if (softmax) {
         float mx = -INFINITY;
         for (int e = lane; e < experts; e += 32) mx = fmaxf(mx, z[e]);
@@ -688,12 +798,18 @@ extern "C" int ss_router(const void* x, const void* w_router, int32_t* ids, floa
         return (int)cudaErrorInvalidValue;
     const int smem = (((hidden + 3) & ~3) + 2 * experts + groups) * 4;
     if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
-    if (dtype == SS_BF16)
-        ss_launch(router_kernel<bf16>, dim3(n_tokens), dim3(ROUTER_THREADS), smem, stream, (const bf16*)x, (const bf16*)w_router, ids,
-                  weights, hidden, experts, top, renormalize, softmax, correction, groups, keep, extra_out, extra, bias);
+    constexpr int TT = 4;
+    const int smem_tt = TT * (hidden * 2 + (2 * experts + groups) * 4);
+    if (dtype == SS_BF16 && hidden % 8 == 0 && (((uintptr_t)x | (uintptr_t)w_router) & 15) == 0 && smem_tt <= 48 * 1024 &&
+        n_tokens >= 2 * TT * ss_sm_count())  // two blocks an SM at least
+        ss_launch(router_kernel<bf16, TT>, dim3((n_tokens + TT - 1) / TT), dim3(ROUTER_THREADS), smem_tt, stream, (const bf16*)x, (const bf16*)w_router,
+                  ids, weights, hidden, experts, top, renormalize, softmax, correction, groups, keep, extra_out, extra, bias, n_tokens);
+    else if (dtype == SS_BF16)
+        ss_launch(router_kernel<bf16, 1>, dim3(n_tokens), dim3(ROUTER_THREADS), smem, stream, (const bf16*)x, (const bf16*)w_router, ids,
+                  weights, hidden, experts, top, renormalize, softmax, correction, groups, keep, extra_out, extra, bias, n_tokens);
     else
-        ss_launch(router_kernel<float>, dim3(n_tokens), dim3(ROUTER_THREADS), smem, stream, (const float*)x, (const float*)w_router,
-                  ids, weights, hidden, experts, top, renormalize, softmax, correction, groups, keep, extra_out, extra, bias);
+        ss_launch(router_kernel<float, 1>, dim3(n_tokens), dim3(ROUTER_THREADS), smem, stream, (const float*)x, (const float*)w_router,
+                  ids, weights, hidden, experts, top, renormalize, softmax, correction, groups, keep, extra_out, extra, bias, n_tokens);
     return SS_LAUNCH_CHECK();
 }
 
@@ -1088,12 +1204,57 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const T* __restr
     out[idx] = from_float<T>(v);
 }
 
+// The same for bfloat16 with a width in steps of 8: 8 elements a thread, the same sums in the same order (2,000 tokens of
+// 3,584 with two choices in sorted rows: 37 us element by element, 9.8 here).
+__global__ void __launch_bounds__(256)
+moe_combine_x8_kernel(const float* __restrict__ y, const bf16* __restrict__ shared, bf16* __restrict__ out, int n_runs, int hidden, int top,
+                      const bf16* __restrict__ sorted, const int32_t* __restrict__ place) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= n_runs) return;
+    const int runs = hidden / 8, t = idx / runs, i = (idx - t * runs) * 8;
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = 0.f;
+    auto add = [&](const uint4& r) {
+        const uint32_t q[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            v[2 * e] += __uint_as_float(q[e] << 16);
+            v[2 * e + 1] += __uint_as_float(q[e] & 0xffff0000u);
+        }
+    };
+#pragma unroll 2
+    for (int k = 0; k < top; ++k) {
+        if (sorted) {
+            add(*reinterpret_cast<const uint4*>(sorted + (int64_t)place[t * top + k] * hidden + i));
+        } else {
+            const float4* p = reinterpret_cast<const float4*>(y + ((int64_t)t * top + k) * hidden + i);
+            const float4 a = p[0], b = p[1];
+            v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+        }
+    }
+    if (shared) add(*reinterpret_cast<const uint4*>(shared + (int64_t)idx * 8));
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+        o[e] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    *reinterpret_cast<uint4*>(out + (int64_t)idx * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 extern "C" int ss_moe_combine(const float* y, const void* shared, void* out, int n_tokens, int hidden, int top, int dtype,
                               const void* sorted, const int32_t* place, cudaStream_t stream) {
     const int64_t n = (int64_t)n_tokens * hidden;
     if (n <= 0) return 0;
     const dim3 grid((unsigned)((n + 255) / 256));
-    if (dtype == SS_BF16)
+    if (dtype == SS_BF16 && hidden % 8 == 0 && n / 8 < (1ll << 31) - 256 &&
+        (((uintptr_t)y | (uintptr_t)shared | (uintptr_t)out | (uintptr_t)sorted) & 15) == 0)
+        ss_launch(moe_combine_x8_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, stream, y, (const bf16*)shared, (bf16*)out,
+                  (int)(n / 8), hidden, top, (const bf16*)sorted, place);
+    else if (dtype == SS_BF16)
         ss_launch(moe_combine_kernel<bf16>, grid, dim3(256), 0, stream, y, (const bf16*)shared, (bf16*)out, n, hidden, top, (const bf16*)sorted, place);
     else
         ss_launch(moe_combine_kernel<float>, grid, dim3(256), 0, stream, y, (const float*)shared, (float*)out, n, hidden, top, (const bf16*)nullptr, (const int32_t*)nullptr);

@@ -891,3 +891,46 @@ def test_experts_with_few_rows_on_tensor_cores(hidden, ff, experts, top, gated, 
                 want[t, k] = down[e].double() @ z.bfloat16().double()
         assert rel_err(y.cpu(), want) < 8e-3  # a hidden value may round to either of two bfloat16 neighbours, 2^-8 apart
     ops().check_errors(torch.device(DEV))
+
+
+# four tokens a block from 1,184 tokens on; a last block of one to four tokens, more experts than warps, extra rows, groups, biases
+@pytest.mark.parametrize("hidden, experts, extra", [(72, 8, 0), (264, 70, 1), (3584, 16, 0)])
+@pytest.mark.parametrize("tokens", [1184, 1187, 1301])
+def test_router_gives_a_token_the_same_bits_beside_many(hidden, experts, extra, tokens):
+    torch.manual_seed(hidden + tokens)
+    x, w = torch.randn(tokens, hidden, device=DEV).bfloat16(), torch.randn(experts + extra, hidden, device=DEV).bfloat16() * hidden ** -0.5
+    for options in (dict(), dict(softmax=True, renormalize=True, bias=torch.randn(experts, device=DEV)),
+                    dict(groups=2, keep=1, correction=torch.randn(experts, device=DEV) * 0.1)):
+        many = ops().router(x, w, 3, extra=extra, **options)
+        few = [ops().router(p, w, 3, extra=extra, **options) for p in x.split(400)]
+        for a, b in zip(many, zip(*few)):
+            assert torch.equal(a, torch.cat(b))
+
+
+# parts of fewer elements than a warp's loads, of exactly a block's, and of the most that stay in registers; widths off the fast path
+@pytest.mark.parametrize("groups, part", [(1, 4), (3, 132), (4, 1024), (2, 1792), (1, 7168), (1, 8192), (1, 8196), (5, 6)])
+def test_gated_norm_of_bfloat16_layers(groups, part):
+    torch.manual_seed(part)
+    n, hidden = 5, groups * part
+    x, weight = torch.randn(n, hidden, device=DEV), torch.randn(hidden, device=DEV)
+    gate = torch.randn(n, hidden + 8, device=DEV).bfloat16()[:, 4: 4 + hidden]
+    got = ops().group_norm(x, weight, groups, 1e-5, torch.bfloat16, gate=gate)
+    y = x.double() * gate.double() * torch.sigmoid(gate.double())
+    y = (y.view(n, groups, part) * torch.rsqrt(y.view(n, groups, part).square().mean(-1, keepdim=True) + 1e-5)).view(n, hidden) * weight.double()
+    assert ((got.double() - y).abs() <= 2.0 ** -8 * y.abs() + 1e-6).all()  # one rounding to bfloat16
+
+
+@pytest.mark.parametrize("tokens, hidden, top", [(3, 8, 1), (70, 200, 3), (33, 1032, 2)])
+def test_experts_sum_eight_elements_at_a_time(tokens, hidden, top):
+    torch.manual_seed(hidden)
+    y, shared = torch.randn(tokens, top, hidden, device=DEV), torch.randn(tokens, hidden, device=DEV).bfloat16()
+    rows = y.view(-1, hidden).bfloat16()
+    place = torch.randperm(tokens * top, device=DEV).int()
+    back = torch.empty_like(rows)
+    back[place.long()] = rows
+    for extra in (None, shared):
+        for got, terms in ((ops().moe_combine(y, extra, torch.bfloat16), y), (ops().moe_combine(back, extra, torch.bfloat16, place, top), rows.view_as(y).float())):
+            total = torch.zeros(tokens, hidden, device=DEV)
+            for k in range(top):
+                total = total + terms[:, k]
+            assert torch.equal(got, (total if extra is None else total + extra.float()).bfloat16())

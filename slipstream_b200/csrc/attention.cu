@@ -120,8 +120,8 @@ extern "C" int ss_attn_decode_mma(const void* q, int64_t q_stride, void* out, in
     return SS_LAUNCH_CHECK();
 }
 
-// ---------------------------------------------------------------- tcgen05 prefill attention (head size 64 or 128)
-#if HEAD_DIM == 64 || HEAD_DIM == 128
+// ---------------------------------------------------------------- tcgen05 prefill attention (head sizes 32 to 128)
+#if HEAD_DIM >= 32 && HEAD_DIM <= 128
 #include "attention_tc5.cuh"
 
 extern "C" int ss_attn_prefill_tc5_supported() { return 1; }
@@ -168,6 +168,12 @@ extern "C" int ss_attn_prefill_tc5(const void* q, int64_t q_stride, int n_tokens
     return SS_LAUNCH_CHECK();
 }
 
+#else
+extern "C" int ss_attn_prefill_tc5_supported() { return 0; }
+#endif
+
+// ---------------------------------------------------------------- decode attention with TMA-fed tiles (head size 64 or 128)
+#if HEAD_DIM == 64 || HEAD_DIM == 128
 #include "attention_decode_tma.cuh"
 
 template <int NS, int FORM>
@@ -293,8 +299,6 @@ extern "C" int ss_attn_decode_across(const void* q, int64_t q_stride, void* out,
     }
     return SS_LAUNCH_CHECK();
 }
-#else
-extern "C" int ss_attn_prefill_tc5_supported() { return 0; }
 #endif
 
 // ---------------------------------------------------------------- the entry point that allocates nothing

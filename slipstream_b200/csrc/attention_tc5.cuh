@@ -1,5 +1,6 @@
 // Paged causal grouped-query attention for prompt portions on the 5th-generation tensor cores
-// (tcgen05.mma with accumulators in tensor memory, operands staged by TMA), bfloat16, head size 64 or 128.
+// (tcgen05.mma with accumulators in tensor memory, operands staged by TMA), bfloat16, head sizes from
+// 32 to 128 in steps of 16 (held as 64 or 128 columns, see padded_head).
 //
 // A block takes up to 128 "rows" of one (request, kv head): TOK = 128 / G consecutive query tokens times the
 // G heads of the kv group, token-major, so the group shares every key/value tile.  Roles:
@@ -23,8 +24,8 @@
 // (:64-88).  Besides the causal rule a row sees what `span` says (a sliding window, a chunk, or everything: the
 // tiles begin at the first one the query tile's first row can see, and each row masks the keys in front of its own
 // lowest one; a window may keep the first keys in sight, whose tiles then stand in front of the window's), and a soft
-// cap may squash the scaled scores.  Other head sizes and page sizes that do not divide 64
-// run the mma.sync kernel of attention_mma.cuh.  Every mbarrier wait is bounded (see gemm_tc5.cu).
+// cap may squash the scaled scores.  Other head sizes and page sizes that do not divide 64 run the mma.sync kernel
+// of attention_mma.cuh.  Every mbarrier wait is bounded (see gemm_tc5.cu).
 #pragma once
 
 #include <cuda.h>
@@ -159,17 +160,32 @@ struct Args {
     DiffPair diff;  // one layer of blocks only (gridDim.z == 1), dim a multiple of 8
 };
 
-template <int D>
+// The columns a head takes in shared and tensor memory: one or two boxes of 64 elements (128 bytes, the swizzle's row).  The
+// tensor maps end at the head's real size, so TMA fills the rest of the last box with zeros: they add nothing to a score and
+// give columns of O that are never written out.
+constexpr int padded_head(int hd) { return hd <= 64 ? 64 : 128; }
+
+template <int HD>
 constexpr int smem_bytes() {
+    constexpr int D = padded_head(HD);
     // Q (128 rows) + three stages of K and two of V (64 keys each) + barriers: 112.5 KB for head size 128, so
     // that two blocks share an SM (one's softmax overlaps the other's products).  P lives in tensor memory.
     return 128 * D * 2 + (FA_KS + 2) * FA_BN * D * 2 + 512;
 }
 
-template <int D>
+template <int HD>
 __global__ void __launch_bounds__(FA_THREADS, 2)
 attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv, const Args a) {
-    constexpr int HALVES = D / 64;
+    static_assert(HD % 16 == 0 && HD <= 128, "whole steps of 16 elements in S = Q K^T");
+    constexpr int D = padded_head(HD), HALVES = D / 64;
+    // The sizes between the boxes come from the mma.sync kernel, whose reference is always a row's largest score so far: its
+    // probability is an exact 1, where a lazy reference leaves a 2^x that rounds to bfloat16.  To be no less exact than that
+    // kernel they keep its reference (LAG 0) and divide by the sum of the probabilities as the PV product takes them, which
+    // costs two operations a pair of keys.  Error against 64 bits of one request of 700 tokens with peaked scores (queries
+    // of 3 sigma), float32 results, 96 elements: mma.sync 5.9e-4; 1.27e-3 with the lazy reference, 8.6e-4 with the rounded
+    // sum alone, 5.7e-4 as it is; two requests of 1,531 tokens take 28.4, 29.6 and 34.1 us (mma.sync 73).
+    constexpr bool BETWEEN = HD != 64 && HD != 128;
+    constexpr float LAG = BETWEEN ? 0.f : 8.f;
     constexpr int Q_BYTES = 128 * D * 2, KV_BYTES = FA_BN * D * 2;
     constexpr int HALF_Q = 128 * 128, HALF_KV = FA_BN * 128;  // bytes of one 64-column half
     constexpr int TMEM_COLS = 256;  // S0 [0,64), S1 [64,128), O [128, 128 + D)
@@ -329,7 +345,7 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             for (int h = 0; h < HALVES; ++h) kd[h] = kst == 0 ? k_desc[0][h] : (kst == 1 ? k_desc[1][h] : k_desc[2][h]);
             if (elect_one()) {
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk)
+                for (int kk = 0; kk < HD / 16; ++kk)
                     umma(tmem + st * FA_BN, q_desc[kk / 4] + (uint64_t)((kk % 4) * 2), kd[kk / 4] + (uint64_t)((kk % 4) * 2), idesc_s, kk != 0);
                 umma_commit(&s_ready[st]);
                 umma_commit(&k_empty[kst]);
@@ -423,11 +439,11 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             for (int c = 0; c < 64; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(sr[c >> 5][c & 31]));
             float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
             if (!valid) mx = 0.f;  // rows without a query: keep the numbers finite
-            if (__any_sync(0xffffffffu, mx > m_ref + 8.0f)) {
+            if (__any_sync(0xffffffffu, mx > m_ref + LAG)) {
                 // some row's maximum moved far: bring O and the sum to the new reference (rows whose maximum
                 // did not move keep theirs: alpha = 1).  O is ours while the PV product of the previous tile
                 // is complete and the next one has not been released.
-                const float m_new = mx > m_ref + 8.0f ? mx : m_ref;
+                const float m_new = mx > m_ref + LAG ? mx : m_ref;
                 if (j > 0) {
                     ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, gave_up));
                     if (!ok) break;
@@ -437,7 +453,7 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                     const float alpha = m_new == -INFINITY ? 1.f : ex2(m_ref - m_new);
                     l *= alpha;
 #pragma unroll 1
-                    for (int c = 0; c < D; c += 32) {
+                    for (int c = 0; c < HD; c += 32) {
                         uint32_t o[32];
                         tmem_ld32(tmem + lane_base + 128 + c, o);
                         tmem_ld_wait();
@@ -461,9 +477,10 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             for (int c = 0; c < 64; c += 2) {
                 const float p0 = ex2(fmaf(__uint_as_float(sr[c >> 5][c & 31]), scale_log2, -m_use));
                 const float p1 = ex2(fmaf(__uint_as_float(sr[(c + 1) >> 5][(c + 1) & 31]), scale_log2, -m_use));
-                l4[(c >> 1) & 3] += p0 + p1;
                 __nv_bfloat162 v = __floats2bfloat162_rn(p0, p1);
                 packed[c >> 1] = *reinterpret_cast<uint32_t*>(&v);
+                if constexpr (BETWEEN) l4[(c >> 1) & 3] += __uint_as_float(packed[c >> 1] << 16) + __uint_as_float(packed[c >> 1] & 0xffff0000u);
+                else l4[(c >> 1) & 3] += p0 + p1;
             }
             l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
             tmem_st32(tmem + lane_base + st * FA_BN, packed);
@@ -489,7 +506,7 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                     // again, and each of the two lanes writes half of the columns.  Columns beyond the values are zero.
                     float ss = 0.f;
 #pragma unroll 1
-                    for (int c = 0; c < D; c += 32) {
+                    for (int c = 0; c < HD; c += 32) {
                         uint32_t o[32];
                         tmem_ld32(tmem + lane_base + 128 + c, o);
                         tmem_ld_wait();
@@ -502,9 +519,9 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                     }
                     diff_scale = a.diff.mult / sqrtf(ss / (float)a.diff.dim + a.diff.eps);
                 }
-                bf16* dst = a.out + (int64_t)(qs + tok0 + tok) * a.out_stride + (int64_t)(u * G + g) * D;
+                bf16* dst = a.out + (int64_t)(qs + tok0 + tok) * a.out_stride + (int64_t)(u * G + g) * HD;
 #pragma unroll 1
-                for (int c = 0; c < D; c += 32) {
+                for (int c = 0; c < HD; c += 32) {
                     uint32_t o[32];
                     tmem_ld32(tmem + lane_base + 128 + c, o);
                     tmem_ld_wait();
@@ -529,11 +546,12 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                         }
                     } else if (a.out_f32) {
                         if (valid) {
-                            float* fdst = reinterpret_cast<float*>(a.out) + (int64_t)(qs + tok0 + tok) * a.out_stride + (int64_t)(u * G + g) * D + c;
+                            float* fdst = reinterpret_cast<float*>(a.out) + (int64_t)(qs + tok0 + tok) * a.out_stride + (int64_t)(u * G + g) * HD + c;
 #pragma unroll
                             for (int e = 0; e < 32; e += 4)
-                                *reinterpret_cast<float4*>(fdst + e) = make_float4(__uint_as_float(o[e]) * inv, __uint_as_float(o[e + 1]) * inv,
-                                                                                  __uint_as_float(o[e + 2]) * inv, __uint_as_float(o[e + 3]) * inv);
+                                if (HD % 32 == 0 || c + e < HD)
+                                    *reinterpret_cast<float4*>(fdst + e) = make_float4(__uint_as_float(o[e]) * inv, __uint_as_float(o[e + 1]) * inv,
+                                                                                      __uint_as_float(o[e + 2]) * inv, __uint_as_float(o[e + 3]) * inv);
                         }
                     } else if (valid) {
 #pragma unroll
@@ -544,7 +562,8 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                                 __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(o[e + 2 * k]) * inv, __uint_as_float(o[e + 2 * k + 1]) * inv);
                                 packed[k] = *reinterpret_cast<uint32_t*>(&v);
                             }
-                            *reinterpret_cast<uint4*>(dst + c + e) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                            if (HD % 32 == 0 || c + e < HD)
+                                *reinterpret_cast<uint4*>(dst + c + e) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
                         }
                     }
                 }
@@ -558,7 +577,7 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
             float* Lsm = Msm + 128;
             const bool have = ok && n_tiles > 0;
 #pragma unroll 1
-            for (int c = 0; c < D; c += 32) {
+            for (int c = 0; c < HD; c += 32) {
                 uint32_t o[32];
                 if (n_tiles > 0) {
                     tmem_ld32(tmem + lane_base + 128 + c, o);
@@ -574,7 +593,8 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     if (splits > 1) {
         cluster_sync_all();  // every block's O, maximum and sum are in its shared memory
         if (warp >= 2 && warp < 6) {
-            // block `part` combines columns part * D / splits .. of all rows: thread = row, as in the softmax
+            // block `part` combines every splits-th group of 8 columns (8 bfloat16 per store) of all rows: thread = row,
+            // as in the softmax
             const int row = (warp & 3) * 32 + lane;
             const float* Osm = reinterpret_cast<const float*>(base);
             const float* Msm = Osm + D * 128;
@@ -591,15 +611,14 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 w[sp] = (sp < splits && ms[sp] != -INFINITY) ? ex2(ms[sp] - m_all) : 0.f;
                 if (sp < splits) l_all += w[sp] * ld_cluster_f32(Lsm + row, (uint32_t)sp);
             }
-            const int cols = D / splits, c0 = part * cols;  // D / splits is a multiple of 8: 8 bfloat16 per store
             const bool valid = row < rows_valid;
             const int tok = valid ? row / G : 0, g = valid ? row - tok * G : 0;
             if (a.sinks && valid)  // once for the row, whichever block of the cluster writes these columns
                 l_all = m_all == -INFINITY ? 1.f : l_all + ex2(a.sinks[kvh * G + g] * 1.4426950408889634f - m_all);
             const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-            bf16* dst = a.out + (int64_t)(qs + tok0 + tok) * a.out_stride + (int64_t)(u * G + g) * D + c0;
+            bf16* dst = a.out + (int64_t)(qs + tok0 + tok) * a.out_stride + (int64_t)(u * G + g) * HD;
 #pragma unroll 1
-            for (int c = 0; c < cols; c += 8) {
+            for (int c = part * 8; c < HD; c += 8 * splits) {
                 float acc[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) acc[e] = 0.f;
@@ -607,11 +626,11 @@ attn_prefill_tc5(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                 for (int sp = 0; sp < 8; ++sp) {
                     if (sp < splits) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) acc[e] += w[sp] * ld_cluster_f32(Osm + (c0 + c + e) * 128 + row, (uint32_t)sp);
+                        for (int e = 0; e < 8; ++e) acc[e] += w[sp] * ld_cluster_f32(Osm + (c + e) * 128 + row, (uint32_t)sp);
                     }
                 }
                 if (valid && a.out_f32) {
-                    float* fdst = reinterpret_cast<float*>(a.out) + (int64_t)(qs + tok0 + tok) * a.out_stride + (int64_t)(u * G + g) * D + c0 + c;
+                    float* fdst = reinterpret_cast<float*>(a.out) + (int64_t)(qs + tok0 + tok) * a.out_stride + (int64_t)(u * G + g) * HD + c;
                     *reinterpret_cast<float4*>(fdst) = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, acc[3] * inv);
                     *reinterpret_cast<float4*>(fdst + 4) = make_float4(acc[4] * inv, acc[5] * inv, acc[6] * inv, acc[7] * inv);
                 } else if (valid) {

@@ -776,17 +776,18 @@ def paged_attention_prefill(q: torch.Tensor, q_stride: int, out: torch.Tensor, k
 
 
 def tcgen05_attention_fits(head_dim: int, n_q: int, n_kv: int, page_size: int, window: int) -> bool:
-    """Whether the TMA-fed decode attention kernel takes this layer (``window`` 0), or the tcgen05 prefill kernel
-    without a sliding window: head size 64 or 128, pages of 8, 16, 32 or 64 tokens, at most 128 query heads per kv
-    head.  (The prefill kernel also takes windows, chunked masks and soft caps: `tcgen05_prefill_fits`.)"""
+    """Whether the TMA-fed decode attention kernel takes this layer (``window`` 0): head size 64 or 128, pages of 8, 16,
+    32 or 64 tokens, at most 128 query heads per kv head.  (The tcgen05 prefill kernel takes more: `tcgen05_prefill_fits`.)"""
     return (head_dim in (64, 128) and not window and page_size in (8, 16, 32, 64) and n_q // n_kv <= 128)
 
 
 def tcgen05_prefill_fits(head_dim: int, n_q: int, n_kv: int, page_size: int) -> bool:
     """Whether the tcgen05 prefill attention kernel takes this layer, whatever its mask (a sliding window, a chunked
     mask or none: the kernel starts at the first key tile a query tile can see and masks by row) and with or without
-    a soft cap on the scores."""
-    return tcgen05_attention_fits(head_dim, n_q, n_kv, page_size, 0)
+    a soft cap on the scores: head sizes from 32 to 128 in steps of 16 (a size that does not fill its boxes of 64 elements
+    is held as if it did, its last columns zero), pages of 8, 16, 32 or 64 tokens, at most 128 query heads per kv head.
+    (At 16 the mma.sync kernel is the faster one up to 700 keys.)"""
+    return (head_dim % 16 == 0 and 32 <= head_dim <= 128 and page_size in (8, 16, 32, 64) and n_q // n_kv <= 128)
 
 
 def paged_attention_prefill_tcgen05(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torch.Tensor,
@@ -809,7 +810,7 @@ def paged_attention_prefill_tcgen05(q: torch.Tensor, q_stride: int, out: torch.T
     _need(kv, torch.bfloat16, "kv pages")
     if q.dtype != torch.bfloat16:
         raise KernelError("the tensor-core attention kernels take bfloat16")
-    if not tcgen05_attention_fits(head_dim, n_q, n_kv, kv.shape[3], 0):
+    if not tcgen05_prefill_fits(head_dim, n_q, n_kv, kv.shape[3]):
         raise KernelError("the tcgen05 attention kernel does not take this head size or page size")
     for name, t in (("block_tables", block_tables), ("tile_req", tile_req), ("tile_tok0", tile_tok0),
                     ("q_start", q_start), ("seq_lens", seq_lens)):
@@ -999,7 +1000,7 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, bloc
     rotated queries; ``ctx`` gives the rows of each request (``q_start``), the cached lengths after
     this step (``seq_lens``) and the lists of query tiles.  float32 runs the CUDA-core kernels (`paged_attention_float32`);
     bfloat16 the tensor-core kernels: the split decode kernel when every request brings one token, else
-    the tcgen05 kernel (head size 64 or 128; windows, chunked masks and soft caps included) or the mma.sync tiled kernel.
+    the tcgen05 kernel (head sizes up to 128; windows, chunked masks and soft caps included) or the mma.sync tiled kernel.
 
     ``rope`` (only where ``fuses_rope``): queries and keys of ``qkv`` are not rotated yet and the newest keys
     and values not yet in their pages; the decode kernel does both.
@@ -1054,7 +1055,7 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, bloc
             diff_combine(heads, diff, n_q // 2, out)
         return
     fused = diff is None or diff_in_attention(diff, n_q, n_kv)
-    if tcgen05_prefill_fits(head_dim, n_q, n_kv, kv.shape[3]):
+    if _prefill_on_tcgen05(ctx, head_dim, n_q, n_kv, kv.shape[3], out, gate):
         tile_req, tile_tok0 = ctx.query_tiles_longest_first(128 // group)
         key = ("prefill_key_parts", 128 // group, n_blocks, (window or chunk) + keep)
         parts = ctx.extras.get(key)
@@ -1078,6 +1079,29 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, bloc
                             diff if fused else None, across)
     if not fused:
         diff_combine(heads, diff, n_q // 2, out)
+
+
+def few_prefill_keys(head_dim: int, longest: int) -> bool:
+    """Whether a prompt step whose longest request holds ``longest`` keys stays on the mma.sync kernel although the tcgen05
+    one takes it: head sizes other than 64 and 128 with few keys.  A query tile is 64 rows in the one and 128 in the other, so
+    half as many blocks there (one request of 63 tokens, 96 elements a head: 7.0 us, and 7.8 on tcgen05; of 128, 48 elements:
+    7.0 and 6.8).  From there on tcgen05 gains with the keys: two requests of 1,531 tokens, 48 elements: 47.7 and 25.0 us, 96
+    elements: 73 and 34; 500 tokens behind 1,500 cached ones 62 and 17, 102 and 20."""
+    return head_dim not in (64, 128) and longest <= (128 if head_dim < 64 else 64)
+
+
+def _prefill_on_tcgen05(ctx, head_dim: int, n_q: int, n_kv: int, page_size: int, out: torch.Tensor, gate: torch.Tensor | None) -> bool:
+    """The kernel of a bfloat16 step with prompt portions: tcgen05 where it takes the layer and the step has the keys for it
+    (a captured step, whose lengths are not known, was told: ``few_keys``).  A gated layer of a head size other than 64 and 128
+    stays on the mma.sync kernel, which gates before it rounds."""
+    if not tcgen05_prefill_fits(head_dim, n_q, n_kv, page_size):
+        return False
+    if head_dim in (64, 128):
+        return True
+    few = ctx.extras.get(("few_keys", head_dim))
+    if few is None:
+        few = few_prefill_keys(head_dim, ctx.max_seq_len)
+    return not few and gate is None and out.data_ptr() % 16 == 0
 
 
 def _heads_f32(out: torch.Tensor, n_q: int, head_dim: int) -> torch.Tensor:
@@ -2748,7 +2772,7 @@ def set_programmatic_launch(enabled: bool) -> None:
 
 
 __all__ = ["KernelError", "KernelBuildError", "embedding", "add_rmsnorm", "hc_norm", "linear_hc_rmsnorm", "rope_norm_cache", "glu_limited", "gate_up_glu", "sigmoid_gate", "key_span", "rope_and_cache", "swiglu",
-           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "paged_attention_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
+           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "few_prefill_keys", "paged_attention_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
            "attention_library", "group_norm", "round_stream", "conv_silu", "ssm_scan", "router", "moe_experts", "moe_combine",
            "norm_rope_cache", "turn_heads", "soft_cap", "embed_sum", "matrix_cell", "cell_output", "gated_recurrence", "xielu",
            "DiffPair", "diff_in_attention", "diff_combine", "heads_to_pages", "branch_norm", "PairedOutput", "WeighedTerms",

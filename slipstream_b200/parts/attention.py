@@ -263,19 +263,22 @@ class PagedAttention(Mixer):
     def capture_variant(self, longest: int, plan: object = None) -> object:
         """Decode steps: long contexts of few requests want the keys cut into more slices than fit one thread-block
         cluster (``ops.decode_slices``).  Steps with prompt portions: into how many parts the tcgen05 prefill kernel
-        cuts the keys of a query tile (``ops.prefill_key_parts``).  Each form is captured as a graph of its own."""
+        cuts the keys of a query tile (``ops.prefill_key_parts``), 0 where the mma.sync kernel runs because there are few
+        keys.  Each form is captured as a graph of its own."""
         bf16 = self.runtime.dtype == torch.bfloat16
         if plan is None or plan.is_decode_only:
             return bool(bf16 and ops.is_long_context(longest))
         group = self.num_heads // self.num_kv_heads
         if not bf16 or not ops.tcgen05_prefill_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_size or 16):
             return None
+        if ops.few_prefill_keys(self.head_dim, longest):
+            return 0
         return int(ops.prefill_key_parts(plan.q_lens, plan.seq_lens, 128 // group, self.kernel_blocks,
                                          ops.sm_count(self.runtime.device), self.sees))
 
     def capture_group(self) -> object:
-        # layers that see equally far answer `capture_variant` alike
-        return ("paged_attention", self.sees)
+        # layers that see equally far with heads of one size answer `capture_variant` alike
+        return ("paged_attention", self.sees, self.head_dim)
 
     def prepare_capture(self, ctx, variant: object, max_model_len: int) -> None:
         if not ctx.is_decode_only:
@@ -283,6 +286,7 @@ class PagedAttention(Mixer):
             # lengths of the step, which a replay does not know on the host)
             ctx.extras[("prefill_key_parts", 128 // (self.num_heads // self.num_kv_heads), self.kernel_blocks,
                         self.sees)] = int(variant or 1)
+            ctx.extras[("few_keys", self.head_dim)] = variant == 0
             return
         # the number of slices must not follow the lengths of the step that happens to be captured
         ctx.extras["static_max_seq_len"] = max_model_len

@@ -121,13 +121,16 @@ class LatentAttention(Mixer):
         return n * self.o_weight.element_size()
 
     def capture_variant(self, longest: int, plan: object = None) -> object:
-        return None  # captured steps run one form of the decode kernel, however long the contexts
+        # one form of the decode kernel, however long the contexts; steps with prompt portions: whether few keys keep the
+        # mma.sync kernel
+        return None if plan is None or plan.is_decode_only else bool(ops.few_prefill_keys(self.row, longest))
 
     def capture_group(self) -> object:
-        return ("latent_attention",)
+        return ("latent_attention", self.row)
 
     def prepare_capture(self, ctx, variant: object, max_model_len: int) -> None:
         if not ctx.is_decode_only:
+            ctx.extras[("few_keys", self.row)] = bool(variant)
             return
         ctx.extras["static_max_seq_len"] = max_model_len  # the number of slices must not follow the captured step
         ctx.extras.setdefault("decode_wide", False)

@@ -75,3 +75,31 @@ def test_where_a_projection_adds_itself_to_the_stream():
     finally:
         F.set_norm_fusion(True)
     assert F.adds_to_stream(8, 3584, 3584, SMS)
+
+
+def test_head_sizes_between_the_boxes_leave_the_mma_sync_kernel_only_for_enough_keys():
+    from types import SimpleNamespace
+    import torch
+
+    out = torch.empty(4, 64, dtype=torch.bfloat16)
+    runs = lambda longest, d, out=out, gate=None, **told: F._prefill_on_tcgen05(
+        SimpleNamespace(max_seq_len=longest, extras={("few_keys", k): v for k, v in ((d, told.get("few")),) if v is not None}), d, 8, 2, 16, out, gate)
+    for d, few in ((32, 128), (48, 128), (80, 64), (96, 64), (112, 64)):
+        assert F.tcgen05_prefill_fits(d, 8, 2, 16) and not F.tcgen05_attention_fits(d, 8, 2, 16, 0)
+        assert not runs(few, d) and runs(few + 1, d)
+        assert runs(0, d, few=False) and not runs(5000, d, few=True)                     # a captured step is told
+        assert not runs(5000, d, gate=out)                                               # gated before rounding there
+        assert not runs(5000, d, out=out.view(-1)[1:65].view(1, 64))                     # 16-byte stores
+    assert runs(1, 64, gate=out) and runs(1, 128)
+    for d, n_q, n_kv, page in ((16, 8, 2, 16), (160, 8, 2, 16), (40, 8, 2, 16), (96, 8, 2, 12), (96, 8, 2, 128), (96, 129, 1, 16)):
+        assert not F.tcgen05_prefill_fits(d, n_q, n_kv, page)
+
+
+def test_expert_tiles_and_float32_key_parts():
+    for experts in (1, 8, 100):
+        widths = [F.expert_tile(p, experts, True, False, True) for p in range(1, 40 * experts)]
+        assert widths == sorted(widths) and set(widths) == {16, 32, 64, 128}
+    assert F.expert_tile(5000, 8, True, True, False) == 256 and F.expert_tile(8, 8, False, False, False) == F.MOE_TILE
+    assert F.float32_key_parts(8, 20, 4, 12, 128, sms=SMS) == 20 and F.float32_key_parts(100, 20, 4, 12, 128, sms=SMS) == 2
+    assert F.float32_key_parts(400, 20, 4, 12, 128, sms=SMS) == 1
+    assert F.float32_key_parts(8, 20, 5000, 28, 128, sms=SMS) == 1  # the slices' scratch would pass its bound

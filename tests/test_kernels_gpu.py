@@ -281,6 +281,43 @@ def test_paged_attention_tiled_kernels(dtype, case):
     ops().check_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("d", [32, 48, 80, 96, 112])
+@pytest.mark.parametrize("n_q, n_kv, page, window", [(4, 2, 16, 0), (14, 2, 8, 37), (40, 2, 64, 150), (3, 3, 32, 64)])
+def test_tcgen05_prefill_of_head_sizes_between_its_boxes(d, n_q, n_kv, page, window):
+    """Head sizes that do not fill one or two boxes of 64 elements: scores over the real columns only, every column
+    written and none beside, alone and with the keys shared by 2, 4 and 8 blocks (at 32 twice
+    as many as there are groups of 8 columns).  Rows behind a request's end hold infinities.  Tolerance: bfloat16 probabilities and outputs, as above."""
+    from slipstream_b200.engine.context import query_tiles_host
+    lens, q_lens = [700, 64, 65, 1, 130], [3, 64, 65, 1, 129]
+    q, kv, table, q_start, seq_lens = make_attention_case(torch.bfloat16, lens, q_lens, n_q, n_kv, d, page, seed=d)
+    for r, n in enumerate(lens):
+        if n % page:
+            kv[int(table[r, (n - 1) // page]), :, :, n % page:] = float("inf")
+    sinks = torch.linspace(-1, 2, n_q, device=DEV)
+    scale = d ** -0.5
+    ref = attention_reference(q, kv, table, q_start, seq_lens, n_kv, page, scale, window, sinks)
+    ql = np.asarray(q_lens, dtype=np.int32)
+    req, t0 = (torch.from_numpy(a).to(DEV) for a in query_tiles_host(ql, 128 // (n_q // n_kv)))
+    args = (q.view(q.shape[0], -1), n_q * d)
+    for kind in (torch.bfloat16, torch.float32):
+        for parts in (1, 2, 4, 8):
+            wide = torch.full((q.shape[0] + 1, n_q * d), float("nan"), device=DEV, dtype=kind)
+            out = wide[:-1]
+            ops().paged_attention_prefill_tcgen05(*args, out, kv, table, req, t0, q_start, seq_lens, n_q, n_kv, d, scale, parts,
+                                                  window=window, sinks=sinks)
+            assert rel_err(out.view_as(ref).cpu(), ref) < 1e-2, (kind, parts)
+            assert wide[-1].isnan().all()
+    if (n_q // n_kv) % 2 == 0:  # differential heads: the mma.sync kernel forms the same combination
+        from slipstream_b200.ops.functions import DiffPair
+        diff = DiffPair(0.3, 0.7, 1e-5, d - 8)
+        a, b = (torch.full((q.shape[0], n_q // 2 * diff.dim), float("nan"), device=DEV, dtype=torch.bfloat16) for _ in range(2))
+        ops().paged_attention_prefill_tcgen05(*args, a, kv, table, req, t0, q_start, seq_lens, n_q, n_kv, d, scale, 1, window=window, diff=diff)
+        req, r0 = (torch.from_numpy(x).to(DEV) for x in query_tiles_host(ql * (n_q // n_kv), 64))
+        ops().paged_attention_prefill(*args, b, kv, table, req, r0, q_start, seq_lens, n_q, n_kv, d, scale, window, diff=diff)
+        assert rel_err(a, b) < 3e-2
+    ops().check_errors(torch.device(DEV))
+
+
 @pytest.mark.parametrize("slices", [1, 2, 5, 16, 32, 64])  # one cluster; 2, 4, 8 clusters of 8 (TMA-fed kernel) or single blocks
 @pytest.mark.parametrize("n_q, n_kv, d, page, window", [(28, 4, 128, 16, 0), (6, 6, 16, 4, 0), (40, 2, 64, 7, 0),
                                                          (8, 2, 32, 16, 100), (3, 1, 256, 16, 0), (40, 2, 64, 8, 0),

@@ -119,7 +119,8 @@ extern "C" int ss_embed_sum(const int32_t* tokens, const int32_t* positions, con
 //   S_t = keep_t S_{t-1} + take_t k_t v_t^T   [D x V],   n_t = keep_t n_{t-1} + take_t k_t.
 // The kernel treats n as one more column of S (the column of a value that is always 1) and writes, per token,
 // the numerators S_t^T q_t [V], the scalar n_t . q_t and m_t; the norm kernel behind it divides.
-// State: memory [slot][H][V + 1][D] float32 (column-major, column V is n), peak [slot][H] (m, starts at 0).
+// State: memory [slot][H][V + 1][D] float32 (column-major, column V is n), peak [slot][H] (m, starts at 0).  All column
+// blocks of a head start from the peak, in no order, so the kernel only reads it; cell_peaks_kernel, behind it, writes it.
 //
 // A block: one request, one head, MC_WARPS * 4 * CPT columns.  A compute warp holds four groups of CPT columns; a group
 // is shared by MC_LANES lanes, lane j holding rows d = i * 4 MC_LANES + 4 j + (0 .. 3), i < NI, of each of its columns
@@ -176,7 +177,7 @@ template <typename T, int NI, int CPT>
 __global__ void __launch_bounds__(MC_THREADS)
 matrix_cell_kernel(const T* __restrict__ qkv, int64_t stride, const float* __restrict__ gates, int64_t gate_stride,
                    const float* __restrict__ bias_i, const float* __restrict__ bias_f, float cap, float q_scale,
-                   float* __restrict__ memory, float* __restrict__ peak, float* __restrict__ num, float* __restrict__ nq,
+                   float* __restrict__ memory, const float* __restrict__ peak, float* __restrict__ num, float* __restrict__ nq,
                    float* __restrict__ peaks_out, const int32_t* __restrict__ q_start, const int32_t* __restrict__ seq_lens,
                    const int32_t* __restrict__ slots, int H, int D, int V, int n_slots, int wide_loads, int* err) {
     pdl_wait();
@@ -374,10 +375,7 @@ matrix_cell_kernel(const T* __restrict__ qkv, int64_t stride, const float* __res
         __syncthreads();
     }
 
-    if (stager) {
-        if (stages_gates && blockIdx.x == 0 && lane == 0) peak[(int64_t)slot * H + h] = m_prev;
-        return;
-    }
+    if (stager) return;
 #pragma unroll
     for (int c = 0; c < CPT; ++c) {
         if (col0 + c > V) continue;
@@ -396,6 +394,27 @@ matrix_cell_kernel(const T* __restrict__ qkv, int64_t stride, const float* __res
     }
 }
 
+// The peak behind a step: m of every request's last row into its slot.
+__global__ void __launch_bounds__(128)
+cell_peaks_kernel(const float* __restrict__ peaks, float* __restrict__ peak, const int32_t* __restrict__ q_start,
+                  const int32_t* __restrict__ seq_lens, const int32_t* __restrict__ slots, int64_t n_pairs, int H, int n_slots) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int64_t pair = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (pair >= n_pairs) return;
+    const int64_t r = pair / H;
+    const int h = (int)(pair - r * H), end = q_start[r + 1], slot = slots[r];
+    if (end <= q_start[r] || seq_lens[r] <= 0 || slot < 0 || slot >= n_slots) return;
+    peak[(int64_t)slot * H + h] = peaks[(int64_t)(end - 1) * H + h];
+}
+
+int launch_cell_peaks(const float* peaks, float* peak, const int32_t* q_start, const int32_t* seq_lens, const int32_t* slots, int R, int H,
+                      int n_slots, cudaStream_t stream) {
+    const int64_t n = (int64_t)R * H;
+    ss_launch(cell_peaks_kernel, dim3((unsigned)((n + 127) / 128)), dim3(128), 0, stream, peaks, peak, q_start, seq_lens, slots, n, H, n_slots);
+    return SS_LAUNCH_CHECK();
+}
+
 template <typename T, int NI, int CPT>
 static int launch_matrix_cell_as(const void* qkv, int64_t stride, const float* gates, int64_t gate_stride, const float* bias_i,
                                  const float* bias_f, float cap, float q_scale, float* memory, float* peak, float* num,
@@ -411,7 +430,8 @@ static int launch_matrix_cell_as(const void* qkv, int64_t stride, const float* g
     ss_launch(matrix_cell_kernel<T, NI, CPT>, grid, dim3(MC_THREADS), smem, stream, (const T*)qkv, stride, gates, gate_stride,
               bias_i, bias_f, cap, q_scale, memory, peak, num, nq, peaks_out, q_start, seq_lens, slots, H, D, V, n_slots, wide,
               err);
-    return SS_LAUNCH_CHECK();
+    if (int rc = SS_LAUNCH_CHECK()) return rc;
+    return launch_cell_peaks(peaks_out, peak, q_start, seq_lens, slots, R, H, n_slots, stream);
 }
 
 template <typename T>

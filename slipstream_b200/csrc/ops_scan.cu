@@ -57,11 +57,14 @@ struct ScanArgs {
     const float* bias_i;
     const float* bias_f;
     float cap, q_scale;
-    float* peak;
+    const float* peak;  // in front of the step, read by all column blocks of a head: a kernel behind this one writes it
     float* nq;
     float* peaks_out;
     int sms;
 };
+
+int launch_cell_peaks(const float* peaks, float* peak, const int32_t* q_start, const int32_t* seq_lens, const int32_t* slots, int R, int H,
+                      int n_slots, cudaStream_t stream);  // ops_cells.cu
 
 namespace {
 
@@ -560,7 +563,6 @@ __global__ void __launch_bounds__(SC_THREADS, N <= 128 ? 2 : 1) scan_chunks_kern
             fetch_values(t0 + nb);
         }
         cp_async_commit();
-        if (CELL && !more && first_cols && tid == 0) g.peak[(int64_t)slot * g.heads + h] = gate_row(buf, 3)[nb - 1];
     }
 #pragma unroll
     for (int m = 0; m < MPW; ++m)
@@ -638,5 +640,6 @@ extern "C" int ss_matrix_cell_chunks(const void* qkv, int64_t stride, const floa
     g.gates = gates; g.gate_stride = gate_stride; g.bias_i = bias_i; g.bias_f = bias_f; g.cap = cap; g.q_scale = q_scale;
     g.peak = peak; g.nq = nq; g.peaks_out = peaks_out;
     if (!scan_fits(g)) return (int)cudaErrorInvalidValue;
-    return launch_scan<true>(g, R, stream);
+    if (int rc = launch_scan<true>(g, R, stream)) return rc;
+    return launch_cell_peaks(peaks_out, peak, q_start, seq_lens, slots, R, H, n_slots, stream);
 }

@@ -2194,6 +2194,7 @@ def matrix_cell(qkv: torch.Tensor, gates: torch.Tensor, bias_i: torch.Tensor | N
     num = torch.empty((n, heads * vdim), dtype=torch.float32, device=qkv.device)
     nq = torch.empty((n, heads), dtype=torch.float32, device=qkv.device)
     peaks = torch.empty((n, heads), dtype=torch.float32, device=qkv.device)
+    _launches[0] += 1  # two kernels: the second one leaves the peak
     if (chunks and not ctx.is_decode_only and qkv.dtype == torch.bfloat16 and dim % 8 == vdim % 8 == qkv.stride(0) % 8 == 0
             and qkv.data_ptr() % 16 == 0 and cap > 0.0):
         _check(ops_library().ss_matrix_cell_chunks(

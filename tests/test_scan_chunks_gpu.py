@@ -127,3 +127,37 @@ def test_what_is_not_finite_reaches_what_it_reaches_token_by_token(token, column
     assert torch.equal(torch.isfinite(got), finite) and 0 < int((~finite).sum()) < finite.numel()
     assert off(got[finite], want[finite].double().cpu()) < 2 * TOLERANCE
     ops.check_errors(DEV)
+
+
+# more column blocks than the GPU holds at once, so that a head's blocks start at different times: one request of many heads, and
+# one-token requests, whose blocks end first, beside a long one
+@pytest.mark.parametrize("heads, dim, vdim, lens", [(28, 256, 256, [70]), (28, 128, 200, [1] * 24 + [130] + [1] * 24), (28, 64, 256, [1] * 60)])
+@pytest.mark.parametrize("chunks", [True, False])
+def test_every_column_block_of_a_matrix_memory_starts_from_the_old_peak(heads, dim, vdim, lens, chunks):
+    from slipstream_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(dim + vdim)
+    draw = lambda *shape: torch.randn(*shape, generator=g, device=DEV)  # noqa: E731
+    n, cap, scale = sum(lens), 6.0, dim ** -0.5
+    qkv, gates = draw(n, heads * (2 * dim + vdim)).bfloat16(), draw(n, 2 * heads) * 4
+    memory, peak = draw(len(lens), heads, vdim + 1, dim), draw(len(lens), heads) - 4.0  # far below what the gates make of it
+    i = cap * torch.tanh(gates[:, :heads].double() / cap)
+    f = torch.nn.functional.logsigmoid(cap * torch.tanh(gates[:, heads:].double() / cap))
+    q, k, x = (qkv[:, o: o + heads * w].reshape(n, heads, w).double() for o, w in ((0, dim), (heads * dim, dim), (2 * heads * dim, vdim)))
+    x = torch.cat([x, torch.ones_like(x[..., :1])], -1)
+    want, memories, peaks, row = [], memory.double(), peak.double(), 0
+    for r, t in enumerate(lens):
+        for at in range(row, row + t):
+            m = torch.maximum(f[at] + peaks[r], i[at])
+            memories[r] = torch.exp(f[at] + peaks[r] - m)[:, None, None] * memories[r] + (torch.exp(i[at] - m)[:, None] * x[at])[:, :, None] * k[at][:, None, :]
+            peaks[r] = m
+            want.append((memories[r] * (q[at] * scale)[:, None, :]).sum(-1))
+        row += t
+    want = torch.stack(want)
+    ctx = step_ctx(lens, list(range(len(lens))))
+    ctx.is_decode_only = max(lens) == 1 and not chunks
+    num, nq, last = ops.matrix_cell(qkv, gates, None, None, cap, scale, memory, peak, ctx, heads, dim, vdim, chunks=chunks)
+    far = lambda got, ref: float((got.double() - ref).norm() / ref.norm())  # noqa: E731
+    assert far(num.view(n, heads, vdim), want[..., :vdim]) < TOLERANCE and far(nq, want[..., vdim]) < TOLERANCE
+    assert far(memory, memories) < TOLERANCE and far(peak, peaks) < TOLERANCE
+    assert torch.equal(peak, last[torch.tensor(lens, device=DEV).cumsum(0) - 1])
+    ops.check_errors(DEV)

@@ -236,14 +236,20 @@ __global__ void __launch_bounds__(SC_THREADS, N <= 128 ? 2 : 1) scan_chunks_kern
             }
             __syncwarp();
         }
+        // A decay below e^-200 is zero in 32 bits, alone or in a product: an infinite one is held there, so that the
+        // differences L_t - L_s of tokens behind it are numbers.  (A NaN stays one.)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) a[e] = a[e] < -200.f ? -200.f : a[e];
         const double a0 = (double)a[0], both = a0 + (double)a[1];
-        double before = both;  // inclusive sum over the lanes, then exclusive
+        double up_to = both;  // inclusive sum over the lanes
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const double up = __shfl_up_sync(0xffffffffu, before, o);
-            if (lane >= o) before += up;
+            const double up = __shfl_up_sync(0xffffffffu, up_to, o);
+            if (lane >= o) up_to += up;
         }
-        before -= both;
+        // the lanes in front, not `up_to` less this lane's two: a NaN of the odd token is not in front of the even one
+        double before = __shfl_up_sync(0xffffffffu, up_to, 1);
+        if (lane == 0) before = 0.0;
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const double sum = before + (e ? both : a0);

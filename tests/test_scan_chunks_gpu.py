@@ -161,3 +161,57 @@ def test_every_column_block_of_a_matrix_memory_starts_from_the_old_peak(heads, d
     assert far(memory, memories) < TOLERANCE and far(peak, peaks) < TOLERANCE
     assert torch.equal(peak, last[torch.tensor(lens, device=DEV).cumsum(0) - 1])
     ops.check_errors(DEV)
+
+
+def same_reach(got, want):
+    """What is finite token by token is finite in chunks, and equal; the rest is not finite in either."""
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), finite)
+    assert 0 < int((~finite).sum()) < finite.numel() and off(got[finite], want[finite].double().cpu()) < 2 * TOLERANCE
+
+
+# the odd and the even token of a lane's pair, at the edges of lanes and chunks; a step size that is infinite forgets everything
+@pytest.mark.parametrize("token, value", [(1, "nan"), (6, "nan"), (63, "inf"), (64, "inf"), (101, "inf"), (149, "nan")])
+def test_step_sizes_that_are_not_finite_reach_no_token_in_front(token, value):
+    from slipstream_b200 import ops
+    torch.manual_seed(token)
+    heads, groups, p, n, t = 4, 2, 64, 128, 150
+    xbc, dt = torch.randn(t, heads * p + 2 * groups * n, device=DEV).bfloat16(), torch.randn(t, heads, device=DEV).bfloat16()
+    consts = [torch.randn(heads, device=DEV) * 0.5 for _ in range(3)]
+    dt[token, 2] = float(value)
+    got, want = (ops.ssm_scan(xbc, dt, *consts, torch.zeros(1, heads, p, n, device=DEV), step_ctx([t], [0]), heads, groups, p, n, chunks=c)
+                 for c in (True, False))
+    assert torch.isfinite(want[:token]).all()
+    same_reach(got, want)
+    ops.check_errors(DEV)
+
+
+@pytest.mark.parametrize("token, column", [(1, 2), (6, 2), (63, 5), (64, 5), (149, 2)])  # input gates, then forget gates
+def test_gates_that_are_not_numbers_reach_no_token_in_front(token, column):
+    from slipstream_b200 import ops
+    torch.manual_seed(token)
+    heads, dim, vdim, t = 3, 64, 72, 150
+    qkv, gates = torch.randn(t, heads * (2 * dim + vdim), device=DEV).bfloat16(), torch.randn(t, 2 * heads, device=DEV) * 3
+    gates[token, column] = float("nan")
+    results = []
+    for chunks in (True, False):
+        memory, peak = torch.zeros(1, heads, vdim + 1, dim, device=DEV), torch.zeros(1, heads, device=DEV)
+        results.append((*ops.matrix_cell(qkv, gates, None, None, 6.0, dim ** -0.5, memory, peak, step_ctx([t], [0]), heads, dim, vdim, chunks=chunks), memory))
+    for which in (0, 1, 3):
+        same_reach(results[0][which], results[1][which])
+    assert torch.isfinite(results[0][0][:token]).all() and torch.equal(results[0][2], results[1][2])
+    ops.check_errors(DEV)
+
+
+def test_a_peak_of_minus_infinity_forgets_the_memory_in_front():
+    from slipstream_b200 import ops
+    torch.manual_seed(0)
+    heads, dim, vdim, t = 3, 64, 72, 100
+    qkv, gates = torch.randn(t, heads * (2 * dim + vdim), device=DEV).bfloat16(), torch.randn(t, 2 * heads, device=DEV) * 3
+    start, results = torch.randn(1, heads, vdim + 1, dim, device=DEV), []
+    for chunks in (True, False):
+        memory, peak = start.clone(), torch.full((1, heads), -float("inf"), device=DEV)
+        results.append((*ops.matrix_cell(qkv, gates, None, None, 6.0, dim ** -0.5, memory, peak, step_ctx([t], [0]), heads, dim, vdim, chunks=chunks), memory, peak))
+    for got, want in zip(*results):
+        assert torch.isfinite(want).all() and off(got, want.double().cpu()) < 2 * TOLERANCE
+    ops.check_errors(DEV)

@@ -315,6 +315,9 @@ __global__ void __launch_bounds__(SC_THREADS, N <= 128 ? 2 : 1) scan_chunks_kern
             __syncthreads();
             for (int i = tid; i < (SC_T - nb) * CT; i += SC_THREADS)
                 *reinterpret_cast<uint4*>(X + (nb + i / CT) * VS + (i % CT) * 8) = make_uint4(0u, 0u, 0u, 0u);
+            // (and the keys: their weights in the state are 0, which an infinite key would make a NaN)
+            for (int i = tid; i < (SC_T - nb) * RUNS; i += SC_THREADS)
+                *reinterpret_cast<uint4*>(K + (nb + i / RUNS) * QS + (i % RUNS) * 8) = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
         }
         const float* lh = gate_row(buf, 0);

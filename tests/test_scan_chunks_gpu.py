@@ -215,3 +215,27 @@ def test_a_peak_of_minus_infinity_forgets_the_memory_in_front():
     for got, want in zip(*results):
         assert torch.isfinite(want).all() and off(got, want.double().cpu()) < 2 * TOLERANCE
     ops.check_errors(DEV)
+
+
+# a value that is not finite cuts a chunk; infinite keys a few tokens behind it in the same 16 tokens and further on, which stand in
+# memory already
+@pytest.mark.parametrize("value_at, key_at", [(10, 14), (10, 40), (0, 1), (70, 75)])
+def test_an_infinite_key_behind_a_cut_reaches_no_token_in_front(value_at, key_at):
+    from slipstream_b200 import ops
+    torch.manual_seed(key_at)
+    heads, dim, vdim, t = 2, 64, 72, 100
+    xbc, dt = torch.randn(t, heads * vdim + 2 * dim, device=DEV).bfloat16(), torch.randn(t, heads, device=DEV).bfloat16()
+    qkv, gates = torch.randn(t, heads * (2 * dim + vdim), device=DEV).bfloat16(), torch.randn(t, 2 * heads, device=DEV)
+    consts = [torch.randn(heads, device=DEV) * 0.5 for _ in range(3)]
+    xbc[value_at, 3], xbc[key_at, heads * vdim + 7] = float("nan"), float("inf")
+    qkv[value_at, 2 * heads * dim + 3], qkv[key_at, heads * dim + 7] = float("nan"), float("inf")
+    results = []
+    for chunks in (True, False):
+        state, memory, peak = torch.zeros(1, heads, vdim, dim, device=DEV), torch.zeros(1, heads, vdim + 1, dim, device=DEV), torch.zeros(1, heads, device=DEV)
+        ctx = step_ctx([t], [0])
+        y = ops.ssm_scan(xbc, dt, *consts, state, ctx, heads, 1, vdim, dim, chunks=chunks)
+        num, nq, _ = ops.matrix_cell(qkv, gates, None, None, 6.0, dim ** -0.5, memory, peak, ctx, heads, dim, vdim, chunks=chunks)
+        results.append((y, state, num, nq, memory))
+    for got, want in zip(*results):
+        same_reach(got, want)
+    ops.check_errors(DEV)

@@ -356,16 +356,23 @@ __device__ __forceinline__ float key_value(uint32_t key) {  // the inverse of or
     return __uint_as_float(key & 0x80000000u ? key & 0x7fffffffu : ~key);
 }
 
-// Token i enters the race with its value plus its Gumbel noise (noise: the four words of its group).  With z = 2^24 - 1 minus
-// the word's upper 24 bits, 1 - u is at least 2^-(n + 1), n the zeros in front of z's 24 bits, and -log(-log u) is below
-// -log(1 - u): a token whose value plus (n + 1) log 2 is below the best entry cannot win, and its logarithms, most of the
-// work, are not formed (z = 0, where u rounds to 1, is never left out).
+// -log(-log u) of u = (word + 1/2) / 2^24, word a noise word's upper 24 bits.  word + 1/2 has more than a float's 24 bits from
+// 2^23 on (the last word's u would be 1 and its noise infinite), so there the noise is formed from 1 - u = (z + 1/2) / 2^24 with
+// z = 2^24 - 1 - word, which is exact.
+__device__ __forceinline__ float gumbel(uint32_t word) {
+    const uint32_t z = 0xffffffu - word;
+    const float e = word < 0x800000u ? -logf(((float)word + 0.5f) * (1.0f / 16777216.0f)) : -log1pf(-((float)z + 0.5f) * (1.0f / 16777216.0f));
+    return -logf(e);
+}
+
+// Token i enters the race with its value plus its Gumbel noise (noise: the four words of its group).  With z as above and n the
+// zeros in front of z's 24 bits (24 for z = 0), 1 - u is at least 2^-(n + 1), and -log(-log u) is below -log(1 - u): a token whose
+// value plus (n + 1) log 2 is below the best entry cannot win, and its logarithms, most of the work, are not formed.
 __device__ __forceinline__ void race(ArgMax& a, float v, int i, const uint32_t* noise, SampleShared& sh) {
-    const uint32_t word = noise[i & 3] >> 8, z = 0xffffffu - word;
-    const float bound = v + (0.69315f * (float)(__clz(z) - 7) + 0.01f);
-    if (z != 0u && bound < key_value(*(volatile uint32_t*)&sh.best_key)) return;
-    const float u = ((float)word + 0.5f) * (1.0f / 16777216.0f);
-    const ArgMax entry{v + (-logf(-logf(u))), i};
+    const uint32_t word = noise[i & 3] >> 8;
+    const float bound = v + (0.69315f * (float)(__clz(0xffffffu - word) - 7) + 0.01f);
+    if (bound < key_value(*(volatile uint32_t*)&sh.best_key)) return;
+    const ArgMax entry{v + gumbel(word), i};
     if (entry.v > a.v) atomicMax(&sh.best_key, order_key(entry.v));
     a = better(a, entry);
 }

@@ -211,3 +211,40 @@ def test_engine_under_random_schedules_gives_the_tokens_of_the_engine_with_room(
             assert got == want, what
         preemptions += tight.scheduler.preemptions
     assert preemptions > 20, "the pools were meant to run out"
+
+
+def noise_words(seed, draw, vocab):
+    from test_generate_gpu import philox4x32_10
+    groups = np.arange((vocab + 3) // 4, dtype=np.uint64)
+    zeros = np.zeros_like(groups)
+    c = philox4x32_10(seed, 0, groups, zeros + np.uint64(draw), zeros, zeros + np.uint64(0x51195))
+    return (np.stack(c, axis=1).reshape(-1)[:vocab] >> np.uint64(8)).astype(np.int64)
+
+
+def test_the_largest_noise_word_is_not_an_infinite_noise():
+    """Its u = 1 - 2^-25 is not a float; a token with that word and a hopeless logit must not be drawn."""
+    vocab, found = 152064, []
+    for draw in range(2000):
+        last = np.flatnonzero(noise_words(7, draw, vocab) == 0xFFFFFF)
+        if last.size:
+            found.append((draw, int(last[0])))
+        if len(found) == 4:
+            break
+    torch.manual_seed(0)
+    logits = torch.randn(len(found), vocab)
+    for i, (_, token) in enumerate(found):
+        logits[i, token] = -40.0
+    for filters in (dict(), dict(top_p=0.999999), dict(min_p=1e-30)):
+        got = run_sample(logits.to(DEV), [dict(temperature=1.0, seed=7, draw=draw, **filters) for draw, _ in found])
+        for i, (draw, token) in enumerate(found):
+            score = logits[i].double().numpy() + gumbel_noise(7, draw, vocab)
+            assert got[i] != token and score[got[i]] >= score.max() - 1e-4, (i, got[i], token)
+
+
+def test_equal_logits_draw_the_token_with_the_largest_noise_word():
+    """The noise of neighbouring words near the end differs by up to 0.5: each word keeps its own."""
+    vocab, rows = 152064, 64
+    got = run_sample(torch.zeros(rows, vocab, device=DEV), [dict(temperature=1.0, seed=3, draw=i) for i in range(rows)])
+    for i in range(rows):
+        words = noise_words(3, i, vocab)
+        assert words[got[i]] == words.max(), i

@@ -1027,7 +1027,7 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, bloc
         raise KernelError("only bfloat16 decode steps rotate inside the attention kernel")
     if qkv.dtype == torch.float32:
         heads = out if diff is None else _heads_f32(out, n_q, head_dim)
-        if n_q // n_kv <= FLOAT32_GROUP:
+        if n_q // n_kv <= FLOAT32_GROUP and kv.data_ptr() % 16 == 0:  # (that kernel copies pages 16 bytes at a time)
             paged_attention_float32(qkv, heads, kv, block_tables, ctx, n_q, n_kv, head_dim, scale, window, chunk, gate, softcap,
                                     sinks, keep, across)
         else:

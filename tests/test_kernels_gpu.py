@@ -971,3 +971,22 @@ def test_experts_sum_eight_elements_at_a_time(tokens, hidden, top):
             for k in range(top):
                 total = total + terms[:, k]
             assert torch.equal(got, (total if extra is None else total + extra.float()).bfloat16())
+
+
+def test_float32_attention_takes_pages_that_start_on_any_float():
+    from slipstream_b200.engine.context import query_tiles_host
+    from types import SimpleNamespace
+    lens, n_q, n_kv, d, page = [40, 9], 4, 2, 32, 16
+    q, kv, table, q_start, seq_lens = make_attention_case(torch.float32, lens, lens, n_q, n_kv, d, page, seed=3)
+    odd = torch.empty(kv.numel() + 1, device=DEV)[1:].view(kv.shape)
+    odd.copy_(kv)
+    tiles = lambda rows, group=1: tuple(torch.tensor(np.asarray(t), dtype=torch.int32, device=DEV)  # noqa: E731
+                                        for t in query_tiles_host(np.asarray(lens, dtype=np.int32) * group, rows))
+    ctx = SimpleNamespace(is_decode_only=False, num_requests=2, max_seq_len=max(lens), seq_lens=seq_lens, q_start=q_start, extras={}, query_tiles=tiles)
+    qkv = torch.cat([q.view(q.shape[0], -1), torch.zeros(q.shape[0], 2 * n_kv * d, device=DEV)], dim=1)
+    outs = [torch.empty(q.shape[0], n_q * d, device=DEV) for _ in range(2)]
+    for out, pages in zip(outs, (kv, odd)):
+        ops().paged_attention(qkv, out, pages, table, ctx, n_q, n_kv, d, 0.3)
+        want = attention_reference(q, kv, table, q_start, seq_lens, n_kv, page, 0.3, 0)
+        assert rel_err(out.cpu(), want.reshape(out.shape)) < 5e-6  # the bound of the float32 kernels, above
+    ops().check_errors(torch.device(DEV))

@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(AF_THREADS, D <= 128 ? 3 : 1) attn_f32_kernel(
             const float now = fmaxf(before, top);
 #pragma unroll
             for (int k = 0; k < KPT; ++k)
-                Ps[(tx + TX * k) * PS + row] = now == -INFINITY ? 0.f : expf(__fsub_rn(sc[k], now));
+                Ps[(tx + TX * k) * PS + row] = sc[k] == -INFINITY ? 0.f : expf(__fsub_rn(sc[k], now));  // (a NaN has no part in `now`, and stays)
             if (tx == 0) {
                 alpha_s[row] = before == -INFINITY ? 0.f : expf(__fsub_rn(before, now));
                 max_s[row] = now;

@@ -990,3 +990,29 @@ def test_float32_attention_takes_pages_that_start_on_any_float():
         want = attention_reference(q, kv, table, q_start, seq_lens, n_kv, page, 0.3, 0)
         assert rel_err(out.cpu(), want.reshape(out.shape)) < 5e-6  # the bound of the float32 kernels, above
     ops().check_errors(torch.device(DEV))
+
+
+@pytest.mark.parametrize("with_sinks", [False, True])
+@pytest.mark.parametrize("parts", [1, 3])
+def test_float32_attention_passes_on_scores_that_are_not_numbers(monkeypatch, with_sinks, parts):
+    """A query of NaN, and slices of keys of which some or all are NaN: every row that sees one is NaN, no other row is."""
+    from types import SimpleNamespace
+    from slipstream_b200.engine.context import query_tiles_host
+    from slipstream_b200.ops import functions
+    lens, n_q, n_kv, d, page = [300, 40], 4, 2, 32, 16
+    q, kv, table, q_start, seq_lens = make_attention_case(torch.float32, lens, lens, n_q, n_kv, d, page, seed=4)
+    q[305, 1] = float("nan")
+    for key in (*range(128, 256), 270):  # request 0: all of its second slice, one key of its third
+        kv[int(table[0, key // page]), 0, 0, key % page] = float("nan")
+    sinks = torch.randn(n_q, device=DEV) if with_sinks else None
+    as_dev = lambda a: torch.tensor(np.asarray(a, dtype=np.int32), device=DEV)  # noqa: E731
+    ctx = SimpleNamespace(is_decode_only=False, num_requests=2, max_seq_len=max(lens), seq_lens=seq_lens, q_start=q_start, extras={},
+                          query_tiles=lambda n, g: tuple(as_dev(t) for t in query_tiles_host(np.asarray(lens) * g, n)))
+    out = torch.zeros(q.shape[0], n_q * d, device=DEV)
+    monkeypatch.setattr(functions, "float32_key_parts", lambda *a, **k: parts)
+    for window in (0, 20):  # 20: rows from 148 on see nothing but NaN, some see one among numbers, the last see none
+        ops().paged_attention_float32(q.reshape(q.shape[0], -1).contiguous(), out, kv, table, ctx, n_q, n_kv, d, 0.3, window, 0, None, 0.0, sinks)
+        want = attention_reference(q, kv, table, q_start, seq_lens, n_kv, page, 0.3, window, sinks).view(out.shape)
+        assert torch.equal(out.isnan().cpu(), want.isnan()) and 0 < int(want.isnan().sum()) < want.numel()
+        assert rel_err(out.cpu()[~want.isnan()], want[~want.isnan()]) < 5e-6
+    ops().check_errors(torch.device(DEV))

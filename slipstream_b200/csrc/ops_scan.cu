@@ -127,11 +127,11 @@ __global__ void __launch_bounds__(SC_THREADS, N <= 128 ? 2 : 1) scan_chunks_kern
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // (1): tokens 16 rt .. of the chunk.  The last tokens see the most keys: of two blocks of an SM they go to different quarters
-    const int rt = (warp + 2 * ((blockIdx.x + gridDim.x * blockIdx.y) / g.sms)) & 3;
+    const int rt = (warp + 2 * (blockIdx.x / g.sms)) & 3;
     const bool makes_gates = warp < 4 && rt == 0;
     const int row_lo = rt * 16 + (lane >> 2), row_hi = row_lo + 8;
     const int col_blocks = (g.vdim + COLS - 1) / COLS;
-    const int h = blockIdx.x / col_blocks, c0 = (blockIdx.x % col_blocks) * COLS, r = blockIdx.y;
+    const int unit = blockIdx.x / col_blocks, c0 = (blockIdx.x % col_blocks) * COLS, r = unit / g.heads, h = unit - r * g.heads;
     const bool first_cols = CELL && c0 == 0;  // the block of a head that also has its normaliser and peaks
     pdl_launch_dependents();
     pdl_wait();
@@ -591,7 +591,9 @@ static int launch_scan_as(const ScanArgs& g, int R, cudaStream_t stream) {
     constexpr int smem = ScanSmem<N, CT>::bytes;
     static SsPerDevice opted;
     if (int rc = ss_opt_in_smem(scan_chunks_kernel<CELL, N, CT>, smem, opted)) return rc;
-    ss_launch(scan_chunks_kernel<CELL, N, CT>, dim3(g.heads * ((g.vdim + CT * 8 - 1) / (CT * 8)), R), dim3(SC_THREADS), smem, stream, g);
+    const int64_t blocks = (int64_t)g.heads * ((g.vdim + CT * 8 - 1) / (CT * 8)) * R;  // along x, which takes any number of requests
+    if (blocks >= (1ll << 31)) return (int)cudaErrorInvalidValue;
+    ss_launch(scan_chunks_kernel<CELL, N, CT>, dim3((unsigned)blocks), dim3(SC_THREADS), smem, stream, g);
     return SS_LAUNCH_CHECK();
 }
 

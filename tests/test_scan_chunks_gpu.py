@@ -239,3 +239,16 @@ def test_an_infinite_key_behind_a_cut_reaches_no_token_in_front(value_at, key_at
     for got, want in zip(*results):
         same_reach(got, want)
     ops.check_errors(DEV)
+
+
+def test_state_space_scan_in_chunks_takes_more_requests_than_a_grid_is_high():
+    from slipstream_b200 import ops
+    torch.manual_seed(0)
+    lens = [2, *[1] * 65536, 70]
+    n, r = sum(lens), len(lens)
+    xbc, dt = torch.randn(n, 24, device=DEV).bfloat16(), torch.randn(n, 1, device=DEV).bfloat16()
+    consts, start = [torch.randn(1, device=DEV) for _ in range(3)], torch.randn(r, 1, 8, 8, device=DEV)
+    states, ctx = [start.clone(), start.clone()], step_ctx(lens, range(r))
+    got, want = (ops.ssm_scan(xbc, dt, *consts, s, ctx, 1, 1, 8, 8, chunks=c) for s, c in zip(states, (True, False)))
+    assert off(got, want.double().cpu()) < TOLERANCE and off(states[0], states[1].double().cpu()) < TOLERANCE
+    ops.check_errors(DEV)

@@ -283,10 +283,12 @@ class PagedAttention(Mixer):
     def prepare_capture(self, ctx, variant: object, max_model_len: int) -> None:
         if not ctx.is_decode_only:
             # a captured step with prompt portions: the number of key parts is the variant's (the choice follows the
-            # lengths of the step, which a replay does not know on the host)
-            ctx.extras[("prefill_key_parts", 128 // (self.num_heads // self.num_kv_heads), self.kernel_blocks,
-                        self.sees)] = int(variant or 1)
-            ctx.extras[("few_keys", self.head_dim)] = variant == 0
+            # lengths of the step, which a replay does not know on the host).  A layer that the tcgen05 kernel does not take (None)
+            # has nothing to say, not for a layer of the same head size and reach that it takes either.
+            if variant is not None:
+                ctx.extras[("prefill_key_parts", 128 // (self.num_heads // self.num_kv_heads), self.kernel_blocks,
+                            self.sees)] = int(variant or 1)
+                ctx.extras[("few_keys", self.head_dim)] = variant == 0
             return
         # the number of slices must not follow the lengths of the step that happens to be captured
         ctx.extras["static_max_seq_len"] = max_model_len

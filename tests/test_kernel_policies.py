@@ -103,3 +103,28 @@ def test_expert_tiles_and_float32_key_parts():
     assert F.float32_key_parts(8, 20, 4, 12, 128, sms=SMS) == 20 and F.float32_key_parts(100, 20, 4, 12, 128, sms=SMS) == 2
     assert F.float32_key_parts(400, 20, 4, 12, 128, sms=SMS) == 1
     assert F.float32_key_parts(8, 20, 5000, 28, 128, sms=SMS) == 1  # the slices' scratch would pass its bound
+
+
+def paged_layer(dim, page_size=16, **kind):
+    from types import SimpleNamespace
+    import torch
+    from slipstream_b200.parts import PagedAttention, RotaryEncoding
+
+    layer = PagedAttention("attn", 64, 4, 2, dim, RotaryEncoding(dim, 1e4), page_size=page_size, **kind)
+    layer.runtime = SimpleNamespace(dtype=torch.bfloat16, device=0)
+    return layer
+
+
+def test_a_layer_off_the_tcgen05_kernel_does_not_answer_for_another_of_its_head_size(monkeypatch):
+    from types import SimpleNamespace
+
+    monkeypatch.setattr(F, "_device_sm_count", lambda index: SMS)
+    taken, other = paged_layer(96), paged_layer(96, page_size=12)
+    for length, wanted in ((30, 0), (9000, 8)):
+        plan = SimpleNamespace(is_decode_only=False, q_lens=np.array([30]), seq_lens=np.array([length]))
+        assert taken.capture_variant(length, plan) == wanted and other.capture_variant(length, plan) is None
+        ctx = SimpleNamespace(is_decode_only=False, extras={})
+        for layer in (taken, other):
+            layer.prepare_capture(ctx, layer.capture_variant(length, plan), 16384)
+        # as in the step that is not captured
+        assert ctx.extras == {("few_keys", 96): wanted == 0, ("prefill_key_parts", 64, 2, 0): max(wanted, 1)}

@@ -259,6 +259,11 @@ class PagedAttention(Mixer):
             self.talk_table = weights[names["talk"]].to(torch.float32).t().contiguous()
         ops.attention_library(self.head_dim)  # compile now, not inside the first step
 
+    @property
+    def gates_inside(self) -> bool:
+        """Whether the attention kernel applies the gate (behind talking heads the mixture does)."""
+        return self.gate and not self.talk
+
     # ------------------------------------------------------------------ decode steps replayed from a graph
     def capture_variant(self, longest: int, plan: object = None) -> object:
         """Decode steps: long contexts of few requests want the keys cut into more slices than fit one thread-block
@@ -271,14 +276,16 @@ class PagedAttention(Mixer):
         group = self.num_heads // self.num_kv_heads
         if not bf16 or not ops.tcgen05_prefill_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_size or 16):
             return None
+        if self.gates_inside and self.head_dim not in (64, 128):
+            return None  # always the mma.sync kernel: one form, one graph
         if ops.few_prefill_keys(self.head_dim, longest):
             return 0
         return int(ops.prefill_key_parts(plan.q_lens, plan.seq_lens, 128 // group, self.kernel_blocks,
                                          ops.sm_count(self.runtime.device), self.sees))
 
     def capture_group(self) -> object:
-        # layers that see equally far with heads of one size answer `capture_variant` alike
-        return ("paged_attention", self.sees, self.head_dim)
+        # layers that see equally far with heads of one size, gated alike, answer `capture_variant` alike
+        return ("paged_attention", self.sees, self.head_dim, self.gates_inside)
 
     def prepare_capture(self, ctx, variant: object, max_model_len: int) -> None:
         if not ctx.is_decode_only:

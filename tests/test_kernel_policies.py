@@ -128,3 +128,14 @@ def test_a_layer_off_the_tcgen05_kernel_does_not_answer_for_another_of_its_head_
             layer.prepare_capture(ctx, layer.capture_variant(length, plan), 16384)
         # as in the step that is not captured
         assert ctx.extras == {("few_keys", 96): wanted == 0, ("prefill_key_parts", 64, 2, 0): max(wanted, 1)}
+
+
+def test_gated_layers_of_the_mma_sync_kernel_are_captured_in_one_form(monkeypatch):
+    from types import SimpleNamespace
+
+    monkeypatch.setattr(F, "_device_sm_count", lambda index: SMS)
+    gated, plain = paged_layer(96, gate=True), paged_layer(96)
+    assert gated.capture_group() != plain.capture_group()
+    answers = [[layer.capture_variant(n, SimpleNamespace(is_decode_only=False, q_lens=np.array([30]), seq_lens=np.array([n])))
+                for n in (30, 300, 9000)] for layer in (gated, plain, paged_layer(64, gate=True))]
+    assert answers[0] == [None] * 3 and answers[1][0] == 0 and len(set(answers[1])) == 3 and len(set(answers[2])) == 2

@@ -1,13 +1,15 @@
 // float32 matrix product on the tensor cores of sm_100a: C[M, N] = X[M, K] * W[N, K]^T (+ bias), all float32.
 //
-// Every operand is cut into three bfloat16 parts, a = a1 + a2 + a3 (each the upper half of what the ones before left, so
-// the three carry the 24 bits of a float32 exactly), on its way into shared memory, and the product is formed from the six pairs
+// Every operand is cut into three bfloat16 parts, a = a1 + a2 + a3 (each what the ones before left, rounded to nearest, so the
+// three carry the 24 bits of a float32 exactly), on its way into shared memory, and the product is formed from the six pairs
 // of parts that matter: a1 b1 in one accumulator, a1 b2 + a2 b1 + a2 b2 + a1 b3 + a3 b1 in another, because the second is
-// 2^-8 of the first and its additions then round at its own size.  What is left out (a2 b3 + a3 b2 and smaller) is below
-// 2^-23 of |a| |b|, 2^-25 on average.  The tensor core adds into an accumulator with truncation, so an accumulator collects only CHUNK = 256 elements
-// of K (16 additions); the chunks' sums are added up in registers, rounded to nearest, in order.  Measured against
-// double precision the error is 1.9e-7 to 2.3e-7 of the result (2-norm) over K of 896 to 18,944, that of a float32 fused
-// multiply-add chain 3.6e-7 to 1.7e-6.
+// 2^-8 of the first and its additions then round at its own size.  What is left out (a2 b3 + a3 b2 and smaller) is at most 2^-24
+// of |a| |b|, 2^-27.4 in the mean square, and has no sign of its own.  (Parts cut off instead of rounded leave out up to 2^-21, always of
+// the product's sign.)  The tensor core adds into an accumulator with truncation, so an accumulator collects only CHUNK = 256 elements
+// of K (16 additions); the chunks' sums are added up in registers, rounded to nearest, in order.  Errors against double precision
+// (2-norm), beside those of a float32 fused multiply-add chain, normal operands: K = 4 2.7e-8 / 3.9e-8, 64 7.0e-8 / 1.4e-7, 256 2.3e-7 /
+// 2.9e-7, 896 2.2e-7 / 5.3e-7, 3,584 2.4e-7 / 1.1e-6.  Positive operands only, where every truncation has the same sign: K = 64 9.0e-8 /
+// 1.2e-7, 128 1.8e-7 / 1.7e-7, 256 3.9e-7 / 2.5e-7, 512 3.8e-7 / 3.5e-7, 896 3.5e-7 / 4.5e-7, 3,584 3.8e-7 / 8.8e-7.
 //
 // An output's value is the same in every form of the kernel and for every M: the same instructions on the same 64-wide
 // steps of K, the same chunks, the chunks' sums added in the same order.  So a token's logits do not depend on what else
@@ -54,12 +56,12 @@ __device__ __forceinline__ float4 f3_load(const float* p) {
     return v;
 }
 
-// The upper halves of two floats, packed: their next parts.  What these leave behind stays in a and b (exactly).
+// Two floats rounded to bfloat16, packed: their next parts.  What these leave behind stays in a and b (exactly).
 __device__ __forceinline__ uint32_t f3_part(float& a, float& b) {
-    const uint32_t x = __float_as_uint(a), y = __float_as_uint(b);
-    a -= __uint_as_float(x & 0xffff0000u);
-    b -= __uint_as_float(y & 0xffff0000u);
-    return __byte_perm(x, y, 0x7632);
+    const uint32_t h = pack_bf16(a, b);
+    a -= __uint_as_float(h << 16);
+    b -= __uint_as_float(h & 0xffff0000u);
+    return h;
 }
 
 __device__ __forceinline__ bool f3_finite(float v) { return fabsf(v) <= 3.4028234e38f; }

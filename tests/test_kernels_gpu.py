@@ -143,7 +143,7 @@ def test_float32_product_on_tensor_cores_carries_24_bits_and_is_independent_of_t
     x[8] *= 1e20
     whole = ops().gemm_float32(x, w, b)
     ref = x.double() @ w.double().T + b.double()
-    # parts left out: 2^-23 of |x| |w|; a chunk's sum: 16 additions that truncate, 2^-23 each at most; the chunks' sums: a
+    # parts left out: 2^-24 of |x| |w|; a chunk's sum: 16 additions that truncate, 2^-23 each at most; the chunks' sums: a
     # rounding of 2^-24 each, with random signs
     bound = (18 + (k / 256) ** 0.5) * 2.0 ** -23 * (x.abs().double() @ w.abs().double().T + b.abs())
     assert ((whole.double() - ref).abs() <= bound).all()
@@ -154,6 +154,26 @@ def test_float32_product_on_tensor_cores_carries_24_bits_and_is_independent_of_t
     for m in (1, 2, 16, 17, 32, 33, 64, 65, 80, 113, 129):
         assert torch.equal(ops().gemm_float32(x[:m].contiguous(), w, b), whole[:m]), m
     ops().check_errors(torch.device(DEV))
+
+
+@pytest.mark.parametrize("k", [4, 8, 16, 64, 192, 256, 512, 896])
+def test_float32_product_is_no_further_from_64_bits_than_the_chain_of_cuda_cores(k):
+    torch.manual_seed(k)
+    x, w = torch.randn(300, k, device=DEV), torch.randn(384, k, device=DEV)
+    ref = x.double() @ w.double().T
+    far = [float((f(x, w).double() - ref).norm()) for f in (ops().gemm_float32, ops().gemm_simt)]
+    assert far[0] < far[1], far
+
+
+@pytest.mark.parametrize("k", [4, 64, 256])
+def test_float32_product_leaves_out_nothing_of_one_sign(k):
+    """Positive operands just below a value of eight bits, whose second part, cut off instead of rounded, would be as large as it can
+    be.  Their parts are exact here, the sums of the first parts' products too (multiples of 2^-14 below 2^10), and those of the
+    others are 2^-8 of them: what is left is one rounding of 2^-24 where the two meet, and 16 truncations of 2^-23 2^-8."""
+    g = torch.Generator(device=DEV).manual_seed(k)
+    x, w = ((torch.randint(0xFF00, 0x10000, (n, k), generator=g, device=DEV) | 0x3F800000).int().view(torch.float32) for n in (90, 130))
+    ref = x.double() @ w.double().T
+    assert float(((ops().gemm_float32(x, w).double() - ref) / ref).abs().max()) < 1.1 * 2.0 ** -24
 
 
 def test_float32_product_passes_infinities_and_nan_on_as_cuda_cores_do():

@@ -384,9 +384,10 @@ __device__ __forceinline__ void group_noise(uint64_t seed, uint64_t draw, int i,
 #define SAMPLE_BINS 1024
 #define SAMPLE_LIST 1024      // values of the threshold's bin that a block keeps
 #define SAMPLE_GATHERED 4096  // ... and all blocks of a row together
+#define SAMPLE_SHARE (1 << 18)  // values of 14 bits that a block can add up in 32
 
 struct SampleBins {
-    uint32_t parts[3][SAMPLE_BINS];         // a block's histogram: counts, or 14 bits of the mass each (no sum overflows)
+    uint32_t parts[3][SAMPLE_BINS];         // a block's histogram: counts, or 14 bits of the mass each (see SAMPLE_SHARE)
     unsigned long long own[SAMPLE_BINS];    // the same added up
     unsigned long long sums[SAMPLE_THREADS / 32];
     unsigned long long before;              // where the threshold falls: what lies in the bins in front of its bin
@@ -444,6 +445,8 @@ __device__ __forceinline__ bool draw_fast(const SampleRow& t, int k, float tp, f
                                           SampleFast& fast, ArgMax& best) {
     const int tid = threadIdx.x;
     const uint32_t n_blocks = cluster_size(), rank = cluster_rank();
+    // (a vocabulary of more than 262,144 and a block to a row, say)
+    if (k <= 0 && (int64_t)((t.vocab + 4 * t.step - 1) / (4 * t.step)) * 4 * blockDim.x > SAMPLE_SHARE) return false;
     float hi = -INFINITY, lo = INFINITY;
     for_groups(t, [&](int, const float (&v)[4], int live) {
 #pragma unroll

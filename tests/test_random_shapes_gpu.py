@@ -248,3 +248,17 @@ def test_equal_logits_draw_the_token_with_the_largest_noise_word():
     for i in range(rows):
         words = noise_words(3, i, vocab)
         assert words[got[i]] == words.max(), i
+
+
+def test_top_p_over_more_values_than_a_block_adds_up_in_32_bits():
+    """263,500 values of one bin whose mass is all ones in its middle 14 bits: those alone pass 2^32.  The draws are ones whose
+    winner would be another token (367,450 and 367,454) if what passes were lost: it stands 6 and 10 tokens behind the threshold."""
+    flat = np.log((4096 * 4000 - 3) / 2.0 ** 24)
+    values = np.concatenate([[0.0], np.full(263500, flat), np.linspace(-0.05, -0.5, 270000)]).astype(np.float32)
+    rows = 150  # one block a row; eight blocks share the single row
+    logits = torch.from_numpy(values).to(DEV).expand(rows, -1).contiguous()
+    for draw, token in ((73818, 42654), (121344, 144665)):
+        ask = dict(temperature=1.0, top_p=0.75, seed=11, draw=draw)
+        kept = plain.filtered_logits(torch.from_numpy(values), temperature=1.0, top_k=-1, top_p=0.75, min_p=0.0).numpy()
+        assert int((kept + gumbel_noise(11, draw, values.size)).argmax()) == token
+        assert run_sample(logits[:1], [ask]) == [token] and run_sample(logits, [ask] * rows) == [token] * rows

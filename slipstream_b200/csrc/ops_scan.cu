@@ -106,6 +106,128 @@ struct ScanSmem {
     static_assert(SC_T * PS * 4 <= 3 * N * VS * 2, "it fits");
 };
 
+// ---- requests with few tokens (decoded ones beside the prompt portions of others): token by token, with the arithmetic of
+// ssm_scan_kernel and matrix_cell_kernel, which run decode steps and steps without a longer portion.  So the bits of such a request do
+// not depend on what else is in its step.  A chunk of 64 tokens for one costs as much as for 64: a portion of 300 tokens
+// beside 48 decoded ones, 112 heads of 64 x 128, 219 us in chunks, 184 so (all token by token 270); 500 beside 200, 821, 666 (740); 32 heads of
+// 128 x 256, 500 beside 200, 1,304, 846 (831).  From two tokens on the time is about that of a chunk (48 requests of 4: 205 and 225 us, of
+// 8: 203 and 299); such requests are few beside a portion.
+#define SC_FEW 8
+
+// State space: columns c0 .. c0 + cols - 1 as ssm_scan_kernel has them, four lanes a column of PER elements each.
+template <int PER>
+__device__ __forceinline__ void scan_few_tokens(const ScanArgs& g, int h, int q0, int q_len, float* sp, int c0, int cols) {
+    const int n0 = (threadIdx.x & 3) * PER, end = min(c0 + cols, g.vdim);
+    const float rate = expf(g.a_log[h]), bias = g.dt_bias[h], skip = g.d_skip[h];
+    const bool vec = (reinterpret_cast<uintptr_t>(sp) & 15) == 0;
+    for (int col = c0 + (threadIdx.x >> 2); col < end; col += SC_THREADS / 4) {  // whole warps: vdim comes in steps of 8
+        float* st = sp + (int64_t)col * g.dim + n0;
+        float S[PER];
+#pragma unroll
+        for (int i = 0; i < PER; i += 4) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (n0 + i < g.dim) v = vec ? *reinterpret_cast<const float4*>(st + i) : make_float4(st[i], st[i + 1], st[i + 2], st[i + 3]);
+            S[i] = v.x; S[i + 1] = v.y; S[i + 2] = v.z; S[i + 3] = v.w;
+        }
+        for (int t = 0; t < q_len; ++t) {
+            const int64_t row = q0 + t;
+            const float z = to_float(g.dt[row * g.dt_stride + h]) + bias, dt = z > 20.f ? z : log1pf(expf(z));
+            const float dec = expf(-rate * dt), xv = to_float(g.x[row * g.stride + (int64_t)h * g.vdim + col]), dx = dt * xv;
+            const bf16* b = g.k + row * g.stride + (int64_t)(h / g.group) * g.dim + n0;
+            const bf16* c = g.q + row * g.stride + (int64_t)(h / g.group) * g.dim + n0;
+            float acc0 = 0.f, acc1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < PER; i += 8) {
+                uint4 bw = make_uint4(0u, 0u, 0u, 0u), cw = bw;
+                if (n0 + i < g.dim) {
+                    bw = *reinterpret_cast<const uint4*>(b + i);
+                    cw = *reinterpret_cast<const uint4*>(c + i);
+                }
+                const uint32_t bb[4] = {bw.x, bw.y, bw.z, bw.w}, cc[4] = {cw.x, cw.y, cw.z, cw.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    S[i + 2 * e] = fmaf(dec, S[i + 2 * e], dx * __uint_as_float(bb[e] << 16));
+                    S[i + 2 * e + 1] = fmaf(dec, S[i + 2 * e + 1], dx * __uint_as_float(bb[e] & 0xffff0000u));
+                    acc0 = fmaf(S[i + 2 * e], __uint_as_float(cc[e] << 16), acc0);
+                    acc1 = fmaf(S[i + 2 * e + 1], __uint_as_float(cc[e] & 0xffff0000u), acc1);
+                }
+            }
+            float acc = acc0 + acc1;
+            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+            if ((threadIdx.x & 3) == 0) g.out[(row * g.heads + h) * g.vdim + col] = fmaf(skip, xv, acc);
+        }
+#pragma unroll
+        for (int i = 0; i < PER; i += 4) {
+            if (n0 + i >= g.dim) continue;
+            if (vec) *reinterpret_cast<float4*>(st + i) = make_float4(S[i], S[i + 1], S[i + 2], S[i + 3]);
+            else { st[i] = S[i]; st[i + 1] = S[i + 1]; st[i + 2] = S[i + 2]; st[i + 3] = S[i + 3]; }
+        }
+    }
+}
+
+// Matrix memory: the same columns, and with the first ones the normaliser, as matrix_cell_kernel has them: eight lanes a column, lane j
+// with elements 32 i + 4 j .. + 3.
+template <int NI>
+__device__ __forceinline__ void cell_few_tokens(const ScanArgs& g, int h, int q0, int q_len, int slot, float* sp, int c0, int cols) {
+    const int j4 = (threadIdx.x & 7) * 4, own = min(c0 + cols, g.vdim) - c0, all = own + (c0 == 0);
+    const float bi = g.bias_i ? g.bias_i[h] : 0.f, bf = g.bias_f ? g.bias_f[h] : 0.f;
+    const bool vec = (reinterpret_cast<uintptr_t>(sp) & 15) == 0;
+    for (int base = 0; base < all; base += SC_THREADS / 8) {  // (the whole warp comes along for the shuffles)
+        const int place = base + (threadIdx.x >> 3), col = place < own ? c0 + place : g.vdim;
+        const bool ok = place < all;
+        float* st = sp + (int64_t)col * g.dim + j4;
+        float S[NI * 4], m = g.peak[(int64_t)slot * g.heads + h];
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float* p = st + 32 * i;
+            if (ok && 32 * i + j4 < g.dim) v = vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+            S[4 * i] = v.x; S[4 * i + 1] = v.y; S[4 * i + 2] = v.z; S[4 * i + 3] = v.w;
+        }
+        for (int t = 0; t < q_len; ++t) {
+            const int64_t row = q0 + t;
+            const float* gate = g.gates + row * g.gate_stride;
+            const float in = g.cap * tanhf((gate[h] + bi) / g.cap), f = sc_log_sigmoid(g.cap * tanhf((gate[g.heads + h] + bf) / g.cap));
+            const float now = fmaxf(f + m, in), keep = expf(f + m - now), take = expf(in - now);
+            if (c0 == 0 && threadIdx.x == 0 && base == 0) g.peaks_out[row * g.heads + h] = now;
+            m = now;
+            const float tv = take * (col < g.vdim ? to_float(g.x[row * g.stride + (int64_t)h * g.vdim + col]) : 1.f);
+            const bf16* k = g.k + row * g.stride + (int64_t)h * g.dim + j4;
+            const bf16* q = g.q + row * g.stride + (int64_t)h * g.dim + j4;
+            float acc = 0.f;
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                uint2 kw = make_uint2(0u, 0u), qw = kw;
+                if (32 * i + j4 < g.dim) {
+                    kw = *reinterpret_cast<const uint2*>(k + 32 * i);
+                    qw = *reinterpret_cast<const uint2*>(q + 32 * i);
+                }
+                const float kk[4] = {__uint_as_float(kw.x << 16), __uint_as_float(kw.x & 0xffff0000u), __uint_as_float(kw.y << 16), __uint_as_float(kw.y & 0xffff0000u)};
+                const float qq[4] = {__uint_as_float(qw.x << 16), __uint_as_float(qw.x & 0xffff0000u), __uint_as_float(qw.y << 16), __uint_as_float(qw.y & 0xffff0000u)};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    S[4 * i + e] = fmaf(keep, S[4 * i + e], kk[e] * tv);
+                    acc = fmaf(S[4 * i + e], __fmul_rn(qq[e], g.q_scale), acc);
+                }
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            if (ok && j4 == 0) {
+                if (col < g.vdim) g.out[(row * g.heads + h) * g.vdim + col] = acc;
+                else g.nq[row * g.heads + h] = acc;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            if (!ok || 32 * i + j4 >= g.dim) continue;
+            float* p = st + 32 * i;
+            if (vec) *reinterpret_cast<float4*>(p) = make_float4(S[4 * i], S[4 * i + 1], S[4 * i + 2], S[4 * i + 3]);
+            else { p[0] = S[4 * i]; p[1] = S[4 * i + 1]; p[2] = S[4 * i + 2]; p[3] = S[4 * i + 3]; }
+        }
+    }
+}
+
 // CELL: the matrix memory, else the state-space scan.
 template <bool CELL, int N, int CT>
 __global__ void __launch_bounds__(SC_THREADS, N <= 128 ? 2 : 1) scan_chunks_kernel(const ScanArgs g) {
@@ -140,6 +262,13 @@ __global__ void __launch_bounds__(SC_THREADS, N <= 128 ? 2 : 1) scan_chunks_kern
     const int slot = g.slots[r];
     if (slot < 0 || slot >= g.n_slots) {
         if (tid == 0) atomicOr(g.err, SS_ERR_SLOT_RANGE);
+        return;
+    }
+    if (q_len <= SC_FEW) {
+        float* state = g.state + ((int64_t)slot * g.heads + h) * (g.vdim + (CELL ? 1 : 0)) * g.dim;
+        if constexpr (CELL) cell_few_tokens<N / 32>(g, h, q0, q_len, slot, state, c0, COLS);
+        else if (N == 64 && g.dim <= 32) scan_few_tokens<8>(g, h, q0, q_len, state, c0, COLS);
+        else scan_few_tokens<N / 4>(g, h, q0, q_len, state, c0, COLS);
         return;
     }
     const bf16* q_src = g.q + (int64_t)q0 * g.stride + (int64_t)(h / g.group) * g.dim;

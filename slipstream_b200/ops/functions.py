@@ -1882,14 +1882,29 @@ def conv_silu(proj: torch.Tensor, col0: int, channels: int, taps: torch.Tensor, 
     return out
 
 
+SCAN_FEW = 8  # tokens up to which a request goes through the recurrences token by token (csrc/ops_scan.cu: SC_FEW)
+
+
+def only_short_portions(ctx) -> bool:
+    """Whether no request of the step brings more than ``SCAN_FEW`` tokens, so that the token-by-token kernels of the state-space scan
+    and the matrix memory run it: they hold more requests on an SM than the kernel that takes chunks, which walks such
+    requests with the same arithmetic (48 requests of 2 tokens, 112 heads of 64 x 128: 150 and 195 us; of 8: 205 and 299).  A captured step,
+    whose lengths the host does not know, was told."""
+    told = getattr(ctx, "extras", {}).get("short_portions")
+    if told is not None:
+        return bool(told)
+    return getattr(ctx, "static_tiles", None) is None and getattr(ctx, "max_q_len", SCAN_FEW + 1) <= SCAN_FEW
+
+
 def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, d_skip: torch.Tensor,
              state: torch.Tensor, ctx, heads: int, groups: int, head_dim: int, state_dim: int, chunks: bool = True) -> torch.Tensor:
     """The diagonal state-space recurrence over each request's tokens, continued from and left in ``state``
     (float32 [slots, heads, head_dim, state_dim]).  ``xbc`` [N, heads * head_dim + 2 * groups * state_dim] holds x, then
     B, then C; ``dt`` [N, heads] is a view of the raw step sizes (unit inner stride).  Per head h (group
     ``h // (heads / groups)``): ``dt' = softplus(dt + dt_bias[h])``, ``S <- exp(-exp(a_log[h]) dt') S + dt' B x^T``,
-    ``y = S^T C + d_skip[h] x``.  Returns y float32 [N, heads * head_dim].  Steps with prompt portions run the kernel that takes
-    chunks of tokens on the tensor cores where it can (``chunks`` False: never): bfloat16 rows, sizes in steps of 8."""
+    ``y = S^T C + d_skip[h] x``.  Returns y float32 [N, heads * head_dim].  Steps with longer portions than ``SCAN_FEW`` tokens
+    run the kernel that takes chunks of tokens on the tensor cores where it can (``chunks`` False: never): bfloat16 rows, sizes in steps
+    of 8.  A request with up to ``SCAN_FEW`` tokens has the same bits in either kernel."""
     _need(xbc, None, "x, B and C")
     for name, t in (("dt_bias", dt_bias), ("a_log", a_log), ("d_skip", d_skip), ("state", state)):
         _need(t, torch.float32, name)
@@ -1900,8 +1915,8 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
     if tuple(state.shape[1:]) != (heads, head_dim, state_dim) or state_dim > 256:
         raise KernelError("ssm_scan: the state must be [slots, heads, head_dim, state_dim] with state_dim <= 256")
     y = torch.empty((n, inner), dtype=torch.float32, device=xbc.device)
-    if (chunks and not ctx.is_decode_only and xbc.dtype == torch.bfloat16 and head_dim % 8 == state_dim % 8 == xbc.shape[1] % 8 == 0
-            and xbc.data_ptr() % 16 == 0):
+    if (chunks and not ctx.is_decode_only and not only_short_portions(ctx) and xbc.dtype == torch.bfloat16
+            and head_dim % 8 == state_dim % 8 == xbc.shape[1] % 8 == 0 and xbc.data_ptr() % 16 == 0):
         _check(ops_library().ss_ssm_scan_chunks(xbc.data_ptr(), xbc.shape[1], dt.data_ptr(), dt.stride(0), dt_bias.data_ptr(),
                                                 a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), y.data_ptr(),
                                                 ctx.q_start.data_ptr(), ctx.seq_lens.data_ptr(), ctx.state_slots.data_ptr(),
@@ -2176,9 +2191,9 @@ def matrix_cell(qkv: torch.Tensor, gates: torch.Tensor, bias_i: torch.Tensor | N
     k: heads * dim | v: heads * vdim]; ``gates`` float32 [N, >= 2 heads] holds the raw input and forget gates.  With
     ``i = cap tanh((a + bias_i) / cap)`` and ``f = logsigmoid(cap tanh((b + bias_f) / cap))``:
     ``m' = max(f + m, i)``, ``S <- exp(f + m - m') S + exp(i - m') k v^T``, n likewise with k alone.
-    Returns (``S^T (q_scale q)`` float32 [N, heads * vdim], ``n . (q_scale q)`` [N, heads], m [N, heads]).  Steps with prompt
-    portions run the kernel that takes chunks of tokens on the tensor cores where it can (``chunks`` False: never): bfloat16
-    rows, sizes in steps of 8."""
+    Returns (``S^T (q_scale q)`` float32 [N, heads * vdim], ``n . (q_scale q)`` [N, heads], m [N, heads]).  Steps with
+    longer portions than ``SCAN_FEW`` tokens run the kernel that takes chunks of tokens on the tensor cores where it can (``chunks``
+    False: never): bfloat16 rows, sizes in steps of 8.  A request with up to ``SCAN_FEW`` tokens has the same bits in either kernel."""
     _need(qkv, None, "q, k and v")
     _need(gates, torch.float32, "gates")
     _need(memory, torch.float32, "memory")
@@ -2195,8 +2210,8 @@ def matrix_cell(qkv: torch.Tensor, gates: torch.Tensor, bias_i: torch.Tensor | N
     nq = torch.empty((n, heads), dtype=torch.float32, device=qkv.device)
     peaks = torch.empty((n, heads), dtype=torch.float32, device=qkv.device)
     _launches[0] += 1  # two kernels: the second one leaves the peak
-    if (chunks and not ctx.is_decode_only and qkv.dtype == torch.bfloat16 and dim % 8 == vdim % 8 == qkv.stride(0) % 8 == 0
-            and qkv.data_ptr() % 16 == 0 and cap > 0.0):
+    if (chunks and not ctx.is_decode_only and not only_short_portions(ctx) and qkv.dtype == torch.bfloat16
+            and dim % 8 == vdim % 8 == qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and cap > 0.0):
         _check(ops_library().ss_matrix_cell_chunks(
             qkv.data_ptr(), qkv.stride(0), gates.data_ptr(), gates.stride(0), _ptr(bias_i), _ptr(bias_f), float(cap), float(q_scale),
             memory.data_ptr(), peak.data_ptr(), num.data_ptr(), nq.data_ptr(), peaks.data_ptr(), ctx.q_start.data_ptr(),
@@ -2774,7 +2789,7 @@ def set_programmatic_launch(enabled: bool) -> None:
 
 __all__ = ["KernelError", "KernelBuildError", "embedding", "add_rmsnorm", "hc_norm", "linear_hc_rmsnorm", "rope_norm_cache", "glu_limited", "gate_up_glu", "sigmoid_gate", "key_span", "rope_and_cache", "swiglu",
            "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "few_prefill_keys", "paged_attention_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
-           "attention_library", "group_norm", "round_stream", "conv_silu", "ssm_scan", "router", "moe_experts", "moe_combine",
+           "attention_library", "group_norm", "round_stream", "conv_silu", "SCAN_FEW", "only_short_portions", "ssm_scan", "router", "moe_experts", "moe_combine",
            "norm_rope_cache", "turn_heads", "soft_cap", "embed_sum", "matrix_cell", "cell_output", "gated_recurrence", "xielu",
            "DiffPair", "diff_in_attention", "diff_combine", "heads_to_pages", "branch_norm", "PairedOutput", "WeighedTerms",
            "latent_rows", "head_product", "decay_attention", "gated_rmsnorm", "block_gates", "gated_linear_recurrence", "head_gate",

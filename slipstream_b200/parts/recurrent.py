@@ -45,6 +45,7 @@ import torch
 from slipstream_b200 import ops
 
 from .base import MIXERS, CacheSpec, IntoNorm, LayerBinding, Mixer, Part, PositionEncoding, Runtime, StateSpec, WeightSpec
+from .state_space import RecurrenceInChunks
 
 
 def _f32(t: torch.Tensor) -> torch.Tensor:
@@ -58,7 +59,7 @@ def _pad_rows(w: torch.Tensor, multiple: int = 8) -> torch.Tensor:
 
 
 @MIXERS.register("matrix_memory")
-class MatrixMemoryMixer(Mixer):
+class MatrixMemoryMixer(RecurrenceInChunks):
     cuda_graph_safe = True
     takes_into = True
     takes_pending_norm = False  # two products read the input

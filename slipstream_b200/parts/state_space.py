@@ -21,8 +21,23 @@ from slipstream_b200 import ops
 from .base import MIXERS, LayerBinding, Mixer, Runtime, StateSpec, WeightSpec
 
 
+class RecurrenceInChunks(Mixer):
+    """A mixer whose recurrence has a kernel for chunks of tokens and one for few tokens: what a captured step with prompt portions
+    is told (``ops.only_short_portions``), so that it runs the kernel that the step would run without the capture."""
+
+    def capture_variant(self, longest: int, plan: object = None) -> object:
+        return None if plan is None or plan.is_decode_only else bool(plan.q_lens.max() <= ops.SCAN_FEW)
+
+    def capture_group(self) -> object:
+        return ("recurrence_in_chunks",)
+
+    def prepare_capture(self, ctx, variant: object, max_model_len: int) -> None:
+        if not ctx.is_decode_only:
+            ctx.extras["short_portions"] = bool(variant)
+
+
 @MIXERS.register("state_space")
-class StateSpaceMixer(Mixer):
+class StateSpaceMixer(RecurrenceInChunks):
     cuda_graph_safe = True
 
     def __init__(self, name: str, hidden_size: int, heads: int, head_dim: int, state_dim: int, groups: int = 1,

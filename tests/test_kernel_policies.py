@@ -139,3 +139,22 @@ def test_gated_layers_of_the_mma_sync_kernel_are_captured_in_one_form(monkeypatc
     answers = [[layer.capture_variant(n, SimpleNamespace(is_decode_only=False, q_lens=np.array([30]), seq_lens=np.array([n])))
                 for n in (30, 300, 9000)] for layer in (gated, plain, paged_layer(64, gate=True))]
     assert answers[0] == [None] * 3 and answers[1][0] == 0 and len(set(answers[1])) == 3 and len(set(answers[2])) == 2
+
+
+def test_steps_of_short_portions_run_the_recurrences_token_by_token_captured_or_not():
+    from types import SimpleNamespace
+    from slipstream_b200.parts.recurrent import MatrixMemoryMixer
+    from slipstream_b200.parts.state_space import StateSpaceMixer
+
+    parts = [StateSpaceMixer("s", 64, 4, 16, 16), MatrixMemoryMixer("m", 64, 2, 16, 16, 15.0)]
+    assert parts[0].capture_group() == parts[1].capture_group()
+    for longest, short in ((2, True), (F.SCAN_FEW, True), (F.SCAN_FEW + 1, False), (700, False)):
+        plan = SimpleNamespace(is_decode_only=False, q_lens=np.array([1, longest]))
+        assert F.only_short_portions(SimpleNamespace(extras={}, max_q_len=longest)) == short
+        for part in parts:
+            # the static context of a captured step says 2 for every length
+            captured = SimpleNamespace(is_decode_only=False, extras={}, max_q_len=2, static_tiles=len)
+            assert not F.only_short_portions(captured)
+            part.prepare_capture(captured, part.capture_variant(longest, plan), 4096)
+            assert F.only_short_portions(captured) == short
+    assert parts[0].capture_variant(5) is None and parts[0].capture_variant(5, SimpleNamespace(is_decode_only=True)) is None

@@ -252,3 +252,44 @@ def test_state_space_scan_in_chunks_takes_more_requests_than_a_grid_is_high():
     got, want = (ops.ssm_scan(xbc, dt, *consts, s, ctx, 1, 1, 8, 8, chunks=c) for s, c in zip(states, (True, False)))
     assert off(got, want.double().cpu()) < TOLERANCE and off(states[0], states[1].double().cpu()) < TOLERANCE
     ops.check_errors(DEV)
+
+
+# decoded tokens and short portions, alone (a decode step, a step of short portions: the token-by-token kernels) and beside a long one
+@pytest.mark.parametrize("short", [[1, 1, 1], [8, 1, 3]])
+@pytest.mark.parametrize("heads, groups, p, n", [(4, 2, 64, 128), (3, 1, 8, 8), (2, 1, 40, 72), (3, 3, 128, 136), (2, 1, 32, 256), (2, 2, 72, 24)])
+def test_few_tokens_have_the_same_state_space_bits_beside_a_prompt_portion(heads, groups, p, n, short):
+    from slipstream_b200 import ops
+    torch.manual_seed(n)
+    lens = [short[0], short[1], 90, short[2]]
+    rows = torch.cat([torch.arange(short[0] + short[1]), torch.arange(sum(lens) - short[2], sum(lens))]).to(DEV)
+    xbc, dt = torch.randn(sum(lens), heads * p + 2 * groups * n, device=DEV).bfloat16(), torch.randn(sum(lens), heads + 1, device=DEV).bfloat16()[:, 1:]
+    consts, start = [torch.randn(heads, device=DEV) * 0.5 for _ in range(3)], torch.randn(4, heads, p, n, device=DEV)
+    alone_ctx, mixed = step_ctx(short, [0, 1, 3]), step_ctx(lens, range(4))
+    alone_ctx.is_decode_only, alone_ctx.max_q_len = max(short) == 1, max(short)
+    states = [start.clone(), start.clone()]
+    alone = ops.ssm_scan(xbc[rows], dt[rows], *consts, states[0], alone_ctx, heads, groups, p, n)
+    beside = ops.ssm_scan(xbc, dt, *consts, states[1], mixed, heads, groups, p, n)
+    assert torch.equal(alone, beside[rows]) and torch.equal(states[0][[0, 1, 3]], states[1][[0, 1, 3]])
+    ops.check_errors(DEV)
+
+
+@pytest.mark.parametrize("short", [[1, 1, 1], [8, 1, 3]])
+@pytest.mark.parametrize("heads, dim, vdim", [(3, 128, 128), (2, 8, 8), (2, 64, 72), (3, 96, 64), (2, 256, 40), (1, 136, 200)])
+def test_few_tokens_have_the_same_matrix_memory_bits_beside_a_prompt_portion(heads, dim, vdim, short):
+    from slipstream_b200 import ops
+    torch.manual_seed(dim)
+    lens = [short[0], short[1], 90, short[2]]
+    rows = torch.cat([torch.arange(short[0] + short[1]), torch.arange(sum(lens) - short[2], sum(lens))]).to(DEV)
+    qkv, gates = torch.randn(sum(lens), heads * (2 * dim + vdim), device=DEV).bfloat16(), torch.randn(sum(lens), 2 * heads, device=DEV) * 3
+    bias_i, bias_f = torch.randn(heads, device=DEV), torch.randn(heads, device=DEV) + 2
+    start = torch.randn(4, heads, vdim + 1, dim, device=DEV), torch.randn(4, heads, device=DEV)
+    alone_ctx, mixed = step_ctx(short, [0, 1, 3]), step_ctx(lens, range(4))
+    alone_ctx.is_decode_only, alone_ctx.max_q_len = max(short) == 1, max(short)
+    states = [[s.clone() for s in start] for _ in range(2)]
+    alone = ops.matrix_cell(qkv[rows], gates[rows], bias_i, bias_f, 6.0, dim ** -0.5, *states[0], alone_ctx, heads, dim, vdim)
+    beside = ops.matrix_cell(qkv, gates, bias_i, bias_f, 6.0, dim ** -0.5, *states[1], mixed, heads, dim, vdim)
+    for a, b in zip(alone, beside):
+        assert torch.equal(a, b[rows])
+    for a, b in zip(*states):
+        assert torch.equal(a[[0, 1, 3]], b[[0, 1, 3]])
+    ops.check_errors(DEV)

@@ -390,7 +390,7 @@ struct SampleBins {
     uint32_t parts[3][SAMPLE_BINS];         // a block's histogram: counts, or 14 bits of the mass each (see SAMPLE_SHARE)
     unsigned long long own[SAMPLE_BINS];    // the same added up
     unsigned long long sums[SAMPLE_THREADS / 32];
-    unsigned long long before;              // where the threshold falls: what lies in the bins in front of its bin
+    unsigned long long before, inside;      // where the threshold falls: what lies in the bins in front of its bin, and in it
     int bin;
 };
 struct SampleGathered {
@@ -433,16 +433,29 @@ __device__ __forceinline__ float2 cluster_range(float hi, float lo, SampleShared
 
 #define SAMPLE_FIX 1099511627776.0f  // 2^40: exp() in (0, 1] as fixed point
 
+__device__ __forceinline__ int sample_bin(float v, float vmax, float scale) {
+    return (int)fminf((vmax - v) * scale, (float)(SAMPLE_BINS - 1));
+}
+
+// What draw_fast found of a row before it gave it up for the length of its lists: the bin of the threshold, and how much of the
+// target (a count, or a mass without top-k) lies in front of it.
+struct SampleKnown {
+    bool is;
+    int bin;
+    float scale, vmax;
+    unsigned long long base, target;
+};
+
 // The draw of a row under top-k or top-p in three passes.  (1) the largest and the smallest value; (2) a histogram over
 // the distance from the largest: a larger value never falls into a later bin, so the bin in which the k-th value stands, or in
 // which the mass reaches top_p, holds the threshold; (3) values in front of that bin race, those in it are listed (under both
 // filters all of them are listed), and block 0 decides value by value which of the list stay: a value stays while what is
 // larger than it counts less than k, or holds less than top_p of the mass.  Returns false where a step does not work
-// out; nothing has been decided then.  Bound by issue (an exponential and up to three shared-memory additions a value) and the
+// out; nothing has been decided then, but `known` says where the threshold falls if it got so far.  Bound by issue (an exponential and up to three shared-memory additions a value) and the
 // pass's way to L2.  64 rows of 152,064 logits, against radix selection with a histogram a digit (four passes for top-k, five
 // for top-p, each forming the values anew): top-k 40 221 -> 77 us, top-p 0.8 272 -> 87, both 349 -> 60.
 __device__ __forceinline__ bool draw_fast(const SampleRow& t, int k, float tp, float mp, uint64_t seed, uint64_t draw, SampleShared& sh,
-                                          SampleFast& fast, ArgMax& best) {
+                                          SampleFast& fast, SampleKnown& known, ArgMax& best) {
     const int tid = threadIdx.x;
     const uint32_t n_blocks = cluster_size(), rank = cluster_rank();
     // (a vocabulary of more than 262,144 and a block to a row, say)
@@ -460,7 +473,7 @@ __device__ __forceinline__ bool draw_fast(const SampleRow& t, int k, float tp, f
     const float vmax = range.x;
     if (!(fabsf(vmax) < INFINITY) || !(range.x - range.y < INFINITY)) return false;
     const float scale = range.x > range.y ? (float)SAMPLE_BINS / fminf(range.x - range.y, 32.f) : 1.f;
-    auto bin_of = [&](float v) { return (int)fminf((vmax - v) * scale, (float)(SAMPLE_BINS - 1)); };
+    auto bin_of = [&](float v) { return sample_bin(v, vmax, scale); };
     const bool counting = k > 0, list_all = counting && tp < 1.0f;  // top-p among the top k needs all of them
 
     SampleBins& b = fast.bins;
@@ -525,14 +538,19 @@ __device__ __forceinline__ bool draw_fast(const SampleRow& t, int k, float tp, f
 #pragma unroll
     for (int u = 0; u < MOST; ++u) {
         if (u >= per) break;
-        const bool first_of_all = tid == 0 && u == 0;
-        if ((before < target || (first_of_all && target == 0ull)) && before + mine[u] >= target) { b.bin = tid * per + u; b.before = before; }
+        if (before < target && before + mine[u] >= target) { b.bin = tid * per + u; b.before = before; b.inside = mine[u]; }
         before += mine[u];
     }
     __syncthreads();
     const int bin = b.bin;
     const unsigned long long base = b.before;
     if (bin < 0) return false;  // (the same in every block)
+    known = SampleKnown{false, bin, scale, vmax, base, target};
+    // (a mass does not tell of how many values it is)
+    if (counting && (list_all ? base + b.inside : b.inside) > (unsigned long long)min(SAMPLE_GATHERED, (int)n_blocks * SAMPLE_LIST)) {
+        known.is = true;
+        return false;
+    }
 
     const float floor_val = mp > 0.0f ? vmax + logf(mp) : -INFINITY;  // min-p: exp(x - x_max) >= min_p
     ArgMax a{-INFINITY, 0x7fffffff};
@@ -572,6 +590,7 @@ __device__ __forceinline__ bool draw_fast(const SampleRow& t, int k, float tp, f
     if (!fits) {
         if (n_blocks > 1) cluster_sync_all();  // sh.word may be written again
         __syncthreads();
+        known.is = true;
         return false;
     }
     if (rank == 0) {
@@ -632,6 +651,154 @@ __device__ __forceinline__ bool draw_fast(const SampleRow& t, int k, float tp, f
     return true;
 }
 
+// The keys between which a threshold lies, and the leading bytes that they share, which need no radix step.
+struct KeyRange {
+    uint32_t hi, lo;
+};
+struct RadixStart {
+    uint32_t prefix, mask;
+    int shift;
+};
+__device__ __forceinline__ RadixStart radix_start(KeyRange a) {
+    const int same = a.lo == a.hi ? 4 : __clz(a.lo ^ a.hi) >> 3;
+    const uint32_t mask = same == 0 ? 0u : 0xffffffffu << (32 - 8 * same);
+    return RadixStart{a.lo & mask, mask, 24 - 8 * same};
+}
+
+// The largest and the smallest key over all threads of all blocks of the cluster.
+__device__ __forceinline__ KeyRange cluster_key_range(KeyRange a, SampleShared& sh) {
+    const int tid = threadIdx.x;
+    a.hi = __reduce_max_sync(0xffffffffu, a.hi);
+    a.lo = __reduce_min_sync(0xffffffffu, a.lo);
+    __syncthreads();
+    if ((tid & 31) == 0) sh.total[tid >> 5] = ((unsigned long long)a.hi << 32) | a.lo;
+    __syncthreads();
+    const uint32_t n = cluster_size();
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+        a.hi = max(a.hi, (uint32_t)(sh.total[w] >> 32));
+        a.lo = min(a.lo, (uint32_t)sh.total[w]);
+    }
+    if (n > 1) {
+        if (tid == 0) sh.word = ((unsigned long long)a.hi << 32) | a.lo;
+        cluster_sync_all();
+        for (uint32_t c = 0; c < n; ++c) {
+            const unsigned long long w = ld_cluster_u64(&sh.word, c);
+            a.hi = max(a.hi, (uint32_t)(w >> 32));
+            a.lo = min(a.lo, (uint32_t)w);
+        }
+        cluster_sync_all();
+    }
+    __syncthreads();
+    return a;
+}
+
+// The thresholds of top-k and top-p by radix selection: the smallest key that stays, and the largest value where it is wanted.  Where `known` has
+// the bin, a pass finds the keys between which its values lie (and whether top-k removes anything that can be drawn), and the
+// selection goes on among them: values that share their leading bytes, or are one value, need fewer steps or none.  A
+// function of its own, not in the way of the rows that do without it.
+struct SampleFloor {
+    uint32_t key;
+    float vmax;
+};
+__device__ __noinline__ SampleFloor radix_floor(const SampleRow t, int k, float tp, bool wants_max, const SampleKnown known,
+                                                unsigned long long* warp_hists, SampleShared& sh) {
+    const float *row = t.row, pen = t.penalty, temp = t.temperature;
+    const uint32_t* seen = t.seen;
+    const int vocab = t.vocab, first = t.first, step = t.step, tid = threadIdx.x, n_warps = blockDim.x >> 5;
+    unsigned long long* my_hist = warp_hists + (tid >> 5) * 256;
+    uint32_t floor_key = 0;
+    KeyRange within{0xffffffffu, 0u};
+    const bool counted = k > 0;  // (what is known is a count)
+    float vmax = known.vmax;
+    if (known.is) {
+        uint32_t hi = 0u, lo = 0xffffffffu, values = 0u;
+        for_groups(t, [&](int, const float (&v)[4], int live) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (e >= live || v[e] == -INFINITY) continue;
+                ++values;
+                if (sample_bin(v[e], known.vmax, known.scale) != known.bin) continue;
+                hi = max(hi, order_key(v[e]));
+                lo = min(lo, order_key(v[e]));
+            }
+        });
+        within = cluster_key_range(KeyRange{hi, lo}, sh);
+        if (counted && cluster_sum((unsigned long long)values, sh) <= (unsigned long long)k) k = 0;
+    }
+
+    // ---- top-k: key of the k-th largest value
+    if (k > 0) {
+        const RadixStart from = radix_start(within);
+        uint32_t prefix = from.prefix, mask = from.mask;
+        unsigned long long want = (unsigned long long)k - (known.is ? known.base : 0ull);  // rank still to find inside the prefix
+        for (int shift = from.shift; shift >= 0; shift -= 8) {
+            for (int b = tid; b < n_warps * 256; b += blockDim.x) warp_hists[b] = 0ull;
+            __syncthreads();
+            BinRun run{0, 0ull};
+            for (int i = first; i < vocab; i += step) {
+                const uint32_t key = order_key(tempered(row, i, seen, pen, temp));
+                if ((key & mask) == prefix && key >= within.lo && key <= within.hi) run_add(run, my_hist, (int)((key >> shift) & 255u), 1ull);
+            }
+            run_flush(run, my_hist);
+            select_bin(sh, warp_hists, n_warps, 0ull, want);
+            prefix |= sh.pick_digit << shift;
+            mask |= 255u << shift;
+            want -= sh.pick_above;
+            __syncthreads();
+        }
+        floor_key = prefix;
+    }
+
+    // ---- maximum of what is left (needed by top-p and min-p)
+    if (wants_max && !known.is) {
+        ArgMax a{-INFINITY, 0x7fffffff};
+        for (int i = first; i < vocab; i += step) {
+            const float v = tempered(row, i, seen, pen, temp);
+            if (order_key(v) >= floor_key) a = better(a, ArgMax{v, i});
+        }
+        vmax = cluster_argmax(a, sh).v;
+    }
+
+    // ---- top-p: keep a token iff the mass of strictly larger values is below top_p
+    if (tp < 1.0f) {
+        unsigned long long limit = known.target, above = known.base;  // above: mass of values whose key exceeds every key under the prefix
+        if (!known.is || counted) {
+            unsigned long long local = 0;  // total mass
+            for (int i = first; i < vocab; i += step) {
+                const float v = tempered(row, i, seen, pen, temp);
+                if (order_key(v) >= floor_key) local += (unsigned long long)(expf(v - vmax) * SAMPLE_FIX);
+            }
+            const unsigned long long total = cluster_sum(local, sh);
+            limit = (unsigned long long)((double)tp * (double)total);
+            above = 0ull;
+            within = KeyRange{0xffffffffu, floor_key};
+        }
+        __syncthreads();
+        const RadixStart from = radix_start(within);
+        uint32_t prefix = from.prefix, mask = from.mask;
+        for (int shift = from.shift; shift >= 0; shift -= 8) {
+            for (int b = tid; b < n_warps * 256; b += blockDim.x) warp_hists[b] = 0ull;
+            __syncthreads();
+            BinRun run{0, 0ull};
+            for (int i = first; i < vocab; i += step) {
+                const float v = tempered(row, i, seen, pen, temp);
+                const uint32_t key = order_key(v);
+                if (key >= within.lo && key <= within.hi && (key & mask) == prefix)
+                    run_add(run, my_hist, (int)((key >> shift) & 255u), (unsigned long long)(expf(v - vmax) * SAMPLE_FIX));
+            }
+            run_flush(run, my_hist);
+            // lowest digit whose bin still starts below the limit
+            select_bin(sh, warp_hists, n_warps, above, limit);
+            prefix |= sh.pick_digit << shift;
+            mask |= 255u << shift;
+            above = sh.pick_above;
+            __syncthreads();
+        }
+        if (prefix > floor_key) floor_key = prefix;
+    }
+    return SampleFloor{floor_key, vmax};
+}
+
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* __restrict__ logits, int64_t stride, int32_t* __restrict__ out,
               const float* __restrict__ temperature, const int32_t* __restrict__ top_k,
@@ -648,9 +815,8 @@ sample_kernel(const float* __restrict__ logits, int64_t stride, int32_t* __restr
     SampleFast& fast = *reinterpret_cast<SampleFast*>(warp_hists);
     // the blocks of a cluster share a row; block c of n takes elements (or groups of four) c * blockDim + tid, + n * blockDim, ...
     const int n_blocks = (int)cluster_size(), rank = (int)cluster_rank();
-    const int r = blockIdx.x / n_blocks, tid = threadIdx.x, warp = tid >> 5, n_warps = blockDim.x >> 5;
+    const int r = blockIdx.x / n_blocks, tid = threadIdx.x;
     const int first = rank * blockDim.x + tid, step = n_blocks * blockDim.x;
-    unsigned long long* my_hist = warp_hists + warp * 256;
     const float* row = logits + (int64_t)r * stride;
     const float temp = temperature[r];
     uint32_t* seen_row = (seen_all && slots && slots[r] >= 0) ? seen_all + (int64_t)slots[r] * seen_words : nullptr;
@@ -680,10 +846,11 @@ sample_kernel(const float* __restrict__ logits, int64_t stride, int32_t* __restr
     const int k = top_k[r] > 0 && top_k[r] < vocab ? top_k[r] : 0;
     const float tp = top_p[r], mp = min_p[r];
     const uint64_t seed = (uint64_t)seeds[r], draw = (uint64_t)draws[r];
+    SampleKnown known{false, 0, 0.f, -INFINITY, 0ull, 0ull};
     if (k > 0 || tp < 1.0f) {
         const SampleRow t{row, seen, pen, temp, vocab, first, step, (reinterpret_cast<uintptr_t>(row) & 15) == 0};
         ArgMax a;
-        if ((k <= SAMPLE_GATHERED / 2 || tp >= 1.0f) && draw_fast(t, k, tp, mp, seed, draw, sh, fast, a)) {
+        if ((k <= SAMPLE_GATHERED / 2 || tp >= 1.0f) && draw_fast(t, k, tp, mp, seed, draw, sh, fast, known, a)) {
             a = cluster_argmax(a, sh);
             if (tid == 0 && rank == 0) {
                 const int tok = a.i == 0x7fffffff ? 0 : a.i;
@@ -694,92 +861,26 @@ sample_kernel(const float* __restrict__ logits, int64_t stride, int32_t* __restr
         }
         __syncthreads();
     }
-    uint32_t floor_key = 0;  // tokens with order_key(value) < floor_key are removed
-
-    // ---- top-k: key of the k-th largest value
-    if (k > 0) {
-        uint32_t prefix = 0, mask = 0;
-        unsigned long long want = (unsigned long long)k;  // rank still to find inside the prefix
-        for (int shift = 24; shift >= 0; shift -= 8) {
-            for (int b = tid; b < n_warps * 256; b += blockDim.x) warp_hists[b] = 0ull;
-            __syncthreads();
-            BinRun run{0, 0ull};
-            for (int i = first; i < vocab; i += step) {
-                const uint32_t key = order_key(tempered(row, i, seen, pen, temp));
-                if ((key & mask) == prefix) run_add(run, my_hist, (int)((key >> shift) & 255u), 1ull);
-            }
-            run_flush(run, my_hist);
-            select_bin(sh, warp_hists, n_warps, 0ull, want);
-            prefix |= sh.pick_digit << shift;
-            mask |= 255u << shift;
-            want -= sh.pick_above;
-            __syncthreads();
-        }
-        floor_key = prefix;
-    }
-
-    // ---- maximum of what is left (needed by top-p and min-p)
-    float vmax = -INFINITY;
-    if (tp < 1.0f || mp > 0.0f) {
-        ArgMax a{-INFINITY, 0x7fffffff};
-        for (int i = first; i < vocab; i += step) {
-            const float v = tempered(row, i, seen, pen, temp);
-            if (order_key(v) >= floor_key) a = better(a, ArgMax{v, i});
-        }
-        vmax = cluster_argmax(a, sh).v;
-    }
-
-    // ---- top-p: keep a token iff the mass of strictly larger values is below top_p
-    if (tp < 1.0f) {
-        // total mass
-        unsigned long long local = 0;
-        for (int i = first; i < vocab; i += step) {
-            const float v = tempered(row, i, seen, pen, temp);
-            if (order_key(v) >= floor_key) local += (unsigned long long)(expf(v - vmax) * SAMPLE_FIX);
-        }
-        const unsigned long long total = cluster_sum(local, sh);
-        const unsigned long long limit = (unsigned long long)((double)tp * (double)total);
-        __syncthreads();
-        uint32_t prefix = 0, mask = 0;
-        unsigned long long above = 0;  // mass of values whose key exceeds every key under the prefix
-        for (int shift = 24; shift >= 0; shift -= 8) {
-            for (int b = tid; b < n_warps * 256; b += blockDim.x) warp_hists[b] = 0ull;
-            __syncthreads();
-            BinRun run{0, 0ull};
-            for (int i = first; i < vocab; i += step) {
-                const float v = tempered(row, i, seen, pen, temp);
-                const uint32_t key = order_key(v);
-                if (key >= floor_key && (key & mask) == prefix)
-                    run_add(run, my_hist, (int)((key >> shift) & 255u), (unsigned long long)(expf(v - vmax) * SAMPLE_FIX));
-            }
-            run_flush(run, my_hist);
-            // lowest digit whose bin still starts below the limit
-            select_bin(sh, warp_hists, n_warps, above, limit);
-            prefix |= sh.pick_digit << shift;
-            mask |= 255u << shift;
-            above = sh.pick_above;
-            __syncthreads();
-        }
-        if (prefix > floor_key) floor_key = prefix;
-    }
+    const SampleRow t{row, seen, pen, temp, vocab, first, step, (reinterpret_cast<uintptr_t>(row) & 15) == 0};
+    SampleFloor least{0u, -INFINITY};  // tokens with order_key(value) < least.key are removed
+    if (k > 0 || tp < 1.0f || mp > 0.0f) least = radix_floor(t, k, tp, tp < 1.0f || mp > 0.0f, known, warp_hists, sh);
 
     // ---- min-p: p_i / p_max = exp(x_i - x_max) >= min_p
     float floor_val = -INFINITY;
-    if (mp > 0.0f) floor_val = vmax + logf(mp);
+    if (mp > 0.0f) floor_val = least.vmax + logf(mp);
 
     // ---- Gumbel-max draw over what is left: one Philox call gives the noise of four consecutive tokens
-    const SampleRow t{row, seen, pen, temp, vocab, first, step, (reinterpret_cast<uintptr_t>(row) & 15) == 0};
     ArgMax a{-INFINITY, 0x7fffffff};
     for_groups(t, [&](int i, const float (&v)[4], int live) {
         bool races = false;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) races |= e < live && order_key(v[e]) >= floor_key && v[e] >= floor_val;
+        for (int e = 0; e < 4; ++e) races |= e < live && order_key(v[e]) >= least.key && v[e] >= floor_val;
         if (!races) return;
         uint32_t c[4];
         group_noise(seed, draw, i, c);
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-            if (e < live && order_key(v[e]) >= floor_key && v[e] >= floor_val) race(a, v[e], i + e, c, sh);
+            if (e < live && order_key(v[e]) >= least.key && v[e] >= floor_val) race(a, v[e], i + e, c, sh);
     });
     a = cluster_argmax(a, sh);
     if (tid == 0 && rank == 0) {

@@ -262,3 +262,27 @@ def test_top_p_over_more_values_than_a_block_adds_up_in_32_bits():
         kept = plain.filtered_logits(torch.from_numpy(values), temperature=1.0, top_k=-1, top_p=0.75, min_p=0.0).numpy()
         assert int((kept + gumbel_noise(11, draw, values.size)).argmax()) == token
         assert run_sample(logits[:1], [ask]) == [token] and run_sample(logits, [ask] * rows) == [token] * rows
+
+
+# rows whose threshold falls among more values than the lists hold: radix selection goes on inside the bin, with the bytes that its
+# values share known; rows with fewer values than top-k keeps
+@pytest.mark.parametrize("m", [1, 20, 150])
+@pytest.mark.parametrize("kind", ["equal", "whole", "close", "signs", "few", "steps"])
+def test_sampling_goes_on_by_radix_selection_inside_the_thresholds_bin(m, kind):
+    g = torch.Generator().manual_seed(m)
+    vocab = 30011
+    x = torch.randn(m, vocab, generator=g)
+    logits = {"equal": torch.full_like(x, -1.5), "whole": (2 * x).round(), "close": 1 + 1e-6 * x, "steps": (x * 40).round() / 40,
+              "signs": torch.where(x > 0, 0.0, -0.0) + torch.where(x < -1, -1.0, 0.0),
+              "few": torch.where(torch.arange(vocab) % 1000 == 7, x, -float("inf"))}[kind]
+    asks = [dict(top_k=40), dict(top_p=0.8), dict(top_k=40, top_p=0.8), dict(top_k=9000), dict(top_k=9000, top_p=0.5), dict(top_k=1500, top_p=0.5, min_p=0.3)]
+    rows = [dict(temperature=1.0, seed=i, draw=i % 5, **asks[i % 6 if kind != "signs" else i % 2 * 3]) for i in range(m)]
+    got = run_sample(logits.to(DEV), rows)
+    for i, r in enumerate(rows):
+        values = logits[i].double()
+        values[(values == 0) & values.signbit()] = -1e-30  # -0 stands below 0
+        kept = plain.filtered_logits(values, temperature=1.0, top_k=r.get("top_k", -1), top_p=r.get("top_p", 1.0), min_p=r.get("min_p", 0.0))
+        kept = np.where(values >= kept[torch.isfinite(kept)].min(), values, -np.inf)  # ties stay
+        score = kept + gumbel_noise(r["seed"], r["draw"], vocab)
+        assert np.isfinite(kept[got[i]]) and score[got[i]] >= score.max() - 1e-4, (i, r, got[i])
+    ops().check_errors(torch.device(DEV))

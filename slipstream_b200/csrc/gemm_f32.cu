@@ -23,7 +23,9 @@
 //   * many tokens: BN = 128 or 64, a chunk's two accumulators double-buffered in tensor memory.
 //   * up to 64 tokens: BN = 16, 32 or 64; K's chunks are spread over the up to 8 blocks of a cluster, each chunk keeps
 //     its own columns of tensor memory, and the blocks add all chunks of their token columns out of one another's shared
-//     memory.  The weights' first loads run ahead of the wait for the kernel in front.
+//     memory.
+// Nothing is read before the wait for the kernels in front, since a weight may be a result of theirs (the first weights ahead of it
+// saved 4 us of a 1.5B layer's decode step, 97 and 101).
 //
 // Why tensor cores: 128 float32 lanes an SM make 74 TFLOP/s at best (the CUDA-core kernel reached 22); six bfloat16
 // products at the measured 1,660 TFLOP/s make 277.  777 tokens at the 7B sizes, before and after (us): q/k/v 1,191 and
@@ -172,17 +174,15 @@ __global__ void __launch_bounds__(F3_THREADS, 1) gemm_f32_kernel(const F32Args g
             for (int p = 0; p < 3; ++p)
                 *reinterpret_cast<uint2*>(dst + p * plane) = make_uint2(f3_part(v.x, v.y), f3_part(v.z, v.w));
         };
+        pdl_wait();  // (for the weights, too: a caller may have formed them a kernel ago)
         if constexpr (FEW) {  // a group of copies a step, empty ones behind the last
-            // the weights before the wait for the kernel in front, X behind it: the first group of X covers all of them
-            for (int u = 0; u < min(AHEAD, steps); ++u) load_w(step0 + u);
-            pdl_wait();
             for (int u = 0; u < AHEAD; ++u) {
+                if (u < steps) load_w(step0 + u);
                 if (X_STAGED && u < steps) load_x(step0 + u);
                 cp_async_commit();
             }
         } else {
             if (steps > 0) load_w(step0);
-            pdl_wait();
         }
         if (!X_STAGED && steps > 0) load_x(step0);
         for (int it = 0; it < steps; ++it) {

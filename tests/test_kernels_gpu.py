@@ -190,6 +190,21 @@ def test_float32_product_passes_infinities_and_nan_on_as_cuda_cores_do():
     ops().check_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("m", [3, 40, 200])
+def test_float32_product_waits_for_weights_that_the_kernel_in_front_forms(m):
+    torch.manual_seed(m)
+    a, b, x = torch.randn(2048, 3584, device=DEV), torch.randn(1024, 3584, device=DEV), torch.randn(m, 1024, device=DEV)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        old = torch.full((2048, 1024), float("nan"), device=DEV)  # what the weights' memory holds before
+        del old
+        w = ops().gemm_float32(a, b)
+        got = ops().gemm_float32(x, w)
+        torch.cuda.synchronize()
+        assert torch.equal(got, ops().gemm_float32(x, w)) and torch.isfinite(got).all()
+    ops().check_errors(torch.device(DEV))
+
+
 def test_float32_product_without_16_byte_rows_takes_the_cuda_cores():
     x, w = torch.randn(5, 70, device=DEV), torch.randn(33, 70, device=DEV)
     assert torch.equal(ops().gemm_float32(x, w), ops().gemm_simt(x, w))

@@ -704,9 +704,11 @@ FLOAT32_SCRATCH = 128 << 20  # bytes of slices that a call may leave in scratch 
 
 
 def float32_key_parts(blocks: int, slices: int, rows: int, heads: int, head_dim: int, sms: int | None = None) -> int:
-    """Blocks that share the ``slices`` slices of a row's keys in the float32 kernel where ``blocks`` would walk all of
-    theirs: as many as make two blocks an SM, the most that do not wait for one another.  The slices then go through
-    scratch memory, which is bounded.  Only the time depends on it: a row's slices are joined in the same order."""
+    """Blocks that share the ``slices`` slices of a row's keys in the float32 kernel.  ``blocks``: the tiles of a step (of 64
+    rows with prompt portions, which two blocks of 32 rows take; of 16 in a decode step) times the heads; as many shares as make two
+    of them an SM, so up to four blocks where three run at a time (us for 64 tokens behind 2,000, 28 heads of 128 on 4: 161, and 183
+    with half the shares; 200 behind 1,500, 12 on 2: 140 and 174).  The slices then go through scratch memory, which is
+    bounded.  Only the time depends on it: a row's slices are joined in the same order."""
     parts = min(slices, 2 * (sms or sm_count()) // max(blocks, 1))
     return parts if parts > 1 and rows * heads * slices * (head_dim + 2) * 4 <= FLOAT32_SCRATCH else 1
 
@@ -716,7 +718,8 @@ def paged_attention_float32(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tens
                             gate: torch.Tensor | None = None, softcap: float = 0.0, sinks: torch.Tensor | None = None,
                             keep: int = 0, across: bool = False) -> None:
     """`paged_attention_simt` for the rows of a step in float32, with the arguments of `paged_attention`: the kernel that
-    tiles 64 rows of a kv head's group with 32 keys and splits a row's keys over several blocks where there are few rows."""
+    tiles rows of a kv head's group (32 of a prompt portion, whose list has tiles of 64; 16 of a decode step) with 32 keys and splits
+    a row's keys over several blocks where there are few rows."""
     _need(out, torch.float32, "attention output")
     _check_sinks(sinks, n_q)
     _need(kv, torch.float32, "kv pages")

@@ -71,6 +71,7 @@ class MatrixMemoryMixer(RecurrenceInChunks):
             raise ValueError("heads and value_dim must be >= 1, dim between 1 and 256, gate_cap positive")
         self.name, self.hidden_size = name, hidden_size
         self.heads, self.dim, self.value_dim = heads, dim, value_dim
+        self.chunk_sizes = (dim, value_dim)
         self.gate_cap, self.norm_eps = float(gate_cap), float(norm_eps)
         self.names = {role: f"{name}.{role}" for role in ("q", "k", "v", "g", "o", "norm", "i", "f")}
         self.names.update({"i_bias": f"{name}.i.b", "f_bias": f"{name}.f.b"})

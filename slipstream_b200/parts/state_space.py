@@ -25,14 +25,22 @@ class RecurrenceInChunks(Mixer):
     """A mixer whose recurrence has a kernel for chunks of tokens and one for few tokens: what a captured step with prompt portions
     is told (``ops.only_short_portions``), so that it runs the kernel that the step would run without the capture."""
 
+    chunk_sizes: tuple[int, ...] = ()  # what the kernel for chunks takes in steps of 8
+
+    @property
+    def takes_chunks(self) -> bool:
+        return self.runtime.dtype == torch.bfloat16 and all(n % 8 == 0 for n in self.chunk_sizes)
+
     def capture_variant(self, longest: int, plan: object = None) -> object:
-        return None if plan is None or plan.is_decode_only else bool(plan.q_lens.max() <= ops.SCAN_FEW)
+        if plan is None or plan.is_decode_only or not self.takes_chunks:
+            return None  # one kernel, one form
+        return bool(plan.q_lens.max() <= ops.SCAN_FEW)
 
     def capture_group(self) -> object:
-        return ("recurrence_in_chunks",)
+        return ("recurrence_in_chunks", self.takes_chunks)
 
     def prepare_capture(self, ctx, variant: object, max_model_len: int) -> None:
-        if not ctx.is_decode_only:
+        if not ctx.is_decode_only and variant is not None:
             ctx.extras["short_portions"] = bool(variant)
 
 
@@ -56,6 +64,7 @@ class StateSpaceMixer(RecurrenceInChunks):
         self.inner = heads * head_dim
         self.channels = self.inner + 2 * groups * state_dim  # what the convolution runs over: x, B, C
         self.proj_width = 2 * self.inner + 2 * groups * state_dim + heads
+        self.chunk_sizes = (head_dim, state_dim)
         n = name
         self.names = {"in": f"{n}.in_proj.weight", "conv": f"{n}.conv1d.weight", "conv_bias": f"{n}.conv1d.bias",
                       "dt_bias": f"{n}.dt_bias", "a_log": f"{n}.A_log", "d": f"{n}.D", "norm": f"{n}.norm.weight",

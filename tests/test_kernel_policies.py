@@ -143,10 +143,13 @@ def test_gated_layers_of_the_mma_sync_kernel_are_captured_in_one_form(monkeypatc
 
 def test_steps_of_short_portions_run_the_recurrences_token_by_token_captured_or_not():
     from types import SimpleNamespace
+    import torch
     from slipstream_b200.parts.recurrent import MatrixMemoryMixer
     from slipstream_b200.parts.state_space import StateSpaceMixer
 
     parts = [StateSpaceMixer("s", 64, 4, 16, 16), MatrixMemoryMixer("m", 64, 2, 16, 16, 15.0)]
+    for part in parts:
+        part.runtime = SimpleNamespace(dtype=torch.bfloat16)
     assert parts[0].capture_group() == parts[1].capture_group()
     for longest, short in ((2, True), (F.SCAN_FEW, True), (F.SCAN_FEW + 1, False), (700, False)):
         plan = SimpleNamespace(is_decode_only=False, q_lens=np.array([1, longest]))
@@ -158,3 +161,23 @@ def test_steps_of_short_portions_run_the_recurrences_token_by_token_captured_or_
             part.prepare_capture(captured, part.capture_variant(longest, plan), 4096)
             assert F.only_short_portions(captured) == short
     assert parts[0].capture_variant(5) is None and parts[0].capture_variant(5, SimpleNamespace(is_decode_only=True)) is None
+
+
+def test_recurrences_without_a_kernel_for_chunks_are_captured_in_one_form():
+    from types import SimpleNamespace
+    import torch
+    from slipstream_b200.parts.recurrent import MatrixMemoryMixer
+    from slipstream_b200.parts.state_space import StateSpaceMixer
+
+    chunked = StateSpaceMixer("s", 64, 4, 16, 16)
+    chunked.runtime = SimpleNamespace(dtype=torch.bfloat16)
+    for part, dtype in ((StateSpaceMixer("s", 64, 4, 16, 16), torch.float32), (StateSpaceMixer("s", 64, 4, 12, 16), torch.bfloat16),
+                        (MatrixMemoryMixer("m", 64, 2, 16, 20, 15.0), torch.bfloat16)):
+        part.runtime = SimpleNamespace(dtype=dtype)
+        assert part.capture_group() != chunked.capture_group()
+        captured = SimpleNamespace(is_decode_only=False, extras={"short_portions": True})
+        for longest in (3, 300):
+            variant = part.capture_variant(longest, SimpleNamespace(is_decode_only=False, q_lens=np.array([longest])))
+            assert variant is None
+            part.prepare_capture(captured, variant, 4096)
+        assert captured.extras == {"short_portions": True}

@@ -120,17 +120,25 @@ class LatentAttention(Mixer):
         n = sum(t.numel() for t in (self.in_weight, self.uq_weight, self.to_latent, self.to_value, self.o_weight))
         return n * self.o_weight.element_size()
 
+    @property
+    def on_tcgen05(self) -> bool:
+        """Whether prompt portions may run the tcgen05 kernel."""
+        return self.runtime.dtype == torch.bfloat16 and ops.tcgen05_prefill_fits(self.row, self.heads, 1, self.page_size or 16)
+
     def capture_variant(self, longest: int, plan: object = None) -> object:
-        # one form of the decode kernel, however long the contexts; steps with prompt portions: whether few keys keep the
-        # mma.sync kernel
-        return None if plan is None or plan.is_decode_only else bool(ops.few_prefill_keys(self.row, longest))
+        # one form of the decode kernel, however long the contexts; steps with prompt portions, where the tcgen05 kernel takes the
+        # rows at all: whether few keys keep the mma.sync kernel
+        if plan is None or plan.is_decode_only or not self.on_tcgen05:
+            return None
+        return bool(ops.few_prefill_keys(self.row, longest))
 
     def capture_group(self) -> object:
-        return ("latent_attention", self.row)
+        return ("latent_attention", self.row, self.on_tcgen05)
 
     def prepare_capture(self, ctx, variant: object, max_model_len: int) -> None:
         if not ctx.is_decode_only:
-            ctx.extras[("few_keys", self.row)] = bool(variant)
+            if variant is not None:
+                ctx.extras[("few_keys", self.row)] = bool(variant)
             return
         ctx.extras["static_max_seq_len"] = max_model_len  # the number of slices must not follow the captured step
         ctx.extras.setdefault("decode_wide", False)

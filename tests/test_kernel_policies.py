@@ -181,3 +181,25 @@ def test_recurrences_without_a_kernel_for_chunks_are_captured_in_one_form():
             assert variant is None
             part.prepare_capture(captured, variant, 4096)
         assert captured.extras == {"short_portions": True}
+
+
+def test_latent_layers_off_the_tcgen05_kernel_are_captured_in_one_form():
+    from types import SimpleNamespace
+    import torch
+    from slipstream_b200.parts import RotaryEncoding
+    from slipstream_b200.parts.latent_attention import LatentAttention
+
+    def layer(dtype, **kind):
+        part = LatentAttention("l", 64, 4, 32, 16, 32, 48, 80, 0.2, RotaryEncoding(16, 1e4), **kind)
+        part.runtime = SimpleNamespace(dtype=dtype)
+        return part
+
+    taken, off = layer(torch.bfloat16), [layer(torch.float32), layer(torch.bfloat16, page_size=12)]
+    plan = lambda: SimpleNamespace(is_decode_only=False)  # noqa: E731
+    assert [taken.capture_variant(n, plan()) for n in (30, 300)] == [True, False]
+    for part in off:
+        assert part.capture_group() != taken.capture_group() and part.capture_variant(30, plan()) is None
+        ctx = SimpleNamespace(is_decode_only=False, extras={})
+        taken.prepare_capture(ctx, True, 4096)
+        part.prepare_capture(ctx, None, 4096)
+        assert ctx.extras == {("few_keys", 96): True}

@@ -284,8 +284,9 @@ class PagedAttention(Mixer):
                                          ops.sm_count(self.runtime.device), self.sees))
 
     def capture_group(self) -> object:
-        # layers that see equally far with heads of one size, gated alike, answer `capture_variant` alike
-        return ("paged_attention", self.sees, self.head_dim, self.gates_inside)
+        # what `capture_variant` answers from beside the step's lengths
+        fits = ops.tcgen05_prefill_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_size or 16)
+        return ("paged_attention", self.sees, self.head_dim, self.gates_inside, fits, 128 // (self.num_heads // self.num_kv_heads), self.kernel_blocks)
 
     def prepare_capture(self, ctx, variant: object, max_model_len: int) -> None:
         if not ctx.is_decode_only:

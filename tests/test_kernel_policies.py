@@ -203,3 +203,22 @@ def test_latent_layers_off_the_tcgen05_kernel_are_captured_in_one_form():
         taken.prepare_capture(ctx, True, 4096)
         part.prepare_capture(ctx, None, 4096)
         assert ctx.extras == {("few_keys", 96): True}
+
+
+def test_attention_layers_share_an_answer_only_where_it_would_be_the_same(monkeypatch):
+    """The runner asks one layer of a group: layers of other heads, pages or head counts are asked themselves."""
+    from types import SimpleNamespace
+    import torch
+    from slipstream_b200.parts import PagedAttention, RotaryEncoding
+
+    monkeypatch.setattr(F, "_device_sm_count", lambda index: SMS)
+    layers = []
+    for heads, kv_heads, page in ((4, 2, 16), (4, 2, 12), (28, 4, 16), (32, 32, 16), (4, 2, 32)):
+        layers.append(PagedAttention("attn", 64, heads, kv_heads, 96, RotaryEncoding(96, 1e4), page_size=page))
+        layers[-1].runtime = SimpleNamespace(dtype=torch.bfloat16, device=0)
+    assert layers[0].capture_group() == layers[4].capture_group()
+    for tokens, length in ((30, 30), (30, 9000), (500, 9000), (2000, 2000)):
+        plan = SimpleNamespace(is_decode_only=False, q_lens=np.array([tokens]), seq_lens=np.array([length]))
+        answers = {}
+        for layer in layers:
+            assert answers.setdefault(layer.capture_group(), layer.capture_variant(length, plan)) == layer.capture_variant(length, plan)

@@ -12,8 +12,8 @@
 //    token whatever else is in the batch;
 //  * top-k and top-p find their threshold in a histogram over the distance from the largest value and among the few
 //    values of the bin where it falls (top-p on fixed-point sums, so the result does not depend on the order of atomics);
-//    rows for which that does not work out (infinities, NaN, too many values in the bin) by radix selection on the value
-//    bits.  Either way the threshold is a value's own bits, and tokens that tie with it are all kept;
+//    rows for which that does not work out by radix selection on the value bits, among the values of the bin (too many in
+//    it) or of the whole row (infinities, NaN).  Either way the threshold is a value's own bits, and tokens that tie with it are all kept;
 //  * rows with temperature 0 take the arg-max of the raw logits (filters skipped,
 //    as sampler.py:55-56); the lowest index wins ties.
 #include "common.cuh"
@@ -449,7 +449,7 @@ struct SampleKnown {
 
 // Decides about a long list (all of it in block 0): its values in order, the largest first, those stay that stand in front of the first of
 // equal values with k or more in front of it, or with top_p of the mass, and they race.  Up to 66 steps of Batcher's bitonic network where
-// comparing all with all takes 0.06 us for every thousand pairs (64 rows, top-k 2,000 and top-p: 883 us, 119 so).
+// comparing all with all takes 0.2 us for every thousand pairs (64 rows, top-k 2,000 and top-p 0.9: 879 us, 114 so).
 __device__ __noinline__ ArgMax draw_from_sorted(SampleFast& fast, int total, int k, unsigned long long base, float tp, bool all_of_it,
                                                 unsigned long long target, float vmax, float floor_val, uint64_t seed, uint64_t draw, ArgMax a,
                                                 SampleShared& sh) {
@@ -528,10 +528,11 @@ __device__ __noinline__ ArgMax draw_from_sorted(SampleFast& fast, int total, int
 // the distance from the largest: a larger value never falls into a later bin, so the bin in which the k-th value stands, or in
 // which the mass reaches top_p, holds the threshold; (3) values in front of that bin race, those in it are listed (under both
 // filters all of them are listed), and block 0 decides value by value which of the list stay: a value stays while what is
-// larger than it counts less than k, or holds less than top_p of the mass (`draw_from_sorted` where they are many).  Returns false where a step does not work
-// out; nothing has been decided then, but `known` says where the threshold falls if it got so far.  Bound by issue (an exponential and up to three shared-memory additions a value) and the
-// pass's way to L2.  64 rows of 152,064 logits, against radix selection with a histogram a digit (four passes for top-k, five
-// for top-p, each forming the values anew): top-k 40 221 -> 77 us, top-p 0.8 272 -> 87, both 349 -> 60.
+// larger than it counts less than k, or holds less than top_p of the mass (`draw_from_sorted` where they are many).  Returns false
+// where a step does not work out; nothing has been decided then, but `known` says where the threshold falls if it got so far.  Bound by
+// issue (an exponential and up to three shared-memory additions a value) and the pass's way to L2.  64 rows of 152,064 logits, against
+// radix selection with a histogram a digit (four passes for top-k, five for top-p, each forming the values anew): top-k 40 223 -> 65
+// us, top-p 0.8 314 -> 98, both 377 -> 66.
 __device__ __forceinline__ bool draw_fast(const SampleRow& t, int k, float tp, float mp, uint64_t seed, uint64_t draw, SampleShared& sh,
                                           SampleFast& fast, SampleKnown& known, ArgMax& best) {
     const int tid = threadIdx.x;

@@ -232,6 +232,47 @@ extern "C" int ss_attn_decode_tma(const void* q, int64_t q_stride, void* out, in
     return launch_decode_tma<2, 0>(map_kv, a, grid, cluster, smem2, stream);
 }
 
+#include "attention_decode_spread.cuh"
+
+// Two blocks an SM share the tiles of all requests (see the kernel): arguments as ss_attn_decode_tma; scratch: for each block
+// (two an SM) 2 x 16 x (HEAD_DIM + 2) floats and 4 more, of which nothing outlives the call.  Two launches.
+extern "C" int ss_attn_decode_spread(const void* q, int64_t q_stride, void* out, int64_t out_stride,
+                                     void* kv, const int32_t* block_tables, int max_blocks, int n_requests,
+                                     const int32_t* q_start, const int32_t* seq_lens, int n_q, int n_kv,
+                                     int page_size, int64_t num_pages, float scale, int window,
+                                     const float* inv_freq, int rot_dim, int fused, float* scratch, const void* gate, int* err,
+                                     cudaStream_t stream, float softcap, const float* sinks, int keep, int out_f32) {
+    if (n_requests <= 0) return 0;
+    if (n_requests > DS_REQUESTS || !scratch) return (int)cudaErrorInvalidValue;
+    if (keep < 0 || (keep > 0 && window <= 0) || (out_f32 && gate)) return (int)cudaErrorInvalidValue;
+    if (page_size % 8 != 0 || 64 % page_size != 0) return -3003;
+    if (fused && (rot_dim < 0 || rot_dim > HEAD_DIM || rot_dim % 2 || (rot_dim > 0 && !inv_freq))) return (int)cudaErrorInvalidValue;
+    // (the row of tiles is counted in 32 bits)
+    if ((int64_t)n_requests * n_kv * ((n_q / n_kv + 15) / 16) * ((int64_t)max_blocks * page_size / 64 + 2) >= (1ll << 31)) return (int)cudaErrorInvalidValue;
+    SpreadArgs s;
+    DecodeTmaArgs& a = s.a;
+    CUtensorMap map_kv;
+    int rc = fa::make_map3(&map_kv, kv, HEAD_DIM, (uint64_t)page_size, (uint64_t)num_pages * 2 * n_kv, (uint64_t)HEAD_DIM * 2,
+                           (uint64_t)page_size * HEAD_DIM * 2, 64, (uint32_t)page_size, 1);
+    if (rc) return rc;
+    a.q = (const bf16*)q; a.q_stride = q_stride; a.out = (bf16*)out; a.out_stride = out_stride; a.kv = (bf16*)kv;
+    a.block_tables = block_tables; a.max_blocks = max_blocks; a.q_start = q_start; a.seq_lens = seq_lens;
+    a.n_q = n_q; a.n_kv = n_kv; a.page_size = page_size; a.num_pages = num_pages; a.scale = scale; a.softcap = softcap; a.window = window;
+    a.n_slices = 1; a.cluster = 1; a.inv_freq = inv_freq; a.rot_dim = fused ? rot_dim : 0; a.fused = fused;
+    a.part_o = nullptr; a.part_lse = nullptr; a.counters = nullptr; a.err = err; a.gate = (const bf16*)gate;
+    a.sinks = sinks; a.keep = keep; a.out_f32 = out_f32; a.across = 0;
+    s.scratch = scratch;
+    s.n_requests = n_requests;
+    s.n_blocks = 2 * ss_sm_count();
+    s.joins = reinterpret_cast<int4*>(scratch + (int64_t)s.n_blocks * 2 * 16 * (HEAD_DIM + 2));
+    constexpr int smem = decode_spread_smem_bytes<HEAD_DIM>();
+    static SsPerDevice opted;
+    if (int rc_smem = ss_opt_in_smem(attn_decode_spread<HEAD_DIM>, smem, opted)) return rc_smem;
+    ss_launch(attn_decode_spread<HEAD_DIM>, dim3(s.n_blocks), dim3(DT_THREADS), smem, stream, map_kv, s);
+    ss_launch(attn_decode_spread_join<HEAD_DIM>, dim3(s.n_blocks - 1), dim3(DS_JOIN_THREADS), 0, stream, s);
+    return SS_LAUNCH_CHECK();
+}
+
 #include "attention_decode_across.cuh"
 
 // What a layer needs of ss_attn_decode_across's scratch: parts per slice (the return value; 0 where the kernel does not take

@@ -143,6 +143,9 @@ _ATTN_SIGNATURES = {
                            c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_float, c_int, c_int,
                            c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float,
                            c_void_p, c_int, c_int, c_int],
+    "ss_attn_decode_spread": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int,
+                              c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_float, c_int,
+                              c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int],
     "ss_attn_decode_mma": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int,
                            c_void_p, c_void_p, c_int, c_int, c_int, c_int64, c_float, c_int, c_int,
                            c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int,
@@ -873,6 +876,25 @@ def decode_scratch(n_requests: int, n_q: int, n_slices: int, head_dim: int, devi
             torch.empty((n_requests, n_q, n_slices), dtype=torch.float32, device=device))
 
 
+def _decode_rope(rope: tuple[torch.Tensor | None, int] | None, q_stride: int, n_q: int, n_kv: int, head_dim: int,
+                 gate: torch.Tensor | None) -> tuple[torch.Tensor | None, int]:
+    """The checked rotation of a decode kernel: (inverse frequencies, rotary size)."""
+    if rope is None:
+        return None, 0
+    inv_freq, rotary_dim = rope
+    if q_stride != (n_q + 2 * n_kv) * head_dim:
+        raise KernelError("the fused rotation takes the stacked q/k/v projection")
+    if rotary_dim % 2 or rotary_dim > head_dim:
+        raise KernelError("rotary_dim must be even and at most head_dim")
+    if rotary_dim:
+        _need(inv_freq, torch.float32, "inv_freq")
+        if inv_freq.numel() != rotary_dim // 2:
+            raise KernelError("inv_freq must hold rotary_dim / 2 values")
+    if gate is not None:
+        raise KernelError("a gated layer does not rotate inside the decode kernel")
+    return inv_freq, rotary_dim
+
+
 def paged_attention_decode(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torch.Tensor,
                            block_tables: torch.Tensor, q_start: torch.Tensor, seq_lens: torch.Tensor,
                            n_requests: int, n_q: int, n_kv: int, head_dim: int, scale: float, window: int = 0,
@@ -918,29 +940,69 @@ def paged_attention_decode(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv
         part_o, part_lse = scratch
         if part_o.numel() < n_requests * n_out * n_slices * head_dim or part_lse.numel() < n_requests * n_out * n_slices:
             raise KernelError("decode scratch is too small")
-    inv_freq, rotary_dim = rope if rope is not None else (None, 0)
-    if rope is not None:
-        if q_stride != (n_q + 2 * n_kv) * head_dim:
-            raise KernelError("the fused rotation takes the stacked q/k/v projection")
-        if rotary_dim % 2 or rotary_dim > head_dim:
-            raise KernelError("rotary_dim must be even and at most head_dim")
-        if rotary_dim:
-            _need(inv_freq, torch.float32, "inv_freq")
-            if inv_freq.numel() != rotary_dim // 2:
-                raise KernelError("inv_freq must hold rotary_dim / 2 values")
+    inv_freq, rotary_dim = _decode_rope(rope, q_stride, n_q, n_kv, head_dim, gate)
     lib = attention_library(head_dim)
     args = (q.data_ptr(), q_stride, out.data_ptr(), out.shape[1], kv.data_ptr(), block_tables.data_ptr(),
             block_tables.shape[1], n_requests, q_start.data_ptr(), seq_lens.data_ptr(), n_q, n_kv, kv.shape[3], kv.shape[0],
             float(scale), key_span(window, chunk), n_slices, _ptr(inv_freq) if rotary_dim else None, rotary_dim,
             int(rope is not None), _ptr(part_o), _ptr(part_lse), _ptr(counters))
-    if gate is not None and rope is not None:
-        raise KernelError("a gated layer does not rotate inside the decode kernel")
     tail = (_gate_ptr(gate, q, q_stride), error_word(q.device).data_ptr(), _stream(), float(softcap or 0.0))
     if tma:
         _check(lib.ss_attn_decode_tma(*args, int(stages), *tail, _ptr(sinks), _kept(keep, window), out_f32, int(across)),
                "paged_attention_decode")
     else:
         _check(lib.ss_attn_decode_mma(*args, *tail, _ptr(sinks), _kept(keep, window), out_f32, int(across)), "paged_attention_decode")
+
+
+def paged_attention_decode_spread(q: torch.Tensor, q_stride: int, out: torch.Tensor, kv: torch.Tensor,
+                                  block_tables: torch.Tensor, q_start: torch.Tensor, seq_lens: torch.Tensor,
+                                  n_requests: int, n_q: int, n_kv: int, head_dim: int, scale: float, window: int = 0,
+                                  rope: tuple[torch.Tensor | None, int] | None = None, chunk: int = 0,
+                                  gate: torch.Tensor | None = None, softcap: float = 0.0, sinks: torch.Tensor | None = None,
+                                  keep: int = 0) -> None:
+    """`paged_attention_decode` for many requests of different lengths (`spreads_decode`): the key tiles of all of them are
+    dealt out evenly to two blocks an SM, by the lengths on the device.  Arguments as there."""
+    if not tcgen05_attention_fits(head_dim, n_q, n_kv, kv.shape[3], 0) or n_requests > DECODE_SPREAD_REQUESTS:
+        raise KernelError("the spread decode kernel takes head size 64 or 128, pages of 8, 16, 32 or 64 tokens and up to 512 requests")
+    _check_sinks(sinks, n_q)
+    out_f32 = _attention_out(out, gate, None)
+    _need(kv, torch.bfloat16, "kv pages")
+    if q.dtype != torch.bfloat16:
+        raise KernelError("the tensor-core attention kernels take bfloat16")
+    for name, t in (("block_tables", block_tables), ("q_start", q_start), ("seq_lens", seq_lens)):
+        _need(t, torch.int32, name)
+    inv_freq, rotary_dim = _decode_rope(rope, q_stride, n_q, n_kv, head_dim, gate)
+    lib = attention_library(head_dim)
+    scratch = torch.empty(2 * sm_count(q.device) * (2 * 16 * (head_dim + 2) + 4), dtype=torch.float32, device=q.device)
+    _check(lib.ss_attn_decode_spread(
+        q.data_ptr(), q_stride, out.data_ptr(), out.shape[1], kv.data_ptr(), block_tables.data_ptr(), block_tables.shape[1], n_requests,
+        q_start.data_ptr(), seq_lens.data_ptr(), n_q, n_kv, kv.shape[3], kv.shape[0], float(scale), key_span(window, chunk),
+        _ptr(inv_freq) if rotary_dim else None, rotary_dim, int(rope is not None), scratch.data_ptr(), _gate_ptr(gate, q, q_stride),
+        error_word(q.device).data_ptr(), _stream(), float(softcap or 0.0), _ptr(sinks), _kept(keep, window), out_f32),
+        "paged_attention_decode_spread")
+
+
+DECODE_SPREAD_REQUESTS = 512  # what the spread decode kernel takes at most
+
+
+def spreads_decode(seq_lens: np.ndarray, n_kv: int, group: int, head_dim: int, reach: int, sms: int) -> bool:
+    """Whether a decode step's key tiles are dealt out evenly (`paged_attention_decode_spread`): its host lengths, the keys a
+    query sees at most (0: all).  Only where a request's head block would have one block, two per SM at a time, and up to 8 heads
+    share a kv head (with more the next unit's queries wait for the merge).  What either way takes, in us, fitted to 28 and 32 heads on 4 and 8
+    kv heads of 128 elements and 14 and 32 on 2 and 4 of 64, 24 to 200 requests of 100 to 3,600 keys on average, equal or between half
+    and one and a half of that: one block a unit walks a tile of 64 keys in 1.1 us (128 elements; 0.8 with 64), 1.56 (0.78) with
+    two on every SM, and the last round lasts as long as its longest unit; dealt out evenly all tiles take the time of the bytes, and the merges and the
+    second kernel 11 (10).  48 requests x 4, 900 keys on average: 27.0 and 25.1 us, 1,800: 49.1 and 38.1, 1,800 each: 35.8 and 36.9."""
+    n = int(seq_lens.size)
+    units = n * n_kv * ((group + 15) // 16)
+    if n_kv < 2 or group > 8 or n > DECODE_SPREAD_REQUESTS or decode_slices(n, n_kv, group, int(seq_lens.max()), False, sms) != 1:
+        return False
+    tiles = (np.minimum(seq_lens, reach) if reach else seq_lens).astype(np.int64) // 64 + 1
+    alone, crowded, fixed = (1.1, 1.56, 11.0) if head_dim == 128 else (0.8, 0.78, 10.0)
+    rounds, rest = divmod(units, 2 * sms)
+    one_block = 3.0 + rounds * crowded * float(tiles.mean()) + (float(tiles.max()) * max(alone, crowded * rest / (2 * sms)) if rest else 0.0)
+    spread = fixed + crowded * float(tiles.sum()) * (units // n) / (2 * sms)
+    return spread < 0.97 * one_block
 
 
 WIDE_CONTEXT = 8192  # from this many cached tokens a decode step of few requests may use more than 8 slices
@@ -1050,6 +1112,18 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, bloc
                                sm_count(qkv.device))
         scratch = ctx.extras.get(("decode_scratch", n_q, head_dim)) if not across else None
         heads = out if diff is None else _heads_f32(out, n_q, head_dim)
+        reach = (window or chunk) + keep
+        key = ("decode_spread", n_kv, group, head_dim, reach)
+        spread = ctx.extras.get(key)
+        if spread is None:  # the same for every layer of the step that sees as far; a captured step was told
+            spread = ctx.extras[key] = not static and spreads_decode(ctx.seq_lens_host, n_kv, group, head_dim, reach, sm_count(qkv.device))
+        if (spread and slices == 1 and not across and tcgen05_attention_fits(head_dim, n_q, n_kv, kv.shape[3], 0)
+                and ctx.num_requests * n_kv * (block_tables.shape[1] * kv.shape[3] // 64 + 2) < 2 ** 31):
+            paged_attention_decode_spread(qkv, qkv.shape[1], heads, kv, block_tables, ctx.q_start, ctx.seq_lens, ctx.num_requests,
+                                          n_q, n_kv, head_dim, scale, window, rope, chunk, gate, softcap, sinks, keep)
+            if diff is not None:
+                diff_combine(heads, diff, n_q // 2, out)
+            return
         paged_attention_decode(qkv, qkv.shape[1], heads, kv, block_tables, ctx.q_start, ctx.seq_lens,
                                ctx.num_requests, n_q, n_kv, head_dim, scale, window, slices, scratch, rope,
                                stages=DECODE_RING_STAGES, chunk=chunk, gate=gate, softcap=softcap, sinks=sinks, keep=keep,
@@ -2791,7 +2865,7 @@ def set_programmatic_launch(enabled: bool) -> None:
 
 
 __all__ = ["KernelError", "KernelBuildError", "embedding", "add_rmsnorm", "hc_norm", "linear_hc_rmsnorm", "rope_norm_cache", "glu_limited", "gate_up_glu", "sigmoid_gate", "key_span", "rope_and_cache", "swiglu",
-           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "few_prefill_keys", "paged_attention_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
+           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "few_prefill_keys", "paged_attention_decode", "paged_attention_decode_spread", "spreads_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
            "attention_library", "group_norm", "round_stream", "conv_silu", "SCAN_FEW", "only_short_portions", "ssm_scan", "router", "moe_experts", "moe_combine",
            "norm_rope_cache", "turn_heads", "soft_cap", "embed_sum", "matrix_cell", "cell_output", "gated_recurrence", "xielu",
            "DiffPair", "diff_in_attention", "diff_combine", "heads_to_pages", "branch_norm", "PairedOutput", "WeighedTerms",

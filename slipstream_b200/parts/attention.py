@@ -267,12 +267,16 @@ class PagedAttention(Mixer):
     # ------------------------------------------------------------------ decode steps replayed from a graph
     def capture_variant(self, longest: int, plan: object = None) -> object:
         """Decode steps: long contexts of few requests want the keys cut into more slices than fit one thread-block
-        cluster (``ops.decode_slices``).  Steps with prompt portions: into how many parts the tcgen05 prefill kernel
+        cluster (``ops.decode_slices``; 1 here), many requests of different lengths their tiles dealt out evenly
+        (``ops.spreads_decode``; 2).  Steps with prompt portions: into how many parts the tcgen05 prefill kernel
         cuts the keys of a query tile (``ops.prefill_key_parts``), 0 where the mma.sync kernel runs because there are few
         keys.  Each form is captured as a graph of its own."""
         bf16 = self.runtime.dtype == torch.bfloat16
         if plan is None or plan.is_decode_only:
-            return bool(bf16 and ops.is_long_context(longest))
+            spread = (bf16 and plan is not None and not self.talk
+                      and ops.spreads_decode(plan.seq_lens, self.num_kv_heads, self.num_heads // self.num_kv_heads, self.head_dim, self.sees,
+                                             ops.sm_count(self.runtime.device)))
+            return int(bf16 and ops.is_long_context(longest)) + 2 * int(spread)
         group = self.num_heads // self.num_kv_heads
         if not bf16 or not ops.tcgen05_prefill_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_size or 16):
             return None
@@ -286,7 +290,8 @@ class PagedAttention(Mixer):
     def capture_group(self) -> object:
         # what `capture_variant` answers from beside the step's lengths
         fits = ops.tcgen05_prefill_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_size or 16)
-        return ("paged_attention", self.sees, self.head_dim, self.gates_inside, fits, 128 // (self.num_heads // self.num_kv_heads), self.kernel_blocks)
+        return ("paged_attention", self.sees, self.head_dim, self.gates_inside, fits, 128 // (self.num_heads // self.num_kv_heads), self.kernel_blocks,
+                self.talk)
 
     def prepare_capture(self, ctx, variant: object, max_model_len: int) -> None:
         if not ctx.is_decode_only:
@@ -300,7 +305,9 @@ class PagedAttention(Mixer):
             return
         # the number of slices must not follow the lengths of the step that happens to be captured
         ctx.extras["static_max_seq_len"] = max_model_len
-        ctx.extras["decode_wide"] = bool(variant)
+        ctx.extras["decode_wide"] = bool(int(variant or 0) & 1)
+        group = self.num_heads // self.num_kv_heads
+        ctx.extras[("decode_spread", self.num_kv_heads, group, self.head_dim, self.sees)] = bool(int(variant or 0) & 2)
         # the float32 kernel's list of query tiles: one tile per row of the batch
         rows = ctx.num_requests
         ctx.set_query_tiles(16, 1, torch.arange(rows, dtype=torch.int32, device=ctx.device),

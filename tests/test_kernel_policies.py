@@ -222,3 +222,31 @@ def test_attention_layers_share_an_answer_only_where_it_would_be_the_same(monkey
         answers = {}
         for layer in layers:
             assert answers.setdefault(layer.capture_group(), layer.capture_variant(length, plan)) == layer.capture_variant(length, plan)
+
+
+def test_decode_tiles_are_dealt_out_where_that_was_measured_to_pay_captured_or_not(monkeypatch):
+    from types import SimpleNamespace
+    import torch
+    from slipstream_b200.parts import PagedAttention, RotaryEncoding
+
+    def uneven(n, mean):
+        weights = np.array([2 + i % 5 for i in range(n)])
+        return (weights * n * mean / weights.sum()).astype(np.int32)
+
+    spreads = lambda lens, n_kv=4, group=7, d=128, reach=0: F.spreads_decode(np.asarray(lens, dtype=np.int32), n_kv, group, d, reach, SMS)  # noqa: E731
+    assert spreads(uneven(48, 1800)) and spreads(uneven(40, 1200)) and spreads(uneven(24, 1800), 8, 4) and spreads(uneven(40, 1200), 4, 8, 64)
+    assert not spreads(uneven(48, 300)) and not spreads([1200] * 64) and not spreads([1200] * 48, 4, 8, 64) and not spreads([1])
+    assert not spreads(uneven(48, 1800), reach=512)           # a window leaves little to deal out
+    assert not spreads(uneven(48, 1800), 4, 9)                # more heads than lie beside the merge
+    assert not spreads(uneven(200, 1800), 1) and not spreads(uneven(8, 1800)) and not spreads(uneven(600, 1800))
+    # a captured step is told what a step run kernel by kernel finds out from its lengths
+    monkeypatch.setattr(F, "_device_sm_count", lambda index: SMS)
+    layer = PagedAttention("attn", 64, 28, 4, 128, RotaryEncoding(128, 1e4), page_size=16)
+    layer.runtime = SimpleNamespace(dtype=torch.bfloat16, device=0)
+    for lens in (uneven(48, 1800), uneven(48, 300), uneven(48, 9000), np.array([9000])):
+        plan = SimpleNamespace(is_decode_only=True, q_lens=np.ones(lens.size, dtype=np.int32), seq_lens=lens)
+        ctx = SimpleNamespace(is_decode_only=True, num_requests=lens.size, device=None, extras={}, set_query_tiles=lambda *a: None)
+        layer.prepare_capture(ctx, layer.capture_variant(int(lens.max()), plan), 16384)
+        assert ctx.extras["decode_wide"] == F.is_long_context(int(lens.max()))
+        assert ctx.extras[("decode_spread", 4, 7, 128, layer.sees)] == spreads(lens)
+    assert layer.capture_variant(5000) == 0  # (no lengths yet: the form for any)

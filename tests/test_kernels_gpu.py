@@ -406,6 +406,58 @@ def test_decode_attention_that_rotates_and_writes_the_newest_token_itself(slices
     ops().check_errors(torch.device(DEV))
 
 
+# few tiles for many blocks (one unit in many parts), more units than requests fit a warp's sum, a request much longer than the rest,
+# requests without a key; groups whose queries lie beside the merge (up to 8 heads) and in its place
+@pytest.mark.parametrize("lens", [[1, 63, 64, 65, 700, 129, 2000, 0, 16, 17], [1 + i % 70 for i in range(300)], [30, 0, 9000, 100], [20000]],
+                         ids=["mixed", "many short", "one long", "alone"])
+@pytest.mark.parametrize("n_q, n_kv, d, page, window, keep", [(28, 4, 128, 16, 0, 0), (6, 3, 64, 8, 0, 0), (40, 2, 64, 32, 150, 0), (16, 2, 128, 64, 70, 5),
+                                                               (18, 2, 128, 16, 0, 0)])
+def test_decode_with_tiles_dealt_out_evenly(lens, n_q, n_kv, d, page, window, keep):
+    """The spread decode kernel against the reference, its options against the kernel with one block a unit, and the rotation
+    inside against the rotary kernel in front, bit for bit.  What lies behind a request's newest token in its pages is
+    infinite.  Tolerance: bfloat16 probabilities and outputs, as above."""
+    R, scale = len(lens), d ** -0.5
+    q, kv, table, q_start, seq_lens = make_attention_case(torch.bfloat16, [max(n, 1) for n in lens], [1] * R, n_q, n_kv, d, page, seed=d + n_q)
+    for r, n in enumerate(lens):
+        if n % page:
+            kv[int(table[r, (n - 1) // page]), :, :, n % page:] = float("inf")
+    there = torch.tensor([n > 0 for n in lens])
+    seq_lens = seq_lens * there.to(DEV).int()
+    sinks = torch.linspace(-1, 2, n_q, device=DEV)
+    flat = q.view(R, -1)
+
+    def run(f, rows=flat, pages=kv, dtype=torch.bfloat16, **options):
+        out = torch.full((R, n_q * d), float("nan"), device=DEV, dtype=dtype)
+        f(rows, rows.shape[1], out, pages, table, q_start, seq_lens, R, n_q, n_kv, d, scale, window, keep=keep, **options)
+        return out
+
+    spread, plain = ops().paged_attention_decode_spread, ops().paged_attention_decode
+    out = run(spread, sinks=sinks)
+    if not keep:
+        ref = attention_reference(q, kv, table, q_start, torch.clamp(seq_lens, min=1), n_kv, page, scale, window, sinks)
+        assert rel_err(out.view_as(ref).cpu()[there], ref[there]) < 1e-2
+    assert (out[~there.to(DEV)] == 0).all()
+    assert torch.equal(out, run(spread, sinks=sinks))  # (the same sums every time)
+    gate = torch.randn(R, n_q * d, device=DEV).bfloat16()
+    wide = torch.cat([flat, gate], dim=1)
+    for options in (dict(sinks=sinks), dict(softcap=3.0), dict(dtype=torch.float32), dict(rows=wide, gate=wide[:, n_q * d:])):
+        assert rel_err(run(spread, **options), run(plain, **options)) < 1e-2, options.keys()
+    g = torch.Generator().manual_seed(5)
+    rot = d // 2 if page == 8 else d
+    qkv = (torch.randn(R, (n_q + 2 * n_kv) * d, generator=g) * 0.7).bfloat16().to(DEV)
+    inv_freq = (1.0 / 10000.0 ** (torch.arange(0, rot, 2, dtype=torch.float32) / rot)).to(DEV)
+    positions = torch.clamp(seq_lens - 1, min=0).int()
+    slots = (table.long()[torch.arange(R, device=DEV), (positions // page).long()] * page + positions % page).int()
+    qkv_a, kv_a, kv_b = qkv.clone(), kv.clone(), kv.clone()
+    ops().rope_and_cache(qkv_a, positions, slots, inv_freq, kv_a, n_q, n_kv, d, rot)
+    a, b = run(spread, rows=qkv_a, pages=kv_a), run(spread, rows=qkv, pages=kv_b, rope=(inv_freq, rot))
+    assert torch.equal(a, b)
+    at = there.to(DEV).nonzero()[:, 0]
+    rows_of = lambda pages: pages[(slots // page).long()[at], :, :, (slots % page).long()[at]]  # noqa: E731
+    assert torch.equal(rows_of(kv_a), rows_of(kv_b)) and torch.isfinite(rows_of(kv_b).float()).all()
+    ops().check_errors(torch.device(DEV))
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_a_far_key_among_hundreds_is_found(dtype):
     """One key 700 tokens back matches the last query far better than all others: its value must

@@ -115,7 +115,7 @@ group_norm_kernel(const TI* __restrict__ in, int64_t in_stride, int terms, const
 
 // The gated form (MODE 1) for float32 rows and bfloat16 gates, 4 elements a load: a block per row and group, its values read and
 // gated once and kept in registers between the sum of squares and the output (element by element and twice over, 2,045 rows
-// of 7,168 in one group took 85 us; 34 here, bound by the exact exponential and division of the gate).
+// of 7,168 in one group took 85 us; 41 with the loads of 8 passes for 7, 35 here, bound by the exact exponential and division of the gate).
 template <int NV>
 __global__ void __launch_bounds__(256)
 gated_norm_kernel(const float* __restrict__ in, const bf16* __restrict__ gate, int64_t gate_stride, const float* __restrict__ weight,
@@ -179,10 +179,16 @@ extern "C" int ss_group_norm(const void* in, int in_f32, int64_t in_stride, int 
         const dim3 grid(n_out * groups), block(threads);
 #define GG_GO(NV) ss_launch(gated_norm_kernel<NV>, grid, block, 0, stream, (const float*)in, (const bf16*)gate, gate_stride, weight, \
                             (bf16*)out, hidden, groups, eps)
-        if (nv == 1) GG_GO(1);
-        else if (nv == 2) GG_GO(2);
-        else if (nv <= 4) GG_GO(4);
-        else GG_GO(8);
+        switch (nv) {
+            case 1: GG_GO(1); break;
+            case 2: GG_GO(2); break;
+            case 3: GG_GO(3); break;
+            case 4: GG_GO(4); break;
+            case 5: GG_GO(5); break;
+            case 6: GG_GO(6); break;
+            case 7: GG_GO(7); break;
+            default: GG_GO(8);
+        }
 #undef GG_GO
         return SS_LAUNCH_CHECK();
     }
@@ -290,100 +296,94 @@ conv_silu_kernel(const T* __restrict__ proj, int64_t stride, int col0, const flo
 }
 
 // The same for bfloat16 with channels in steps of 4 (and the projection's rows and the first channel on 8-byte boundaries) and
-// at most 4 taps: a thread takes 4 neighbouring channels, 8 bytes a load and a store, over CONV_ROWS rows, the loads of 4 rows
-// in flight.  The window of a row that is not a request's first in this tile is already in registers.  Bound by the exact
-// exponentials and divisions of silu, so by how many warps an SM holds: 2,045 rows of 9,216 channels took 60 us with 8 channels a
-// thread and a row at a time, 81 with 8 channels and 8 rows in flight (164 registers), 56 so.
-__global__ void __launch_bounds__(128)
+// at most 4 taps: a thread takes 4 neighbouring channels, 8 bytes a load and a store, over CONV_ROWS4 rows, four at a time, of which the next
+// four are on their way meanwhile.  The number of taps and what follows the sum are template arguments: behind run-time values every tap cost a
+// selection and every row a shift of the window, 57 instructions an element where the sum and its exact silu take 25.  2,045 rows of
+// 9,216 channels: 60 us with 8 channels a thread and a row at a time, 53 with 4 and run-time taps, 32 so (32 rows a block: 32, but 12.7 where 600
+// rows of 1,152 channels take 8.1 with 16); bound by issue (the exponential and the division).
+#define CONV_ROWS4 16
+template <int TAPS, int KIND>  // KIND: plus_input
+__global__ void __launch_bounds__(128, 6)
 conv_silu_bf16x4_kernel(const bf16* __restrict__ proj, int64_t stride, int col0, const float* __restrict__ taps,
                         const float* __restrict__ bias, const float* __restrict__ state, bf16* __restrict__ out,
                         const int32_t* __restrict__ q_start, const int32_t* __restrict__ seq_lens,
-                        const int32_t* __restrict__ slots, int R, int n_rows, int C, int n_taps, int n_slots, int* err, int plus_input) {
+                        const int32_t* __restrict__ slots, int R, int n_rows, int C, int n_slots, int* err) {
     pdl_launch_dependents();
     pdl_wait();
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (c >= C) return;
-    constexpr int MAXB = 3;  // taps - 1 at most
-    const int back = n_taps - 1;
-    float w[4][MAXB + 1], x[4][MAXB], b[4];
+    constexpr int BACK = TAPS - 1, BATCH = 4;  // rows of a request whose loads are in flight before the first is used
+    float w[4][TAPS], b[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         b[e] = bias ? bias[c + e] : 0.f;
 #pragma unroll
-        for (int j = 0; j <= MAXB; ++j) w[e][j] = j < n_taps ? taps[(int64_t)(c + e) * n_taps + j] : 0.f;
-#pragma unroll
-        for (int j = 0; j < MAXB; ++j) x[e][j] = 0.f;
+        for (int j = 0; j < TAPS; ++j) w[e][j] = taps[(int64_t)(c + e) * TAPS + j];
     }
     auto widen = [](const uint2& raw, float (&v)[4]) {
         v[0] = __uint_as_float(raw.x << 16); v[1] = __uint_as_float(raw.x & 0xffff0000u);
         v[2] = __uint_as_float(raw.y << 16); v[3] = __uint_as_float(raw.y & 0xffff0000u);
     };
-    const int row_first = blockIdx.x * CONV_ROWS, row_end = min(n_rows, row_first + CONV_ROWS);
-    int r = -1, r_end = -1;
-    bool on = false;
-    constexpr int BATCH = 4;  // rows of a request whose loads are in flight before the first is used
+    const int row_first = blockIdx.x * CONV_ROWS4, row_end = min(n_rows, row_first + CONV_ROWS4);
     for (int row = row_first; row < row_end;) {
-        if (row >= r_end) {
-            r = request_of_row(q_start, R, row);
-            if (r < 0) break;
-            r_end = q_start[r + 1];
-            const int slot = slots[r];
-            on = seq_lens[r] > 0 && slot >= 0 && slot < n_slots;
-            if (seq_lens[r] > 0 && !on && threadIdx.x == 0) atomicOr(err, SS_ERR_SLOT_RANGE);
-            const float* st = state + (int64_t)(on ? slot : 0) * back * C + c;
-            const int i = row - q_start[r];
-#pragma unroll
-            for (int j = 0; j < MAXB; ++j) {
-                if (j >= back || !on) break;
-                const int src = i - (back - j);
-                float v[4];
-                if (src >= 0) {
-                    widen(*reinterpret_cast<const uint2*>(proj + (int64_t)(row - (back - j)) * stride + col0 + c), v);
-                } else {
-                    const float4 old = *reinterpret_cast<const float4*>(st + (int64_t)(back + src) * C);
-                    v[0] = old.x; v[1] = old.y; v[2] = old.z; v[3] = old.w;
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) x[e][j] = v[e];
-            }
-        }
-        const int n = min(min(row_end, r_end) - row, BATCH);
+        const int r = request_of_row(q_start, R, row);
+        if (r < 0) return;
+        const int stop = min(row_end, q_start[r + 1]), slot = slots[r];
+        const bool on = seq_lens[r] > 0 && slot >= 0 && slot < n_slots;
+        if (seq_lens[r] > 0 && !on && threadIdx.x == 0) atomicOr(err, SS_ERR_SLOT_RANGE);
         if (!on) {
-            row += n;
+            row = stop;
             continue;
         }
-        uint2 raw[BATCH];
+        const bf16* src = proj + (int64_t)row * stride + col0 + c;
+        uint2 next[BATCH];
+        auto load = [&](int left) {
 #pragma unroll
-        for (int u = 0; u < BATCH; ++u)
-            if (u < n) raw[u] = *reinterpret_cast<const uint2*>(proj + (int64_t)(row + u) * stride + col0 + c);
+            for (int u = 0; u < BATCH; ++u)
+                if (u < left) next[u] = *reinterpret_cast<const uint2*>(src + (int64_t)u * stride);
+        };
+        load(stop - row);
+        // x[u]: the inputs of rows row - BACK .. row + BATCH - 1, in front of the first the request's state
+        float x[BACK + BATCH][4];
+        const float* st = state + (int64_t)slot * BACK * C + c;
+        const int i = row - q_start[r];
 #pragma unroll
-        for (int u = 0; u < BATCH; ++u) {
-            if (u >= n) break;
-            float cur[4];
-            widen(raw[u], cur);
-            uint32_t packed[2];
-#pragma unroll
-            for (int e = 0; e < 4; e += 2) {
-                float o2[2];
-#pragma unroll
-                for (int d = 0; d < 2; ++d) {
-                    float acc = b[e + d];
-#pragma unroll
-                    for (int j = 0; j <= MAXB; ++j)
-                        if (j <= back) acc = fmaf(w[e + d][j], j < back ? x[e + d][j < MAXB ? j : 0] : cur[e + d], acc);
-                    o2[d] = plus_input == 1 ? cur[e + d] + acc : (plus_input == 2 ? acc : silu_exact(acc));
-                }
-                const __nv_bfloat162 h2 = __floats2bfloat162_rn(o2[0], o2[1]);
-                packed[e >> 1] = *reinterpret_cast<const uint32_t*>(&h2);
+        for (int j = 0; j < BACK; ++j) {
+            const int back = i - (BACK - j);
+            if (back >= 0) {
+                widen(*reinterpret_cast<const uint2*>(src - (int64_t)(BACK - j) * stride), x[j]);
+            } else {
+                const float4 old = *reinterpret_cast<const float4*>(st + (int64_t)(BACK + back) * C);
+                x[j][0] = old.x; x[j][1] = old.y; x[j][2] = old.z; x[j][3] = old.w;
             }
-            *reinterpret_cast<uint2*>(out + (int64_t)(row + u) * C + c) = make_uint2(packed[0], packed[1]);
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-#pragma unroll
-                for (int j = 0; j < MAXB; ++j)
-                    if (j < back) x[e][j] = (j + 1 < back) ? x[e][j + 1 < MAXB ? j + 1 : 0] : cur[e];
         }
-        row += n;
+        bf16* dst = out + (int64_t)row * C + c;
+        for (; row < stop; row += BATCH) {
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) widen(next[u], x[BACK + u]);
+            src += BATCH * stride;
+            load(stop - row - BATCH);
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) {
+                if (row + u >= stop) break;
+                float y[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float acc = b[e];
+#pragma unroll
+                    for (int j = 0; j < TAPS; ++j) acc = fmaf(w[e][j], x[u + j][e], acc);
+                    y[e] = KIND == 1 ? x[u + BACK][e] + acc : (KIND == 2 ? acc : silu_exact(acc));
+                }
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[1]), hi = __floats2bfloat162_rn(y[2], y[3]);
+                *reinterpret_cast<uint2*>(dst + (int64_t)u * C) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            }
+            dst += (int64_t)BATCH * C;
+#pragma unroll
+            for (int j = 0; j < BACK; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[j][e] = x[BATCH + j][e];
+        }
+        row = stop;
     }
 }
 
@@ -416,9 +416,17 @@ extern "C" int ss_conv_silu(const void* proj, int64_t stride, int col0, const fl
     const dim3 grid((n_rows + CONV_ROWS - 1) / CONV_ROWS, (C + 127) / 128);
     if (dtype == SS_BF16 && !fused_update && n_taps <= 4 && C % 4 == 0 && col0 % 4 == 0 && stride % 4 == 0 && ((uintptr_t)proj & 7) == 0 &&
         ((uintptr_t)out & 7) == 0 && ((uintptr_t)state & 15) == 0) {
-        const dim3 grid4((n_rows + CONV_ROWS - 1) / CONV_ROWS, (C / 4 + 127) / 128);
-        ss_launch(conv_silu_bf16x4_kernel, grid4, dim3(128), 0, stream, (const bf16*)proj, stride, col0, taps, bias, state,
-                  (bf16*)out, q_start, seq_lens, slots, R, n_rows, C, n_taps, n_slots, err, plus_input);
+        const dim3 grid4((n_rows + CONV_ROWS4 - 1) / CONV_ROWS4, (C / 4 + 127) / 128);
+        auto go = [&](auto kernel) {
+            ss_launch(kernel, grid4, dim3(128), 0, stream, (const bf16*)proj, stride, col0, taps, bias, (const float*)state, (bf16*)out, q_start,
+                      seq_lens, slots, R, n_rows, C, n_slots, err);
+        };
+#define CONV_GO(TAPS) (plus_input == 1 ? go(conv_silu_bf16x4_kernel<TAPS, 1>) : plus_input == 2 ? go(conv_silu_bf16x4_kernel<TAPS, 2>) : go(conv_silu_bf16x4_kernel<TAPS, 0>))
+        if (n_taps == 1) CONV_GO(1);
+        else if (n_taps == 2) CONV_GO(2);
+        else if (n_taps == 3) CONV_GO(3);
+        else CONV_GO(4);
+#undef CONV_GO
     } else if (dtype == SS_BF16)
         ss_launch(conv_silu_kernel<bf16>, grid, dim3(128), 0, stream, (const bf16*)proj, stride, col0, taps, bias, state,
                   (bf16*)out, q_start, seq_lens, slots, R, n_rows, C, n_taps, n_slots, fused_update, err, plus_input);

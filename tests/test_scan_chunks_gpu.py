@@ -293,3 +293,26 @@ def test_few_tokens_have_the_same_matrix_memory_bits_beside_a_prompt_portion(hea
     for a, b in zip(*states):
         assert torch.equal(a[[0, 1, 3]], b[[0, 1, 3]])
     ops.check_errors(DEV)
+
+
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+@pytest.mark.parametrize("kind", [dict(), dict(plus_input=True), dict(activation=False)], ids=["silu", "plus input", "plain"])
+def test_convolution_of_four_channels_a_thread_gives_the_bits_of_the_other_kernel(taps, kind):
+    """Requests that end inside a batch of four rows and a block's sixteen, or bring fewer rows than the window has, one without
+    tokens: channels that start on 8 bytes against the same channels one element further."""
+    from slipstream_b200 import ops
+    g = torch.Generator().manual_seed(taps)
+    lens, slots, channels = [1, 2, 3, 5, 0, 16, 17, 33, 4, 7], [9, 0, 1, 2, 3, 4, 5, 6, 7, 8], 516
+    rows = torch.randn(sum(lens), channels + 8, generator=g).bfloat16().to(DEV)
+    shifted = torch.cat([rows[:, :1], rows[:, :-1]], dim=1)
+    w, b = torch.randn(channels, taps, generator=g).to(DEV), torch.randn(channels, generator=g).to(DEV)
+    start = torch.randn(10, taps - 1, channels, generator=g).to(DEV)
+    ctx, got = step_ctx(lens, slots), []
+    for proj, col0 in ((rows, 4), (shifted, 5)):
+        for bias in (b, None):
+            state = start.clone()
+            got.append((ops.conv_silu(proj, col0, channels, w, bias, state, ctx, **kind), state))
+    for a, c in ((got[0], got[2]), (got[1], got[3])):
+        assert torch.equal(a[0], c[0]) and torch.equal(a[1], c[1])
+    assert not torch.equal(got[0][0], got[1][0])
+    ops.check_errors(DEV)

@@ -28,7 +28,8 @@ extern "C" int ss_attn_simt(const void* q, int64_t q_stride, void* out, int64_t 
                                              page_size, num_pages, scale, window, gate, err, stream, softcap, sinks, keep, across);
 }
 
-// tile_req null: a decode step (one token a request).  parts > 1: a row's slices of keys on that many blocks; `part` and
+// tile_req null: a decode step (one token a request), of the kernel that takes whole slices for heads of up to 128 if there is
+// scratch for them or one slice is all (max_slices).  parts > 1: a row's slices of keys on that many blocks; `part` and
 // `part_ml` then hold max_slices slices a (row, output head), at least as many as the longest request has.
 extern "C" int ss_attn_f32(const float* q, int64_t q_stride, float* out, int64_t out_stride, const float* kv,
                            const int32_t* tables, int max_blocks, const int32_t* tile_req, const int32_t* tile_q0, int n_tiles,

@@ -15,8 +15,8 @@
 //
 // Bound by issue: 70 % of its instructions are the multiply-adds, and three blocks of four warps an SM issue on about half
 // of the cycles.  Against attention_simt.cuh (a tile of 16 tokens of one query head, keys in series, no copies ahead):
-// 777 tokens of two requests, one behind 300 cached ones, 28 heads of 128 on 4: 551 -> 209 us; four decoded tokens behind
-// 500 on average, 12 heads of 128 on 2: 266 -> 33 us; 20 behind 800, 28 on 4: 602 -> 102 us.
+// 777 tokens of two requests, one behind 300 cached ones, 28 heads of 128 on 4: 551 -> 209 us.  Decode steps with heads of up
+// to 128 have a kernel of their own (attn_f32_decode_kernel).
 #pragma once
 
 #include "common.cuh"
@@ -320,74 +320,317 @@ __global__ void __launch_bounds__(AF_THREADS, D <= 128 ? 3 : 1) attn_f32_kernel(
     }
 }
 
-// Joins the slices of every row: a warp to a (row, output head).
-template <int D>
-__global__ void __launch_bounds__(AF_THREADS) attn_f32_join_kernel(const AttnF32Args g) {
+// One token a request: a block takes AFD_RT rows of a request and a slice of keys (gridDim.z blocks deal a request's slices
+// out among them), whose keys and values it fetches in one go.  The scores of the slice's tiles are formed side by side, a
+// warp to 16 keys; a tile's maximum so far is that of the tiles before it and its own, whoever formed them, so the
+// exponentials, the sums (a thread to 4 rows and 2 elements) and the joins are those of attn_f32_kernel, bit for bit.
+//
+// BOTH: keys and values have buffers of their own and travel together, one block an SM: for a grid of one wave, whose time
+// is the latency of its loads.  Otherwise values follow into the keys' buffer and three blocks an SM cover for each other.
+//
+// Bound by shared memory: a load brings 128 bytes a cycle to an SM's registers, also where lanes share a word, so a slice's
+// scores take 3,700 cycles and its outputs as many, beside 3,000 in which its 131 KB arrive.  (Products of 4 x 4 a thread, on
+// two warps, need half of that and run longer all the same: 439 us where these take 359, a warp has no other beside it.)
+// With its join, against attn_f32_kernel (four tiles of a slice one after another), us, 12 heads of 128 on 2: four requests
+// of 2,000 tokens 33.8 -> 17.0; 28 on 4: 20 of 800 79 -> 30, 20 of 16,000 1320 -> 359 (the memory takes 180), 200 of 300
+// 150 -> 88, one of 100 17.5 -> 8.5; 14 of 64 on 2: 256 of 1,000 240 -> 113.
+#define AFD_RT 8
+#define AFD_THREADS 256
+#define AFD_PS 8
+
+template <int D, bool BOTH>
+constexpr int afd_smem_bytes() {
+    return (AFD_RT * (D + 4) + (BOTH ? 2 : 1) * AF_SLICE * (D + 4) + AF_SLICE * AFD_PS + (8 + AF_SLICE / AF_BN + 2) * AFD_RT) * 4;
+}
+
+template <int D, bool BOTH>
+__global__ void __launch_bounds__(AFD_THREADS, BOTH ? 1 : 3) attn_f32_decode_kernel(const AttnF32Args g) {
+    static_assert(AF_SLICE == 128 && AF_BN == 32 && D <= 128, "eight warps of 16 keys, 128 threads a half of the rows");
+    constexpr int KS = D + 4, TPS = AF_SLICE / AF_BN, C4 = D / 4;
+    extern __shared__ __align__(16) float afd_smem[];
+    float* Qs = afd_smem;
+    float* Ks = Qs + AFD_RT * KS;
+    float* Vs = BOTH ? Ks + AF_SLICE * KS : Ks;
+    float* Ps = Ks + (BOTH ? 2 : 1) * AF_SLICE * KS;  // [key][row]
+    float* top_s = Ps + AF_SLICE * AFD_PS;            // [warp][row]: the largest score of the warp's 16 keys
+    float* alpha_s = top_s + 8 * AFD_RT;              // [tile][row]: the factor of what was summed before the tile
+    float* ml_s = alpha_s + TPS * AFD_RT;              // [row]: maximum and sum of the only slice
+
     pdl_launch_dependents();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int G = g.n_q / g.n_kv, n_heads = g.across ? g.n_kv * g.n_kv : g.n_kv, u = blockIdx.x % n_heads;
+    const int per_request = (G + AFD_RT - 1) / AFD_RT, block = blockIdx.x / n_heads;
+    const HeadPair hp = head_pair(u, g.n_kv, g.across);
+    const int r = block / per_request, row0 = (block % per_request) * AFD_RT, rows = min(AFD_RT, G - row0);
     pdl_wait();
-    const int lane = threadIdx.x & 31;
-    const int G = g.n_q / g.n_kv, heads = g.across ? g.n_q * g.n_kv : g.n_q;
-    const int64_t item = (int64_t)blockIdx.x * (AF_THREADS / 32) + (threadIdx.x >> 5);
-    const int row = (int)(item / heads), h_out = (int)(item % heads);
-    if (row >= g.n_rows || row >= g.q_start[g.n_requests]) return;
-    int lo = 0, hi = g.n_requests;  // the request of the row: the last one that starts at or before it
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (g.q_start[mid] <= row) lo = mid;
-        else hi = mid;
+    const int token = g.q_start[r], token_end = g.q_start[r + 1], seq_len = g.seq_lens[r];
+    const int q_len = token_end - token;
+    if (q_len <= 0) return;  // a padding request of a captured step
+    const int pos = seq_len - q_len, lowest = key_floor(pos, g.window);
+    const int32_t* table = g.tables + (int64_t)r * g.max_blocks;
+    const KeyTiles walk = key_tiles(lowest, pos, g.keep, AF_BN);
+    const int s_first = walk.kept > 0 ? 0 : walk.first / TPS, s_end = pos < 0 ? 0 : pos / AF_SLICE + 1;
+    const bool alone = g.part == nullptr;  // no request has a second slice
+    if (!alone && s_first + (int)blockIdx.z >= s_end) return;
+
+    const int64_t to_value = (int64_t)(g.n_kv + hp.value - hp.key) * g.page_size * D;  // from a key to its value
+    const int tx = lane & 7, ty = lane >> 3;              // scores: keys 16 warp + tx (+ 8), rows ty (+ 4)
+    const int half = tid >> 6 & 1, d = (tid & 63) * 2;   // outputs: rows 4 half .. + 3, elements d and d + 1
+    // the output of a row of which the only slice has maximum m, sum l and output v
+    auto finish = [&](int row, float m, float l, float v0, float v1) {
+        const int h = hp.key * G + row0 + row;
+        float tot_m = g.sinks ? g.sinks[h] : -INFINITY, tot_l = g.sinks ? 1.f : 0.f;
+        const float2 f = af_join(tot_m, tot_l, m, l);
+        float* out = g.out + (int64_t)token * g.out_stride + (int64_t)(u * G + row0 + row) * D + d;
+        const float* gate = g.gate ? g.gate + (int64_t)token * g.q_stride + (int64_t)h * D + d : nullptr;
+        out[0] = af_finish(af_mix(0.f, f, v0), tot_l, gate);
+        out[1] = af_finish(af_mix(0.f, f, v1), tot_l, gate ? gate + 1 : nullptr);
+    };
+    // (asked for in front of the keys, behind which it would queue)
+    float4 query = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tid < AFD_RT * C4 && tid / C4 < rows) {
+        const float* src = g.q + (int64_t)token * g.q_stride + (int64_t)(hp.key * G + row0 + tid / C4) * D + tid % C4 * 4;
+        query = make_float4(src[0], src[1], src[2], src[3]);
     }
-    const int r = lo, pos = g.seq_lens[r] - (g.q_start[r + 1] - row);
+    bool first = true;
+    for (int slice = s_first + (int)blockIdx.z; slice < s_end; slice += (int)gridDim.z) {
+        int seen = 0;  // the tiles of the slice that hold a key in sight
+#pragma unroll
+        for (int t = 0; t < TPS; ++t)
+            if (slice * TPS + t < walk.kept || (slice * TPS + t >= walk.first && slice * TPS + t <= pos / AF_BN)) seen |= 1 << t;
+        if (seen == 0) continue;
+        const bool mine = seen >> (warp / 2) & 1;
+        // ---- keys (and values): a warp fetches the 16 whose scores it forms; those out of sight are zero
+        int64_t key_at = -1;
+        if (mine && lane < 16) {
+            const int key = slice * AF_SLICE + warp * 16 + lane;
+            if ((key >= lowest || key < g.keep) && key <= pos) {
+                const int64_t page = table[key / g.page_size];
+                if (page >= g.num_pages) atomicOr(g.err, SS_ERR_PAGE_RANGE);
+                else if (page >= 0) key_at = ((page * 2 * g.n_kv + hp.key) * g.page_size + key % g.page_size) * D;
+            }
+        }
+        auto fetch = [&](float* to, int64_t further) {
+            // whole rows to an instruction where they fill its lanes, otherwise 8 lanes to a row (359 against 374 us for 20
+            // requests behind 16,000 with heads of 128; 339 against 265 for 100 behind 700 with heads of 96)
+            constexpr bool WHOLE = 32 % C4 == 0;
+            constexpr int LANES = WHOLE ? C4 : 8, RPI = 32 / LANES;
+            const int c0 = lane % LANES * 4;
+#pragma unroll
+            for (int i = 0; i < 16 / RPI; ++i) {
+                const int64_t at = __shfl_sync(0xffffffffu, key_at, i * RPI + lane / LANES);
+                const float* src = g.kv + (at >= 0 ? at + further + c0 : 0);
+                float* dst = to + (warp * 16 + i * RPI + lane / LANES) * KS + c0;
+#pragma unroll
+                for (int c = 0; c < D; c += LANES * 4)
+                    if (WHOLE || c + c0 < D) cp_async16(dst + c, src + c, at >= 0);
+            }
+        };
+        if (!first) __syncthreads();  // everyone is done with the slice before
+        if (mine) fetch(Ks, 0);
+        cp_async_commit();
+        if (BOTH && mine) fetch(Vs, to_value);
+        cp_async_commit();
+        if (first) {
+            if (tid < AFD_RT * C4) *reinterpret_cast<float4*>(&Qs[tid / C4 * KS + tid % C4 * 4]) = query;
+            __syncthreads();
+            first = false;
+        }
+        cp_async_wait<1>();
+        __syncwarp();
+
+        // ---- scores
+        float s[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+        if (mine) {
+            const float *q0 = Qs + ty * KS, *k0 = Ks + (warp * 16 + tx) * KS;
+#pragma unroll (BOTH ? 8 : 4)
+            for (int e = 0; e < D; e += 4) {
+                float4 q4[2], k4[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    q4[i] = *reinterpret_cast<const float4*>(q0 + i * 4 * KS + e);
+                    k4[i] = *reinterpret_cast<const float4*>(k0 + i * 8 * KS + e);
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        s[i][k] = fmaf(q4[i].x, k4[k].x, s[i][k]);
+                        s[i][k] = fmaf(q4[i].y, k4[k].y, s[i][k]);
+                        s[i][k] = fmaf(q4[i].z, k4[k].z, s[i][k]);
+                        s[i][k] = fmaf(q4[i].w, k4[k].w, s[i][k]);
+                    }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            float top = -INFINITY;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int key = slice * AF_SLICE + warp * 16 + tx + 8 * k;
+                const bool ok = mine && ty + 4 * i < rows && key <= pos && (key >= lowest || key < g.keep);
+                const float x = __fmul_rn(s[i][k], g.scale);
+                s[i][k] = ok ? (g.softcap > 0.f ? __fmul_rn(g.softcap, tanhf(x / g.softcap)) : x) : -INFINITY;
+                top = fmaxf(top, s[i][k]);
+            }
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            if (tx == 0) top_s[warp * AFD_RT + ty + 4 * i] = top;
+        }
+        __syncthreads();
+        if (!BOTH && mine) fetch(Vs, to_value);  // (over the warp's own keys)
+        if (!BOTH) cp_async_commit();
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int row = ty + 4 * i;
+            float before = -INFINITY, now = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                const float top = top_s[w * AFD_RT + row];
+                if (w < (warp & ~1)) before = fmaxf(before, top);
+                if (w <= (warp | 1)) now = fmaxf(now, top);
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+                Ps[(warp * 16 + tx + 8 * k) * AFD_PS + row] = s[i][k] == -INFINITY ? 0.f : expf(__fsub_rn(s[i][k], now));  // (a NaN has no part in `now`, and stays)
+            if (tx == 0 && !(warp & 1)) alpha_s[warp / 2 * AFD_RT + row] = before == -INFINITY ? 0.f : expf(__fsub_rn(before, now));
+        }
+        cp_async_wait<0>();
+        __syncthreads();
+
+        // ---- outputs: warps 0 to 3; meanwhile a lane of warp 4 to each row sums the probabilities
+        float acc[4][2], l = 0.f;
+        if (warp < 4) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.f;
+            if (d < D)
+                for (int t = 0; t < TPS; ++t) {
+                    if (!(seen >> t & 1)) continue;
+                    if (seen & ((1 << t) - 1)) {
+                        const float4 a = *reinterpret_cast<const float4*>(&alpha_s[t * AFD_RT + half * 4]);
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            acc[0][e] = __fmul_rn(acc[0][e], a.x); acc[1][e] = __fmul_rn(acc[1][e], a.y);
+                            acc[2][e] = __fmul_rn(acc[2][e], a.z); acc[3][e] = __fmul_rn(acc[3][e], a.w);
+                        }
+                    }
+#pragma unroll 8
+                    for (int k = t * AF_BN; k < (t + 1) * AF_BN; ++k) {
+                        const float4 p = *reinterpret_cast<const float4*>(&Ps[k * AFD_PS + half * 4]);
+                        const float2 v = *reinterpret_cast<const float2*>(&Vs[k * KS + d]);
+                        acc[0][0] = fmaf(p.x, v.x, acc[0][0]); acc[0][1] = fmaf(p.x, v.y, acc[0][1]);
+                        acc[1][0] = fmaf(p.y, v.x, acc[1][0]); acc[1][1] = fmaf(p.y, v.y, acc[1][1]);
+                        acc[2][0] = fmaf(p.z, v.x, acc[2][0]); acc[2][1] = fmaf(p.z, v.y, acc[2][1]);
+                        acc[3][0] = fmaf(p.w, v.x, acc[3][0]); acc[3][1] = fmaf(p.w, v.y, acc[3][1]);
+                    }
+                }
+        } else if (warp == 4 && lane < rows) {
+            for (int t = 0; t < TPS; ++t) {
+                if (!(seen >> t & 1)) continue;
+                if (seen & ((1 << t) - 1)) l = __fmul_rn(l, alpha_s[t * AFD_RT + lane]);
+#pragma unroll 16
+                for (int k = t * AF_BN; k < (t + 1) * AF_BN; ++k) l = __fadd_rn(l, Ps[k * AFD_PS + lane]);
+            }
+            float slice_m = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) slice_m = fmaxf(slice_m, top_s[w * AFD_RT + lane]);
+            if (alone) {
+                ml_s[lane * 2] = slice_m;
+                ml_s[lane * 2 + 1] = l;
+            } else {
+                g.part_ml[((int64_t)token * (n_heads * G) + u * G + row0 + lane) * g.max_slices + slice] = make_float2(slice_m, l);
+            }
+        }
+        if (alone) __syncthreads();
+        if (warp < 4 && d < D)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int row = half * 4 + i;
+                if (row >= rows) break;
+                if (alone) {
+                    finish(row, ml_s[row * 2], ml_s[row * 2 + 1], acc[i][0], acc[i][1]);
+                } else {
+                    const int64_t at = ((int64_t)token * (n_heads * G) + u * G + row0 + row) * g.max_slices + slice;
+                    *reinterpret_cast<float2*>(&g.part[at * D + d]) = make_float2(acc[i][0], acc[i][1]);
+                }
+            }
+    }
+    if (alone && first && warp < 4 && d < D)  // a request without a key
+        for (int i = half * 4; i < min(half * 4 + 4, rows); ++i) finish(i, -INFINITY, 0.f, 0.f, 0.f);
+}
+
+// Joins the slices of every row: a block to a (row, output head), a thread to an element.
+template <int D>
+__global__ void __launch_bounds__((D + 31) / 32 * 32) attn_f32_join_kernel(const AttnF32Args g) {
+    pdl_launch_dependents();
+    const int d = threadIdx.x, lane = d & 31;
+    const int G = g.n_q / g.n_kv, heads = g.across ? g.n_q * g.n_kv : g.n_q;
+    const int64_t item = blockIdx.x;
+    const int row = (int)(item / heads), h_out = (int)(item % heads);
     const HeadPair hp = head_pair(h_out / G, g.n_kv, g.across);
     const int h = hp.key * G + h_out % G;
-    constexpr int NC = (D + 127) / 128;
-    float m = g.sinks ? g.sinks[h] : -INFINITY, l = g.sinks ? 1.f : 0.f;
-    float tot[NC][4];
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) tot[c][e] = 0.f;
+    pdl_wait();
+    // the request of the row: its own number where every request has one token, otherwise the last that starts at or before it
+    int r = row, ends = 0;
+    if (row >= g.n_requests || g.q_start[row] != row || (ends = g.q_start[row + 1]) != row + 1) {
+        if (row >= g.q_start[g.n_requests]) return;
+        int hi = g.n_requests;
+        r = 0;
+        while (hi - r > 1) {
+            const int mid = (r + hi) >> 1;
+            if (g.q_start[mid] <= row) r = mid;
+            else hi = mid;
+        }
+        ends = g.q_start[r + 1];
+    }
+    const int pos = g.seq_lens[r] - (ends - row);
+    float m = g.sinks ? g.sinks[h] : -INFINITY, l = g.sinks ? 1.f : 0.f, total = 0.f;
     // the slices that hold a key the row sees: those of the kept keys, then those from its lowest key on
     const int first = key_floor(pos, g.window) / AF_SLICE, last = pos < 0 ? -1 : pos / AF_SLICE;
     const int kept = g.keep > 0 ? min((g.keep - 1) / AF_SLICE + 1, first) : 0;
     const int count = last < 0 ? 0 : kept + last - first + 1;
     const int64_t at0 = item * g.max_slices;
-    constexpr int AHEAD = 4;
-    for (int j0 = 0; j0 < count; j0 += AHEAD) {
-        float2 ml[AHEAD];
-        float4 v[AHEAD][NC];
+    auto slice_at = [&](int j) { return at0 + (j < kept ? j : first + (j - kept)); };
+    // 32 slices at a time, whose loads travel together: their factors side by side, a lane to each (a maximum over those
+    // before is the same in any order); what is left to do in order is a product, a product and a sum a slice
+    for (int j0 = 0; j0 < count; j0 += 32) {
+        const int n = min(32, count - j0);
+        float2 ml = make_float2(-INFINITY, 0.f);
+        if (lane < n) ml = g.part_ml[slice_at(j0 + lane)];
+        float v[32];
 #pragma unroll
-        for (int a = 0; a < AHEAD; ++a) {
-            const int j = j0 + a;
-            if (j >= count) break;
-            const int64_t at = at0 + (j < kept ? j : first + (j - kept));
-            ml[a] = g.part_ml[at];
-#pragma unroll
-            for (int c = 0; c < NC; ++c)
-                if ((lane + 32 * c) * 4 < D) v[a][c] = *reinterpret_cast<const float4*>(&g.part[at * D + (lane + 32 * c) * 4]);
+        for (int i = 0; i < 32; ++i) {
+            if (i % 8 == 0 && i >= n) break;
+            v[i] = d < D && i < n ? g.part[slice_at(j0 + i) * D + d] : 0.f;
         }
+        float top = ml.x;
 #pragma unroll
-        for (int a = 0; a < AHEAD; ++a) {
-            if (j0 + a >= count) break;
-            const float2 f = af_join(m, l, ml[a].x, ml[a].y);
+        for (int o = 1; o < 32; o <<= 1) {
+            const float below = __shfl_up_sync(0xffffffffu, top, o);
+            if (lane >= o) top = fmaxf(top, below);
+        }
+        const float before = __shfl_up_sync(0xffffffffu, top, 1), all = __shfl_sync(0xffffffffu, top, 31);
+        float m_lane = lane == 0 ? m : fmaxf(m, before), l_lane = 0.f;
+        const float2 f = af_join(m_lane, l_lane, ml.x, ml.y);
+        m = fmaxf(m, all);
 #pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                if ((lane + 32 * c) * 4 >= D) break;
-                tot[c][0] = af_mix(tot[c][0], f, v[a][c].x);
-                tot[c][1] = af_mix(tot[c][1], f, v[a][c].y);
-                tot[c][2] = af_mix(tot[c][2], f, v[a][c].z);
-                tot[c][3] = af_mix(tot[c][3], f, v[a][c].w);
-            }
+        for (int i = 0; i < 32; ++i) {
+            if (i >= n) break;
+            const float2 fi = make_float2(__shfl_sync(0xffffffffu, f.x, i), __shfl_sync(0xffffffffu, f.y, i));
+            l = af_mix(l, fi, __shfl_sync(0xffffffffu, ml.y, i));
+            total = af_mix(total, fi, v[i]);
         }
     }
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int d = (lane + 32 * c) * 4 + e;
-            if (d < D)
-                g.out[(int64_t)row * g.out_stride + (int64_t)h_out * D + d] =
-                    af_finish(tot[c][e], l, g.gate ? g.gate + (int64_t)row * g.q_stride + (int64_t)h * D + d : nullptr);
-        }
+    if (d < D)
+        g.out[(int64_t)row * g.out_stride + (int64_t)h_out * D + d] =
+            af_finish(total, l, g.gate ? g.gate + (int64_t)row * g.q_stride + (int64_t)h * D + d : nullptr);
+}
+
+template <int D>
+int launch_attn_f32_join(const AttnF32Args& g, cudaStream_t stream) {
+    const int64_t items = (int64_t)g.n_rows * (g.across ? g.n_q * g.n_kv : g.n_q);
+    ss_launch(attn_f32_join_kernel<D>, dim3((unsigned)items), dim3((D + 31) / 32 * 32), 0, stream, g);
+    return SS_LAUNCH_CHECK();
 }
 
 template <int D, int RT>
@@ -398,17 +641,33 @@ int launch_attn_f32_rows(const AttnF32Args& g, int n_tiles, int parts, cudaStrea
     const int blocks = g.tile_req ? n_tiles * (64 / RT) : g.n_requests * ((g.n_q / g.n_kv + RT - 1) / RT);
     const int heads = g.across ? g.n_kv * g.n_kv : g.n_kv;
     ss_launch(attn_f32_kernel<D, RT>, dim3(blocks * heads, 1, parts), dim3(AF_THREADS), smem, stream, g);
-    if (g.part) {
-        const int64_t items = (int64_t)g.n_rows * heads * (g.n_q / g.n_kv);
-        ss_launch(attn_f32_join_kernel<D>, dim3((unsigned)((items + AF_THREADS / 32 - 1) / (AF_THREADS / 32))), dim3(AF_THREADS), 0, stream, g);
-    }
-    return SS_LAUNCH_CHECK();
+    const int rc = SS_LAUNCH_CHECK();
+    return rc || !g.part ? rc : launch_attn_f32_join<D>(g, stream);
 }
 
 // 32 rows of a prompt portion to a block (64, with 8 warps and half the blocks: 257 us where 32 take 209, 777 tokens at the 7B sizes); a decode
-// step's rows of one request in tiles of 16.
+// step's rows of one request in tiles of 16, where attn_f32_decode_kernel does not take them (wider heads, whose slice passes
+// an SM's shared memory, and slices that pass the scratch memory's bound).
+template <int D, bool BOTH>
+int launch_attn_f32_decode(const AttnF32Args& g, dim3 grid, cudaStream_t stream) {
+    constexpr int smem = afd_smem_bytes<D, BOTH>();
+    static SsPerDevice opted;
+    if (int rc = ss_opt_in_smem(attn_f32_decode_kernel<D, BOTH>, smem, opted)) return rc;
+    ss_launch(attn_f32_decode_kernel<D, BOTH>, grid, dim3(AFD_THREADS), smem, stream, g);
+    return SS_LAUNCH_CHECK();
+}
+
 template <int D>
 int launch_attn_f32(const AttnF32Args& g, int n_tiles, int parts, cudaStream_t stream) {
+    if constexpr (D <= 128)
+        if (g.tile_req == nullptr && (g.part != nullptr || g.max_slices == 1)) {
+            const int G = g.n_q / g.n_kv, heads = g.across ? g.n_kv * g.n_kv : g.n_kv;
+            const int64_t blocks = (int64_t)g.n_requests * heads * ((G + AFD_RT - 1) / AFD_RT);
+            const dim3 grid((unsigned)blocks, 1, parts);
+            const int rc = blocks * parts <= ss_sm_count() ? launch_attn_f32_decode<D, true>(g, grid, stream)
+                                                           : launch_attn_f32_decode<D, false>(g, grid, stream);
+            return rc || !g.part ? rc : launch_attn_f32_join<D>(g, stream);
+        }
     if (g.tile_req == nullptr) return launch_attn_f32_rows<D, 16>(g, n_tiles, parts, stream);
     return launch_attn_f32_rows<D, 32>(g, n_tiles, parts, stream);
 }

@@ -716,18 +716,29 @@ def float32_key_parts(blocks: int, slices: int, rows: int, heads: int, head_dim:
     return parts if parts > 1 and rows * heads * slices * (head_dim + 2) * 4 <= FLOAT32_SCRATCH else 1
 
 
+def float32_decode_parts(blocks: int, slices: int, rows: int, heads: int, head_dim: int, sms: int | None = None) -> int:
+    """Blocks to which the ``slices`` slices of a request's keys are dealt out in a decode step; ``blocks``: the tiles of at
+    most 8 rows times the heads.  Up to 8 waves of one block an SM, so that requests of unlike lengths even out.  1 with more than one
+    slice: the slices would pass the scratch memory's bound, and `float32_key_parts` decides."""
+    if slices == 1 or rows * heads * slices * (head_dim + 2) * 4 > FLOAT32_SCRATCH:
+        return 1
+    return max(2, min(slices, 8 * (sms or sm_count()) // max(blocks, 1)))
+
+
 def paged_attention_float32(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, block_tables: torch.Tensor, ctx, n_q: int,
                             n_kv: int, head_dim: int, scale: float, window: int = 0, chunk: int = 0,
                             gate: torch.Tensor | None = None, softcap: float = 0.0, sinks: torch.Tensor | None = None,
                             keep: int = 0, across: bool = False) -> None:
     """`paged_attention_simt` for the rows of a step in float32, with the arguments of `paged_attention`: the kernel that
     tiles rows of a kv head's group (32 of a prompt portion, whose list has tiles of 64; 16 of a decode step) with 32 keys and splits
-    a row's keys over several blocks where there are few rows."""
+    a row's keys over several blocks where there are few rows; in decode steps with heads of up to 128 the one that takes a
+    slice of 128 keys at a time."""
     _need(out, torch.float32, "attention output")
     _check_sinks(sinks, n_q)
     _need(kv, torch.float32, "kv pages")
     group, heads = n_q // n_kv, n_kv * n_q if across else n_q
-    if ctx.is_decode_only:
+    decode_only = ctx.is_decode_only
+    if decode_only:
         tile_req = tile_row0 = None
         tiles = ctx.num_requests * ((group + 15) // 16)
         longest = ctx.extras.get("static_max_seq_len") or ctx.max_seq_len
@@ -737,7 +748,12 @@ def paged_attention_float32(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tens
     for name, t in (("block_tables", block_tables), ("q_start", ctx.q_start), ("seq_lens", ctx.seq_lens)):
         _need(t, torch.int32, name)
     slices = max(1, -(-longest // FLOAT32_SLICE))
-    parts = float32_key_parts(tiles * heads // group, slices, qkv.shape[0], heads, head_dim, sm_count(qkv.device))
+    parts = 1
+    if decode_only and head_dim <= 128:  # (wider heads: a slice's keys and values pass an SM's shared memory)
+        parts = float32_decode_parts(ctx.num_requests * ((group + 7) // 8) * (heads // group), slices, qkv.shape[0], heads,
+                                     head_dim, sm_count(qkv.device))
+    if parts == 1:
+        parts = float32_key_parts(tiles * heads // group, slices, qkv.shape[0], heads, head_dim, sm_count(qkv.device))
     part = part_ml = None
     if parts > 1:
         part = torch.empty((qkv.shape[0], heads, slices, head_dim), dtype=torch.float32, device=qkv.device)
@@ -2865,7 +2881,7 @@ def set_programmatic_launch(enabled: bool) -> None:
 
 
 __all__ = ["KernelError", "KernelBuildError", "embedding", "add_rmsnorm", "hc_norm", "linear_hc_rmsnorm", "rope_norm_cache", "glu_limited", "gate_up_glu", "sigmoid_gate", "key_span", "rope_and_cache", "swiglu",
-           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "few_prefill_keys", "paged_attention_decode", "paged_attention_decode_spread", "spreads_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
+           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "float32_decode_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "few_prefill_keys", "paged_attention_decode", "paged_attention_decode_spread", "spreads_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
            "attention_library", "group_norm", "round_stream", "conv_silu", "SCAN_FEW", "only_short_portions", "ssm_scan", "router", "moe_experts", "moe_combine",
            "norm_rope_cache", "turn_heads", "soft_cap", "embed_sum", "matrix_cell", "cell_output", "gated_recurrence", "xielu",
            "DiffPair", "diff_in_attention", "diff_combine", "heads_to_pages", "branch_norm", "PairedOutput", "WeighedTerms",

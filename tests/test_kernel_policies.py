@@ -105,6 +105,17 @@ def test_expert_tiles_and_float32_key_parts():
     assert F.float32_key_parts(8, 20, 5000, 28, 128, sms=SMS) == 1  # the slices' scratch would pass its bound
 
 
+def test_float32_decode_deals_out_slices_within_the_scratch_memory():
+    for blocks in (1, 8, 100, 5000):
+        for slices in (2, 16, 250):
+            parts = F.float32_decode_parts(blocks, slices, 4, 12, 128, sms=SMS)
+            assert 2 <= parts <= slices and (parts == 2 or blocks * parts <= 8 * SMS)  # (2: the slices meet in scratch memory)
+    assert F.float32_decode_parts(8, 1, 4, 12, 128, sms=SMS) == 1
+    bound = F.FLOAT32_SCRATCH // (12 * 16 * (128 + 2) * 4)  # rows whose slices just fit
+    assert F.float32_decode_parts(8, 16, bound, 12, 128, sms=SMS) > 1 == F.float32_decode_parts(8, 16, bound + 1, 12, 128, sms=SMS)
+
+
+
 def paged_layer(dim, page_size=16, **kind):
     from types import SimpleNamespace
     import torch

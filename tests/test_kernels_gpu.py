@@ -982,6 +982,39 @@ def test_float32_attention_gives_a_row_the_same_bits_however_its_step_was_cut(mo
     ops().check_errors(torch.device(DEV))
 
 
+# one slice and several, few blocks (keys and values side by side) and many, groups of more than 8 and of an odd number, heads
+# that do and do not fill a copy's lanes; windows with kept keys, chunks, sinks, a soft cap, a gate, values of every kv head
+@pytest.mark.parametrize("d, n_q, n_kv, n, longest, window, chunk, keep, options", [
+    (128, 12, 2, 4, 900, 0, 0, 0, ""), (128, 14, 2, 40, 700, 0, 0, 0, "sinks"), (64, 20, 2, 3, 128, 0, 0, 0, "gate"),
+    (48, 9, 1, 70, 300, 0, 0, 0, "softcap"), (80, 6, 2, 30, 600, 37, 0, 70, "sinks"), (96, 8, 8, 2, 500, 0, 160, 0, "gate"),
+    (16, 4, 2, 5, 400, 0, 0, 0, "across"), (112, 3, 3, 60, 129, 1, 0, 0, "softcap sinks"), (32, 2, 2, 1, 1, 0, 0, 0, "sinks")])
+def test_float32_decode_of_whole_slices_gives_the_bits_of_tiles_in_line(monkeypatch, d, n_q, n_kv, n, longest, window, chunk, keep, options):
+    from types import SimpleNamespace
+    from slipstream_b200.ops import functions
+    rng = np.random.default_rng(d + n)
+    lens = [longest] + [int(v) for v in rng.integers(1, longest + 1, n - 1)]
+    q, kv, table, _, seq_lens = make_attention_case(torch.float32, lens, [1] * n, n_q, n_kv, d, 16, seed=d)
+    width = n_q * d * (2 if "gate" in options else 1)
+    rows = torch.randn(n, width, device=DEV)
+    rows[:, :n_q * d] = q.reshape(n, -1)
+    sinks = torch.randn(n_q, device=DEV) if "sinks" in options else None
+    across = "across" in options
+    starts = torch.arange(n + 1, dtype=torch.int32, device=DEV)
+    ctx = SimpleNamespace(is_decode_only=True, num_requests=n, max_seq_len=longest, seq_lens=seq_lens, q_start=starts, extras={})
+    outs = []
+    for whole in (True, False):
+        if not whole:  # no scratch memory, and a slice more than the requests have: the kernel of tiles, a block to a row
+            monkeypatch.setattr(functions, "FLOAT32_SCRATCH", 0)
+            ctx.extras["static_max_seq_len"] = longest + 128
+        out = torch.full((n, n_q * d * (n_kv if across else 1)), 7.0, device=DEV)
+        ops().paged_attention_float32(rows, out, kv, table, ctx, n_q, n_kv, d, 0.3, window, chunk,
+                                      rows[:, n_q * d:] if "gate" in options else None, 20.0 if "softcap" in options else 0.0,
+                                      sinks, keep, across)
+        outs.append(out)
+    assert not (outs[0] == 7.0).any() and torch.equal(*outs)
+    ops().check_errors(torch.device(DEV))
+
+
 # widths and depths off the 128-row weight tiles and 64-wide steps of K; tokens that make every tile width (16, 32, 64, 128), all on
 # one expert (several tiles of it) or spread out, some experts without a token
 @pytest.mark.parametrize("hidden, ff, experts, top, gated", [(200, 64, 5, 2, True), (72, 192, 3, 1, True), (264, 320, 8, 3, True),

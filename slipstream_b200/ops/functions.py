@@ -233,14 +233,16 @@ def attention_library(head_dim: int) -> ctypes.CDLL:
     return lib  # type: ignore[return-value]
 
 
+_error_words: dict[torch.device, torch.Tensor] = {}
+
+
 def error_word(device: torch.device) -> torch.Tensor:
-    key = ("err", device)
-    word = _state.get(key)
+    word = _error_words.get(device)
     if word is None:
         with torch.inference_mode(False):  # the word is cleared in place later, from any mode
             word = torch.zeros(1, dtype=torch.int32, device=device)
-        _state[key] = word
-    return word  # type: ignore[return-value]
+        _error_words[device] = word
+    return word
 
 
 _ERR_NAMES = {1: "a token id outside the vocabulary", 2: "a cache slot outside the pool",
@@ -276,13 +278,15 @@ def sm_count(device: torch.device | int | None = None) -> int:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_get_device = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream() -> int:
     """Handle of the current CUDA stream (every wrapper below asks for it, so the short way is taken when
-    this torch has it)."""
-    if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+    this torch has it: without `torch.cuda.current_device`, which first asks whether CUDA is initialised; the tensors of
+    the call are on the device, so it is)."""
+    if _raw_stream is not None and _get_device is not None:
+        return _raw_stream(_get_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -558,7 +562,7 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor | None = None, block: int | 
     if block < 1 or inter % block:
         raise KernelError(f"block {block} does not divide the {inter} features")
     if out is None:
-        out = torch.empty((n, inter), dtype=gate_up.dtype, device=gate_up.device)
+        out = gate_up.new_empty((n, inter))
     _need(out, gate_up.dtype, "swiglu output")
     _check(ops_library().ss_swiglu(gate_up.data_ptr(), out.data_ptr(), n, inter, block, _code(gate_up.dtype),
                                    _stream()), "swiglu")
@@ -609,7 +613,7 @@ def gemm_float32(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | Non
         _need(bias, torch.float32, "bias")
         if bias.numel() != n:
             raise KernelError("bias has the wrong size or dtype")
-    out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+    out = x.new_empty((m, n))
     _check(gemm_library().ss_gemm_f32(x.data_ptr(), weight.data_ptr(), _ptr(bias), out.data_ptr(), m, n, k, n,
                                       error_word(x.device).data_ptr(), _stream()), "gemm_f32")
     return out
@@ -754,16 +758,18 @@ def paged_attention_float32(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tens
                                      head_dim, sm_count(qkv.device))
     if parts == 1:
         parts = float32_key_parts(tiles * heads // group, slices, qkv.shape[0], heads, head_dim, sm_count(qkv.device))
-    part = part_ml = None
-    if parts > 1:
-        part = torch.empty((qkv.shape[0], heads, slices, head_dim), dtype=torch.float32, device=qkv.device)
-        part_ml = torch.empty((qkv.shape[0], heads, slices, 2), dtype=torch.float32, device=qkv.device)
+    part = part_at = part_ml_at = None
+    if parts > 1:  # the slices' outputs, and behind them their maxima and sums
+        count = qkv.shape[0] * heads * slices
+        part = qkv.new_empty(count * (head_dim + 2))
+        part_at = part.data_ptr()
+        part_ml_at = part_at + count * head_dim * 4
     _check(attention_library(head_dim).ss_attn_f32(
         qkv.data_ptr(), qkv.shape[1], out.data_ptr(), out.shape[1], kv.data_ptr(), block_tables.data_ptr(),
         block_tables.shape[1], _ptr(tile_req), _ptr(tile_row0), tiles, ctx.q_start.data_ptr(), ctx.seq_lens.data_ptr(),
         ctx.num_requests, n_q, n_kv, kv.shape[3], kv.shape[0], float(scale), key_span(window, chunk),
         _gate_ptr(gate, qkv, qkv.shape[1]), error_word(qkv.device).data_ptr(), _stream(), float(softcap or 0.0), _ptr(sinks),
-        _kept(keep, window), int(across), _ptr(part), _ptr(part_ml), slices, qkv.shape[0], parts), "attn_f32")
+        _kept(keep, window), int(across), part_at, part_ml_at, slices, qkv.shape[0], parts), "attn_f32")
     if parts > 1:
         _launches[0] += 1  # the kernel that joins the slices
 

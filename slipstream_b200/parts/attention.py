@@ -383,7 +383,7 @@ class PagedAttention(Mixer):
             out = ops.talking_attention(q, layer.kv, meta.block_tables, ctx, self.num_heads, self.num_kv_heads, self.head_dim, self.scale,
                                         self.talk_table, gate, **mask)
         else:
-            out = torch.empty((x.shape[0], width), dtype=x.dtype, device=x.device)
+            out = qkv.new_empty((qkv.shape[0], width))
             ops.paged_attention(q, out, layer.kv, meta.block_tables, ctx, self.num_heads, self.num_kv_heads, self.head_dim, self.scale,
                                 rope=(inv_freq, rotary_dim) if fused else None, gate=gate, **mask)
         if self.head_gate:

@@ -981,8 +981,18 @@ static int gemm_tc5(const void* A, const void* B, const void* bias, int bias_f32
         for (int i = 0; i < S * S; ++i) g.hc_mix[i] = ends.hc_weights[i];
         for (int i = 0; i < S; ++i) { g.hc_out[i] = ends.hc_weights[S * S + i]; g.hc_in[i] = ends.hc_weights[S * S + S + i]; }
     }
-    const bool deep = swapped && ((K + TC_BK - 1) / TC_BK + slices - 1) / slices >= 24;
+    const int per = ((K + TC_BK - 1) / TC_BK + slices - 1) / slices;  // K steps of a block
+    const bool deep = swapped && per >= 24;
     dim3 grid((N + bn - 1) / bn, (M + TC_BM - 1) / TC_BM, slices);
+    // No more blocks than SMs: a ring that fills the SM.  Most or all of a block's weights are then under way before the kernel in
+    // front has ended, and clusters do not pile up on a few SMs (with four stages, three blocks fit on one, beside
+    // empty ones).  Where the blocks have no more K steps than the four stages hold, only the second counts, and it
+    // pays as long as the kernel behind, which starts early, finds SMs without such a block: up to half of them.  A
+    // request of 16 tokens in 24 layers of 896 (q/k/v 72 blocks of 2 steps, o 56 of 2, down 56 of 10): 11.47 -> 10.53 ms,
+    // 11.35 with down alone; 12 layers of 1,536 (down 96 blocks of 18; q/k/v 128 of 3, o 96 of 3): 8.86 -> 8.50,
+    // 8.97 with all three.
+    const int64_t blocks = (int64_t)grid.x * grid.y * grid.z;
+    const bool alone = swapped && blocks <= ss_sm_count() && (per > 4 || blocks <= ss_sm_count() / 2);
     if (!swapped) grid = dim3((M + TC_BM - 1) / TC_BM, (N + bn - 1) / bn, slices);
     switch (bn) {
         // Swapped and many K steps per block (down, gate/up, the LM head: 37 to 56): a deeper ring, still two blocks
@@ -993,10 +1003,13 @@ static int gemm_tc5(const void* A, const void* B, const void* bias, int bias_f32
         // hold beside two of these matters more: six stages for every product took 2.96 ms.
         case 16: {
             const int e = ends.residual ? 1 : ends.in_squares ? 2 : 0;
+            if (alone) return launch16<10>(e, ma, mb, g, grid, stream);
             return deep ? launch16<6>(e, ma, mb, g, grid, stream) : launch16<4>(e, ma, mb, g, grid, stream);
         }
-        case 32: return launch<32, 4>(ma, mb, g, grid, stream);  // (five stages when deep: 3.27 ms instead of 3.24 at 32 requests)
-        case 64: return launch<64, 4>(ma, mb, g, grid, stream);  // two blocks fit on an SM
+        case 32:  // (five stages when deep: 3.27 ms instead of 3.24 at 32 requests)
+            return alone ? launch<32, 10>(ma, mb, g, grid, stream) : launch<32, 4>(ma, mb, g, grid, stream);
+        case 64:  // two blocks of four stages fit on an SM
+            return alone ? launch<64, 8>(ma, mb, g, grid, stream) : launch<64, 4>(ma, mb, g, grid, stream);
         case 128: return launch<128, 6>(ma, mb, g, grid, stream);
         case 256: return launch<256, 4>(ma, mb, g, grid, stream);
         default: return -2006;

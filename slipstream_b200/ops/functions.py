@@ -1474,22 +1474,32 @@ def takes_pending_norm(x: "torch.Tensor | PendingNorm", features: int, swiglu: b
     return many_tokens_fits(x.shape[0], features, x.shape[1], sms)
 
 
-def gemm_plan(tokens: int, features: int, k: int, sms: int | None = None) -> tuple[bool, int, int]:
-    """(swapped, tile width, K slices) for ``x[tokens, k] @ w[features, k].T`` on ``sms`` multiprocessors."""
-    return _gemm_plan(tokens, features, k, sms or sm_count())
+def gemm_plan(tokens: int, features: int, k: int, sms: int | None = None, swiglu: bool = False) -> tuple[bool, int, int]:
+    """(swapped, tile width, K slices) for ``x[tokens, k] @ w[features, k].T`` on ``sms`` multiprocessors; ``swiglu``: with a
+    gated unit in the epilogue."""
+    return _gemm_plan(tokens, features, k, sms or sm_count(), swiglu)
 
 
 @functools.lru_cache(maxsize=None)
-def _gemm_plan(tokens: int, features: int, k: int, sms: int) -> tuple[bool, int, int]:
+def _gemm_plan(tokens: int, features: int, k: int, sms: int, swiglu: bool) -> tuple[bool, int, int]:
     k_iters = (k + 63) // 64
     if tokens <= 64:
         bn = 16 if tokens <= 16 else (32 if tokens <= 32 else 64)
         tiles = (features + 127) // 128
+        # a gated unit joins its slices with half of the lanes, and a block alone on its SM has most of its weights under
+        # way early: one slice, if that leaves few SMs without a block, or more of them where K is short.  us on 148 SMs, one
+        # slice against the rule below: 112 tiles, K 896 to 8,192: 6.2 / 6.9, 8.9 / 9.5, 13.0 / 13.8, 19.9 / 20.0, 37.9 / 43.9
+        # (48 tokens 9.8 / 11.9 to 43 / 45); 96 tiles, K 1,536 and 4,096: 8.4 / 8.5 and 18.2 / 17.8 (48 tokens 12.0 / 14.1
+        # and, K 8,192, 39 / 41); 76 tiles, K 896 and 1,536: 5.5 / 5.9 and 8.2 / 7.5; 60 tiles: 4.9 / 5.7 and 7.1 / 6.8
+        if swiglu and tiles <= sms and (10 * tiles >= 7 * sms or 8 * tiles >= 5 * sms and (k_iters <= 40 or bn > 16)
+                                        or 5 * tiles >= 2 * sms and k_iters <= 16):
+            return True, bn, 1
         # at most 8 slices: they then form one thread-block cluster and are added through shared memory
         slices = max(1, min(k_iters, (2 * sms + tiles - 1) // tiles if tiles < sms else 1, 8))
-        # the widest tile leaves room for two blocks per SM, and clusters do not pack an SM's last slot: stay
-        # within one wave of blocks (36 tiles x 8 slices ran as two waves: 18.1 us against 13.2 with 7 slices)
-        while bn == 64 and slices > 1 and tiles * slices > sms + (3 * sms) // 4:
+        # the wider tiles leave room for two blocks per SM, and clusters do not pack an SM's last slot: stay
+        # within one wave of blocks (48 tokens, 36 tiles x 8 slices ran as two waves: 18.1 us against 13.2 with 7 slices; 24
+        # tokens, K 896 and 8,192: 76 tiles x 4 11.2 and 37.3, x 3 6.6 and 27.7, 140 x 3 12.5 and 52.6, x 1 9.3 and 48.3)
+        while bn > 16 and slices > 1 and tiles * slices > sms + (3 * sms) // 4:
             slices -= 1
         return True, bn, slices
     bn = 256 if features >= 256 else (128 if features >= 128 else (64 if features >= 64 else (32 if features >= 32 else 16)))
@@ -1542,7 +1552,7 @@ def gemm_tcgen05(x: "torch.Tensor | PendingNorm", weight: torch.Tensor, bias: to
         bias_f32 = int(bias.dtype == torch.float32)
         if bias.numel() != features or bias.dtype not in (torch.float32, torch.bfloat16):
             raise KernelError("bias has the wrong size or dtype")
-    swapped, bn, slices = plan or gemm_plan(tokens, features, k, sm_count(x.device))
+    swapped, bn, slices = plan or gemm_plan(tokens, features, k, sm_count(x.device), swiglu)
     partial = counters = None
     if slices > 1 and not (swapped and slices <= 8 and tokens <= bn):
         partial, counters = _gemm_workspace(x.device)

@@ -55,6 +55,16 @@ def test_streaming_product_plan_and_routing():
         assert not F.many_tokens_fits(4096, features, k, SMS)
 
 
+def test_gated_products_of_about_one_tile_a_multiprocessor_keep_their_sums_in_one_block():
+    for tokens in (1, 16, 24, 64):
+        assert all(F.gemm_plan(tokens, f, k, SMS, True)[2] == 1 for f, k in ((9728, 896), (17920, 1536), (13440, 20000), (18944, 8192)))
+        assert F.gemm_plan(tokens, 9728, 1536, SMS, True) == F.gemm_plan(tokens, 9728, 1536, SMS)
+        assert F.gemm_plan(tokens, 37888, 3584, SMS, True) == F.gemm_plan(tokens, 37888, 3584, SMS)
+        for f, k in ((7680, 896), (9728, 8192), (17920, 896)):  # more than 16 columns: within one wave of two blocks an SM
+            _, bn, slices = F.gemm_plan(tokens, f, k, SMS)
+            assert bn == 16 or slices * (f // 128) <= SMS + 3 * SMS // 4
+
+
 def test_where_a_projection_adds_itself_to_the_stream():
     """The last projection of a branch takes over the add and prepares the norm behind it in decode steps of up to
     16 tokens, where its K slices are a cluster and the width is a multiple of 128; for long prompt portions only

@@ -591,6 +591,27 @@ def test_tcgen05_fused_swiglu(tokens, inter, k, bias):
     ops().check_errors(torch.device(DEV))
 
 
+# rings that fill an SM: fewer, as many and more K steps than the ring's 10 (8 with 64 columns) stages and than twice as many,
+# with a last step that is not full; blocks up to half of the SMs with few steps, up to all of them with more, and beyond
+@pytest.mark.parametrize("tokens", [1, 16, 17, 33, 64])
+@pytest.mark.parametrize("features, k, slices", [(896, 104, 2), (128, 640, 1), (128, 648, 1), (9472, 320, 1), (9600, 264, 1), (18944, 360, 1),
+                                                 (19072, 328, 1), (896, 4864, 8), (1000, 1416, 1)])
+def test_tcgen05_with_blocks_alone_on_their_multiprocessors(tokens, features, k, slices):
+    torch.manual_seed(features + k)
+    x, w = torch.randn(tokens, k, device=DEV).bfloat16(), torch.randn(features, k, device=DEV).bfloat16()
+    bn = 16 if tokens <= 16 else 32 if tokens <= 32 else 64
+    ref = x.double() @ w.double().T
+    got = ops().gemm_tcgen05(x, w, None, torch.float32, plan=(True, bn, slices))
+    # exact products; sums of 16 of them added to the accumulator, up to 4,864 / 16 times, each losing up to 2^-23 of it
+    assert rel_err(got, ref) < 304 * 2.0 ** -23
+    if features % 128 == 0:
+        gate, up = ref.view(tokens, features // 128, 2, 64).unbind(2)
+        want = (gate * torch.sigmoid(gate) * up).reshape(tokens, features // 2)
+        assert rel_err(ops().gemm_tcgen05(x, w, None, swiglu=True, plan=(True, bn, slices)), want) < 8e-3
+        assert rel_err(ops().gemm_tcgen05(x, w, None, swiglu=True), want) < 8e-3  # the plan's own slices
+    ops().check_errors(torch.device(DEV))
+
+
 @pytest.mark.parametrize("tokens, features, k, bias, w_f32", [(8, 3584, 3584, False, False), (1, 3584, 18944, False, False),
                                                              (16, 896, 4864, True, True), (5, 256, 136, True, False),
                                                              (3, 1024, 512, False, True), (11, 5120, 13824, False, False),

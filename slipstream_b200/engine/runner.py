@@ -52,7 +52,7 @@ class ModelRunner:
         if dtype_name not in _DTYPES:
             raise ValueError(f"unsupported dtype: {dtype_name} (bfloat16 or float32)")
         self.dtype_name = dtype_name
-        self.runtime = Runtime(self.device, _DTYPES[dtype_name])
+        self.runtime = Runtime(self.device, _DTYPES[dtype_name], page_size)
         self.max_model_len = max_model_len or self.config.max_position_embeddings
         self.page_size = page_size
         self.max_num_seqs = max_num_seqs

@@ -264,7 +264,26 @@ class PagedAttention(Mixer):
         """Whether the attention kernel applies the gate (behind talking heads the mixture does)."""
         return self.gate and not self.talk
 
+    @property
+    def page_tokens(self) -> int:
+        """Tokens that a page of this layer holds."""
+        return self.page_size or getattr(self.runtime, "page_size", 16)
+
     # ------------------------------------------------------------------ decode steps replayed from a graph
+    @property
+    def _may_spread(self) -> bool:
+        """Whether the decode kernel that deals key tiles out evenly takes this layer."""
+        return (self.runtime.dtype == torch.bfloat16 and not self.talk
+                and ops.tcgen05_attention_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_tokens, 0))
+
+    def _spreads(self, plan: object) -> bool:
+        """Whether the decode step of ``plan`` has its key tiles dealt out evenly.  A layer that the kernel does not take never
+        asks: its second graph would hold the kernels of the first."""
+        if plan is None or not self._may_spread:
+            return False
+        return ops.spreads_decode(plan.seq_lens, self.num_kv_heads, self.num_heads // self.num_kv_heads, self.head_dim, self.sees,
+                                  ops.sm_count(self.runtime.device))
+
     def capture_variant(self, longest: int, plan: object = None) -> object:
         """Decode steps: long contexts of few requests want the keys cut into more slices than fit one thread-block
         cluster (``ops.decode_slices``; 1 here), many requests of different lengths their tiles dealt out evenly
@@ -273,12 +292,9 @@ class PagedAttention(Mixer):
         keys.  Each form is captured as a graph of its own."""
         bf16 = self.runtime.dtype == torch.bfloat16
         if plan is None or plan.is_decode_only:
-            spread = (bf16 and plan is not None and not self.talk
-                      and ops.spreads_decode(plan.seq_lens, self.num_kv_heads, self.num_heads // self.num_kv_heads, self.head_dim, self.sees,
-                                             ops.sm_count(self.runtime.device)))
-            return int(bf16 and ops.is_long_context(longest)) + 2 * int(spread)
+            return int(bf16 and ops.is_long_context(longest)) + 2 * int(self._spreads(plan))
         group = self.num_heads // self.num_kv_heads
-        if not bf16 or not ops.tcgen05_prefill_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_size or 16):
+        if not bf16 or not ops.tcgen05_prefill_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_tokens):
             return None
         if self.gates_inside and self.head_dim not in (64, 128):
             return None  # always the mma.sync kernel: one form, one graph
@@ -289,7 +305,7 @@ class PagedAttention(Mixer):
 
     def capture_group(self) -> object:
         # what `capture_variant` answers from beside the step's lengths
-        fits = ops.tcgen05_prefill_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_size or 16)
+        fits = ops.tcgen05_prefill_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_tokens)
         return ("paged_attention", self.sees, self.head_dim, self.gates_inside, fits, 128 // (self.num_heads // self.num_kv_heads), self.kernel_blocks,
                 self.talk)
 
@@ -306,8 +322,9 @@ class PagedAttention(Mixer):
         # the number of slices must not follow the lengths of the step that happens to be captured
         ctx.extras["static_max_seq_len"] = max_model_len
         ctx.extras["decode_wide"] = bool(int(variant or 0) & 1)
-        group = self.num_heads // self.num_kv_heads
-        ctx.extras[("decode_spread", self.num_kv_heads, group, self.head_dim, self.sees)] = bool(int(variant or 0) & 2)
+        if self._may_spread:  # (a layer that is not taken does not speak for one that is)
+            group = self.num_heads // self.num_kv_heads
+            ctx.extras[("decode_spread", self.num_kv_heads, group, self.head_dim, self.sees)] = bool(int(variant or 0) & 2)
         # the float32 kernel's list of query tiles: one tile per row of the batch
         rows = ctx.num_requests
         ctx.set_query_tiles(16, 1, torch.arange(rows, dtype=torch.int32, device=ctx.device),

@@ -94,6 +94,7 @@ class Runtime:
 
     device: torch.device
     dtype: torch.dtype  # torch.bfloat16 or torch.float32
+    page_size: int = 16  # tokens a page of the layers that ask for no size of their own holds
 
     @property
     def is_fp32(self) -> bool:

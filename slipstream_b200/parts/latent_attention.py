@@ -123,7 +123,7 @@ class LatentAttention(Mixer):
     @property
     def on_tcgen05(self) -> bool:
         """Whether prompt portions may run the tcgen05 kernel."""
-        return self.runtime.dtype == torch.bfloat16 and ops.tcgen05_prefill_fits(self.row, self.heads, 1, self.page_size or 16)
+        return self.runtime.dtype == torch.bfloat16 and ops.tcgen05_prefill_fits(self.row, self.heads, 1, self.page_size or getattr(self.runtime, "page_size", 16))
 
     def capture_variant(self, longest: int, plan: object = None) -> object:
         # one form of the decode kernel, however long the contexts; steps with prompt portions, where the tcgen05 kernel takes the

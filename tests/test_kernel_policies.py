@@ -271,3 +271,32 @@ def test_decode_tiles_are_dealt_out_where_that_was_measured_to_pay_captured_or_n
         assert ctx.extras["decode_wide"] == F.is_long_context(int(lens.max()))
         assert ctx.extras[("decode_spread", 4, 7, 128, layer.sees)] == spreads(lens)
     assert layer.capture_variant(5000) == 0  # (no lengths yet: the form for any)
+
+
+def test_layers_off_the_spread_decode_kernel_are_captured_in_one_form(monkeypatch):
+    """Head sizes and pages that the kernel does not take, the engine's own page size among them: the rule is not asked, and
+    such a layer does not change what one of the same heads and reach was told."""
+    from types import SimpleNamespace
+    import torch
+    from slipstream_b200.parts import PagedAttention, RotaryEncoding
+    from slipstream_b200.parts.base import Runtime
+
+    monkeypatch.setattr(F, "_device_sm_count", lambda index: SMS)
+    lens = (np.array([2 + i % 5 for i in range(48)]) * 450).astype(np.int32)
+    plan = SimpleNamespace(is_decode_only=True, q_lens=np.ones(48, dtype=np.int32), seq_lens=lens)
+
+    def layer(dim=128, page=None, pages=16, dtype=torch.bfloat16):
+        made = PagedAttention("attn", 64, 28, 4, dim, RotaryEncoding(dim, 1e4), page_size=page)
+        made.runtime = Runtime(torch.device("cuda:0"), dtype, pages)
+        return made
+
+    taken = [layer(), layer(64), layer(page=32, pages=128), layer(pages=8)]
+    others = [layer(d) for d in (32, 80, 96, 192, 256)] + [layer(page=48), layer(pages=128), layer(dtype=torch.float32)]
+    assert F.spreads_decode(lens, 4, 7, 96, 0, SMS)  # (the rule alone would say yes)
+    assert [x.capture_variant(int(lens.max()), plan) for x in taken] == [2] * 4
+    assert [x.capture_variant(int(lens.max()), plan) for x in others] == [0] * 8
+    assert len({layer().capture_group(), layer(pages=128).capture_group(), layer(page=48).capture_group()}) == 2
+    ctx = SimpleNamespace(is_decode_only=True, num_requests=48, device=None, extras={}, set_query_tiles=lambda *a: None)
+    for x in (layer(), layer(pages=128)):
+        x.prepare_capture(ctx, x.capture_variant(int(lens.max()), plan), 16384)
+    assert ctx.extras[("decode_spread", 4, 7, 128, 0)] is True

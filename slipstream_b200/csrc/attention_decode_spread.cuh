@@ -463,8 +463,8 @@ attn_decode_spread(const __grid_constant__ CUtensorMap map_kv, const SpreadArgs 
             fetch_queries();
         }
     }
-    if (begin >= end && tid < 16) {  // nothing, for a join that comes past
-        *reinterpret_cast<float2*>(s.scratch + (int64_t)blockIdx.x * 2 * 16 * (D + 2) + 16 * D + tid * 2) = make_float2(-INFINITY, 0.f);
+    if (begin >= end && tid < 16) {  // no sums, for a join that comes past: a denominator that no piece has
+        *reinterpret_cast<float2*>(s.scratch + (int64_t)blockIdx.x * 2 * 16 * (D + 2) + 16 * D + tid * 2) = make_float2(-INFINITY, -1.f);
     }
     // rows of requests without a key
     for (int r = blockIdx.x; r < s.n_requests; r += gridDim.x)
@@ -505,9 +505,10 @@ attn_decode_spread_join(const SpreadArgs s) {
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                if (k0 + k >= parts || ml[k].x == -INFINITY) continue;  // no part, nothing seen, or a block without a tile
+                if (k0 + k >= parts || ml[k].y < 0.f) continue;  // no part, or a block without a tile
+                // a piece without a score above -infinity has no weight, but its sums count: those of scores that are not numbers are not either
                 const float top = fmaxf(mx, ml[k].x);
-                const float old = mx == -INFINITY ? 0.f : fast_exp2(mx - top), now = fast_exp2(ml[k].x - top);
+                const float old = mx == -INFINITY ? 0.f : fast_exp2(mx - top), now = ml[k].x == -INFINITY ? 0.f : fast_exp2(ml[k].x - top);
                 sum.x = fmaf(v[k].x, now, sum.x * old);
                 sum.y = fmaf(v[k].y, now, sum.y * old);
                 sum.z = fmaf(v[k].z, now, sum.z * old);

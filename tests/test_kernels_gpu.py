@@ -458,6 +458,35 @@ def test_decode_with_tiles_dealt_out_evenly(lens, n_q, n_kv, d, page, window, ke
     ops().check_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("with_sinks", [False, True])
+def test_tiles_dealt_out_evenly_pass_on_scores_that_are_not_numbers(with_sinks):
+    """A query of NaN, keys of NaN (one; all of some tiles), a value of infinity among keys whose scores are -infinity, in requests that
+    cuts divide and in one that lies in a block: NaN where the kernel with one block a unit has it."""
+    lens, n_q, n_kv, d, page = [3000, 40, 2500, 700, 3000, 90], 4, 2, 64, 16
+    R = len(lens)
+    q, kv, table, q_start, seq_lens = make_attention_case(torch.bfloat16, lens, [1] * R, n_q, n_kv, d, page, seed=4)
+    q = q.clone()
+    q[0, 1] = q[1, 2] = float("nan")
+    for r, keys in ((2, (1300,)), (3, range(700)), (4, range(320, 2000))):
+        for key in keys:
+            kv[int(table[r, key // page]), 0, 0, key % page] = float("nan")
+    q[5, 0] = 1.0
+    for key in range(90):
+        kv[int(table[5, key // page]), 0, 0, key % page] = -float("inf")
+    kv[int(table[5, 2]), 1, 0, 3, 5] = float("inf")
+    sinks = torch.randn(n_q, device=DEV) if with_sinks else None
+    outs = []
+    for f in (ops().paged_attention_decode_spread, ops().paged_attention_decode):
+        out = torch.zeros(R, n_q * d, device=DEV, dtype=torch.bfloat16)
+        f(q.view(R, -1), n_q * d, out, kv, table, q_start, seq_lens, R, n_q, n_kv, d, d ** -0.5, sinks=sinks)
+        outs.append(out)
+    there = outs[1].isnan()
+    assert torch.equal(outs[0].isnan(), there) and there.any(dim=1).all() and not there.all()
+    assert there.view(R, n_q, d)[0, 1].all() and there.view(R, n_q, d)[2:5, 0].all()
+    assert rel_err(outs[0][~there], outs[1][~there]) < 1e-2
+    ops().check_errors(torch.device(DEV))
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_a_far_key_among_hundreds_is_found(dtype):
     """One key 700 tokens back matches the last query far better than all others: its value must

@@ -1474,14 +1474,15 @@ def takes_pending_norm(x: "torch.Tensor | PendingNorm", features: int, swiglu: b
     return many_tokens_fits(x.shape[0], features, x.shape[1], sms)
 
 
-def gemm_plan(tokens: int, features: int, k: int, sms: int | None = None, swiglu: bool = False) -> tuple[bool, int, int]:
+def gemm_plan(tokens: int, features: int, k: int, sms: int | None = None, swiglu: bool = False,
+              out_f32: bool = False) -> tuple[bool, int, int]:
     """(swapped, tile width, K slices) for ``x[tokens, k] @ w[features, k].T`` on ``sms`` multiprocessors; ``swiglu``: with a
-    gated unit in the epilogue."""
-    return _gemm_plan(tokens, features, k, sms or sm_count(), swiglu)
+    gated unit in the epilogue; ``out_f32``: with float32 outputs."""
+    return _gemm_plan(tokens, features, k, sms or sm_count(), swiglu, out_f32)
 
 
 @functools.lru_cache(maxsize=None)
-def _gemm_plan(tokens: int, features: int, k: int, sms: int, swiglu: bool) -> tuple[bool, int, int]:
+def _gemm_plan(tokens: int, features: int, k: int, sms: int, swiglu: bool, out_f32: bool = False) -> tuple[bool, int, int]:
     k_iters = (k + 63) // 64
     if tokens <= 64:
         bn = 16 if tokens <= 16 else (32 if tokens <= 32 else 64)
@@ -1498,8 +1499,10 @@ def _gemm_plan(tokens: int, features: int, k: int, sms: int, swiglu: bool) -> tu
         slices = max(1, min(k_iters, (2 * sms + tiles - 1) // tiles if tiles < sms else 1, 8))
         # the wider tiles leave room for two blocks per SM, and clusters do not pack an SM's last slot: stay
         # within one wave of blocks (48 tokens, 36 tiles x 8 slices ran as two waves: 18.1 us against 13.2 with 7 slices; 24
-        # tokens, K 896 and 8,192: 76 tiles x 4 11.2 and 37.3, x 3 6.6 and 27.7, 140 x 3 12.5 and 52.6, x 1 9.3 and 48.3)
-        while bn > 16 and slices > 1 and tiles * slices > sms + (3 * sms) // 4:
+        # tokens, K 896 and 8,192: 76 tiles x 4 11.2 and 37.3, x 3 6.6 and 27.7, 140 x 3 12.5 and 52.6, x 1 9.3 and 48.3).
+        # Float32 outputs of up to 32 tokens keep their slices: longer sums show in them (relative error at 5,120 x 5,120, 8 slices
+        # and 6: 6.0e-7 and 8.3e-7; rounded to bfloat16 1.65888e-3 both)
+        while bn > (32 if out_f32 else 16) and slices > 1 and tiles * slices > sms + (3 * sms) // 4:
             slices -= 1
         return True, bn, slices
     bn = 256 if features >= 256 else (128 if features >= 128 else (64 if features >= 64 else (32 if features >= 32 else 16)))
@@ -1552,7 +1555,7 @@ def gemm_tcgen05(x: "torch.Tensor | PendingNorm", weight: torch.Tensor, bias: to
         bias_f32 = int(bias.dtype == torch.float32)
         if bias.numel() != features or bias.dtype not in (torch.float32, torch.bfloat16):
             raise KernelError("bias has the wrong size or dtype")
-    swapped, bn, slices = plan or gemm_plan(tokens, features, k, sm_count(x.device), swiglu)
+    swapped, bn, slices = plan or gemm_plan(tokens, features, k, sm_count(x.device), swiglu, out_dtype == torch.float32)
     partial = counters = None
     if slices > 1 and not (swapped and slices <= 8 and tokens <= bn):
         partial, counters = _gemm_workspace(x.device)

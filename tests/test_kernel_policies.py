@@ -65,6 +65,11 @@ def test_gated_products_of_about_one_tile_a_multiprocessor_keep_their_sums_in_on
             assert bn == 16 or slices * (f // 128) <= SMS + 3 * SMS // 4
 
 
+def test_float32_outputs_keep_their_slices():
+    assert F.gemm_plan(24, 5120, 5120, SMS)[2] == 6 and F.gemm_plan(24, 5120, 5120, SMS, out_f32=True)[2] == 8
+    assert F.gemm_plan(48, 5120, 5120, SMS)[2] == F.gemm_plan(48, 5120, 5120, SMS, out_f32=True)[2]
+
+
 def test_where_a_projection_adds_itself_to_the_stream():
     """The last projection of a branch takes over the add and prepares the norm behind it in decode steps of up to
     16 tokens, where its K slices are a cluster and the width is a multiple of 128; for long prompt portions only

@@ -70,6 +70,7 @@ struct GemmArgs {
     int out_f32;
     int bias_f32;
     int cluster;        // 1: the slices of a tile are one thread-block cluster and are added through shared memory
+    int part_steps;     // swiglu with one slice whose sums stay apart: K steps of each
     int swiglu;         // 1 (swapped only): rows 0..63 of a tile are gate features, rows 64..127 the matching up
                         // features; the output has M / 2 features: out[n][tile * 64 + r] = silu(gate) * up
     // A branch's last projection (cluster mode, M a multiple of 128) may add its output, rounded to bfloat16, to the
@@ -131,12 +132,16 @@ __device__ __forceinline__ void store_out(const GemmArgs& g, int m, int n, float
 // decode step of 8 requests took 2.73 ms instead of 2.69 without using either).
 // PATH: 0 every form, chosen by the arguments; the forms of a decode step as kernels of their own (swapped, 16
 // columns): 1 K slices in a cluster, plain bfloat16 output (q/k/v, o, down), 4 the same with exactly 8 slices;
-// 2 one slice with SwiGLU (gate/up); 3 one slice, plain output (the LM head).
+// 2 one slice with SwiGLU (gate/up); 3 one slice, plain output (the LM head).  5 (16, 32 and 64 columns): as 2, where other products
+// would have slices: the block keeps the sums of every g.part_steps K steps apart, each in columns of its own, and adds them in
+// order.  They are the accumulators of those slices, so the result has their bits: one long sum loses more (each addition up to
+// 2^-23 of it: 1.4e-6 where four slices lose 5e-7, K 1,536).  A request in 24 layers of 896, 76 tiles: the step 581 us with clusters of 4, 549
+// with one sum, 557 so; 12 layers of 1,536, 140 tiles, 3 slices: 478, 445, 450.
 template <int BN, int STAGES, int ENDS, int PATH>
 __global__ void __launch_bounds__(TC_THREADS)
 gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmArgs g) {
     constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2;
-    constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
+    constexpr int TMEM_COLS = PATH == 5 ? (BN == 16 ? 128 : 256) : BN < 32 ? 32 : BN;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* full = reinterpret_cast<uint64_t*>(tiles + STAGES * (A_BYTES + B_BYTES));
@@ -151,9 +156,9 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     // what the generic kernel (PATH 0) asks of its arguments, the others know: a decode step's kernels branch less
     const bool f_swapped = PATH == 0 ? g.swapped != 0 : true;
     const bool f_cluster = PATH == 0 ? g.cluster != 0 : (PATH == 1 || PATH == 4);
-    const bool f_swiglu = PATH == 0 ? g.swiglu != 0 : PATH == 2;
-    const bool f_single = PATH == 0 ? g.slices == 1 : (PATH == 2 || PATH == 3);  // one K slice
-    const int n_sl = PATH == 4 ? 8 : (PATH == 2 || PATH == 3) ? 1 : g.slices;    // K slices
+    const bool f_swiglu = PATH == 0 ? g.swiglu != 0 : (PATH == 2 || PATH == 5);
+    const bool f_single = PATH == 0 ? g.slices == 1 : (PATH == 2 || PATH == 3 || PATH == 5);  // one K slice
+    const int n_sl = PATH == 4 ? 8 : (PATH == 2 || PATH == 3 || PATH == 5) ? 1 : g.slices;    // K slices
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // swapped: (token tile, weight tile); else the row tiles of the activations run fastest, so that the blocks
     // that are resident together share a weight tile and the weights are read from memory once
@@ -228,17 +233,23 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         // both K-major, N = BN, M = 128.
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
         bool ok = true;
-        for (int it = 0; it < k_iters && ok; ++it) {
+        uint32_t acc = tmem_acc;
+        int step = 0;  // of the sum in columns acc ..
+        for (int it = 0; it < k_iters && ok; ++it, ++step) {
             const int s = it % STAGES;
             ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (it / STAGES) & 1, gave_up));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             unsigned char* a_tile = tiles + s * (A_BYTES + B_BYTES);
             const uint64_t a_desc = smem_desc(a_tile), b_desc = smem_desc(a_tile + A_BYTES);
+            if (PATH == 5 && step == g.part_steps) {
+                acc += BN;
+                step = 0;
+            }
             if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < TC_BK / 16; ++kk)  // 16 K elements = 32 bytes further along the swizzled row
-                    umma_f16(tmem_acc, a_desc + (uint64_t)(kk * 2), b_desc + (uint64_t)(kk * 2), idesc, (it | kk) != 0);
+                    umma_f16(acc, a_desc + (uint64_t)(kk * 2), b_desc + (uint64_t)(kk * 2), idesc, (step | kk) != 0);
                 umma_commit(&empty[s]);
             }
             __syncwarp();
@@ -300,7 +311,32 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll 1
             for (int c = 0; c < BN; c += 16) {
                 uint32_t r[16];
-                if (k_iters > 0) {
+                if constexpr (PATH == 5) {
+                    // the sums in their order, as the slices of a cluster are added
+                    const uint32_t from = tmem_acc + ((uint32_t)(quarter * 32) << 16) + c;
+                    const int sums = (k_iters + g.part_steps - 1) / g.part_steps;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) r[j] = 0u;
+                    if constexpr (BN == 16) {
+                        for (int p0 = 0; p0 < sums; p0 += 4) {
+                            uint32_t four[64];
+                            tmem_ld64(from + p0 * 16, four);
+#pragma unroll
+                            for (int p = 0; p < 4; ++p) {
+                                if (p0 + p >= sums) break;
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(four[p * 16 + j])));
+                            }
+                        }
+                    } else {
+                        for (int p = 0; p < sums; ++p) {
+                            uint32_t one[16];
+                            tmem_ld16(from + p * BN, one);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(one[j])));
+                        }
+                    }
+                } else if (k_iters > 0) {
                     tmem_ld16(tmem_acc + ((uint32_t)(quarter * 32) << 16) + c, r);
                 } else {
 #pragma unroll
@@ -929,7 +965,9 @@ extern "C" int64_t ss_gemm_tc5_scratch_floats(int tiles, int slices, int bn) { r
 // or 256).  swapped: write C transposed (C[n * ldc + m]).  swiglu (swapped, M a multiple of 128): A's rows
 // alternate 64 gate and 64 up features; C gets M / 2 features, silu(gate) * up.  slices > 1 needs `partial` (see
 // ss_gemm_tc5_scratch_floats) and `counters` (one int per tile, zero; left zero), except in swapped mode with
-// 2..8 slices and N <= bn, where the slices are added through the shared memory of a thread-block cluster.
+// 2..8 slices and N <= bn, where the slices are added through the shared memory of a thread-block cluster.  swiglu, slices = -p, p up to
+// 8 and p x bn up to 256: one block a tile that keeps the sums of p slices apart and adds them in their order; refused where the
+// block would not be alone on its multiprocessor (see below).
 extern "C" void ss_set_pdl(int on) { ss_pdl_flag() = on; }
 
 struct NormEnds {  // see GemmArgs: the output added to the float32 stream, the output scaled by the norm in front
@@ -953,6 +991,9 @@ static int gemm_tc5(const void* A, const void* B, const void* bias, int bias_f32
     if (swiglu && (!swapped || M % TC_BM != 0)) return -2007;
     if (K <= 0 || K % 8 != 0 || lda % 8 != 0 || ldb % 8 != 0) return -2003;
     if (((uintptr_t)A & 15) || ((uintptr_t)B & 15)) return -2004;
+    const int parts = slices < 0 ? -slices : 1;  // sums of one slice that stay apart
+    if (slices < 0) slices = 1;
+    if (parts > 8 || (parts > 1 && (!swiglu || bn > 64 || parts * bn > (bn == 16 ? 128 : 256)))) return -2005;
     const int cluster = swapped && slices >= 2 && slices <= 8 && N <= bn;
     if (slices < 1 || (slices > 1 && !cluster && (!partial || !counters))) return -2005;
     if (ends.residual && (!cluster || swiglu || M % TC_BM != 0 || !ends.tile_squares || !ends.scaled || !ends.norm_weight ||
@@ -982,6 +1023,7 @@ static int gemm_tc5(const void* A, const void* B, const void* bias, int bias_f32
         for (int i = 0; i < S; ++i) { g.hc_out[i] = ends.hc_weights[S * S + i]; g.hc_in[i] = ends.hc_weights[S * S + S + i]; }
     }
     const int per = ((K + TC_BK - 1) / TC_BK + slices - 1) / slices;  // K steps of a block
+    g.part_steps = parts > 1 ? (per + parts - 1) / parts : 0;
     const bool deep = swapped && per >= 24;
     dim3 grid((N + bn - 1) / bn, (M + TC_BM - 1) / TC_BM, slices);
     // No more blocks than SMs: a ring that fills the SM.  Most or all of a block's weights are then under way before the kernel in
@@ -993,6 +1035,8 @@ static int gemm_tc5(const void* A, const void* B, const void* bias, int bias_f32
     // 8.97 with all three.
     const int64_t blocks = (int64_t)grid.x * grid.y * grid.z;
     const bool alone = swapped && blocks <= ss_sm_count() && (per > 4 || blocks <= ss_sm_count() / 2);
+    // (more than 64 columns of tensor memory only where no other block that takes some can stand beside this one and wait for it)
+    if (parts > 1 && !alone) return -2005;
     if (!swapped) grid = dim3((M + TC_BM - 1) / TC_BM, (N + bn - 1) / bn, slices);
     switch (bn) {
         // Swapped and many K steps per block (down, gate/up, the LM head: 37 to 56): a deeper ring, still two blocks
@@ -1003,12 +1047,15 @@ static int gemm_tc5(const void* A, const void* B, const void* bias, int bias_f32
         // hold beside two of these matters more: six stages for every product took 2.96 ms.
         case 16: {
             const int e = ends.residual ? 1 : ends.in_squares ? 2 : 0;
+            if (parts > 1) return e == 2 ? launch<16, 10, 2, 5>(ma, mb, g, grid, stream) : launch<16, 10, 0, 5>(ma, mb, g, grid, stream);
             if (alone) return launch16<10>(e, ma, mb, g, grid, stream);
             return deep ? launch16<6>(e, ma, mb, g, grid, stream) : launch16<4>(e, ma, mb, g, grid, stream);
         }
         case 32:  // (five stages when deep: 3.27 ms instead of 3.24 at 32 requests)
+            if (parts > 1) return launch<32, 10, 0, 5>(ma, mb, g, grid, stream);
             return alone ? launch<32, 10>(ma, mb, g, grid, stream) : launch<32, 4>(ma, mb, g, grid, stream);
         case 64:  // two blocks of four stages fit on an SM
+            if (parts > 1) return launch<64, 8, 0, 5>(ma, mb, g, grid, stream);
             return alone ? launch<64, 8>(ma, mb, g, grid, stream) : launch<64, 4>(ma, mb, g, grid, stream);
         case 128: return launch<128, 6>(ma, mb, g, grid, stream);
         case 256: return launch<256, 4>(ma, mb, g, grid, stream);

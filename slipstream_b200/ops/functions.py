@@ -1481,19 +1481,47 @@ def gemm_plan(tokens: int, features: int, k: int, sms: int | None = None, swiglu
     return _gemm_plan(tokens, features, k, sms or sm_count(), swiglu, out_f32)
 
 
+def gated_sums(tokens: int, features: int, k: int, sms: int | None = None) -> int:
+    """Sums of K that the one block of a gated product's tile keeps apart: as many as the product would have slices without
+    that rule of `gemm_plan`, so that their additions, and the bits of the result, are those of the slices."""
+    return _gated_sums(tokens, features, k, sms or sm_count())
+
+
+def _small_batch_tiles(tokens: int, features: int, k: int) -> tuple[int, int, int]:
+    """(tile width, weight tiles, K steps) of a product of up to 64 tokens."""
+    return 16 if tokens <= 16 else (32 if tokens <= 32 else 64), (features + 127) // 128, (k + 63) // 64
+
+
+def _gated_in_one_block(bn: int, tiles: int, k_iters: int, sms: int) -> bool:
+    """Whether a block forms a whole tile of a gated product that other products would cut along K: it would join its slices with
+    half of the lanes, and a block alone on its SM has most of its weights under way early.  Where that leaves few SMs without a block,
+    or more of them where K is short.  us on 148 SMs, slices against one block, 4 tokens (24, 48): 147 tiles, K 896 and 4,096: 12.1 /
+    8.0 and 32.0 / 24.9; 112, K 896, 2,560, 4,096, 8,192: 7.1 / 6.8, 13.9 / 13.4, 20.1 / 20.3 (22.4 / 21.8, 24.9 / 23.2), 43.4 / 37.1;
+    104: 6.8 / 6.5 and, K 4,096, 19.0 / 19.0; 96, K 896, 1,536, 2,560: 6.7 / 6.2, 8.7 / 9.2 (11.2 / 10.4, 13.8 / 11.9), 12.5 / 12.7 (14.8 /
+    14.0, 17.5 / 15.5); 76, K 512, 896, 1,024: 5.4 / 4.4, 6.2 / 6.2 (7.8 / 7.6, 9.9 / 9.4), 6.4 / 7.2 (8.1 / 8.5, 10.3 / 10.4); 60, K 896 and
+    1,024: 5.9 / 5.6 and 6.1 / 6.1 (7.5 / 7.5, 9.1 / 9.3).  Behind one another in a decode step the short ones give more: 76 tiles, K 896,
+    24 layers: 581 / 557."""
+    return tiles <= sms and (k_iters > 4 or 2 * tiles <= sms) and (
+        10 * tiles >= 7 * sms or 8 * tiles >= 5 * sms and bn > 16 or 5 * tiles >= 2 * sms and k_iters <= 14)
+
+
+@functools.lru_cache(maxsize=None)
+def _gated_sums(tokens: int, features: int, k: int, sms: int) -> int:
+    bn, tiles, k_iters = _small_batch_tiles(tokens, features, k)
+    if tokens > 64 or not _gated_in_one_block(bn, tiles, k_iters, sms):
+        return 1
+    slices = max(1, min(k_iters, (2 * sms + tiles - 1) // tiles if tiles < sms else 1, 8))
+    while bn == 64 and slices > 1 and tiles * slices > sms + (3 * sms) // 4:
+        slices -= 1
+    return slices
+
+
 @functools.lru_cache(maxsize=None)
 def _gemm_plan(tokens: int, features: int, k: int, sms: int, swiglu: bool, out_f32: bool = False) -> tuple[bool, int, int]:
     k_iters = (k + 63) // 64
     if tokens <= 64:
-        bn = 16 if tokens <= 16 else (32 if tokens <= 32 else 64)
-        tiles = (features + 127) // 128
-        # a gated unit joins its slices with half of the lanes, and a block alone on its SM has most of its weights under
-        # way early: one slice, if that leaves few SMs without a block, or more of them where K is short.  us on 148 SMs, one
-        # slice against the rule below: 112 tiles, K 896 to 8,192: 6.2 / 6.9, 8.9 / 9.5, 13.0 / 13.8, 19.9 / 20.0, 37.9 / 43.9
-        # (48 tokens 9.8 / 11.9 to 43 / 45); 96 tiles, K 1,536 and 4,096: 8.4 / 8.5 and 18.2 / 17.8 (48 tokens 12.0 / 14.1
-        # and, K 8,192, 39 / 41); 76 tiles, K 896 and 1,536: 5.5 / 5.9 and 8.2 / 7.5; 60 tiles: 4.9 / 5.7 and 7.1 / 6.8
-        if swiglu and tiles <= sms and (10 * tiles >= 7 * sms or 8 * tiles >= 5 * sms and (k_iters <= 40 or bn > 16)
-                                        or 5 * tiles >= 2 * sms and k_iters <= 16):
+        bn, tiles, _ = _small_batch_tiles(tokens, features, k)
+        if swiglu and _gated_in_one_block(bn, tiles, k_iters, sms):
             return True, bn, 1
         # at most 8 slices: they then form one thread-block cluster and are added through shared memory
         slices = max(1, min(k_iters, (2 * sms + tiles - 1) // tiles if tiles < sms else 1, 8))
@@ -1556,6 +1584,8 @@ def gemm_tcgen05(x: "torch.Tensor | PendingNorm", weight: torch.Tensor, bias: to
         if bias.numel() != features or bias.dtype not in (torch.float32, torch.bfloat16):
             raise KernelError("bias has the wrong size or dtype")
     swapped, bn, slices = plan or gemm_plan(tokens, features, k, sm_count(x.device), swiglu, out_dtype == torch.float32)
+    if swiglu and plan is None and slices == 1:
+        slices = -max(1, gated_sums(tokens, features, k, sm_count(x.device)))  # (one block a tile, its sums apart)
     partial = counters = None
     if slices > 1 and not (swapped and slices <= 8 and tokens <= bn):
         partial, counters = _gemm_workspace(x.device)
@@ -2900,7 +2930,7 @@ def set_programmatic_launch(enabled: bool) -> None:
 
 
 __all__ = ["KernelError", "KernelBuildError", "embedding", "add_rmsnorm", "hc_norm", "linear_hc_rmsnorm", "rope_norm_cache", "glu_limited", "gate_up_glu", "sigmoid_gate", "key_span", "rope_and_cache", "swiglu",
-           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "float32_decode_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "few_prefill_keys", "paged_attention_decode", "paged_attention_decode_spread", "spreads_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
+           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "float32_decode_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "few_prefill_keys", "paged_attention_decode", "paged_attention_decode_spread", "spreads_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gated_sums", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
            "attention_library", "group_norm", "round_stream", "conv_silu", "SCAN_FEW", "only_short_portions", "ssm_scan", "router", "moe_experts", "moe_combine",
            "norm_rope_cache", "turn_heads", "soft_cap", "embed_sum", "matrix_cell", "cell_output", "gated_recurrence", "xielu",
            "DiffPair", "diff_in_attention", "diff_combine", "heads_to_pages", "branch_norm", "PairedOutput", "WeighedTerms",

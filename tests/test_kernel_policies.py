@@ -70,6 +70,19 @@ def test_float32_outputs_keep_their_slices():
     assert F.gemm_plan(48, 5120, 5120, SMS)[2] == F.gemm_plan(48, 5120, 5120, SMS, out_f32=True)[2]
 
 
+def test_gated_products_in_one_block_keep_the_sums_of_their_slices():
+    for tokens in (1, 16, 24, 64):
+        for features in range(128, 20000, 128):
+            for k in (64, 200, 256, 320, 896, 4096, 8192):
+                sums, slices = F.gated_sums(tokens, features, k, SMS), F.gemm_plan(tokens, features, k, SMS, out_f32=True)[2]
+                _, bn, gated = F.gemm_plan(tokens, features, k, SMS, True)
+                tiles = features // 128
+                # the sums of the slices, in as many columns of tensor memory as a block alone on its SM may take
+                assert sums == 1 or gated == 1 and sums == slices and sums <= 8 and sums * bn <= 256
+                assert gated == 1 or sums == 1
+                assert sums == 1 or tiles <= SMS and ((k + 63) // 64 > 4 or tiles <= SMS // 2)
+
+
 def test_where_a_projection_adds_itself_to_the_stream():
     """The last projection of a branch takes over the add and prepares the norm behind it in decode steps of up to
     16 tokens, where its K slices are a cluster and the width is a multiple of 128; for long prompt portions only

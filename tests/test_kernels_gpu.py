@@ -620,6 +620,23 @@ def test_tcgen05_fused_swiglu(tokens, inter, k, bias):
     ops().check_errors(torch.device(DEV))
 
 
+# sums of 3, 4 and 5 slices in one block, the last of fewer K steps than the others (14 steps in 4 and in 5, 6 in 5, 24 in 3, 9 in 3), a last
+# step that is not full, blocks for up to half and for all of the SMs
+@pytest.mark.parametrize("tokens", [1, 16, 17, 33, 64])
+@pytest.mark.parametrize("features, k", [(9728, 896), (7680, 840), (8960, 328), (17920, 1536), (13440, 1704), (18816, 520)])
+def test_a_gated_product_in_one_block_gives_the_bits_of_its_slices(tokens, features, k):
+    torch.manual_seed(features + k)
+    x, w = torch.randn(tokens, k, device=DEV).bfloat16(), (torch.randn(features, k, device=DEV) * k ** -0.5).bfloat16()
+    bias = torch.randn(features, device=DEV)
+    bn = 16 if tokens <= 16 else 32 if tokens <= 32 else 64
+    sums = ops().gated_sums(tokens, features, k)
+    assert ops().gemm_plan(tokens, features, k, None, True) == (True, bn, 1) and (sums > 1 or bn == 64)
+    for options in (dict(), dict(out_dtype=torch.float32, bias=bias), dict(glu=(1.7, 7.0, 1.0, 0.0))):
+        got = [ops().gemm_tcgen05(x, w, swiglu=True, plan=plan, **options) for plan in (None, (True, bn, sums))]
+        assert torch.equal(*got)
+    ops().check_errors(torch.device(DEV))
+
+
 # rings that fill an SM: fewer, as many and more K steps than the ring's 10 (8 with 64 columns) stages and than twice as many,
 # with a last step that is not full; blocks up to half of the SMs with few steps, up to all of them with more, and beyond
 @pytest.mark.parametrize("tokens", [1, 16, 17, 33, 64])

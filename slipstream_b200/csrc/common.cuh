@@ -233,6 +233,29 @@ static inline void ss_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 b
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// How many clusters of `n` blocks (along grid.z) of a kernel run at the same time: clusters do not cross the GPU's processor clusters, so
+// fewer than its multiprocessors hold blocks.  0 where the runtime has no answer.  The kernel has its shared memory opted in.
+template <typename K>
+static inline int ss_resident_clusters(K kernel, int threads, int smem, int n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, n);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = n;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int count = 0;
+    if (cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return count;
+}
+
 // Blocks along grid.x grouped into clusters of `cluster_x`.
 template <typename... KArgs, typename... Args>
 static inline void ss_launch_cluster_x(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

@@ -368,23 +368,8 @@ static int f3_resident_clusters(int n) {
         using Form = F32Form<16, 2, 3, true>;
         static SsPerDevice opted;
         int count = 0;
-        if (ss_opt_in_smem(gemm_f32_kernel<16, 2, 3, true>, Form::SMEM, opted) == 0) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(1, 1, n);
-            cfg.blockDim = dim3(F3_THREADS);
-            cfg.dynamicSmemBytes = Form::SMEM;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = 1;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = n;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&count, gemm_f32_kernel<16, 2, 3, true>, &cfg) != cudaSuccess) {
-                cudaGetLastError();
-                count = 0;
-            }
-        }
+        if (ss_opt_in_smem(gemm_f32_kernel<16, 2, 3, true>, Form::SMEM, opted) == 0)
+            count = ss_resident_clusters(gemm_f32_kernel<16, 2, 3, true>, F3_THREADS, Form::SMEM, n);
         known[dev][n] = count > 0 ? count : (ss_sm_count() / n > 0 ? ss_sm_count() / n : 1);
     }
     return known[dev][n];

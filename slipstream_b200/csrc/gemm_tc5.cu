@@ -931,6 +931,22 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& 
     return SS_LAUNCH_CHECK();
 }
 
+// How many clusters of n blocks with a ring that fills an SM run at the same time (asked one time a device; the kernels of 32 and 64 columns
+// leave no room for a second block either).
+static int clusters_alone(int n) {
+    static int known[SS_MAX_DEVICES][9];  // 0: not asked yet
+    const int dev = ss_current_device();
+    if (dev < 0 || n < 1 || n > 8) return 0;
+    if (known[dev][n] == 0) {
+        constexpr int smem = 10 * (TC_BM * TC_BK * 2 + 16 * TC_BK * 2) + 1024 + 512;
+        static SsPerDevice opted;
+        int count = 0;
+        if (ss_opt_in_smem(gemm_tc5_kernel<16, 10, 0, 4>, smem, opted) == 0) count = ss_resident_clusters(gemm_tc5_kernel<16, 10, 0, 4>, TC_THREADS, smem, n);
+        known[dev][n] = count > 0 ? count : -1;
+    }
+    return known[dev][n];
+}
+
 // The 16-column kernels of a decode step: the form (PATH) and the ends (ENDS) as kernels of their own.
 template <int STAGES>
 static int launch16(int ends, const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& g, dim3 grid, cudaStream_t stream) {
@@ -1026,15 +1042,17 @@ static int gemm_tc5(const void* A, const void* B, const void* bias, int bias_f32
     g.part_steps = parts > 1 ? (per + parts - 1) / parts : 0;
     const bool deep = swapped && per >= 24;
     dim3 grid((N + bn - 1) / bn, (M + TC_BM - 1) / TC_BM, slices);
-    // No more blocks than SMs: a ring that fills the SM.  Most or all of a block's weights are then under way before the kernel in
-    // front has ended, and clusters do not pile up on a few SMs (with four stages, three blocks fit on one, beside
-    // empty ones).  Where the blocks have no more K steps than the four stages hold, only the second counts, and it
+    // A ring that fills the SM where all blocks stand at the same time so.  Most or all of a block's weights are then under way before the
+    // kernel in front has ended, and clusters do not pile up on a few SMs (with four stages, three blocks fit on one, beside
+    // empty ones).  Clusters that wait for a second round cost more than that gives: 4 tokens, K 8,192 in 8 slices, 15 tiles 8.8 -> 8.4 us,
+    // 16 to 18 9.1 to 9.7 -> 13.2 to 13.4 (and 2,176 x 2,176 4.7 -> 7.3), so clusters are counted as the runtime places them.
+    // Where the blocks have no more K steps than the four stages hold, only the room counts, and it
     // pays as long as the kernel behind, which starts early, finds SMs without such a block: up to half of them.  A
-    // request of 16 tokens in 24 layers of 896 (q/k/v 72 blocks of 2 steps, o 56 of 2, down 56 of 10): 11.47 -> 10.53 ms,
-    // 11.35 with down alone; 12 layers of 1,536 (down 96 blocks of 18; q/k/v 128 of 3, o 96 of 3): 8.86 -> 8.50,
-    // 8.97 with all three.
+    // request's step through 24 layers of 896 (q/k/v 72 blocks of 2 steps, o 56 of 2, down 56 of 10), replayed from its graph: 641 -> 581 us;
+    // through 12 of 1,536 (down 96 blocks of 18; q/k/v 128 of 3 and o 96 of 3 stay): 498 -> 478.
     const int64_t blocks = (int64_t)grid.x * grid.y * grid.z;
-    const bool alone = swapped && blocks <= ss_sm_count() && (per > 4 || blocks <= ss_sm_count() / 2);
+    const bool resident = cluster ? blocks / slices <= clusters_alone(slices) : blocks <= ss_sm_count();
+    const bool alone = swapped && resident && (per > 4 || blocks <= ss_sm_count() / 2);
     // (more than 64 columns of tensor memory only where no other block that takes some can stand beside this one and wait for it)
     if (parts > 1 && !alone) return -2005;
     if (!swapped) grid = dim3((M + TC_BM - 1) / TC_BM, (N + bn - 1) / bn, slices);

@@ -641,7 +641,7 @@ def test_a_gated_product_in_one_block_gives_the_bits_of_its_slices(tokens, featu
 # with a last step that is not full; blocks up to half of the SMs with few steps, up to all of them with more, and beyond
 @pytest.mark.parametrize("tokens", [1, 16, 17, 33, 64])
 @pytest.mark.parametrize("features, k, slices", [(896, 104, 2), (128, 640, 1), (128, 648, 1), (9472, 320, 1), (9600, 264, 1), (18944, 360, 1),
-                                                 (19072, 328, 1), (896, 4864, 8), (1000, 1416, 1)])
+                                                 (19072, 328, 1), (896, 4864, 8), (1000, 1416, 1), (1920, 4160, 8), (2176, 4160, 8)])
 def test_tcgen05_with_blocks_alone_on_their_multiprocessors(tokens, features, k, slices):
     torch.manual_seed(features + k)
     x, w = torch.randn(tokens, k, device=DEV).bfloat16(), torch.randn(features, k, device=DEV).bfloat16()

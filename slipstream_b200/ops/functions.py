@@ -1002,6 +1002,7 @@ def paged_attention_decode_spread(q: torch.Tensor, q_stride: int, out: torch.Ten
         _ptr(inv_freq) if rotary_dim else None, rotary_dim, int(rope is not None), scratch.data_ptr(), _gate_ptr(gate, q, q_stride),
         error_word(q.device).data_ptr(), _stream(), float(softcap or 0.0), _ptr(sinks), _kept(keep, window), out_f32),
         "paged_attention_decode_spread")
+    _launches[0] += 1  # the kernel that combines the units that a cut divides
 
 
 DECODE_SPREAD_REQUESTS = 512  # what the spread decode kernel takes at most

@@ -458,6 +458,48 @@ def test_decode_with_tiles_dealt_out_evenly(lens, n_q, n_kv, d, page, window, ke
     ops().check_errors(torch.device(DEV))
 
 
+def spread_step(lens, n_kv, d, page, pages, seed, rows=None):
+    """A decode step's context on the device and its pages' table: ``rows`` requests, those behind ``lens`` without keys."""
+    from types import SimpleNamespace
+    rows = rows or len(lens)
+    host = np.array([*lens, *[0] * (rows - len(lens))], dtype=np.int32)
+    perm, table = iter(np.random.default_rng(seed).permutation(pages).tolist()), np.full((rows, pages), -1, dtype=np.int32)
+    for r, n in enumerate(host):
+        table[r, :-(-int(n) // page)] = [next(perm) for _ in range(-(-int(n) // page))]
+    ctx = SimpleNamespace(is_decode_only=True, num_requests=rows, max_seq_len=int(host.max()), seq_lens_host=host, extras={},
+                          seq_lens=torch.tensor(host, device=DEV), q_start=torch.arange(rows + 1, dtype=torch.int32, device=DEV))
+    return ctx, torch.tensor(table, device=DEV)
+
+
+UNEVEN = [(2 + i % 5) * 300 for i in range(40)]
+
+
+def test_decode_attention_of_uneven_requests_takes_the_kernel_that_deals_tiles_out():
+    n_q, n_kv, d, page = 32, 4, 64, 16
+    ctx, table = spread_step(UNEVEN, n_kv, d, page, 4000, 1)
+    kv = torch.randn(4000, 2, n_kv, page, d, device=DEV).bfloat16()
+    qkv = torch.randn(40, n_q * d, device=DEV).bfloat16()
+    diff = ops().DiffPair(0.4, 0.6, 1e-5, d)
+
+    def run(pages, told=None, pair=None):
+        ctx.extras.clear()
+        if told is not None:
+            ctx.extras[("decode_spread", n_kv, n_q // n_kv, d, 0)] = told
+        out = torch.full((40, n_q * d // (2 if pair else 1)), float("nan"), device=DEV, dtype=torch.bfloat16)
+        before = ops().launch_count()
+        ops().paged_attention(qkv, out, pages, table, ctx, n_q, n_kv, d, d ** -0.5, diff=pair)
+        return out, ops().launch_count() - before
+
+    (a, two), (b, one) = run(kv), run(kv, False)
+    assert (two, one) == (2, 1) and rel_err(a, b) < 1e-2  # bfloat16 outputs, as above
+    (a, three), (b, two) = run(kv, pair=diff), run(kv, False, diff)
+    assert (three, two) == (3, 2) and rel_err(a, b) < 1e-2
+    odd = torch.randn(1400, 2, n_kv, 48, d, device=DEV).bfloat16()  # pages that it does not take
+    table.clamp_(max=1399)
+    assert run(odd)[1] == 1
+    ops().check_errors(torch.device(DEV))
+
+
 @pytest.mark.parametrize("with_sinks", [False, True])
 def test_tiles_dealt_out_evenly_pass_on_scores_that_are_not_numbers(with_sinks):
     """A query of NaN, keys of NaN (one; all of some tiles), a value of infinity among keys whose scores are -infinity, in requests that

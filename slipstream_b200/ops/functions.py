@@ -1017,14 +1017,17 @@ def spreads_decode(seq_lens: np.ndarray, n_kv: int, group: int, head_dim: int, r
     two on every SM, and the last round lasts as long as its longest unit; dealt out evenly all tiles take the time of the bytes, and the merges and the
     second kernel 11 (10).  48 requests x 4, 900 keys on average: 27.0 and 25.1 us, 1,800: 49.1 and 38.1, 1,800 each: 35.8 and 36.9."""
     n = int(seq_lens.size)
-    units = n * n_kv * ((group + 15) // 16)
-    if n_kv < 2 or group > 8 or n > DECODE_SPREAD_REQUESTS or decode_slices(n, n_kv, group, int(seq_lens.max()), False, sms) != 1:
+    per_request = n_kv * ((group + 15) // 16)
+    # (as many blocks as SMs, or fewer: `decode_slices` cuts the keys of all but the shortest requests)
+    if n_kv < 2 or group > 8 or n > DECODE_SPREAD_REQUESTS or n * per_request <= sms:
         return False
-    tiles = (np.minimum(seq_lens, reach) if reach else seq_lens).astype(np.int64) // 64 + 1
+    units = n * per_request
+    seen = np.minimum(seq_lens, reach) if reach else seq_lens
+    longest, total = int(seen.max()) // 64 + 1, int((seen >> 6).sum()) + n  # tiles of 64 keys
     alone, crowded, fixed = (1.1, 1.56, 11.0) if head_dim == 128 else (0.8, 0.78, 10.0)
     rounds, rest = divmod(units, 2 * sms)
-    one_block = 3.0 + rounds * crowded * float(tiles.mean()) + (float(tiles.max()) * max(alone, crowded * rest / (2 * sms)) if rest else 0.0)
-    spread = fixed + crowded * float(tiles.sum()) * (units // n) / (2 * sms)
+    one_block = 3.0 + rounds * crowded * (total / n) + (longest * max(alone, crowded * rest / (2 * sms)) if rest else 0.0)
+    spread = fixed + crowded * total * per_request / (2 * sms)
     return spread < 0.97 * one_block
 
 
@@ -1135,13 +1138,16 @@ def paged_attention(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tensor, bloc
                                sm_count(qkv.device))
         scratch = ctx.extras.get(("decode_scratch", n_q, head_dim)) if not across else None
         heads = out if diff is None else _heads_f32(out, n_q, head_dim)
-        reach = (window or chunk) + keep
-        key = ("decode_spread", n_kv, group, head_dim, reach)
-        spread = ctx.extras.get(key)
-        if spread is None:  # the same for every layer of the step that sees as far; a captured step was told
-            spread = ctx.extras[key] = not static and spreads_decode(ctx.seq_lens_host, n_kv, group, head_dim, reach, sm_count(qkv.device))
-        if (spread and slices == 1 and not across and tcgen05_attention_fits(head_dim, n_q, n_kv, kv.shape[3], 0)
-                and ctx.num_requests * n_kv * (block_tables.shape[1] * kv.shape[3] // 64 + 2) < 2 ** 31):
+        # asked only where the kernel takes the layer, one time for every layer of the step that sees as far; a captured step was told
+        spread = (slices == 1 and not across and tcgen05_attention_fits(head_dim, n_q, n_kv, kv.shape[3], 0)
+                  and ctx.num_requests * n_kv * (block_tables.shape[1] * kv.shape[3] // 64 + 2) < 2 ** 31)
+        if spread:
+            reach = (window or chunk) + keep
+            key = ("decode_spread", n_kv, group, head_dim, reach)
+            spread = ctx.extras.get(key)
+            if spread is None:
+                spread = ctx.extras[key] = not static and spreads_decode(ctx.seq_lens_host, n_kv, group, head_dim, reach, sm_count(qkv.device))
+        if spread:
             paged_attention_decode_spread(qkv, qkv.shape[1], heads, kv, block_tables, ctx.q_start, ctx.seq_lens, ctx.num_requests,
                                           n_q, n_kv, head_dim, scale, window, rope, chunk, gate, softcap, sinks, keep)
             if diff is not None:

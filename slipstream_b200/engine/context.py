@@ -153,6 +153,7 @@ class HostPlan:
     slot_maps: np.ndarray  # [groups, N]
     page_sizes: list[int]  # per cache group
     requests: list = field(default_factory=list)  # the cache manager's record of each entry's request
+    rows: int = 0  # requests of the captured step that runs this one (0: none does)
 
     @property
     def num_requests(self) -> int:

@@ -154,6 +154,7 @@ class ModelRunner:
         attention, say, cuts the keys of few long requests into more slices than those of many short ones, and
         the number of slices is fixed when a graph is captured)."""
         longest = int(plan.seq_lens.max())
+        plan.rows = bucket
         variants = tuple(part.capture_variant(longest, plan) for part in self.variant_parts)
         graph = self._graphs.get((bucket, variants))
         if graph is None:

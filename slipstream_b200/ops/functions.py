@@ -1008,18 +1008,19 @@ def paged_attention_decode_spread(q: torch.Tensor, q_stride: int, out: torch.Ten
 DECODE_SPREAD_REQUESTS = 512  # what the spread decode kernel takes at most
 
 
-def spreads_decode(seq_lens: np.ndarray, n_kv: int, group: int, head_dim: int, reach: int, sms: int) -> bool:
+def spreads_decode(seq_lens: np.ndarray, n_kv: int, group: int, head_dim: int, reach: int, sms: int, rows: int = 0) -> bool:
     """Whether a decode step's key tiles are dealt out evenly (`paged_attention_decode_spread`): its host lengths, the keys a
-    query sees at most (0: all).  Only where a request's head block would have one block, two per SM at a time, and up to 8 heads
+    query sees at most (0: all), the requests of the captured step that runs it (0: its own; the kernels of that step are launched for as
+    many, and those without a token cost nothing).  Only where a request's head block would have one block, two per SM at a time, and up to 8 heads
     share a kv head (with more the next unit's queries wait for the merge).  What either way takes, in us, fitted to 28 and 32 heads on 4 and 8
     kv heads of 128 elements and 14 and 32 on 2 and 4 of 64, 24 to 200 requests of 100 to 3,600 keys on average, equal or between half
     and one and a half of that: one block a unit walks a tile of 64 keys in 1.1 us (128 elements; 0.8 with 64), 1.56 (0.78) with
     two on every SM, and the last round lasts as long as its longest unit; dealt out evenly all tiles take the time of the bytes, and the merges and the
     second kernel 11 (10).  48 requests x 4, 900 keys on average: 27.0 and 25.1 us, 1,800: 49.1 and 38.1, 1,800 each: 35.8 and 36.9."""
     n = int(seq_lens.size)
-    per_request = n_kv * ((group + 15) // 16)
+    rows, per_request = rows or n, n_kv * ((group + 15) // 16)
     # (as many blocks as SMs, or fewer: `decode_slices` cuts the keys of all but the shortest requests)
-    if n_kv < 2 or group > 8 or n > DECODE_SPREAD_REQUESTS or n * per_request <= sms:
+    if n_kv < 2 or group > 8 or rows > DECODE_SPREAD_REQUESTS or rows * per_request <= sms:
         return False
     units = n * per_request
     seen = np.minimum(seq_lens, reach) if reach else seq_lens

@@ -282,7 +282,7 @@ class PagedAttention(Mixer):
         if plan is None or not self._may_spread:
             return False
         return ops.spreads_decode(plan.seq_lens, self.num_kv_heads, self.num_heads // self.num_kv_heads, self.head_dim, self.sees,
-                                  ops.sm_count(self.runtime.device))
+                                  ops.sm_count(self.runtime.device), getattr(plan, "rows", 0))
 
     def capture_variant(self, longest: int, plan: object = None) -> object:
         """Decode steps: long contexts of few requests want the keys cut into more slices than fit one thread-block

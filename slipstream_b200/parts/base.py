@@ -128,7 +128,7 @@ class Part:
     def capture_variant(self, longest: int, plan: object = None) -> object:
         """Which captured form of this part a step whose longest request holds ``longest`` tokens should run
         (any hashable; None: there is only one form).  ``plan`` is the step's host-side metadata
-        (``engine.context.HostPlan``: ``q_lens``, ``seq_lens``, ``is_decode_only``) or None.  The runner keeps one
+        (``engine.context.HostPlan``: ``q_lens``, ``seq_lens``, ``is_decode_only``, ``rows``) or None.  The runner keeps one
         graph per bucket and combination of variants."""
         return None
 

@@ -318,3 +318,41 @@ def test_layers_off_the_spread_decode_kernel_are_captured_in_one_form(monkeypatc
     for x in (layer(), layer(pages=128)):
         x.prepare_capture(ctx, x.capture_variant(int(lens.max()), plan), 16384)
     assert ctx.extras[("decode_spread", 4, 7, 128, 0)] is True
+
+
+def bare_runner(monkeypatch, layer, max_num_seqs, max_model_len=4096):
+    """A model runner of one layer that records the graphs it captures instead of capturing them."""
+    from types import SimpleNamespace
+    from slipstream_b200.engine import runner as module
+    monkeypatch.setattr(F, "_device_sm_count", lambda index: SMS)
+    monkeypatch.setattr(module, "DecodeGraph", lambda runner, bucket, variants: SimpleNamespace(bucket=bucket, variants=variants))
+    made = module.ModelRunner.__new__(module.ModelRunner)
+    made.use_cuda_graphs, made.max_num_seqs, made.max_model_len, made.variant_parts, made._graphs = True, max_num_seqs, max_model_len, [layer], {}
+    return made
+
+
+def decode_plan(lens):
+    from types import SimpleNamespace
+    lens = np.asarray(lens, dtype=np.int32)
+    return SimpleNamespace(is_decode_only=True, q_lens=np.ones(lens.size, dtype=np.int32), seq_lens=lens, rows=0)
+
+
+def spread_layer(heads=28, kv_heads=4, **kind):
+    import torch
+    from slipstream_b200.parts import PagedAttention, RotaryEncoding
+    from slipstream_b200.parts.base import Runtime
+    layer = PagedAttention("attn", 64, heads, kv_heads, 128, RotaryEncoding(128, 1e4), **kind)
+    layer.runtime = Runtime(torch.device("cuda:0"), torch.bfloat16)
+    return layer
+
+
+def test_the_rule_for_dealing_tiles_out_asks_for_the_requests_of_the_captured_step(monkeypatch):
+    """36 requests run in the graph for 48, whose blocks are too many to cut a request's keys: they ask as those would.  In a graph of
+    as many blocks as multiprocessors, where keys are cut, none does; nor behind 512 requests."""
+    runner = bare_runner(monkeypatch, spread_layer(), 600)
+    lens = [(2 + i % 5) * 450 for i in range(48)]
+    for live, bucket, form in ((33, 48, 2), (36, 48, 2), (37, 48, 2), (48, 48, 2), (30, 32, 0), (24, 24, 0)):
+        graph = runner._decode_graph(bucket, decode_plan(lens[:live]))
+        assert (graph.bucket, graph.variants) == (bucket, (form,)), live
+    one_long = np.array([20000] + [100] * 400, dtype=np.int32)
+    assert [F.spreads_decode(one_long, 4, 7, 128, 0, SMS, rows=n) for n in (0, 512, 600)] == [True, True, False]

@@ -14,6 +14,7 @@ class; neither has a forward pass, cache or loader of its own.
 
 from __future__ import annotations
 
+import itertools
 from pathlib import Path
 
 import numpy as np
@@ -190,19 +191,21 @@ class ModelRunner:
         return bucket if bucket is not None and bucket <= max(self.max_num_seqs, 1) * 2 else None
 
     def capture_decode_graphs(self, max_requests: int | None = None) -> int:
-        """Capture the decode graph of every batch bucket up to ``max_requests`` (default: the most requests
-        the cache manager admits) now, instead of at the first step that needs it: a capture takes tens of
-        milliseconds, during which every running request waits.  Returns how many graphs were captured."""
+        """Capture the decode graphs of every batch bucket up to ``max_requests`` (default: the most requests
+        the cache manager admits) now, instead of at the first step that needs them: a capture takes tens of
+        milliseconds, during which every running request waits.  A bucket has a graph for every form that its parts may ask for
+        (``Part.prepared_variants``; not those of contexts from 8,192 tokens on).  Returns how many graphs were captured."""
         if not self.use_cuda_graphs:
             return 0
         limit = self.max_num_seqs if max_requests is None else max_requests
         made = 0
         for bucket in BUCKETS:
-            variants = tuple(part.capture_variant(1) for part in self.variant_parts)  # the form for short requests
-            if self._graph_bucket(bucket) != bucket or (bucket, variants) in self._graphs:
+            if self._graph_bucket(bucket) != bucket:
                 continue
-            self._graphs[(bucket, variants)] = DecodeGraph(self, bucket, variants)
-            made += 1
+            for variants in itertools.product(*(part.prepared_variants(bucket, self.max_model_len) for part in self.variant_parts)):
+                if (bucket, variants) not in self._graphs:
+                    self._graphs[(bucket, variants)] = DecodeGraph(self, bucket, variants)
+                    made += 1
             if bucket >= limit:
                 break
         return made

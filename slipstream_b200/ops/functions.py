@@ -1032,6 +1032,18 @@ def spreads_decode(seq_lens: np.ndarray, n_kv: int, group: int, head_dim: int, r
     return spread < 0.97 * one_block
 
 
+def may_spread_decode(rows: int, n_kv: int, group: int, head_dim: int, reach: int, longest: int, sms: int) -> bool:
+    """Whether a captured step of ``rows`` requests of up to ``longest`` tokens is worth preparing with its tiles dealt out:
+    `spreads_decode` says yes to one, a quarter, half or all of them at that length, the others short, or to half or three quarters as many."""
+    for live in (rows, 3 * rows // 4, rows // 2 + 1):
+        lens = np.ones(max(live, 1), dtype=np.int32)
+        for long_ones in (1, live // 4, live // 2, live):
+            lens[:long_ones] = longest
+            if spreads_decode(lens, n_kv, group, head_dim, reach, sms, rows):
+                return True
+    return False
+
+
 WIDE_CONTEXT = 8192  # from this many cached tokens a decode step of few requests may use more than 8 slices
 
 
@@ -2938,7 +2950,7 @@ def set_programmatic_launch(enabled: bool) -> None:
 
 
 __all__ = ["KernelError", "KernelBuildError", "embedding", "add_rmsnorm", "hc_norm", "linear_hc_rmsnorm", "rope_norm_cache", "glu_limited", "gate_up_glu", "sigmoid_gate", "key_span", "rope_and_cache", "swiglu",
-           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "float32_decode_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "few_prefill_keys", "paged_attention_decode", "paged_attention_decode_spread", "spreads_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gated_sums", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
+           "gemm_simt", "gemm_float32", "paged_attention_simt", "paged_attention_float32", "float32_key_parts", "float32_decode_parts", "paged_attention", "fuses_rope", "paged_attention_prefill", "paged_attention_prefill_tcgen05", "prefill_key_parts", "tcgen05_attention_fits", "tcgen05_prefill_fits", "few_prefill_keys", "paged_attention_decode", "paged_attention_decode_spread", "spreads_decode", "may_spread_decode", "decode_scratch", "decode_slices", "is_long_context", "require_cuda", "argmax", "sample", "mark_seen", "gather_tokens", "prepare_decode", "gemm_tcgen05", "gemm_tcgen05_many", "many_tokens_fits", "many_tokens_swiglu_fits", "gemm_plan", "gated_sums", "gemm_library", "gate_up_swiglu", "set_programmatic_launch", "launch_count", "count_launches", "sm_count", "linear", "linear_add_rmsnorm", "adds_to_stream", "takes_pending_norm", "PendingNorm", "set_norm_fusion", "check_errors", "raise_for_status", "error_word", "ops_library",
            "attention_library", "group_norm", "round_stream", "conv_silu", "SCAN_FEW", "only_short_portions", "ssm_scan", "router", "moe_experts", "moe_combine",
            "norm_rope_cache", "turn_heads", "soft_cap", "embed_sum", "matrix_cell", "cell_output", "gated_recurrence", "xielu",
            "DiffPair", "diff_in_attention", "diff_combine", "heads_to_pages", "branch_norm", "PairedOutput", "WeighedTerms",

@@ -303,6 +303,12 @@ class PagedAttention(Mixer):
         return int(ops.prefill_key_parts(plan.q_lens, plan.seq_lens, 128 // group, self.kernel_blocks,
                                          ops.sm_count(self.runtime.device), self.sees))
 
+    def prepared_variants(self, rows: int, max_model_len: int) -> list:
+        # short requests, and requests of different lengths where a step of so many may ask for that form
+        may = self._may_spread and ops.may_spread_decode(rows, self.num_kv_heads, self.num_heads // self.num_kv_heads, self.head_dim,
+                                                         self.sees, max_model_len, ops.sm_count(self.runtime.device))
+        return [0, 2] if may else [0]
+
     def capture_group(self) -> object:
         # what `capture_variant` answers from beside the step's lengths
         fits = ops.tcgen05_prefill_fits(self.head_dim, self.num_heads, self.num_kv_heads, self.page_tokens)

@@ -132,6 +132,10 @@ class Part:
         graph per bucket and combination of variants."""
         return None
 
+    def prepared_variants(self, rows: int, max_model_len: int) -> list:
+        """What `capture_variant` answers for decode steps of ``rows`` requests that are to be captured before the first of them runs."""
+        return [self.capture_variant(1)]
+
     def capture_group(self) -> object:
         """Parts that return the same value here always answer ``capture_variant`` alike (every attention layer
         of a model, say), so the runner asks one of them per step."""

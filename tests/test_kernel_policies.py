@@ -1,6 +1,7 @@
 """The host-side rules that pick a kernel's shape (no GPU needed): slices of the decode attention, key parts of
 the prefill attention, tile and K slices of the streaming matrix product, and which product a projection runs."""
 import numpy as np
+import pytest
 
 from slipstream_b200.ops import functions as F
 
@@ -356,3 +357,16 @@ def test_the_rule_for_dealing_tiles_out_asks_for_the_requests_of_the_captured_st
         assert (graph.bucket, graph.variants) == (bucket, (form,)), live
     one_long = np.array([20000] + [100] * 400, dtype=np.int32)
     assert [F.spreads_decode(one_long, 4, 7, 128, 0, SMS, rows=n) for n in (0, 512, 600)] == [True, True, False]
+
+
+@pytest.mark.parametrize("kind, most, graphs", [(dict(), 64, 11), (dict(kv_heads=28), 64, 15), (dict(heads=4, kv_heads=1), 64, 9), (dict(page_size=48), 64, 9),
+                                                (dict(window=128), 64, 9)])
+def test_a_prepared_runner_captures_nothing_when_requests_become_uneven(monkeypatch, kind, most, graphs):
+    runner = bare_runner(monkeypatch, spread_layer(**kind), most)
+    assert runner.capture_decode_graphs() == graphs == len(runner._graphs)
+    rng = np.random.default_rng(0)
+    for live in (1, 5, 20, 24, 33, 40, 48, 50, 64):
+        for mean in (1, 100, 700, 1500, 2300):
+            for lens in ([mean] * live, rng.uniform(0.3, 1.7, live) * mean + 1, [4000] + [mean] * (live - 1)):
+                runner._decode_graph(runner._graph_bucket(live), decode_plan(lens))
+    assert len(runner._graphs) == graphs and runner.capture_decode_graphs() == 0

@@ -500,6 +500,46 @@ def test_decode_attention_of_uneven_requests_takes_the_kernel_that_deals_tiles_o
     ops().check_errors(torch.device(DEV))
 
 
+def test_a_captured_step_deals_tiles_out_by_the_lengths_of_each_replay():
+    """Two layers' attention with the rotation inside, captured for 48 requests and replayed with fewer of them, with other cuts, with one
+    request much longer and with one alone: the bits of the kernel called directly, and within bfloat16 of one block a unit."""
+    n_q, n_kv, d, page, pages, rows = 16, 4, 64, 16, 6000, 48
+    g = torch.Generator(device=DEV).manual_seed(3)
+    kv = [torch.randn(pages, 2, n_kv, page, d, device=DEV, generator=g).bfloat16() for _ in range(2)]
+    qkv = [torch.randn(rows, (n_q + 2 * n_kv) * d, device=DEV, generator=g).bfloat16() for _ in range(2)]
+    rope = ((1.0 / 10000.0 ** (torch.arange(0, d, 2, dtype=torch.float32) / d)).to(DEV), d)
+    outs = [torch.empty(rows, n_q * d, device=DEV, dtype=torch.bfloat16) for _ in range(2)]
+    ctx, table = spread_step([], n_kv, d, page, pages, 0, rows)
+    ctx.extras.update({"static_max_seq_len": 96000, "decode_wide": False, ("decode_spread", n_kv, n_q // n_kv, d, 0): True})
+
+    def step():
+        for layer in range(2):
+            ops().paged_attention(qkv[layer], outs[layer], kv[layer], table, ctx, n_q, n_kv, d, d ** -0.5, rope=rope)
+
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        step()
+    torch.cuda.synchronize()
+    graph, before = torch.cuda.CUDAGraph(), ops().launch_count()
+    with torch.cuda.graph(graph):
+        step()
+    assert ops().launch_count() - before == 4
+    for seed, lens in enumerate([UNEVEN[:36], [1 + 37 * i for i in range(48)], [20000] + [5 + i for i in range(40)], [0, 0, 777], [640] * 48]):
+        now, pages_of = spread_step(lens, n_kv, d, page, pages, seed, rows)
+        ctx.seq_lens.copy_(now.seq_lens)
+        table.copy_(pages_of)
+        copies = [t.clone() for t in kv]
+        graph.replay()
+        for layer in range(2):
+            for f, pool in ((ops().paged_attention_decode_spread, copies[layer]), (ops().paged_attention_decode, copies[layer].clone())):
+                want = torch.full_like(outs[0], float("nan"))
+                f(qkv[layer], qkv[layer].shape[1], want, pool, pages_of, now.q_start, now.seq_lens, rows, n_q, n_kv, d, d ** -0.5, rope=rope)
+                assert torch.equal(pool, kv[layer])
+                assert torch.equal(outs[layer], want) if f is ops().paged_attention_decode_spread else rel_err(outs[layer], want) < 1e-2
+            assert (outs[layer][len(lens):] == 0).all()
+    ops().check_errors(torch.device(DEV))
+
+
 @pytest.mark.parametrize("with_sinks", [False, True])
 def test_tiles_dealt_out_evenly_pass_on_scores_that_are_not_numbers(with_sinks):
     """A query of NaN, keys of NaN (one; all of some tiles), a value of infinity among keys whose scores are -infinity, in requests that

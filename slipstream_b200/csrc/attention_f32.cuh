@@ -331,9 +331,11 @@ __global__ void __launch_bounds__(AF_THREADS, D <= 128 ? 3 : 1) attn_f32_kernel(
 // Bound by shared memory: a load brings 128 bytes a cycle to an SM's registers, also where lanes share a word, so a slice's
 // scores take 3,700 cycles and its outputs as many, beside 3,000 in which its 131 KB arrive.  (Products of 4 x 4 a thread, on
 // two warps, need half of that and run longer all the same: 439 us where these take 359, a warp has no other beside it.)
-// With its join, against attn_f32_kernel (four tiles of a slice one after another), us, 12 heads of 128 on 2: four requests
-// of 2,000 tokens 33.8 -> 17.0; 28 on 4: 20 of 800 79 -> 30, 20 of 16,000 1320 -> 359 (the memory takes 180), 200 of 300
-// 150 -> 88, one of 100 17.5 -> 8.5; 14 of 64 on 2: 256 of 1,000 240 -> 113.
+// With its join, against attn_f32_kernel (four tiles of a slice one after another), us, requests of equal length replayed from a
+// graph, 12 heads of 128 on 2: four of 2,000 tokens 28 -> 11 (33.8 -> 17.0 behind a layer's products); 28 on 4: 20 of 800 80 -> 27, 20 of
+// 16,000 1,080 -> 356 (the memory takes 180), 200 of 300 135 -> 85, one of 100 17.8 -> 8.8; 14 of 64 on 2: 256 of 1,000 239 -> 104.
+// Groups of more than 8 heads, whose keys come once for every 8, against tiles of 16 rows: heads of 128 on 1, 64 requests of 800
+// tokens, 9 heads 58 -> 35, 24 109 -> 49, 64 168 -> 125, 128 302 -> 228.
 #define AFD_RT 8
 #define AFD_THREADS 256
 #define AFD_PS 8
@@ -645,9 +647,6 @@ int launch_attn_f32_rows(const AttnF32Args& g, int n_tiles, int parts, cudaStrea
     return rc || !g.part ? rc : launch_attn_f32_join<D>(g, stream);
 }
 
-// 32 rows of a prompt portion to a block (64, with 8 warps and half the blocks: 257 us where 32 take 209, 777 tokens at the 7B sizes); a decode
-// step's rows of one request in tiles of 16, where attn_f32_decode_kernel does not take them (wider heads, whose slice passes
-// an SM's shared memory, and slices that pass the scratch memory's bound).
 template <int D, bool BOTH>
 int launch_attn_f32_decode(const AttnF32Args& g, dim3 grid, cudaStream_t stream) {
     constexpr int smem = afd_smem_bytes<D, BOTH>();
@@ -657,6 +656,9 @@ int launch_attn_f32_decode(const AttnF32Args& g, dim3 grid, cudaStream_t stream)
     return SS_LAUNCH_CHECK();
 }
 
+// 32 rows of a prompt portion to a block (64, with 8 warps and half the blocks: 257 us where 32 take 209, 777 tokens at the 7B sizes); a decode
+// step's rows of one request in tiles of 16, where attn_f32_decode_kernel does not take them (heads of more than 128, for which it has
+// no threads: 64 of them take 2 elements each of a half of the rows; and slices that pass the scratch memory's bound).
 template <int D>
 int launch_attn_f32(const AttnF32Args& g, int n_tiles, int parts, cudaStream_t stream) {
     if constexpr (D <= 128)

@@ -169,7 +169,7 @@ class LLMEngine:
 
     def warm_up(self, max_requests: int | None = None) -> int:
         """Capture the decode graphs of all batch sizes up to ``max_requests`` (default ``max_num_seqs``) before
-        the first request, so that no request ever waits for a capture.  Returns the number captured."""
+        the first request, so that no decode step of contexts below 8,192 tokens waits for a capture.  Returns the number captured."""
         return self.runner.capture_decode_graphs(max_requests)
 
     def add_request(self, request: Request) -> Sequence:

@@ -753,7 +753,7 @@ def paged_attention_float32(qkv: torch.Tensor, out: torch.Tensor, kv: torch.Tens
         _need(t, torch.int32, name)
     slices = max(1, -(-longest // FLOAT32_SLICE))
     parts = 1
-    if decode_only and head_dim <= 128:  # (wider heads: a slice's keys and values pass an SM's shared memory)
+    if decode_only and head_dim <= 128:  # (wider heads: the kernel has no threads for them)
         parts = float32_decode_parts(ctx.num_requests * ((group + 7) // 8) * (heads // group), slices, qkv.shape[0], heads,
                                      head_dim, sm_count(qkv.device))
     if parts == 1:
@@ -983,7 +983,8 @@ def paged_attention_decode_spread(q: torch.Tensor, q_stride: int, out: torch.Ten
                                   gate: torch.Tensor | None = None, softcap: float = 0.0, sinks: torch.Tensor | None = None,
                                   keep: int = 0) -> None:
     """`paged_attention_decode` for many requests of different lengths (`spreads_decode`): the key tiles of all of them are
-    dealt out evenly to two blocks an SM, by the lengths on the device.  Arguments as there."""
+    dealt out evenly to two blocks an SM, by the lengths on the device.  Arguments as there.  It takes groups of any size;
+    the rule chooses it for up to 8 heads a kv head."""
     if not tcgen05_attention_fits(head_dim, n_q, n_kv, kv.shape[3], 0) or n_requests > DECODE_SPREAD_REQUESTS:
         raise KernelError("the spread decode kernel takes head size 64 or 128, pages of 8, 16, 32 or 64 tokens and up to 512 requests")
     _check_sinks(sinks, n_q)
@@ -1016,7 +1017,9 @@ def spreads_decode(seq_lens: np.ndarray, n_kv: int, group: int, head_dim: int, r
     kv heads of 128 elements and 14 and 32 on 2 and 4 of 64, 24 to 200 requests of 100 to 3,600 keys on average, equal or between half
     and one and a half of that: one block a unit walks a tile of 64 keys in 1.1 us (128 elements; 0.8 with 64), 1.56 (0.78) with
     two on every SM, and the last round lasts as long as its longest unit; dealt out evenly all tiles take the time of the bytes, and the merges and the
-    second kernel 11 (10).  48 requests x 4, 900 keys on average: 27.0 and 25.1 us, 1,800: 49.1 and 38.1, 1,800 each: 35.8 and 36.9."""
+    second kernel 11 (10).  48 requests x 4, 900 keys on average: 27.0 and 25.1 us, 1,800: 49.1 and 38.1, 1,800 each: 35.8 and 36.9.
+    The microseconds are a B200's.  One kv head stays with one block a unit, to which they are not fitted (8 heads of 128 on 1, 160 requests
+    of 600 keys on average: 20.8 and 23.4, of 1,800 49.9 and 34.7)."""
     n = int(seq_lens.size)
     rows, per_request = rows or n, n_kv * ((group + 15) // 16)
     # (as many blocks as SMs, or fewer: `decode_slices` cuts the keys of all but the shortest requests)
